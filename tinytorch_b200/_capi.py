@@ -1,9 +1,12 @@
-"""ctypes binding of libtt_attn.so (declared in include/tt_attn.h).
+"""Loads libtt_attn.so (declared in include/tt_attn.h): through ctypes, struct by
+struct, for C-ABI callers and queries (lib()), and through the torch extension
+module built from csrc/binding.cpp for the ops (native()).
 
-This is the only route from Python to the kernels.  There is no fallback: if the
-shared library is missing or fails to load, importing the ops raises.
+There is no other route from Python to the kernels and no fallback: if a library
+is missing or fails to load, the ops raise.
 """
 import ctypes as C
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -126,6 +129,7 @@ EXPORTS = ("tt_attn_fwd", "tt_attn_bwd", "tt_attn_decode", "tt_attn_decode_appen
            "tt_attn_last_cuda_error", "tt_attn_version")
 
 _lib = None
+_native = None
 
 
 class AttnError(RuntimeError):
@@ -167,6 +171,23 @@ def lib():
         L.tt_attn_last_cuda_error.restype = C.c_char_p
         _lib = L
     return _lib
+
+
+def native():
+    """The extension module lib/_native.so, bound to the library at LIB_PATH.  Raises if it has not been built."""
+    global _native
+    if _native is None:
+        lib()
+        import torch  # noqa: F401 (the module's symbols come from torch's libraries)
+        path = os.path.join(HERE, "lib", "_native.so")
+        if not os.path.exists(path):
+            raise ImportError("%s not found: build it with `python -m tinytorch_b200.build`" % path)
+        spec = importlib.util.spec_from_file_location("tinytorch_b200._native", path)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        m.bind(LIB_PATH, AttnError)
+        _native = m
+    return _native
 
 
 def check(rc):

@@ -1,4 +1,5 @@
-"""Compile the CUDA sources under csrc/ into lib/libtt_attn.so (sm_100a only).
+"""Compile the CUDA sources under csrc/ into lib/libtt_attn.so (sm_100a only) and
+the torch binding csrc/binding.cpp into the extension module lib/_native.so.
 
 nvcc cross-compiles without a GPU.  Object files are rebuilt only when a source
 or header is newer.  Run as ``python -m tinytorch_b200.build``.
@@ -70,7 +71,32 @@ def build(verbose=False, force=False, out_dir=None, defines=()):
     return LIB
 
 
+def build_native():
+    """The torch binding: libtt_attn.so is loaded by it at run time (see _capi.native), torch's libraries are the
+    ones the process has already loaded."""
+    import sysconfig
+    from torch.utils import cpp_extension
+    src, out = os.path.join(CSRC, "binding.cpp"), os.path.join(OUT, "_native.so")
+    if os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), _headers_mtime()):
+        return out
+    os.makedirs(OUT, exist_ok=True)
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    incs = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", src, "-o", out]
+    for i in incs:
+        cmd += ["-isystem", i]
+    for p in cpp_extension.library_paths():
+        cmd += ["-L" + p]
+    cmd += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("building the torch binding failed:\n%s\n%s" % (r.stdout, r.stderr))
+    return out
+
+
 if __name__ == "__main__":
     defs = [a[2:] for a in sys.argv[1:] if a.startswith("-D")]
     outs = [a[6:] for a in sys.argv[1:] if a.startswith("--out=")]
     print(build(verbose="-v" in sys.argv, force="-f" in sys.argv, out_dir=outs[0] if outs else None, defines=defs))
+    if not outs:
+        print(build_native())
