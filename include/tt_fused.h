@@ -67,19 +67,30 @@ typedef struct tt_silu_mul_params {
  * fp32 before the single rounding to the tensor dtype.  ldx / ldw / ldy are the row strides
  * in elements (0 = dense); K, N and the strides must be multiples of 8 and the pointers
  * 16-byte aligned (TT_ATTN_ERR_ALIGN otherwise).  `status` (optional device word) receives a
- * non-zero value if a bounded device-side wait expired. */
+ * non-zero value if a bounded device-side wait expired.
+ * The gradient products of FuncLinear::backward (src/Function/FuncNNLayer.h:20-34) contract
+ * over the rows of an operand; x_t / w_t (added to the end of the struct; a caller with the
+ * shorter struct_size gets 0) say that the operand is stored with the contraction as its slow
+ * dimension, so that no transposed copy is needed:
+ *   dX[M,K] = dY W     x = dY, w = W (stored [contraction N, K]), w_t = 1
+ *   dW[N,K] = dY^T X   x = dY (stored [contraction M, N]), w = X (stored [contraction M, K]),
+ *                      x_t = w_t = 1; K (the contraction) may then be any size
+ * x_sum (optional, with x_t): [M] receives the sums of x over the contraction, in the tensor
+ * dtype (fp32 accumulation): db = sum of dY over its rows, beside dW. */
 typedef struct tt_linear_params {
   uint32_t struct_size;
   int32_t dtype;
   int64_t M, N, K;
-  const void* x;    /* [M, K] */
-  const void* w;    /* [N, K] */
+  const void* x;    /* [M, K]; with x_t [K, M] */
+  const void* w;    /* [N, K]; with w_t [K, N] */
   const void* bias; /* [N] or NULL */
   void* y;          /* [M, N] */
   int64_t ldx, ldw, ldy;
   int32_t device;
   void* stream;
   int32_t* status;
+  int32_t x_t, w_t;
+  void* x_sum; /* [M] or NULL */
 } tt_linear_params;
 
 TT_ATTN_API int tt_linear(const tt_linear_params* p);

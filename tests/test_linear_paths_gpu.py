@@ -1,0 +1,57 @@
+"""GPU: the projection kernels and their gradient products at the edges of their tiles and dispatch rules.
+
+linear_split.cu takes outputs with few tiles (any M up to 128, or fewer 256 x 256 tiles than about two rounds of CTA
+pairs, by cost), linear_tc.cu the rest; both read operands stored with the contraction slow or fast.  Reference: the
+same sums in fp64.  Bound per element: half a unit in the last place of the tensor dtype for the one rounding, plus
+fp32 accumulation in any order: (terms + 2) * 2^-24 * sum of |products|.
+"""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+HALF_ULP = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}  # relative to the value's binade, from below
+TINY = {torch.bfloat16: 1e-30, torch.float16: 2.0 ** -25}          # spacing of fp16 subnormals
+
+
+def _check(got, a, b, bias, dtype):  # got ~ a b (+ bias), a [m, k], b [k, n] in fp64
+    want, terms, size = a @ b, a.shape[1] + (bias is not None), a.abs() @ b.abs()
+    if bias is not None:
+        want, size = want + bias, size + bias.abs()
+    bound = HALF_ULP[dtype] * want.abs() * 1.01 + (terms + 2) * 2.0 ** -24 * size + TINY[dtype]
+    err = (got.double() - want).abs()
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N", [
+    (1, 8, 8), (16, 64, 128), (17, 72, 136), (3, 4096, 264),                 # one tile of x; clusters of 1 .. 8
+    (128, 520, 1024), (129, 1032, 4096), (255, 64, 4096), (300, 1024, 3000),  # several tiles of x, K tails
+    (511, 192, 264), (257, 4160, 512),
+    (1100, 72, 9736), (2050, 456, 4872), (4000, 64, 2568),                    # the persistent pairs, ragged on every side
+])
+def test_projection_and_gradients_at_tile_edges(dtype, M, K, N):
+    from tinytorch_b200 import fused
+    g = torch.Generator("cuda").manual_seed(M + 3 * K + 7 * N)
+    x, w, b, dy = (torch.randn(s, device="cuda", generator=g).to(dtype) for s in ((M, K), (N, K), (N,), (M, N)))
+    for t in (x, w, b):
+        t.requires_grad_()
+    y = fused.linear(x, w, b)
+    dx, dw, db = torch.autograd.grad(y, (x, w, b), dy)
+    xd, wd, bd, dyd = (t.detach().double() for t in (x, w, b, dy))
+    _check(y, xd, wd.t(), bd, dtype)
+    _check(dx, dyd, wd, None, dtype)
+    _check(dw, dyd.t(), xd, None, dtype)
+    _check(db[:, None], dyd.t(), torch.ones(M, 1, device="cuda", dtype=torch.float64), None, dtype)
+
+
+def test_strided_rows_and_repeat():
+    """Row-strided operands, the same answer twice (the sums over a cluster are in rank order)."""
+    from tinytorch_b200 import fused
+    g = torch.Generator("cuda").manual_seed(5)
+    big = torch.randn(40, 2048 + 64, device="cuda", generator=g).bfloat16()
+    w = torch.randn(1024, 2048 + 8, device="cuda", generator=g).bfloat16()[:, :2048]
+    x = big[::2, 64:]
+    y1, y2 = fused.linear(x, w), fused.linear(x, w)
+    assert torch.equal(y1, y2)
+    _check(y1, x.double(), w.double().t(), None, torch.bfloat16)

@@ -119,6 +119,7 @@ class LinearParams(C.Structure):
         ("x", C.c_void_p), ("w", C.c_void_p), ("bias", C.c_void_p), ("y", C.c_void_p),
         ("ldx", C.c_int64), ("ldw", C.c_int64), ("ldy", C.c_int64),
         ("device", C.c_int32), ("stream", C.c_void_p), ("status", C.c_void_p),
+        ("x_t", C.c_int32), ("w_t", C.c_int32), ("x_sum", C.c_void_p),
     ]
 
 

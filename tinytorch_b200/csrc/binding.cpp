@@ -275,29 +275,29 @@ void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
 }
 
 // ------------------------------------------------------------------------------------------------- linear --
-// x2 [M, K] rows may be strided, w [N, K]; y [.., N] dense
-void linear_raw(const Tensor& x, int64_t M, int64_t K, int64_t ldx, const Tensor& w, const Tensor& bias, const Tensor& y,
-                const Tensor& status) {
+// Row stride of a matrix with contiguous columns (a single row's stride may be anything).
+int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
+
+// y[M, N] (dense memory) = x[M, K] w[N, K]^T + bias; x_t / w_t: the operand is given as [K, M] / [K, N]
+void linear_raw(const Tensor& x, bool x_t, const Tensor& w, bool w_t, const Tensor& bias, const Tensor& y, const Tensor& status,
+                const Tensor& x_sum) {
   tt_linear_params p{};
   set_common(&p, x);
   p.dtype = dtype_of(x.scalar_type());
-  p.M = M, p.N = w.size(0), p.K = K;
+  p.M = x.size(x_t ? 1 : 0), p.K = x.size(x_t ? 0 : 1), p.N = w.size(w_t ? 1 : 0);
   p.x = x.data_ptr(), p.w = w.data_ptr(), p.y = y.data_ptr();
   p.bias = bias.defined() ? bias.data_ptr() : nullptr;
-  p.ldx = ldx, p.ldw = w.stride(0), p.ldy = p.N;
+  p.ldx = row_stride(x), p.ldw = row_stride(w), p.ldy = p.N;
   p.status = status.defined() ? static_cast<int32_t*>(status.data_ptr()) : nullptr;
+  p.x_t = x_t, p.w_t = w_t;
+  p.x_sum = x_sum.defined() ? x_sum.data_ptr() : nullptr;
   check(api.linear(&p));
-}
-
-Tensor linear_2d(const Tensor& x2, const Tensor& w, const Tensor& bias) {
-  Tensor y = empty({x2.size(0), w.size(0)}, x2.scalar_type(), x2.device());
-  linear_raw(x2, x2.size(0), x2.size(1), x2.stride(0), w, bias, y, Tensor());
-  return y;
 }
 
 Tensor rows_of(const Tensor& t) {  // [.., C] as [rows, C] with contiguous columns
   Tensor r = t.dim() == 2 ? t : t.reshape({-1, t.size(-1)});
-  return r.stride(1) == 1 ? r : r.contiguous();
+  if (r.stride(1) != 1 || (r.size(0) > 1 && r.stride(0) < r.size(1))) r = r.clone(at::MemoryFormat::Contiguous);
+  return r;
 }
 
 // function::FuncLinear::backward (src/Function/FuncNNLayer.h:20-34)
@@ -312,11 +312,19 @@ struct LinearBackward : public torch::autograd::Node {
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
     const Tensor g2 = rows_of(grads[0]), xt = x2.unpack(), wt = w.unpack();
-    // dX[M,K] = dY[M,N] W[N,K] = dY (W^T)^T: the kernel contracts over the last dimension of both operands
-    if (task_should_compute_output(0)) out[0] = linear_2d(g2, wt.t().contiguous(), Tensor()).reshape(in_shape);
-    // dW[N,K] = dY^T[N,M] X[M,K] = (dY^T) (X^T)^T
-    if (task_should_compute_output(1)) out[1] = linear_2d(g2.t().contiguous(), xt.t().contiguous(), Tensor());
-    if (has_bias && task_should_compute_output(2)) out[2] = g2.to(at::kFloat).sum(0).to(g2.scalar_type());
+    // the products contract over the slow dimension of W, and of dY and X: read as they are stored
+    if (task_should_compute_output(0)) {  // dX[M,K] = dY[M,N] W[N,K]
+      out[0] = empty(in_shape, g2.scalar_type(), g2.device());
+      linear_raw(g2, false, wt, true, Tensor(), out[0], Tensor(), Tensor());
+    }
+    const bool need_db = has_bias && task_should_compute_output(2);
+    if (need_db) out[2] = empty({g2.size(1)}, g2.scalar_type(), g2.device());
+    if (task_should_compute_output(1)) {  // dW[N,K] = dY[M,N]^T X[M,K], with db[N] = sum of dY over its rows
+      out[1] = empty({g2.size(1), xt.size(1)}, g2.scalar_type(), g2.device());
+      linear_raw(g2, true, xt, true, Tensor(), out[1], Tensor(), out[2]);
+    } else if (need_db) {
+      out[2] = g2.to(at::kFloat).sum(0).to(g2.scalar_type());
+    }
     return out;
   }
 };
@@ -336,11 +344,11 @@ Tensor linear_autograd(const Tensor& x, const Tensor& w, const Tensor& bias) {
   {
     at::NoGradGuard no_grad;
     x2 = rows_of(x);
-    wc = w.stride(1) == 1 ? w : w.contiguous();
+    wc = rows_of(w);
     at::DimVector shape(x.sizes().begin(), x.sizes().end());
     shape.back() = w.size(0);
     y = empty(shape, x.scalar_type(), x.device());
-    linear_raw(x2, x2.size(0), x2.size(1), x2.stride(0), wc, bias, y, Tensor());
+    linear_raw(x2, false, wc, false, bias, y, Tensor(), Tensor());
   }
   if (grad) {
     auto node = std::shared_ptr<LinearBackward>(new LinearBackward(), torch::autograd::deleteNode);
@@ -621,7 +629,7 @@ PyObject* py_linear_raw(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     NoGil nogil;
     y = empty({x.size(0), w.size(0)}, x.scalar_type(), x.device());
-    linear_raw(x, x.size(0), x.size(1), x.stride(0), w, bias, y, status);
+    linear_raw(x, false, w, false, bias, y, status, Tensor());
   }
   return wrap(y);
   END_HANDLE_TH_ERRORS

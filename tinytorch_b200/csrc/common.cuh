@@ -128,9 +128,27 @@ cudaError_t launch_fused_add_rms_norm(int dtype, void* input, void* residual, co
                                       int64_t dim, float eps, cudaStream_t stream);
 cudaError_t launch_silu_mul(int dtype, void* out, const void* x, int64_t rows, int64_t d, cudaStream_t stream);
 
-// y = x w^T + bias on the tensor cores (linear_tc.cu); ld* are row strides in elements
-cudaError_t launch_linear_tc(int dtype, const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
-                             int64_t ldx, int64_t ldw, int64_t ldy, int32_t* status, int device, cudaStream_t stream);
+// y = x w^T + bias on the tensor cores; ld* are row strides in elements, x_t / w_t as in tt_linear_params
+struct LinearCall {
+  int dtype;
+  const void* x;
+  const void* w;
+  const void* bias;
+  void* y;
+  int M, N, K;
+  int64_t ldx, ldw, ldy;
+  bool x_t, w_t;
+  int32_t* status;
+  int device;
+  cudaStream_t stream;
+};
+cudaError_t launch_linear_tc(const LinearCall& c);
+// ... for outputs with too few tiles to occupy the machine: contraction split over clusters (linear_split.cu)
+double linear_split_us(const LinearCall& c);  // what it is expected to take
+cudaError_t launch_linear_split(const LinearCall& c);
+// out[n] = sum over the rows of x[rows, n] (fused_ops.cu); n and ldx are multiples of 8
+cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, int device,
+                               cudaStream_t stream);
 
 // one CTA waiting `limit_ns` on an mbarrier nobody arrives on (selftest.cu)
 cudaError_t launch_wait_expiry(int32_t* status, uint64_t limit_ns, unsigned long long* waited_ns, cudaStream_t stream);

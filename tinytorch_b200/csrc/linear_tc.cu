@@ -1,26 +1,26 @@
 // y[M,N] = x[M,K] w[N,K]^T + bias[N] for fp16 / bf16 on sm_100a tensor cores: the
 // projections either side of attention (reference: function::linear =
 // op::matmul(input, weight, false, true, bias), src/Function/FuncNNLayer.h:14-19, which
-// calls a library gemm and, for the bias, pre-fills C, src/Operation/OpLinalgCuda.cuh:141-215).
+// calls a library gemm and, for the bias, pre-fills C, src/Operation/OpLinalgCuda.cuh:141-215),
+// and its two gradient products.
 //
-// Persistent kernel, one CTA per SM, output tiles of MT x 128 rows by 256 columns (MT = 1 or 2):
-//   warp 0     producer: cp.async.bulk.tensor loads (128-byte swizzle) of the (MT x 128) x 64
-//              slice of x and the 256 x 64 slice of w into a ring of 4 (MT = 1) or 3 (MT = 2) stages
-//   warp 1     issuer: the warp runs the loop, one elected lane issues tcgen05.mma (kind::f16, M = 128, N = 256, both
-//              operands K-major) into 256-column TMEM accumulators.  MT = 1: two accumulators used in
-//              turn, so that the epilogue of a tile runs under the main loop of the next.  MT = 2: one
-//              accumulator per 128-row half of the tile; both halves read the same slice of w from shared
-//              memory, and the next tile's upper half starts while the lower half is still being drained.
-//              Shared memory moves 128 bytes per clock, and the operands of an M = 128, N = 256 MMA are
-//              12 KB per 128 clocks on top of the TMA writes that bring them in: with MT = 1 that is
-//              192 bytes per clock of tensor time (the pipe cannot be busy more than two thirds of the
-//              time; a profile showed 67 %), with MT = 2, where w is brought in once for two MMAs, 160.
-//   warps 4-7  epilogue: thread r owns output row r (TMEM lane r); 64 columns at a time
-//              are read with tcgen05.ld, get the bias (fp32), are rounded to the tensor
-//              dtype and leave through a swizzled staging tile and a TMA store (rows and
+// Persistent CTA PAIRS (clusters of two, tcgen05 cta_group::2), one CTA per SM, output tiles of 256 x 256: each CTA of
+// a pair holds 128 rows of the tile and of x, and HALF of the tile's rows of w; an MMA of M = 256, N = 256, K = 16
+// reads 8 KB from each CTA's shared memory in 128 clocks and the fills bring in another 8 KB, i.e. 128 bytes per clock
+// of tensor time where two independent 128 x 256 tiles need 192 (shared memory moves 128).
+//   warp 0     producer (both CTAs): cp.async.bulk.tensor loads (128-byte swizzle) of its 128 x 64 slices of x and w
+//              into a 5-stage ring; both CTAs' loads complete on the LEADER's barrier of the stage
+//   warp 1     issuer (leader only): one elected lane issues the MMAs into one of two 256-column TMEM accumulators per
+//              CTA, used in turn, so that the epilogue of a tile runs under the main loop of the next; its commits
+//              reach the barriers of both CTAs
+//   warps 4-7, epilogue (both CTAs): two warpgroups take the 64-column blocks alternately, thread r of each owns output
+//   warps 8-11 row r of the CTA's half (TMEM lane r); a block is read with tcgen05.ld, gets the bias (fp32), is rounded
+//              to the tensor dtype and leaves through one of the warpgroup's two swizzled staging tiles and a TMA store (rows and
 //              columns beyond M, N are clipped by the tensor map; the K tail reads as zero)
-// Tiles are ordered in groups of eight row-tiles so that CTAs running at the same time
-// share slices of x and w in L2.  Every wait is bounded.
+// Tiles are ordered in groups of four row-tiles so that CTAs running at the same time share slices of x and w in L2.
+// X_MN / W_MN: the operand is stored with the contraction as its slow dimension (x as [K, M], w as [K, N]) and is read
+// as an MN-major MMA operand, so that the gradients dX = dY W and dW = dY^T X need no transposed copies.
+// Every mbarrier wait is bounded; after an expired one the CTA still meets the cluster barrier at the end.
 #include <type_traits>
 
 #include "common.cuh"
@@ -30,33 +30,25 @@
 namespace ttattn {
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int kMaxStage = 4;
-constexpr int kThreads = 256;
-constexpr int kEpi = 128;
-constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;
-constexpr int kOutBytes = BM * 128;  // staging: 128 rows x 64 columns of 16 bits
-
-// MT: 128-row halves per output tile
-template <int MT>
-struct Cfg {
-  static constexpr int kStages = MT == 1 ? 4 : 3;
-  static constexpr int kStageBytes = MT * kABytes + kBBytes;
-  static constexpr int kGroupM = 8 / MT;  // row-tiles per L2 group: 1024 rows either way
-};
+constexpr int BM = 256, BN = 256, BK = 64;  // tile of a pair
+constexpr int HM = BM / 2, HN = BN / 2;     // what one CTA loads of it
+constexpr int NSTAGE = 5;
+constexpr int kThreads = 384;
+constexpr int kEpi = 128;  // threads of an epilogue warpgroup
+constexpr int kABytes = HM * BK * 2, kBBytes = HN * BK * 2;
+constexpr int kStageBytes = kABytes + kBBytes;
+constexpr int kOutBytes = HM * 128;  // staging: 128 rows x 64 columns of 16 bits
+constexpr int kGroupM = 4;           // row-tiles per L2 group
 
 struct __align__(8) SmemCtl {
-  uint64_t full[kMaxStage], empty[kMaxStage];
+  uint64_t full[NSTAGE], empty[NSTAGE];
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
 
-template <int MT>
-constexpr int smem_bytes() {
-  return Cfg<MT>::kStages * Cfg<MT>::kStageBytes + 2 * kOutBytes + BN * 4 + static_cast<int>(sizeof(SmemCtl));
-}
-static_assert(smem_bytes<1>() <= 232448 && smem_bytes<2>() <= 232448, "exceeds the shared memory a CTA may request");
+constexpr int kSmemBytes = NSTAGE * kStageBytes + 4 * kOutBytes + BN * 4 + static_cast<int>(sizeof(SmemCtl));
+static_assert(kSmemBytes <= 232448, "exceeds the shared memory a CTA may request");
 
 struct LinArgs {
   const void* bias;  // [N] in the tensor dtype, or null
@@ -75,7 +67,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-template <int kGroupM>
 __device__ __forceinline__ void tile_of(int t, int tiles_m, int tiles_n, int* m_tile, int* n_tile) {
   const int per_group = kGroupM * tiles_n;
   const int g = t / per_group, in_g = t - g * per_group;
@@ -85,27 +76,23 @@ __device__ __forceinline__ void tile_of(int t, int tiles_m, int tiles_n, int* m_
   *n_tile = in_g / gm;
 }
 
-template <bool BF16, int MT>
-__global__ void __launch_bounds__(kThreads, 1)
+template <bool BF16, bool X_MN, bool W_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     linear_tc_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
                      const __grid_constant__ CUtensorMap tmY, const LinArgs a) {
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   extern __shared__ __align__(1024) uint8_t smem[];
-  if ((ptx::smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need a 1024-byte boundary
-    if (threadIdx.x == 0 && a.status) atomicOr(a.status, kStatusBadSmemAlign);
-    return;
-  }
-  constexpr int NSTAGE = Cfg<MT>::kStages, kStageBytes = Cfg<MT>::kStageBytes, kGroupM = Cfg<MT>::kGroupM;
-  constexpr int TM = MT * BM;  // rows of an output tile
   uint8_t* sOut = smem + NSTAGE * kStageBytes;
-  float* sBias = reinterpret_cast<float*>(sOut + 2 * kOutBytes);
+  float* sBias = reinterpret_cast<float*>(sOut + 4 * kOutBytes);
   SmemCtl* ctl = reinterpret_cast<SmemCtl*>(sBias + BN);
   volatile int* abort_flag = &ctl->abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tiles_m = (a.M + TM - 1) / TM, tiles_n = (a.N + BN - 1) / BN;
+  const uint32_t rank = ptx::cluster_rank();
+  const int tiles_m = (a.M + BM - 1) / BM, tiles_n = (a.N + BN - 1) / BN;
   const int n_tiles = tiles_m * tiles_n;
   const int n_kb = (a.K + BK - 1) / BK;
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;  // the pair's tiles
 
   if (warp == 0 && lane == 0) {
 #pragma unroll
@@ -116,131 +103,134 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&ctl->acc_full[i], 1);
-      ptx::mbar_init(&ctl->acc_empty[i], kEpi);
+      ptx::mbar_init(&ctl->acc_empty[i], 16);  // the epilogue warps of both CTAs
     }
-    ctl->abort_flag = 0;
+    ctl->abort_flag = (ptx::smem_u32(smem) & 1023u) != 0;  // the swizzled tiles need a 1024-byte boundary
     ptx::fence_barrier_init();
     ptx::tma_prefetch_desc(&tmX);
     ptx::tma_prefetch_desc(&tmW);
     ptx::tma_prefetch_desc(&tmY);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(&ctl->tmem_base, 512);
-    ptx::tmem_relinquish();
+    ptx::tmem_alloc_pair(&ctl->tmem_base, 512);
+    ptx::tmem_relinquish_pair();
   }
   ptx::tc_fence_before();
   __syncthreads();
+  ptx::cluster_sync();  // the barriers of both CTAs are initialised
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
+  ptx::grid_dep_launch();  // (the next kernel may come up: this grid has its TMEM)
+  ptx::grid_dep_wait();    // everything below reads or writes global memory
+  const bool usable = *abort_flag == 0;
 
   if (warp == 0) {
     // -------------------------------------------------------------- producer --
-    if (lane == 0) {
-      uint32_t g = 0;  // k-slices requested so far (ring position)
+    if (lane == 0 && usable) {
+      int s = 0;
+      uint32_t ph = 1;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      uint32_t full0 = ptx::map_rank(ptx::smem_u32(&ctl->full[0]), 0);  // the leader's
+      for (int t = first; t < n_tiles && ok; t += step) {
         int mt, nt;
-        tile_of<kGroupM>(t, tiles_m, tiles_n, &mt, &nt);
-        for (int kb = 0; kb < n_kb; ++kb, ++g) {
-          const int s = g % NSTAGE;
-          if (!(ok = ptx::mbar_wait(&ctl->empty[s], ((g / NSTAGE) & 1) ^ 1, abort_flag))) break;
+        tile_of(t, tiles_m, tiles_n, &mt, &nt);
+        const int m0 = mt * BM + static_cast<int>(rank) * HM, n0 = nt * BN + static_cast<int>(rank) * HN;
+        for (int kb = 0; kb < n_kb; ++kb) {
+          if (!(ok = ptx::mbar_wait(&ctl->empty[s], ph, abort_flag))) break;
           uint8_t* sa = smem + s * kStageBytes;
-          ptx::mbar_arrive_expect_tx(&ctl->full[s], kStageBytes);
-#pragma unroll
-          for (int h = 0; h < MT; ++h)  // rows beyond M read as zero
-            ptx::tma_load_4d(sa + h * kABytes, &tmX, &ctl->full[s], kb * BK, mt * TM + h * BM, 0, 0);
-          ptx::tma_load_4d(sa + MT * kABytes, &tmW, &ctl->full[s], kb * BK, nt * BN, 0, 0);
-          ptx::tma_load_4d(sa + MT * kABytes + kBBytes / 2, &tmW, &ctl->full[s], kb * BK, nt * BN + 128, 0, 0);
+          uint8_t* sb = sa + kABytes;
+          const uint32_t bar = full0 + s * 8;
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], 2 * kStageBytes);  // both CTAs' loads
+          if constexpr (X_MN) {  // blocks of [64 contraction rows][64 columns]
+            ptx::tma_load_4d_pair(sa, &tmX, bar, m0, kb * BK, 0, 0);
+            ptx::tma_load_4d_pair(sa + kABytes / 2, &tmX, bar, m0 + 64, kb * BK, 0, 0);
+          } else {
+            ptx::tma_load_4d_pair(sa, &tmX, bar, kb * BK, m0, 0, 0);  // rows beyond M read as zero
+          }
+          if constexpr (W_MN) {
+            ptx::tma_load_4d_pair(sb, &tmW, bar, n0, kb * BK, 0, 0);
+            ptx::tma_load_4d_pair(sb + kBBytes / 2, &tmW, bar, n0 + 64, kb * BK, 0, 0);
+          } else {
+            ptx::tma_load_4d_pair(sb, &tmW, bar, kb * BK, n0, 0, 0);
+          }
+          if (++s == NSTAGE) s = 0, ph ^= 1;
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     // ---------------------------------------------------------------- issuer --
     // the whole warp runs the loop (waits made uniform by a vote), one elected lane issues: addresses and
     // descriptors stay warp-uniform
-    {
-      const bool leader = ptx::elect_one();
-      constexpr uint32_t kHi = ptx::smem_desc_hi_sw128(1024);
-      const uint32_t idesc = ptx::make_idesc_f16(BM, BN, BF16 ? 1 : 0, 0, 0);
-      const uint32_t alo = ptx::smem_desc_lo(ptx::smem_u32(smem), 16);
-      const uint32_t blo = ptx::smem_desc_lo(ptx::smem_u32(smem + MT * kABytes), 16);
-      uint32_t g = 0;
-      bool ok = true;
-      int i = 0;
-      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++i) {
-        // Accumulator of half h of tile i, and how often it has been used before: with MT = 1 the two
-        // accumulators alternate between tiles, with MT = 2 each half of the tile has its own.
-        auto acc_of = [&](int h) { return MT == 1 ? (i & 1) : h; };
-        const uint32_t use = MT == 1 ? (i >> 1) : i;
-        for (int kb = 0; kb < n_kb && ok; ++kb, ++g) {
-          const int s = g % NSTAGE;
-          if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->full[s], (g / NSTAGE) & 1, abort_flag)) != 0)) break;
-          ptx::tc_fence_after();
-          const uint32_t so = s * (kStageBytes >> 4);
+    const bool leader = ptx::elect_one();
+    constexpr uint32_t kHi = ptx::smem_desc_hi_sw128(1024);
+    const uint32_t idesc = ptx::make_idesc_f16(BM, BN, BF16 ? 1 : 0, X_MN ? 1 : 0, W_MN ? 1 : 0);
+    const uint32_t alo = ptx::smem_desc_lo(ptx::smem_u32(smem), X_MN ? kABytes / 2 : 16);
+    const uint32_t blo = ptx::smem_desc_lo(ptx::smem_u32(smem + kABytes), W_MN ? kBBytes / 2 : 16);
+    // one k-step: 16 contraction rows of 128 bytes (MN-major), or 32 bytes of the 128-byte swizzled row
+    constexpr uint32_t kAStep = X_MN ? 128 : 2, kBStep = W_MN ? 128 : 2;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = usable;
+    int i = 0;
+    for (int t = first; t < n_tiles && ok; t += step, ++i) {
+      const int buf = i & 1;
+      // the epilogues of both CTAs have read what this accumulator held before
+      if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_empty[buf], ((i >> 1) & 1) ^ 1, abort_flag)) != 0)) break;
+      ptx::tc_fence_after();
+      const uint32_t d = tmem + buf * BN;
+      for (int kb = 0; kb < n_kb; ++kb) {
+        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) != 0)) break;
+        ptx::tc_fence_after();
+        const uint32_t so = s * (kStageBytes >> 4);
 #pragma unroll
-          for (int h = 0; h < MT; ++h) {
-            const int ai = acc_of(h);
-            if (kb == 0) {
-              // the epilogue has read what this accumulator held before
-              if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_empty[ai], (use & 1) ^ 1, abort_flag)) != 0)) break;
-              ptx::tc_fence_after();
-            }
-            const uint32_t d = tmem + ai * BN, ah = alo + so + h * (kABytes >> 4);
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k)  // 32 bytes per k-step inside the 128-byte swizzled row
-              if (leader) ptx::mma_ss2(d, ah + k * 2, kHi, blo + so + k * 2, kHi, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            if (leader && kb == n_kb - 1) ptx::mma_commit(&ctl->acc_full[ai]);
-          }
-          if (ok && leader) ptx::mma_commit(&ctl->empty[s]);
-        }
+        for (int k = 0; k < BK / 16; ++k)
+          if (leader)
+            ptx::mma_ss2_pair(d, alo + so + k * kAStep, kHi, blo + so + k * kBStep, kHi, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        if (leader) ptx::mma_commit_pair(&ctl->empty[s]);
+        if (++s == NSTAGE) s = 0, ph ^= 1;
       }
+      if (leader && ok) ptx::mma_commit_pair(&ctl->acc_full[buf]);
     }
   } else if (warp >= 4) {
     // -------------------------------------------------------------- epilogue --
-    const int r = tid - 128;  // output row within the tile = TMEM lane
+    const int wg = (warp - 4) >> 2, r = tid & (kEpi - 1);  // output row within the CTA's half = TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    bool ok = true;
+    const uint32_t acc_empty0 = ptx::map_rank(ptx::smem_u32(&ctl->acc_empty[0]), 0);  // the leader's
+    float* bias = sBias + wg * (BN / 2);  // of this warpgroup's two blocks
+    bool ok = usable;
     int i = 0;
-    uint32_t stores = 0;  // staging buffer toggle
-    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++i) {
+    for (int t = first; t < n_tiles; t += step, ++i) {
       int mt, nt;
-      tile_of<kGroupM>(t, tiles_m, tiles_n, &mt, &nt);
-      const int n0 = nt * BN;
-      const uint32_t use = MT == 1 ? (i >> 1) : i;
-      // this tile's slice of the bias, as fp32 (threads that see an expired wait still meet the barriers)
-      ptx::named_barrier(1, kEpi);  // the previous tile's readers of sBias are done
-#pragma unroll
-      for (int j = 0; j < BN / kEpi; ++j) {
-        const int n = n0 + r + j * kEpi;
-        sBias[r + j * kEpi] = (a.bias && n < a.N) ? to_f32<T>(reinterpret_cast<const T*>(a.bias)[n]) : 0.f;
+      tile_of(t, tiles_m, tiles_n, &mt, &nt);
+      const int n0 = nt * BN, m0 = mt * BM + static_cast<int>(rank) * HM, buf = i & 1;
+      {  // (threads that see an expired wait still meet the barriers)
+        const int n = n0 + wg * 64 + (r >> 6) * 128 + (r & 63);  // blocks wg and wg + 2
+        bias[r] = (a.bias && n < a.N) ? to_f32<T>(reinterpret_cast<const T*>(a.bias)[n]) : 0.f;
       }
-      ptx::named_barrier(1, kEpi);
-#pragma unroll 1
-      for (int h = 0; h < MT; ++h) {
-      const int buf = MT == 1 ? (i & 1) : h, m0 = mt * TM + h * BM;
-      if (ok) ok = ptx::mbar_wait(&ctl->acc_full[buf], use & 1, abort_flag);
+      if (ok) ok = ptx::mbar_wait(&ctl->acc_full[buf], (i >> 1) & 1, abort_flag);
       ptx::tc_fence_after();
 #pragma unroll 1
-      for (int c = 0; c < BN / 64; ++c) {
+      for (int cc = 0; cc < 2; ++cc) {
+        const int c = wg + 2 * cc;
+        uint8_t* stage = sOut + (wg * 2 + cc) * kOutBytes;
         uint32_t v[64];
         ptx::tmem_ld32p(tmem + buf * BN + lane_addr + c * 64, v);
         ptx::tmem_ld32p(tmem + buf * BN + lane_addr + c * 64 + 32, v + 32);
-        ptx::tmem_wait_ld();
-        if (c == BN / 64 - 1) {
-          // the whole accumulator is in registers / already stored: the issuer may reuse it
-          ptx::tc_fence_before();
-          ptx::mbar_arrive(&ctl->acc_empty[buf]);
-        }
-        uint8_t* stage = sOut + (stores & 1) * kOutBytes;
-        ++stores;
-        // at most one earlier store (the other staging buffer) may still be reading shared memory
+        // at most one earlier store (the other staging tile) may still be reading shared memory
         if (r == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        ptx::named_barrier(1, kEpi);
+        ptx::tmem_wait_ld();
+        if (cc == 1) {
+          // this warp's share of the accumulator is in registers / already stored
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster(acc_empty0 + buf * 8);
+        }
+        ptx::named_barrier(1 + wg, kEpi);
 #pragma unroll
         for (int ch = 0; ch < 8; ++ch) {
           const int e = ch * 8;
-          const float4 b0 = *reinterpret_cast<const float4*>(sBias + c * 64 + e);
-          const float4 b1 = *reinterpret_cast<const float4*>(sBias + c * 64 + e + 4);
+          const float4 b0 = *reinterpret_cast<const float4*>(bias + cc * 64 + e);
+          const float4 b1 = *reinterpret_cast<const float4*>(bias + cc * 64 + e + 4);
           uint4 w;
           w.x = pack2<BF16>(__uint_as_float(v[e + 0]) + b0.x, __uint_as_float(v[e + 1]) + b0.y);
           w.y = pack2<BF16>(__uint_as_float(v[e + 2]) + b0.z, __uint_as_float(v[e + 3]) + b0.w);
@@ -249,62 +239,70 @@ __global__ void __launch_bounds__(kThreads, 1)
           *reinterpret_cast<uint4*>(stage + r * 128 + ((ch ^ (r & 7)) << 4)) = w;
         }
         ptx::fence_proxy_async_smem();
-        ptx::named_barrier(1, kEpi);
+        // (also: every thread has read the bias before the next tile's is written)
+        ptx::named_barrier(1 + wg, kEpi);
         if (r == 0 && ok && n0 + c * 64 < a.N && m0 < a.M) {
           ptx::tma_store_4d(&tmY, stage, n0 + c * 64, m0, 0, 0);
           ptx::bulk_commit();
         }
       }
-      }
     }
     if (r == 0) ptx::bulk_wait_all();
   }
 
+  __syncwarp();
   ptx::tc_fence_before();
-  __syncthreads();
+  ptx::cluster_sync();  // neither CTA leaves while the other may still signal its barriers
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, 512);
+    ptx::tmem_dealloc_pair(tmem, 512);
   }
   if (tid == 0 && ctl->abort_flag && a.status) atomicOr(a.status, kStatusWaitExpired);
 }
 
-template <bool BF16, int MT>
-cudaError_t launch_t(int dtype, const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
-                     int64_t ldx, int64_t ldw, int64_t ldy, int32_t* status, int device, cudaStream_t stream) {
-  CUtensorMap tx, tw, ty;
-  // 2-D tensors as [1, 1, rows, cols] maps: box = 64 columns x 128 rows, 128-byte swizzle
-  if (!make_map(&tx, dtype, x, K, M, 1, 1, Str3{ldx * M, ldx * M, ldx}) ||
-      !make_map(&tw, dtype, w, K, N, 1, 1, Str3{ldw * N, ldw * N, ldw}) ||
-      !make_map(&ty, dtype, y, N, M, 1, 1, Str3{ldy * M, ldy * M, ldy}))
-    return cudaErrorInvalidValue;
-  auto kern = linear_tc_kernel<BF16, MT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<MT>());
+template <bool BF16, bool X_MN, bool W_MN>
+cudaError_t launch_t(const LinearCall& c, int ctas) {
+  auto kern = linear_tc_kernel<BF16, X_MN, W_MN>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return e;
-  const long long tiles = static_cast<long long>((M + MT * BM - 1) / (MT * BM)) * ((N + BN - 1) / BN);
-  const int sms = sm_count(device);
-  LinArgs a{bias, M, N, K, status};
-  kern<<<static_cast<unsigned>(tiles < sms ? tiles : sms), kThreads, smem_bytes<MT>(), stream>>>(tx, tw, ty, a);
-  return cudaGetLastError();
+  CUtensorMap tx, tw, ty;
+  // 128-byte swizzle; boxes of 64 contiguous elements (the contraction, or for an MN-major operand its other dimension)
+  if (!make_map_2d(&tx, c.dtype, c.x, X_MN ? c.M : c.K, X_MN ? c.K : c.M, c.ldx, X_MN ? BK : HM) ||
+      !make_map_2d(&tw, c.dtype, c.w, W_MN ? c.N : c.K, W_MN ? c.K : c.N, c.ldw, W_MN ? BK : HN) ||
+      !make_map_2d(&ty, c.dtype, c.y, c.N, c.M, c.ldy, HM))
+    return cudaErrorInvalidValue;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = c.stream;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, c.status});
 }
 
-// 256-row tiles when they still fill the machine at least once; otherwise 128-row tiles (twice the CTAs)
-inline bool tall_tiles(int M, int N, int device) {
-  const long long tiles = static_cast<long long>((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-  return tiles >= sm_count(device);
+template <bool BF16>
+cudaError_t launch_bf(const LinearCall& c, int ctas) {
+  if (c.x_t) return c.w_t ? launch_t<BF16, true, true>(c, ctas) : launch_t<BF16, true, false>(c, ctas);
+  return c.w_t ? launch_t<BF16, false, true>(c, ctas) : launch_t<BF16, false, false>(c, ctas);
 }
 
 }  // namespace
 
-cudaError_t launch_linear_tc(int dtype, const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
-                             int64_t ldx, int64_t ldw, int64_t ldy, int32_t* status, int device, cudaStream_t stream) {
-  if (dtype != TT_ATTN_BF16 && dtype != TT_ATTN_F16) return cudaErrorInvalidValue;
-  const bool bf = dtype == TT_ATTN_BF16;
-  if (tall_tiles(M, N, device))
-    return bf ? launch_t<true, 2>(dtype, x, w, bias, y, M, N, K, ldx, ldw, ldy, status, device, stream)
-              : launch_t<false, 2>(dtype, x, w, bias, y, M, N, K, ldx, ldw, ldy, status, device, stream);
-  return bf ? launch_t<true, 1>(dtype, x, w, bias, y, M, N, K, ldx, ldw, ldy, status, device, stream)
-            : launch_t<false, 1>(dtype, x, w, bias, y, M, N, K, ldx, ldw, ldy, status, device, stream);
+cudaError_t launch_linear_tc(const LinearCall& c) {
+  if (c.dtype != TT_ATTN_BF16 && c.dtype != TT_ATTN_F16) return cudaErrorInvalidValue;
+  // The persistent pairs where they are expected to be the faster: whole rounds of 256 x 256 tiles at 0.29 us per 64 of
+  // the contraction (or an epilogue each, where the contraction is short), 4.5 us for ramp and drain.  Few rows leave
+  // most of a 256-row tile empty, and then the weight's way from HBM is what takes the time.
+  const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + BN - 1) / BN);
+  const int pairs = sm_count(c.device) / 2;
+  const double round_us = 0.29 * ((c.K + BK - 1) / BK);
+  const double pair_us = 4.5 + static_cast<double>((tiles + pairs - 1) / pairs) * (round_us > 1.6 ? round_us : 1.6);
+  if (tiles < 2 * pairs && (c.M <= HM || linear_split_us(c) < pair_us)) return launch_linear_split(c);
+  const int ctas = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
+  return c.dtype == TT_ATTN_BF16 ? launch_bf<true>(c, ctas) : launch_bf<false>(c, ctas);
 }
 
 }  // namespace ttattn

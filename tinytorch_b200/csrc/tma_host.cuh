@@ -46,6 +46,11 @@ inline bool make_map(CUtensorMap* m, int dtype, const void* ptr, int D, int S, i
   return r == CUDA_SUCCESS;
 }
 
+// [rows, cols] matrix with row stride `ld` (elements), box = 64 columns x `box_rows` rows.
+inline bool make_map_2d(CUtensorMap* m, int dtype, const void* ptr, int cols, int rows, int64_t ld, int box_rows) {
+  return make_map(m, dtype, ptr, cols, rows, 1, 1, Str3{ld * rows, ld * rows, ld}, box_rows);
+}
+
 // Dense fp32 [B, H, S, D] buffer, box = 32 floats (128 bytes) x `box_rows` rows, for TMA reductions.
 inline bool make_map_f32(CUtensorMap* m, const float* ptr, int D, int S, int H, int B, int box_rows = 128) {
   EncodeTiledFn fn = encode_fn();
