@@ -1,4 +1,4 @@
-// Attention backward on CUDA cores with fp32 arithmetic, for every dtype.
+// Attention backward on CUDA cores with fp32 arithmetic for Float32 tensors, and the delta pre-pass of both backwards.
 //
 // The reference's FuncSDPAttention::backward is unimplemented
 // (src/Function/FuncNNLayer.h:267); its gradient is defined by the chain
@@ -8,57 +8,24 @@
 //   dS = P o (dP - rowsum(P o dP)) * scale,   rowsum(P o dP) = rowsum(dO o O) = delta
 //   dQ = dS K            dK = dS^T Q
 // P is recomputed from Q, K and the forward's log-sum-exp, so no [L,S] matrix is
-// ever stored.  Three kernels:
+// ever stored.  Two kernels:
 //   bwd_delta_kernel   delta[b,h,i] = sum_d dO[i,d] * O[i,d]           (fp32 workspace)
-//   bwd_dkdv_kernel    one CTA per 64-key tile: loops over the query tiles (and
-//                      over the query heads of the group), accumulates dK, dV in
-//                      registers -> deterministic, no atomics
-//   bwd_dq_kernel      one CTA per 64-query tile: loops over key tiles, accumulates dQ
-#include "common.cuh"
-#include "ptx.cuh"
+//   bwd_simt_kernel    CTAs of two kinds in one launch, so that a small problem pays one launch and both kinds fill
+//                      the machine together:
+//     key CTAs    one per 64-key tile: loop over the query tiles (and over the query heads of the group),
+//                 accumulate dK, dV in registers -> deterministic, no atomics
+//     query CTAs  one per 64-query tile: loop over the key tiles, accumulate dQ
+// Bound by the FMA pipes: seven products where five would do if dQ left through atomics, whose order is not
+// deterministic.  16 x TY threads per tile (simt_tile.cuh): 8 rows per thread for D = 64; 4 for D = 128, where 8
+// would need more accumulators than there are registers.  B4 H16 S2048 D64 causal: 4986 -> 2807 us (24 -> 43 TFLOP/s),
+// B2 H4 S128 D64: 63 -> 23 us; ncu: FMA pipe 63 % busy.
+#include "simt_tile.cuh"
 
 namespace ttattn {
 namespace {
 
-constexpr int TM = 64, TN = 64, kThreads = 256;
-
-template <typename T, int D>
-__device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t row_stride, int row0, int rows_valid,
-                                          int tid) {
-  constexpr int LD = D + 1;
-  for (int idx = tid; idx < TM * (D / 4); idx += kThreads) {
-    int r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-    if (row0 + r < rows_valid) {
-      const T* p = src + static_cast<int64_t>(row0 + r) * row_stride + c4;
-      v0 = to_f32<T>(p[0]), v1 = to_f32<T>(p[1]), v2 = to_f32<T>(p[2]), v3 = to_f32<T>(p[3]);
-    }
-    float* d = dst + r * LD + c4;
-    d[0] = v0, d[1] = v1, d[2] = v2, d[3] = v3;
-  }
-}
-
-// out[i][j] = sum_d A[(ty+16i)][d] * B[(tx+16j)][d]
-template <int D>
-__device__ __forceinline__ void tile_nt(const float* A, const float* B, int ty, int tx, float (&out)[4][4]) {
-  constexpr int LD = D + 1;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) out[i][j] = 0.f;
-#pragma unroll 8
-  for (int d = 0; d < D; ++d) {
-    float av[4], bv[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) av[i] = A[(ty + 16 * i) * LD + d];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) bv[j] = B[(tx + 16 * j) * LD + d];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) out[i][j] = fmaf(av[i], bv[j], out[i][j]);
-  }
-}
+using namespace simt;
+constexpr int kThreads = 256;  // of the delta kernel
 
 // delta[b,h,i] = sum_d dO[i,d] * O[i,d].  Each thread reads 16 bytes of a row of
 // O and of dO; the D*sizeof(T)/16 threads of a row reduce with shuffles.  For the
@@ -96,229 +63,198 @@ __global__ void __launch_bounds__(kThreads) bwd_delta_kernel(const BwdArgs a) {
   if (part == 0 && row < total) a.delta[row] = s;
 }
 
-// Computes P and dS for the (query tile, key tile) pair held in shared memory and
-// writes them to Ps / dSs ([row][col], leading dimension TN+1).
-// `shift` is the causal alignment (key j participates iff j <= i + shift), `mask_base` the
-// mask offset of this (b, h).
-template <typename T, int D>
+template <int D>
+struct Cfg {
+  static constexpr int TY = D == 64 ? 8 : 16, NT = 16 * TY, R = TS / TY;
+  static constexpr int kSmemBytes = (4 * kTileFloats<D> + 2 * kScoreFloats + 2 * TS) * static_cast<int>(sizeof(float));
+};
+
+// The (query tile, key tile) pair in shared memory: P into Ps (if KEYS) and dS into dSs, [query][key] both.
+// `shift` is the causal alignment (key j participates iff j <= i + shift), `mask_base` the mask offset of (b, h).
+template <int D, bool MASK, bool KEYS>
 __device__ __forceinline__ void tile_p_ds(const BwdArgs& a, const float* Qs, const float* Ks, const float* Vs,
-                                          const float* dOs, const float* lse_s, const float* delta_s, float* Ps,
+                                          const float* dOs, const float* lse2_s, const float* delta_s, float* Ps,
                                           float* dSs, int row0, int col0, int kv_len, int shift, int64_t mask_base,
                                           int ty, int tx) {
-  constexpr int LP = TN + 1;
+  constexpr int TY = Cfg<D>::TY, R = Cfg<D>::R;
   const float c = a.scale * kLog2e;
-  float s[4][4], dp[4][4];
-  tile_nt<D>(Qs, Ks, ty, tx, s);
-  tile_nt<D>(dOs, Vs, ty, tx, dp);
+  float bias[MASK ? R : 1][4];
+  if constexpr (MASK) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty + 16 * i, row = row0 + r;
-    const float lse2 = lse_s[r] * kLog2e, dl = delta_s[r];
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int row = row0 + ty + TY * i, col = col0 + tx + 16 * j;
+        bias[i][j] = row < a.Lq && col < kv_len ? mask_bias2<float>(a.mask, mask_base + row * a.mask.sl + col) : 0.f;
+      }
+  }
+  float p[R][4], dp[R][4];
+  product_nt<D, TY>(Qs, Ks, ty, tx, p);
+  const bool edge = row0 + TS > a.Lq || col0 + TS > kv_len || (a.causal && col0 + TS - 1 > row0 + shift);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int r = ty + TY * i, row = row0 + r;
+    const float lse2 = lse2_s[r];  // lse * log2(e); +inf for a row without any participating key, whose P is 0
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int cidx = tx + 16 * j, col = col0 + cidx;
-      // a row without any participating key has LSE = -inf and P = 0
-      const bool keep = row < a.Lq && col < kv_len && (!a.causal || col <= row + shift) && lse_s[r] != -INFINITY;
-      float x = fmaf(s[i][j], c, -lse2);
-      if (a.mask.ptr && keep) x += mask_bias2<T>(a.mask, mask_base + row * a.mask.sl + col);
-      const float p = keep ? exp2f(x) : 0.f;
-      if (Ps) Ps[r * LP + cidx] = p;
-      dSs[r * LP + cidx] = p * (dp[i][j] - dl) * a.scale;
+      float x = fmaf(p[i][j], c, -lse2);
+      if constexpr (MASK) x += bias[i][j];
+      p[i][j] = exp2f(x);
+      const int col = col0 + tx + 16 * j;
+      if (edge && !(row < a.Lq && col < kv_len && (!a.causal || col <= row + shift))) p[i][j] = 0.f;
+      if constexpr (KEYS) Ps[r * LP + tx + 16 * j] = p[i][j];
     }
+  }
+  product_nt<D, TY>(dOs, Vs, ty, tx, dp);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int r = ty + TY * i;
+    const float dl = delta_s[r];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) dSs[r * LP + tx + 16 * j] = p[i][j] * (dp[i][j] - dl) * a.scale;
   }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) bwd_dkdv_kernel(const BwdArgs a) {
-  constexpr int LD = D + 1, LP = TN + 1, DC = D / 16;
-  extern __shared__ float sm[];
-  float* Ks = sm;
-  float* Vs = Ks + TN * LD;
-  float* Qs = Vs + TN * LD;
-  float* dOs = Qs + TM * LD;
-  float* Ps = dOs + TM * LD;
-  float* dSs = Ps + TM * LP;
-  float* lse_s = dSs + TM * LP;
-  float* delta_s = lse_s + TM;
-
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int nt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const int group = a.Hq / a.Hkv;
-  const int col0 = nt * TN;
-  int kv_len = a.Skv;
-  if (a.kv_lens) {
-    int l = a.kv_lens[b];
-    kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
+// lse (times log2 e, +inf where -inf) and delta of the 64 queries from row0 on
+__device__ __forceinline__ void load_vectors(const BwdArgs& a, float* lse2_s, float* delta_s, int64_t base, int row0, int tid) {
+  if (tid < TS) {
+    const bool in = row0 + tid < a.Lq;
+    const float l = in ? a.lse[base + row0 + tid] : 0.f;
+    lse2_s[tid] = l == -INFINITY ? INFINITY : l * kLog2e;
+    delta_s[tid] = in ? a.delta[base + row0 + tid] : 0.f;
   }
-  const T* k = reinterpret_cast<const T*>(a.k) + b * a.ks.b + hk * a.ks.h;
-  const T* v = reinterpret_cast<const T*>(a.v) + b * a.vs.b + hk * a.vs.h;
-  load_tile<T, D>(Ks, k, a.ks.s, col0, a.Skv, tid);
-  load_tile<T, D>(Vs, v, a.vs.s, col0, a.Skv, tid);
+}
 
-  float dk[4][DC], dv[4][DC];
+template <int D>
+__device__ __forceinline__ void store_rows(float* out, const Str3& st, int row0, int step, int n_rows, int first, int tx,
+                                           const float2 (&acc)[Cfg<D>::R][D / 32]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < Cfg<D>::R; ++i) {
+    const int row = row0 + first + step * i;
+    if (row >= n_rows) continue;
 #pragma unroll
-    for (int j = 0; j < DC; ++j) dk[i][j] = 0.f, dv[i][j] = 0.f;
+    for (int c = 0; c < D / 64; ++c)
+      *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * st.s + tx * 4 + c * 64) =
+          make_float4(acc[i][2 * c].x, acc[i][2 * c].y, acc[i][2 * c + 1].x, acc[i][2 * c + 1].y);
+  }
+}
 
-  const int n_q_tiles = (a.Lq + TM - 1) / TM;
-  const int shift = causal_shift(a.causal, kv_len, a.Lq);
-  // first query tile with a row i such that col0 <= i + shift
-  const int qt_begin = a.causal ? (col0 - shift > 0 ? (col0 - shift) / TM : 0) : 0;
-  if (col0 < kv_len) {
-    for (int g = 0; g < group; ++g) {
-      const int h = hk * group + g;
-      const T* q = reinterpret_cast<const T*>(a.q) + b * a.qs.b + h * a.qs.h;
-      const T* dO = reinterpret_cast<const T*>(a.d_o) + b * a.dos.b + h * a.dos.h;
-      const float* lse = a.lse + (static_cast<int64_t>(b) * a.Hq + h) * a.Lq;
-      const float* delta = a.delta + (static_cast<int64_t>(b) * a.Hq + h) * a.Lq;
-      for (int qt = qt_begin; qt < n_q_tiles; ++qt) {
-        const int row0 = qt * TM;
-        __syncthreads();
-        load_tile<T, D>(Qs, q, a.qs.s, row0, a.Lq, tid);
-        load_tile<T, D>(dOs, dO, a.dos.s, row0, a.Lq, tid);
-        if (tid < TM) {
-          const bool in = row0 + tid < a.Lq;
-          lse_s[tid] = in ? lse[row0 + tid] : 0.f;
-          delta_s[tid] = in ? delta[row0 + tid] : 0.f;
-        }
-        __syncthreads();
-        tile_p_ds<T, D>(a, Qs, Ks, Vs, dOs, lse_s, delta_s, Ps, dSs, row0, col0, kv_len, shift,
-                        b * a.mask.sb + h * a.mask.sh, ty, tx);
-        __syncthreads();
-        // dV[kv][d] += sum_row P[row][kv] dO[row][d];  dK[kv][d] += sum_row dS[row][kv] Q[row][d]
-#pragma unroll 2
-        for (int r = 0; r < TM; ++r) {
-          float pv[4], sv[4], gv[DC], qv[DC];
+template <int D, bool MASK>
+__global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(const BwdArgs a, int key_tiles, int key_ctas) {
+  using C = Cfg<D>;
+  constexpr int TY = C::TY, R = C::R, NT = C::NT;
+  extern __shared__ __align__(16) float sm[];
+  float* Qs = sm;
+  float* dOs = Qs + kTileFloats<D>;
+  float* Ks = dOs + kTileFloats<D>;
+  float* Vs = Ks + kTileFloats<D>;
+  float* Ps = Vs + kTileFloats<D>;
+  float* dSs = Ps + kScoreFloats;
+  float* lse2_s = dSs + kScoreFloats;
+  float* delta_s = lse2_s + TS;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const bool keys = static_cast<int>(blockIdx.x) < key_ctas;
+  const int group = a.Hq / a.Hkv;
+
+  float2 acc0[R][D / 32], acc1[R][D / 32];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) pv[i] = Ps[r * LP + ty + 16 * i], sv[i] = dSs[r * LP + ty + 16 * i];
+  for (int i = 0; i < R; ++i)
 #pragma unroll
-          for (int j = 0; j < DC; ++j) gv[j] = dOs[r * LD + tx + 16 * j], qv[j] = Qs[r * LD + tx + 16 * j];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < DC; ++j) {
-              dv[i][j] = fmaf(pv[i], gv[j], dv[i][j]);
-              dk[i][j] = fmaf(sv[i], qv[j], dk[i][j]);
-            }
+    for (int j = 0; j < D / 32; ++j) acc0[i][j] = make_float2(0.f, 0.f), acc1[i][j] = make_float2(0.f, 0.f);
+
+  const float* qb = reinterpret_cast<const float*>(a.q);
+  const float* kb = reinterpret_cast<const float*>(a.k);
+  const float* vb = reinterpret_cast<const float*>(a.v);
+  const float* gb = reinterpret_cast<const float*>(a.d_o);
+  const int q_tiles = (a.Lq + TS - 1) / TS;
+
+  if (keys) {
+    // ------------------------------------------------------------- dK, dV of a key tile --
+    const int nt = blockIdx.x % key_tiles, bh = blockIdx.x / key_tiles;  // (the first key tile is seen by most queries)
+    const int hk = bh % a.Hkv, b = bh / a.Hkv, col0 = nt * TS;
+    int kv_len = a.Skv;
+    if (a.kv_lens) {
+      int l = a.kv_lens[b];
+      kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
+    }
+    const int shift = causal_shift(a.causal, kv_len, a.Lq);
+    // first query tile with a row i such that col0 <= i + shift
+    const int qt0 = a.causal ? (col0 - shift > 0 ? (col0 - shift) / TS : 0) : 0;
+    load_tile<D, NT>(Ks, kb + b * a.ks.b + hk * a.ks.h, a.ks.s, col0, a.Skv, tid);
+    load_tile<D, NT>(Vs, vb + b * a.vs.b + hk * a.vs.h, a.vs.s, col0, a.Skv, tid);
+    bool first = true;
+    if (col0 < kv_len) {
+      for (int g = 0; g < group; ++g) {
+        const int h = hk * group + g;
+        const float* q = qb + b * a.qs.b + h * a.qs.h;
+        const float* dO = gb + b * a.dos.b + h * a.dos.h;
+        const int64_t base = (static_cast<int64_t>(b) * a.Hq + h) * a.Lq;
+        for (int qt = qt0; qt < q_tiles; ++qt) {
+          const int row0 = qt * TS;
+          __syncthreads();  // the tiles of the step before have been read
+          load_tile<D, NT>(Qs, q, a.qs.s, row0, a.Lq, tid);
+          load_tile<D, NT>(dOs, dO, a.dos.s, row0, a.Lq, tid);
+          copies_commit();
+          if (first) ptx::grid_dep_wait();  // launched early behind the delta pre-pass
+          first = false;
+          load_vectors(a, lse2_s, delta_s, base, row0, tid);
+          copies_wait<0>();
+          __syncthreads();
+          tile_p_ds<D, MASK, true>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift,
+                                   b * a.mask.sb + h * a.mask.sh, ty, tx);
+          __syncthreads();
+          product_tn<D, TY>(Ps, dOs, ty, tx, acc0);
+          product_tn<D, TY>(dSs, Qs, ty, tx, acc1);
         }
       }
     }
-  }
-  T* dK = a.dk ? reinterpret_cast<T*>(a.dk) + b * a.dks.b + hk * a.dks.h : nullptr;
-  T* dV = a.dv ? reinterpret_cast<T*>(a.dv) + b * a.dvs.b + hk * a.dvs.h : nullptr;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int col = col0 + ty + 16 * i;
-    if (col >= a.Skv) continue;
-#pragma unroll
-    for (int j = 0; j < DC; ++j) {
-      if (dK) dK[static_cast<int64_t>(col) * a.dks.s + tx + 16 * j] = from_f32<T>(dk[i][j]);
-      if (dV) dV[static_cast<int64_t>(col) * a.dvs.s + tx + 16 * j] = from_f32<T>(dv[i][j]);
+    copies_wait<0>();
+    if (first) ptx::grid_dep_wait();
+    if (a.dv)
+      store_rows<D>(reinterpret_cast<float*>(a.dv) + b * a.dvs.b + hk * a.dvs.h, a.dvs, col0, 1, a.Skv, ty * R, tx, acc0);
+    if (a.dk)
+      store_rows<D>(reinterpret_cast<float*>(a.dk) + b * a.dks.b + hk * a.dks.h, a.dks, col0, 1, a.Skv, ty * R, tx, acc1);
+  } else {
+    // ----------------------------------------------------------------- dQ of a query tile --
+    const int x = blockIdx.x - key_ctas;
+    const int mt = q_tiles - 1 - x % q_tiles, bh = x / q_tiles;  // (under a causal mask the last tile is longest)
+    const int h = bh % a.Hq, b = bh / a.Hq, hk = h / group, row0 = mt * TS;
+    int kv_len = a.Skv;
+    if (a.kv_lens) {
+      int l = a.kv_lens[b];
+      kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
     }
-  }
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) bwd_dq_kernel(const BwdArgs a) {
-  constexpr int LD = D + 1, LP = TN + 1, DC = D / 16;
-  extern __shared__ float sm[];
-  float* Qs = sm;
-  float* dOs = Qs + TM * LD;
-  float* Ks = dOs + TM * LD;
-  float* Vs = Ks + TN * LD;
-  float* dSs = Vs + TN * LD;
-  float* lse_s = dSs + TM * LP;
-  float* delta_s = lse_s + TM;
-
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int mt = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
-  const int row0 = mt * TM;
-  int kv_len = a.Skv;
-  if (a.kv_lens) {
-    int l = a.kv_lens[b];
-    kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
-  }
-  const int shift = causal_shift(a.causal, kv_len, a.Lq);
-  int kv_end = kv_len;
-  if (a.causal && row0 + TM + shift < kv_end) kv_end = row0 + TM + shift > 0 ? row0 + TM + shift : 0;
-  const int n_tiles = (kv_end + TN - 1) / TN;
-
-  const T* q = reinterpret_cast<const T*>(a.q) + b * a.qs.b + h * a.qs.h;
-  const T* dO = reinterpret_cast<const T*>(a.d_o) + b * a.dos.b + h * a.dos.h;
-  const T* k = reinterpret_cast<const T*>(a.k) + b * a.ks.b + hk * a.ks.h;
-  const T* v = reinterpret_cast<const T*>(a.v) + b * a.vs.b + hk * a.vs.h;
-  load_tile<T, D>(Qs, q, a.qs.s, row0, a.Lq, tid);
-  load_tile<T, D>(dOs, dO, a.dos.s, row0, a.Lq, tid);
-  if (tid < TM) {
-    const bool in = row0 + tid < a.Lq;
-    const int64_t base = (static_cast<int64_t>(b) * a.Hq + h) * a.Lq + row0 + tid;
-    lse_s[tid] = in ? a.lse[base] : 0.f;
-    delta_s[tid] = in ? a.delta[base] : 0.f;
-  }
-  float dq[4][DC];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < DC; ++j) dq[i][j] = 0.f;
-
-  for (int t = 0; t < n_tiles; ++t) {
-    const int col0 = t * TN;
-    __syncthreads();
-    load_tile<T, D>(Ks, k, a.ks.s, col0, a.Skv, tid);
-    load_tile<T, D>(Vs, v, a.vs.s, col0, a.Skv, tid);
-    __syncthreads();
-    tile_p_ds<T, D>(a, Qs, Ks, Vs, dOs, lse_s, delta_s, nullptr, dSs, row0, col0, kv_len, shift,
-                    b * a.mask.sb + h * a.mask.sh, ty, tx);
-    __syncthreads();
-#pragma unroll 4
-    for (int cc = 0; cc < TN; ++cc) {
-      float sv[4], kv[DC];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sv[i] = dSs[(ty + 16 * i) * LP + cc];
-#pragma unroll
-      for (int j = 0; j < DC; ++j) kv[j] = Ks[cc * LD + tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < DC; ++j) dq[i][j] = fmaf(sv[i], kv[j], dq[i][j]);
+    const int shift = causal_shift(a.causal, kv_len, a.Lq);
+    int kv_end = kv_len;
+    if (a.causal && row0 + TS + shift < kv_end) kv_end = row0 + TS + shift > 0 ? row0 + TS + shift : 0;
+    const int n_tiles = (kv_end + TS - 1) / TS;
+    const float* k = kb + b * a.ks.b + hk * a.ks.h;
+    const float* v = vb + b * a.vs.b + hk * a.vs.h;
+    load_tile<D, NT>(Qs, qb + b * a.qs.b + h * a.qs.h, a.qs.s, row0, a.Lq, tid);
+    load_tile<D, NT>(dOs, gb + b * a.dos.b + h * a.dos.h, a.dos.s, row0, a.Lq, tid);
+    if (n_tiles > 0) {
+      load_tile<D, NT>(Ks, k, a.ks.s, 0, a.Skv, tid);
+      load_tile<D, NT>(Vs, v, a.vs.s, 0, a.Skv, tid);
     }
+    copies_commit();
+    ptx::grid_dep_wait();  // launched early behind the delta pre-pass
+    load_vectors(a, lse2_s, delta_s, (static_cast<int64_t>(b) * a.Hq + h) * a.Lq, row0, tid);
+    for (int t = 0; t < n_tiles; ++t) {
+      const int col0 = t * TS;
+      copies_wait<0>();
+      __syncthreads();
+      tile_p_ds<D, MASK, false>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, nullptr, dSs, row0, col0, kv_len, shift,
+                                b * a.mask.sb + h * a.mask.sh, ty, tx);
+      __syncthreads();
+      if (t + 1 < n_tiles) load_tile<D, NT>(Vs, v, a.vs.s, col0 + TS, a.Skv, tid);
+      product_nn<D, TY>(dSs, Ks, ty, tx, acc0);
+      __syncthreads();
+      if (t + 1 < n_tiles) load_tile<D, NT>(Ks, k, a.ks.s, col0 + TS, a.Skv, tid);
+      copies_commit();
+    }
+    copies_wait<0>();
+    store_rows<D>(reinterpret_cast<float*>(a.dq) + b * a.dqs.b + h * a.dqs.h, a.dqs, row0, TY, a.Lq, ty, tx, acc0);
   }
-  T* dQ = reinterpret_cast<T*>(a.dq) + b * a.dqs.b + h * a.dqs.h;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = row0 + ty + 16 * i;
-    if (row >= a.Lq) continue;
-#pragma unroll
-    for (int j = 0; j < DC; ++j) dQ[static_cast<int64_t>(row) * a.dqs.s + tx + 16 * j] = from_f32<T>(dq[i][j]);
-  }
-}
-
-template <typename T, int D>
-cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
-  const int64_t rows = static_cast<int64_t>(a.B) * a.Hq * a.Lq;
-  bwd_delta_kernel<T, D><<<static_cast<unsigned>((rows * (D * sizeof(T) / 16) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(a);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (a.dk || a.dv) {
-    constexpr int smem = (4 * TM * (D + 1) + 2 * TM * (TN + 1) + 2 * TM) * sizeof(float);
-    auto kern = bwd_dkdv_kernel<T, D>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<dim3((a.Skv + TN - 1) / TN, a.Hkv, a.B), kThreads, smem, stream>>>(a);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if (a.dq) {
-    constexpr int smem = (4 * TM * (D + 1) + TM * (TN + 1) + 2 * TM) * sizeof(float);
-    auto kern = bwd_dq_kernel<T, D>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    kern<<<dim3((a.Lq + TM - 1) / TM, a.Hq, a.B), kThreads, smem, stream>>>(a);
-    e = cudaGetLastError();
-  }
-  return e;
 }
 
 template <typename T, int D>
@@ -326,6 +262,28 @@ cudaError_t launch_delta_t(const BwdArgs& a, cudaStream_t stream) {
   const int64_t rows = static_cast<int64_t>(a.B) * a.Hq * a.Lq;
   bwd_delta_kernel<T, D><<<static_cast<unsigned>((rows * (D * sizeof(T) / 16) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(a);
   return cudaGetLastError();
+}
+
+template <int D, bool MASK>
+cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
+  cudaError_t e = launch_delta_t<float, D>(a, stream);
+  if (e != cudaSuccess) return e;
+  auto kern = bwd_simt_kernel<D, MASK>;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const long long key_tiles = (a.Skv + TS - 1) / TS, q_tiles = (a.Lq + TS - 1) / TS;
+  const long long key_ctas = a.dk || a.dv ? key_tiles * a.Hkv * a.B : 0, q_ctas = a.dq ? q_tiles * a.Hq * a.B : 0;
+  if (key_ctas + q_ctas > 0x7fffffffll) return cudaErrorInvalidValue;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(key_ctas + q_ctas));
+  cfg.blockDim = dim3(Cfg<D>::NT);
+  cfg.dynamicSmemBytes = Cfg<D>::kSmemBytes;
+  cfg.stream = stream;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, a, static_cast<int>(key_tiles), static_cast<int>(key_ctas));
 }
 
 }  // namespace
@@ -338,9 +296,11 @@ cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t st
 }
 
 cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, cudaStream_t stream) {
-  if (dtype == TT_ATTN_F32) return D == 64 ? launch_t<float, 64>(a, stream) : launch_t<float, 128>(a, stream);
-  if (dtype == TT_ATTN_F16) return D == 64 ? launch_t<__half, 64>(a, stream) : launch_t<__half, 128>(a, stream);
-  return D == 64 ? launch_t<__nv_bfloat16, 64>(a, stream) : launch_t<__nv_bfloat16, 128>(a, stream);
+  if (dtype != TT_ATTN_F32) return cudaErrorInvalidValue;
+  const bool mask = a.mask.ptr != nullptr;
+  if (D == 64) return mask ? launch_t<64, true>(a, stream) : launch_t<64, false>(a, stream);
+  if (D == 128) return mask ? launch_t<128, true>(a, stream) : launch_t<128, false>(a, stream);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace ttattn
