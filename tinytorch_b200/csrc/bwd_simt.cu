@@ -274,16 +274,8 @@ cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
   const long long key_tiles = (a.Skv + TS - 1) / TS, q_tiles = (a.Lq + TS - 1) / TS;
   const long long key_ctas = a.dk || a.dv ? key_tiles * a.Hkv * a.B : 0, q_ctas = a.dq ? q_tiles * a.Hq * a.B : 0;
   if (key_ctas + q_ctas > 0x7fffffffll) return cudaErrorInvalidValue;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(key_ctas + q_ctas));
-  cfg.blockDim = dim3(Cfg<D>::NT);
-  cfg.dynamicSmemBytes = Cfg<D>::kSmemBytes;
-  cfg.stream = stream;
-  cfg.attrs = attr, cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a, static_cast<int>(key_tiles), static_cast<int>(key_ctas));
+  return launch_early(kern, dim3(static_cast<unsigned>(key_ctas + q_ctas)), dim3(Cfg<D>::NT), Cfg<D>::kSmemBytes, stream, 1,
+                      a, static_cast<int>(key_tiles), static_cast<int>(key_ctas));
 }
 
 }  // namespace

@@ -158,6 +158,24 @@ void decode_plan(int capacity, int* nsplit, int* chunk);
 // ... for the tensor-core path (several query heads per kv head): longer chunks, see decode.cu
 void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int* nsplit, int* chunk);
 
+// Launches a kernel that calls ptx::grid_dep_wait() before it touches global memory: it may come up, and set itself up,
+// while the kernel before it in the stream ends (or, if that one allows it, still runs).  `cluster`: CTAs per cluster.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kern)(P...), dim3 grid, dim3 block, int smem, cudaStream_t stream, int cluster, A... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 template <typename T>
 __device__ __forceinline__ float to_f32(T x);
 template <>

@@ -268,17 +268,8 @@ cudaError_t sums_t(const void* x, void* out, int64_t rows, int64_t n, int64_t ld
   // the rows of a column block are divided while a CTA keeps at least 64 of them
   int cluster = 1;
   while (cluster < 8 && rows >= cluster * 2 * 64) cluster *= 2;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>((n + kSumCols - 1) / kSumCols) * cluster);
-  cfg.blockDim = dim3(kThreads);
-  cfg.stream = stream;
-  cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, column_sums_kernel<T>, static_cast<const T*>(x), static_cast<T*>(out), rows, n, ld, cluster);
+  return launch_early(column_sums_kernel<T>, dim3(static_cast<unsigned>((n + kSumCols - 1) / kSumCols) * cluster), dim3(kThreads), 0, stream, cluster,
+                      static_cast<const T*>(x), static_cast<T*>(out), rows, n, ld, cluster);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

@@ -5,10 +5,19 @@
 // writes the [L,S] score matrix to HBM.
 //
 // Persistent kernel, one CTA per SM, all 512 TMEM columns.  A work item is a pair
-// of 128-row query tiles of one (batch, head); CTAs draw items from a global
+// of 128-row query blocks of one (batch, kv head), numbered query tile by query
+// tile with the heads of the group together: where heads share keys, both blocks
+// see the same ones, and short sequences fill both.  CTAs draw items from a global
 // counter, heads in order and, within a head, the longest (latest causal) pair
 // first, so that the CTAs running at any moment share few heads' K/V in L2 and
 // the last items to be drawn are the shortest.
+// SPLIT: where the items leave most SMs idle (a chunk of new queries against a
+// long cache), the key tiles of an item are divided among the CTAs of a cluster,
+// one item per cluster; the unnormalised O, maxima and sums meet in distributed
+// shared memory at the end and every CTA of the cluster writes a share of the rows.
+// Measured (us, before -> now): 2 x 256 new queries against 8192 rows, 32/8 heads
+// 120 -> 75; 64 against 4096, 8/2 heads 60 -> 20; 32 against 15000, 8 heads, D = 64
+// 166 -> 29; grouped causal 8 x 2048, 32/8 heads 268 -> 262, 777, 32/8 heads 21 -> 19.
 //   warp 8   producer : draws items and publishes them to the other warps; TMA
 //                       tiled loads (128-byte swizzle, one copy per CTA) of the item's
 //                       two Q tiles and of each K and V tile into a 2-stage ring.
@@ -33,6 +42,7 @@
 // the CTA unwind.
 #include <cuda.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -88,20 +98,22 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 // One work item, decoded identically by every role.
 struct Item {
-  int b, h, hk, row0, kv_len, nt0, nt1, n_max, shift;
+  int b, hk, h0, h1, row00, row01;  // head and first row of the two blocks
+  int kv_len, shift;                // key j participates iff j <= i + shift (causal)
+  int j0, nt0, nt1, n_max;          // first key tile, and how many each block walks from there
 };
 
 // GEN: the general variant of the kernel (a mask and / or a causal triangle that is
 // not top-left aligned); the fast variant compiles all of that out.
 template <bool GEN>
-__device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs) {
+__device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs, int rank = 0, int cluster = 1) {
   Item it;
   // Heads in order, the longest (latest causal) pair of a head first: the CTAs running at any moment share few
   // heads' K/V in L2.  Only the last items are ordered differently: over the final kTailWaves waves the pairs of
   // the remaining heads are taken longest first ACROSS those heads, so that what is drawn last is short and the
   // CTAs finish together (in head order the last head's longest pair, an eighth of a CTA's whole share of
-  // config 2, would be drawn when most CTAs are nearly done).  Those heads' K/V together fit L2.
-  const int n_heads = a.B * a.Hq;
+  // 128 heads of 4096 rows, would be drawn when most CTAs are nearly done).  Those heads' K/V together fit L2.
+  const int n_heads = a.B * a.Hkv, group = a.Hq / a.Hkv;
   int tail_heads = (kTailWaves * static_cast<int>(gridDim.x) + n_pairs - 1) / n_pairs;
   if (tail_heads > n_heads) tail_heads = n_heads;
   const int w0 = (n_heads - tail_heads) * n_pairs;
@@ -110,31 +122,42 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs
     bh = w / n_pairs;
     mp = n_pairs - 1 - (w - bh * n_pairs);
   } else {
-    const int x = w - w0, rank = x / tail_heads;
-    bh = n_heads - tail_heads + (x - rank * tail_heads);
-    mp = n_pairs - 1 - rank;
+    const int x = w - w0, rank_in = x / tail_heads;
+    bh = n_heads - tail_heads + (x - rank_in * tail_heads);
+    mp = n_pairs - 1 - rank_in;
   }
-  it.b = bh / a.Hq;
-  it.h = bh - it.b * a.Hq;
-  it.hk = it.h / (a.Hq / a.Hkv);
-  it.row0 = mp * (QT * BM);
+  it.b = bh / a.Hkv;
+  it.hk = bh - it.b * a.Hkv;
   int kv_len = a.Skv;
   if (a.kv_lens) {
     int l = a.kv_lens[it.b];
     kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
   }
   it.kv_len = kv_len;
-  // Number of key tiles each query tile walks (0 for a tile wholly beyond Lq).
-  int e0 = kv_len, e1 = kv_len;
   it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
-  if (a.causal) {
-    int c0 = it.row0 + BM + it.shift, c1 = it.row0 + 2 * BM + it.shift;
-    if (GEN) c0 = c0 > 0 ? c0 : 0, c1 = c1 > 0 ? c1 : 0;
-    if (c0 < e0) e0 = c0;
-    if (c1 < e1) e1 = c1;
+  const int x = mp * QT, qt0 = x / group, qt1 = (x + 1) / group;
+  it.h0 = it.hk * group + x - qt0 * group, it.h1 = it.hk * group + x + 1 - qt1 * group;
+  it.row00 = qt0 * BM, it.row01 = qt1 * BM;
+  // key tiles that a block sees (0 for one wholly beyond Lq)
+  auto tiles = [&](int row0) {
+    int e = kv_len;
+    if (a.causal) {
+      int c = row0 + BM + it.shift;
+      if (GEN) c = c > 0 ? c : 0;
+      if (c < e) e = c;
+    }
+    return row0 < a.Lq ? (e + BN - 1) / BN : 0;
+  };
+  int nt0 = tiles(it.row00), nt1 = tiles(it.row01);
+  it.j0 = 0;
+  if (cluster > 1) {
+    // this CTA's share of the key tiles
+    const int n = nt0 > nt1 ? nt0 : nt1, lo = n * rank / cluster, hi = n * (rank + 1) / cluster;
+    it.j0 = lo;
+    nt0 = (nt0 < hi ? nt0 : hi) - lo, nt1 = (nt1 < hi ? nt1 : hi) - lo;
+    nt0 = nt0 > 0 ? nt0 : 0, nt1 = nt1 > 0 ? nt1 : 0;
   }
-  it.nt0 = (it.row0 < a.Lq) ? (e0 + BN - 1) / BN : 0;
-  it.nt1 = (it.row0 + BM < a.Lq) ? (e1 + BN - 1) / BN : 0;
+  it.nt0 = nt0, it.nt1 = nt1;
   it.n_max = it.nt0 > it.nt1 ? it.nt0 : it.nt1;
   return it;
 }
@@ -182,11 +205,64 @@ __device__ __forceinline__ void add_mask_row(uint32_t (&s)[BN], const MaskArgs& 
   }
 }
 
-template <int D, bool BF16, bool GEN>
+// SPLIT: the 256 rows of an item over the CS CTAs of the cluster.  `stats`: (reference, sum) of every row, `xo`: its
+// unnormalised O, at the same place in the shared memory of each CTA.  D / 4 lanes read a row (a warp's reads are whole
+// 512-byte rows), 8 vectors are in flight per thread; this CTA's own share is read as ordinary shared memory.
+template <int D, bool BF16, int CS>
+__device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, int rank, int warp, int lane, uint32_t stats,
+                                             uint32_t xo) {
+  using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+  constexpr int kPer = 128 / D;  // rows that a warp reads at a time
+  constexpr int kBatch = 8 / CS, kRows = QT * BM / CS;
+  const int c4 = lane % (D / 4);
+  uint32_t pstats[CS], pxo[CS];  // this CTA's first, then the others in turn
+#pragma unroll
+  for (int r = 1; r < CS; ++r) pstats[r] = ptx::map_rank(stats, (rank + r) % CS), pxo[r] = ptx::map_rank(xo, (rank + r) % CS);
+  pstats[0] = stats, pxo[0] = xo;
+#pragma unroll 1
+  for (int i = warp * kPer + lane / (D / 4); i < kRows; i += 8 * kPer * kBatch) {
+    float4 x[kBatch][CS];
+    float2 ml[kBatch][CS];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int rr = rank * kRows + i + u * 8 * kPer;
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+        const uint32_t sa = pstats[r] + rr * 8, xa = pxo[r] + rr * D * 4 + ((c4 ^ rr) & (D / 4 - 1)) * 16;
+        ml[u][r] = r == 0 ? ptx::ld_shared_f2(sa) : ptx::ld_cluster_f2(sa);
+        x[u][r] = r == 0 ? ptx::ld_shared_f4(xa) : ptx::ld_cluster_f4(xa);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int rr = rank * kRows + i + u * 8 * kPer, t = rr / BM;
+      const int row = (t == 0 ? it.row00 : it.row01) + (rr & (BM - 1)), head = t == 0 ? it.h0 : it.h1;
+      float m = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int r = 0; r < CS; ++r) m = fmaxf(m, ml[u][r].x);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+        if (ml[u][r].x == -INFINITY) continue;  // (a CTA without key tiles for the row left no O)
+        const float w = ptx::ex2(ml[u][r].x - m);
+        l = fmaf(ml[u][r].y, w, l);
+        v.x = fmaf(x[u][r].x, w, v.x), v.y = fmaf(x[u][r].y, w, v.y), v.z = fmaf(x[u][r].z, w, v.z), v.w = fmaf(x[u][r].w, w, v.w);
+      }
+      if (row >= a.Lq) continue;
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      *reinterpret_cast<uint2*>(reinterpret_cast<T*>(a.o) + it.b * a.os.b + head * a.os.h + static_cast<int64_t>(row) * a.os.s +
+                                c4 * 4) = make_uint2(pack2<BF16>(v.x * inv, v.y * inv), pack2<BF16>(v.z * inv, v.w * inv));
+      if (a.lse && c4 == 0)
+        a.lse[(static_cast<int64_t>(it.b) * a.Hq + head) * a.Lq + row] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+    }
+  }
+}
+
+template <int D, bool BF16, bool GEN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
     fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
-                  const FwdArgs a) {
+                  const FwdArgs a, int cluster) {
   extern __shared__ uint8_t smem_raw[];
   // 128-byte-swizzled tiles must start on a 1024-byte boundary.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -201,8 +277,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const int n_pairs = (a.Lq + QT * BM - 1) / (QT * BM);
-  const int n_items = n_pairs * a.Hq * a.B;
+  const int n_pairs = ((a.Lq + BM - 1) / BM * (a.Hq / a.Hkv) + QT - 1) / QT;
+  const int n_items = n_pairs * a.Hkv * a.B;
+  const int rank = SPLIT ? static_cast<int>(ptx::cluster_rank()) : 0;
+  auto item_of = [&](int w) { return SPLIT ? decode_item<GEN>(a, w, n_pairs, rank, cluster) : decode_item<GEN>(a, w, n_pairs); };
 
   constexpr int HALVES = D / 64;  // 64-element (128-byte) column blocks per row
   constexpr int HALF_BYTES = BM * 128;
@@ -246,6 +324,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
+  ptx::grid_dep_launch();  // (the next kernel may come up: this grid has its TMEM)
+  ptx::grid_dep_wait();    // (launched early: everything below reads or writes global memory)
 
   // Register budget: the softmax warpgroups hold a whole 128-column S row per
   // thread; the producer / issuer warpgroup needs little.
@@ -260,11 +340,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t g = 0;             // K/V tiles requested so far (ring position)
         uint32_t qc0 = 0, qc1 = 0;  // items whose Q tile 0 / 1 was requested so far
         for (uint32_t i = 0;; ++i) {
-          int w = atomicAdd(a.sched, 1);
+          // the first item is the CTA's own number; the counter, where one is needed, hands out the rest
+          int w;
+          if (SPLIT)
+            w = i == 0 ? static_cast<int>(blockIdx.x) / cluster : -1;
+          else
+            w = i == 0 ? static_cast<int>(blockIdx.x) : (a.sched ? static_cast<int>(gridDim.x) + atomicAdd(a.sched, 1) : -1);
           if (w >= n_items) w = -1;
           const int slot = i & 1;
           Item it{};
-          if (w >= 0) it = decode_item<GEN>(a, w, n_pairs);
+          if (w >= 0) it = item_of(w);
           if (!ptx::mbar_wait(&ctl->item_empty[slot], ((i >> 1) & 1) ^ 1, abort_flag)) break;
           ctl->item[slot] = w;
           ctl->item_nt0[slot] = w >= 0 ? it.nt0 : 0;
@@ -280,7 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             ptx::mbar_arrive_expect_tx(&ctl->q_full[t], TB);
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf)
-              ptx::tma_load_4d(sQ + t * TB + hf * HALF_BYTES, &tmQ, &ctl->q_full[t], hf * 64, it.row0 + t * BM, it.h, it.b);
+              ptx::tma_load_4d(sQ + t * TB + hf * HALF_BYTES, &tmQ, &ctl->q_full[t], hf * 64,
+                              t == 0 ? it.row00 : it.row01, t == 0 ? it.h0 : it.h1, it.b);
             ++qc;
             return true;
           };
@@ -292,13 +378,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             ptx::mbar_arrive_expect_tx(&ctl->k_full[st], TB);
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf)
-              ptx::tma_load_4d(sK + st * TB + hf * HALF_BYTES, &tmK, &ctl->k_full[st], hf * 64, j * BN, it.hk, it.b);
+              ptx::tma_load_4d(sK + st * TB + hf * HALF_BYTES, &tmK, &ctl->k_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
             if (j == 0 && !(ok = load_q(1, qc1))) break;
             if (!(ok = ptx::mbar_wait(&ctl->v_empty[st], ph ^ 1, abort_flag))) break;
             ptx::mbar_arrive_expect_tx(&ctl->v_full[st], TB);
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf)
-              ptx::tma_load_4d(sV + st * TB + hf * HALF_BYTES, &tmV, &ctl->v_full[st], hf * 64, j * BN, it.hk, it.b);
+              ptx::tma_load_4d(sV + st * TB + hf * HALF_BYTES, &tmV, &ctl->v_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
           }
           if (!ok) break;
         }
@@ -377,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           __syncwarp();  // every lane has read the slot before it is handed back
           if (leader) ptx::mbar_arrive(&ctl->item_empty[slot]);
           if (w < 0) break;
-          const Item it = decode_item<GEN>(a, w, n_pairs);
+          const Item it = item_of(w);
           if (it.n_max == 0) continue;
           const int nt0 = it.nt0, nt1 = it.nt1, n_max = it.n_max;
           auto nt = [&](int t) { return t == 0 ? nt0 : nt1; };
@@ -469,15 +555,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int w = ctl->item[slot];
       ptx::mbar_arrive(&ctl->item_empty[slot]);
       if (w < 0) break;
-      const Item it = decode_item<GEN>(a, w, n_pairs);
+      const Item it = item_of(w);
       const int n_t = t == 0 ? it.nt0 : it.nt1;
-      const int tile_row0 = it.row0 + t * BM;
+      const int tile_row0 = t == 0 ? it.row00 : it.row01, head = t == 0 ? it.h0 : it.h1;
       const int row = tile_row0 + r_in;  // global query row of this thread
       const int kv_len = it.kv_len;
-      T* orow = reinterpret_cast<T*>(a.o) + it.b * a.os.b + it.h * a.os.h + static_cast<int64_t>(row) * a.os.s;
-      float* lse_row = a.lse ? a.lse + (static_cast<int64_t>(it.b) * a.Hq + it.h) * a.Lq + row : nullptr;
+      T* orow = reinterpret_cast<T*>(a.o) + it.b * a.os.b + head * a.os.h + static_cast<int64_t>(row) * a.os.s;
+      float* lse_row = a.lse ? a.lse + (static_cast<int64_t>(it.b) * a.Hq + head) * a.Lq + row : nullptr;
 
-      if (n_t == 0) {
+      if (!SPLIT && n_t == 0) {
         // no participating key (or tile beyond Lq): O = 0, LSE = -inf
         if (row < a.Lq) {
 #pragma unroll
@@ -497,10 +583,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int cc = 0; cc < 4; ++cc) ptx::tmem_ld32p(tS + cc * 32, s + cc * 32);
         ptx::tmem_wait_ld();
 
-        const int col0 = j * BN;
+        const int col0 = (it.j0 + j) * BN;
         if constexpr (GEN) {
           if (a.mask.ptr && row < a.Lq)
-            add_mask_row<T>(s, a.mask, it.b * a.mask.sb + it.h * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
+            add_mask_row<T>(s, a.mask, it.b * a.mask.sb + head * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
         }
         const bool mask_tile = (col0 + BN > kv_len) || (a.causal && col0 + BN - 1 > tile_row0 + it.shift);
         if (mask_tile) {
@@ -590,6 +676,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       cnt += n_t;
 
+      if constexpr (SPLIT) {
+        // The unnormalised O (over the K / V stages), reference and sum (over the Q tiles) of this CTA's key tiles go
+        // to shared memory once every MMA of the CTA is complete; the rows are put together below.
+        if (ok && it.nt0 > 0) ok = ptx::mbar_wait(&ctl->o_full[0], 0, abort_flag);
+        if (ok && it.nt1 > 0) ok = ptx::mbar_wait(&ctl->o_full[1], 0, abort_flag);
+        __syncwarp();
+        ptx::tc_fence_after();
+        float* xo = reinterpret_cast<float*>(sK) + (t * BM + r_in) * D;
+        reinterpret_cast<float2*>(sQ)[t * BM + r_in] = make_float2(n_t > 0 ? m_ref : -INFINITY, l2.x + l2.y);
+        if (n_t > 0) {
+#pragma unroll
+          for (int cc = 0; cc < D / 32; ++cc) ptx::tmem_ld32p(tO + cc * 32, s + cc * 32);
+          ptx::tmem_wait_ld();
+#pragma unroll
+          for (int ch = 0; ch < D / 4; ++ch)  // (16-byte pieces of a row permuted by the row: no bank conflicts)
+            *reinterpret_cast<uint4*>(xo + ((ch ^ r_in) & (D / 4 - 1)) * 4) =
+                make_uint4(s[ch * 4], s[ch * 4 + 1], s[ch * 4 + 2], s[ch * 4 + 3]);
+        }
+        break;
+      }
+
       // epilogue: O / l -> global, LSE.  The issuer may already be computing the
       // next item's first S_t; its first PV waits for this warpgroup's next P.
       if (ok) ok = ptx::mbar_wait(&ctl->o_full[t], ec & 1, abort_flag);
@@ -622,13 +729,29 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::fence_proxy_async_smem();
         ptx::named_barrier(1 + t, BM);
         if (r_in == 0 && ok) {
-          ptx::tma_store_4d(&tmO, stage, hf * 64, tile_row0, it.h, it.b);
+          ptx::tma_store_4d(&tmO, stage, hf * 64, tile_row0, head, it.b);
           ptx::bulk_commit();
         }
       }
       if (ok && row < a.Lq && lse_row) *lse_row = l > 0.f ? (m_ref + log2f(l)) * kLn2 : -INFINITY;
     }
     if (r_in == 0) ptx::bulk_wait_all();
+  }
+
+  if constexpr (SPLIT) {
+    __syncwarp();
+    ptx::cluster_sync();
+    if (warp < 8 && *abort_flag == 0) {
+      const Item it = item_of(blockIdx.x / cluster);
+      if (cluster == 2)
+        combine_rows<D, BF16, 2>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+      else if (cluster == 4)
+        combine_rows<D, BF16, 4>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+      else
+        combine_rows<D, BF16, 8>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+    }
+    __syncwarp();
+    ptx::cluster_sync();  // no CTA leaves while another still reads its shared memory
   }
 
   ptx::tc_fence_before();
@@ -641,23 +764,70 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ------------------------------------------------------------------ host ----
-template <int D, bool BF16, bool GEN>
-cudaError_t launch_t(const FwdArgs& a, int dtype, int device, cudaStream_t stream) {
+template <int D, bool BF16, bool GEN, bool SPLIT>
+cudaError_t launch_k(const FwdArgs& a, int dtype, int grid, int cluster, cudaStream_t stream) {
   CUtensorMap tq, tk, tv, to;
   if (!make_map(&tq, dtype, a.q, D, a.Lq, a.Hq, a.B, a.qs) || !make_map(&tk, dtype, a.k, D, a.Skv, a.Hkv, a.B, a.ks) ||
       !make_map(&tv, dtype, a.v, D, a.Skv, a.Hkv, a.B, a.vs) || !make_map(&to, dtype, a.o, D, a.Lq, a.Hq, a.B, a.os))
     return cudaErrorInvalidValue;
-  auto kern = fwd_tc_kernel<D, BF16, GEN>;
+  auto kern = fwd_tc_kernel<D, BF16, GEN, SPLIT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D>());
   if (e != cudaSuccess) return e;
-  // the work counter must start at zero for every launch
-  e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);
-  if (e != cudaSuccess) return e;
-  const long long n_items = static_cast<long long>((a.Lq + QT * BM - 1) / (QT * BM)) * a.Hq * a.B;
+  return launch_early(kern, dim3(grid), dim3(kThreads), smem_bytes<D>(), stream, cluster, tq, tk, tv, to, a, cluster);
+}
+
+// CTAs of clusters of this size that can be resident at once, one to an SM (a cluster lives inside one GPC, and GPCs
+// differ in size).  Asked once per device.
+template <int D, bool BF16, bool GEN>
+int split_slots(int device, int cluster) {
+  static std::atomic<int> known[64][3];
+  if (device < 0 || device >= 64) return 0;
+  std::atomic<int>& k = known[device][cluster == 2 ? 0 : (cluster == 4 ? 1 : 2)];
+  int n = k.load(std::memory_order_relaxed);
+  if (n == 0) {
+    auto kern = fwd_tc_kernel<D, BF16, GEN, true>;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count(device) / cluster * cluster);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem_bytes<D>();
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D>()) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    n = clusters > 0 ? clusters * cluster : -1;
+    k.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+template <int D, bool BF16, bool GEN>
+cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
+  const long long n_pairs = ((a.Lq + BM - 1ll) / BM * (a.Hq / a.Hkv) + QT - 1) / QT, n_items = n_pairs * a.Hkv * a.B;
+  if (n_items > 0x7fffffffll) return cudaErrorInvalidValue;
   const int sms = sm_count(device);
+  // Keys divided over clusters: the largest cluster whose CTAs are all resident at once and walk at least three key
+  // tiles each (a step takes 1.6 us; the exchange and the cluster barriers about five).
+  const int n_tiles = ((a.causal == TT_ATTN_CAUSAL_TOP_LEFT && a.Lq < a.Skv ? a.Lq : a.Skv) + BN - 1) / BN;
+  for (int cs = 8; cs >= 2; cs >>= 1)
+    if (n_tiles >= 3 * cs && n_items * cs <= sms && n_items * cs <= split_slots<D, BF16, GEN>(device, cs)) {
+      a.sched = nullptr;
+      return launch_k<D, BF16, GEN, true>(a, dtype, static_cast<int>(n_items) * cs, cs, stream);
+    }
   const int grid = static_cast<int>(n_items < sms ? n_items : sms);
-  kern<<<grid, kThreads, smem_bytes<D>(), stream>>>(tq, tk, tv, to, a);
-  return cudaGetLastError();
+  if (n_items > grid) {
+    // the counter that hands out what comes after the CTAs' first items must start at zero for every launch
+    cudaError_t e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);
+    if (e != cudaSuccess) return e;
+  } else {
+    a.sched = nullptr;
+  }
+  return launch_k<D, BF16, GEN, false>(a, dtype, grid, 1, stream);
 }
 
 }  // namespace

@@ -324,18 +324,8 @@ cudaError_t launch_t(const LinearCall& c, const Plan& p) {
   uint32_t cols = 32;
   while (static_cast<int>(cols) < p.mt) cols *= 2;
   const SplitArgs a{c.bias, c.y, c.ldy, c.M, c.N, c.K, p.mt, p.tiles_m, p.stages, p.cluster, cols, c.status};
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = p.cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(p.tiles) * p.cluster);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = p.smem;
-  cfg.stream = c.stream;
-  cfg.attrs = attr, cfg.numAttrs = p.cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kern, tw, tx, a);
+  return launch_early(kern, dim3(static_cast<unsigned>(p.tiles) * p.cluster), dim3(kThreads), p.smem, c.stream, p.cluster,
+                      tw, tx, a);
 }
 
 template <bool BF16>

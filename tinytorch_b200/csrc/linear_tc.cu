@@ -271,16 +271,8 @@ cudaError_t launch_t(const LinearCall& c, int ctas) {
       !make_map_2d(&tw, c.dtype, c.w, W_MN ? c.N : c.K, W_MN ? c.K : c.N, c.ldw, W_MN ? BK : HN) ||
       !make_map_2d(&ty, c.dtype, c.y, c.N, c.M, c.ldy, HM))
     return cudaErrorInvalidValue;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = c.stream;
-  cfg.attrs = attr, cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, c.status});
+  return launch_early(kern, dim3(ctas), dim3(kThreads), kSmemBytes, c.stream, 1,
+                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, c.status});
 }
 
 template <bool BF16>
