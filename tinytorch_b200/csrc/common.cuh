@@ -102,7 +102,9 @@ struct DecodeArgs {
   void* q_rot;                     // append on the tensor-core path: scratch [B, Hq, D] for the rotated q
   int32_t* lens_scratch;           // ... and [B] for the lengths after the append
   int chained;                     // tensor-core path: the kernel before this one in the stream has zeroed the
-                                   // work counter and lets its dependents start early (programmatic launch)
+                                   // work counter
+  const int32_t* lens_hint;        // tensor-core path: lengths that may be read while the kernel before this one
+                                   // still runs, good enough to ask for cache rows in L2 (or null)
 };
 
 // Each returns a cudaError_t from the launch (no synchronisation).
@@ -154,7 +156,7 @@ cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows
 cudaError_t launch_wait_expiry(int32_t* status, uint64_t limit_ns, unsigned long long* waited_ns, cudaStream_t stream);
 
 // Split planning for decode, shared by the launcher and the workspace query.
-void decode_plan(int capacity, int* nsplit, int* chunk);
+void decode_plan(int B, int Hkv, int capacity, int* nsplit, int* chunk);
 // ... for the tensor-core path (several query heads per kv head): longer chunks, see decode.cu
 void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int* nsplit, int* chunk);
 

@@ -116,6 +116,7 @@ __device__ __forceinline__ void rope_slice(float (&x)[N], const float* cos, cons
 template <typename T, int D, int G, bool APPEND>
 __global__ void __launch_bounds__(kThreads, G == 1 ? 3 : 1) decode_kernel(const DecodeArgs a) {
   ptx::grid_dep_launch();  // the combine kernel's CTAs may come up under the last wave of this grid
+  ptx::grid_dep_wait();    // (launched early behind whatever is before it in the stream)
   constexpr int N = Vec16<T>::N;  // elements per 16-byte slice
   constexpr int LPK = D / N;      // lanes per cache row
   constexpr int KPW = 32 / LPK;   // rows per warp-wide load
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 3 : 1) decode_kernel(const 
   }
   const int begin = split * a.chunk;
   const int end = min(len, begin + a.chunk);
+  if (begin >= end && split > 0) return;  // (the combine kernel reads the splits that have rows, and the first)
   const float c = a.scale * kLog2e;
 
   for (int g0 = 0; g0 < group; g0 += G) {
@@ -305,64 +307,80 @@ __global__ void __launch_bounds__(kThreads, G == 1 ? 3 : 1) decode_kernel(const 
   }
 }
 
-// One CTA per (head, batch): fold the per-split partials into O and LSE.
-template <typename T, int D>
+// Splits of a sequence that left a partial result: those with rows, and in any case the first.  `appended`: the step's
+// token has been added to kv_lens[b] rows.
+__device__ __forceinline__ int splits_of(const DecodeArgs& a, int b, bool appended) {
+  int len = a.capacity;
+  if (a.kv_lens) {
+    const int l = a.kv_lens[b];
+    len = l < 0 ? 0 : (l < a.capacity ? l : a.capacity);
+    if (appended && len < a.capacity) ++len;
+  }
+  const int n = (len + a.chunk - 1) / a.chunk;
+  return n > 1 ? n : 1;
+}
+
+constexpr int kMaxSplit = 64;
+
+// One CTA per (head, batch): fold the per-split partials into O and LSE.  A thread per split fetches maximum and sum,
+// then a thread per channel adds the weighted partials, eight loads in flight.
+template <typename T, int D, bool APPEND>
 __global__ void __launch_bounds__(D) decode_combine_kernel(const DecodeArgs a) {
+  __shared__ float s_w[kMaxSplit], s_l[kMaxSplit];
   const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
-  ptx::grid_dep_wait();  // (launched early after the tensor-core scan: its partials are complete from here on)
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();  // (launched early after the scan: its partials are complete from here on)
+  const int n = splits_of(a, b, APPEND);
   const float* pp = a.partial + (static_cast<int64_t>(b) * a.Hq + h) * a.nsplit * (D + 2);
+  for (int s = d; s < n; s += D) s_w[s] = pp[s * (D + 2) + D], s_l[s] = pp[s * (D + 2) + D + 1];
+  __syncthreads();
   float mn = -INFINITY;
-  for (int s = 0; s < a.nsplit; ++s) mn = fmaxf(mn, pp[s * (D + 2) + D]);
+  for (int s = 0; s < n; ++s) mn = fmaxf(mn, s_w[s]);
   float lt = 0.f, at = 0.f;
-  for (int s = 0; s < a.nsplit; ++s) {
-    const float ms = pp[s * (D + 2) + D];
-    const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - mn);
-    lt += pp[s * (D + 2) + D + 1] * w;
-    at += pp[s * (D + 2) + d] * w;
+  for (int s0 = 0; s0 < n; s0 += 8) {
+    float p[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) p[u] = s0 + u < n ? pp[(s0 + u) * (D + 2) + d] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (s0 + u >= n) break;
+      const float ms = s_w[s0 + u];
+      const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - mn);
+      lt += s_l[s0 + u] * w;
+      at += p[u] * w;
+    }
   }
   const float inv = lt > 0.f ? 1.f / lt : 0.f;
   reinterpret_cast<T*>(a.o)[b * a.os.b + h * a.os.h + d] = from_f32<T>(at * inv);
   if (a.lse && d == 0) a.lse[static_cast<int64_t>(b) * a.Hq + h] = lt > 0.f ? (mn + log2f(lt)) * kLn2 : -INFINITY;
 }
 
-// `early`: the scan kernel before it lets its dependents start; the combine kernel's CTAs
-// then come up while the scan still runs and wait in grid_dep_wait() for its partials.
-template <typename T, int D>
-cudaError_t combine_t(const DecodeArgs& a, cudaStream_t stream, bool early = false) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a.Hq, a.B);
-  cfg.blockDim = dim3(D);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  if (early) cfg.attrs = attr, cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, decode_combine_kernel<T, D>, a);
+template <typename T, int D, bool APPEND>
+cudaError_t combine_t(const DecodeArgs& a, cudaStream_t stream) {
+  return launch_early(decode_combine_kernel<T, D, APPEND>, dim3(a.Hq, a.B), dim3(D), 0, stream, 1, a);
 }
 
 template <typename T, int D, bool APPEND>
 cudaError_t launch_t(const DecodeArgs& a, cudaStream_t stream) {
   const int group = a.Hq / a.Hkv;
   dim3 grid(a.nsplit, a.Hkv, a.B);
-  if (group % 8 == 0)
-    decode_kernel<T, D, 8, APPEND><<<grid, kThreads, 0, stream>>>(a);
-  else if (group % 4 == 0)
-    decode_kernel<T, D, 4, APPEND><<<grid, kThreads, 0, stream>>>(a);
-  else if (group % 2 == 0)
-    decode_kernel<T, D, 2, APPEND><<<grid, kThreads, 0, stream>>>(a);
-  else
-    decode_kernel<T, D, 1, APPEND><<<grid, kThreads, 0, stream>>>(a);
-  cudaError_t e = cudaGetLastError();
+  auto kern = group % 8 == 0   ? decode_kernel<T, D, 8, APPEND>
+              : group % 4 == 0 ? decode_kernel<T, D, 4, APPEND>
+              : group % 2 == 0 ? decode_kernel<T, D, 2, APPEND>
+                               : decode_kernel<T, D, 1, APPEND>;
+  cudaError_t e = launch_early(kern, grid, dim3(kThreads), 0, stream, 1, a);
   if (e != cudaSuccess || a.nsplit == 1) return e;
-  return combine_t<T, D>(a, stream, true);
+  return combine_t<T, D, APPEND>(a, stream);
 }
 
 }  // namespace
 
-void decode_plan(int capacity, int* nsplit, int* chunk) {
-  // 512-row chunks keep CTAs short enough that mixed sequence lengths balance
-  // across the SMs; at most 64 splits per sequence.
+// Splits of the scan: 512-row chunks keep CTAs short enough that mixed sequence lengths balance across the SMs; shorter
+// ones (down to 64 rows, one pass of a CTA) where a small batch would leave SMs without a CTA and every CTA with a long
+// serial scan (one sequence of 1024 rows and 8 heads: 16 CTAs of 512 rows, or 128 of 64); at most 64 per sequence.
+void decode_plan(int B, int Hkv, int capacity, int* nsplit, int* chunk) {
   int ck = 512;
+  while (ck > 64 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 148) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 63) / 64 * 64;
   *chunk = ck;
   *nsplit = capacity <= ck ? 1 : (capacity + ck - 1) / ck;
@@ -380,17 +398,18 @@ cudaError_t launch_d(int dtype, int D, const DecodeArgs& a, cudaStream_t stream)
 // The plan a call with these sizes uses (the launcher, the workspace query and the entry points agree
 // through this one function).  The tensor-core path pays a few thousand cycles at every item boundary
 // (the two softmax chains are merged there), so its chunks are 2048 rows - 16 tiles - unless that would
-// leave fewer than about two items per SM.
+// leave fewer than about two items per SM; below 512 rows only where those leave half of the SMs without one.
 void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int* nsplit, int* chunk) {
   DecodeArgs probe{};
   probe.Hq = Hq, probe.Hkv = Hkv;
   if (!decode_tc_applies(dtype, D, probe)) {
-    decode_plan(capacity, nsplit, chunk);
+    decode_plan(B, Hkv, capacity, nsplit, chunk);
     return;
   }
   int ck = 2048;
   const long long want = D == 64 ? 592 : 296;  // two items per resident CTA (D = 64 runs two CTAs per SM)
   while (ck > 512 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < want) ck >>= 1;
+  while (ck > 128 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 74) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 127) / 128 * 128;
   *chunk = ck;
   *nsplit = capacity <= ck ? 1 : (capacity + ck - 1) / ck;
@@ -401,8 +420,9 @@ cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t st
     // several query heads per kv head: the tensor-core scan, then the same combine kernel
     cudaError_t e = launch_decode_tc(dtype, D, a, stream);
     if (e != cudaSuccess || a.nsplit == 1) return e;
-    if (D == 128) return dtype == TT_ATTN_F16 ? combine_t<__half, 128>(a, stream, true) : combine_t<__nv_bfloat16, 128>(a, stream, true);
-    return dtype == TT_ATTN_F16 ? combine_t<__half, 64>(a, stream, true) : combine_t<__nv_bfloat16, 64>(a, stream, true);
+    if (D == 128)
+      return dtype == TT_ATTN_F16 ? combine_t<__half, 128, false>(a, stream) : combine_t<__nv_bfloat16, 128, false>(a, stream);
+    return dtype == TT_ATTN_F16 ? combine_t<__half, 64, false>(a, stream) : combine_t<__nv_bfloat16, 64, false>(a, stream);
   }
   return launch_d<false>(dtype, D, a, stream);
 }
@@ -417,6 +437,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(D / 2) rope_append_kernel(const DecodeArgs a, int32_t* lens_out) {
   const int hh = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
   ptx::grid_dep_launch();  // the decode kernel may set itself up; it waits for this grid before it reads anything
+  ptx::grid_dep_wait();
   if (hh == 0 && b == 0 && t == 0 && a.sched) *a.sched = 0;  // its work counter
   int pos = a.kv_lens[b];
   pos = pos < 0 ? 0 : pos;
@@ -455,13 +476,13 @@ __global__ void __launch_bounds__(D / 2) rope_append_kernel(const DecodeArgs a, 
 
 template <typename T, int D>
 cudaError_t append_tc_t(int dtype, const DecodeArgs& a, cudaStream_t stream) {
-  rope_append_kernel<T, D><<<dim3(a.Hq + a.Hkv, a.B), D / 2, 0, stream>>>(a, a.lens_scratch);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_early(rope_append_kernel<T, D>, dim3(a.Hq + a.Hkv, a.B), dim3(D / 2), 0, stream, 1, a, a.lens_scratch);
   if (e != cudaSuccess) return e;
   DecodeArgs d = a;
   d.q = a.q_rot;
   d.qs = Str3{static_cast<int64_t>(a.Hq) * D, D, D};
   d.kv_lens = a.lens_scratch;
+  d.lens_hint = a.kv_lens;
   d.chained = 1;
   return launch_decode(dtype, D, d, stream);
 }

@@ -97,15 +97,17 @@ __device__ __forceinline__ float warp_max(float x) {
   return __int_as_float(r);
 }
 
-__device__ __forceinline__ ItemDesc item_of(const DecodeArgs& a, int w) {
+// HINT: the lengths may still be being written; they are read past L1, so that no later reader on this SM finds a stale line.
+template <bool HINT = false>
+__device__ __forceinline__ ItemDesc item_of(const DecodeArgs& a, int w, const int32_t* kv_lens) {
   ItemDesc it;
   it.split = w % a.nsplit;
   const int bh = w / a.nsplit;
   it.hk = bh % a.Hkv;
   it.b = bh / a.Hkv;
   int len = a.capacity;
-  if (a.kv_lens) {
-    const int l = a.kv_lens[it.b];
+  if (kv_lens) {
+    const int l = HINT ? __ldcg(kv_lens + it.b) : kv_lens[it.b];
     len = l < 0 ? 0 : (l < a.capacity ? l : a.capacity);
   }
   it.begin = it.split * a.chunk;
@@ -173,28 +175,45 @@ __global__ void __launch_bounds__(kThreads, OCC)
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
   const uint32_t tS = tmem, tO = tmem + 2 * GP;  // buffer i of each at + 16 i
-  // Everything above touched no global memory.  In a chained launch the kernel before this one (rotation and
-  // append) may still be running: wait for its results, then let the combine kernel's CTAs come up.
+  // Everything above touched no global memory, and the kernel before this one (in the fused step: rotation and append)
+  // may still be running.  Under its end the first tiles of this CTA's first item are asked for in L2, by lengths that
+  // need only be about right (L2 is the point of coherence: a row that is still being written is not read stale).
+  ptx::grid_dep_launch();  // (the combine kernel's CTAs may come up: this grid has its TMEM)
+  if (warp == kProducerWarp && lane == 0 && (a.lens_hint || !a.kv_lens)) {
+    const ItemDesc it = item_of<true>(a, blockIdx.x, a.lens_hint);
+    for (int j = 0; j < it.n_tiles && j < NSTAGE; ++j)
+#pragma unroll
+      for (int hf = 0; hf < D / 64; ++hf) {
+        ptx::tma_prefetch_4d(&tmK, hf * 64, it.begin + j * BK, it.hk, it.b);
+        ptx::tma_prefetch_4d(&tmV, hf * 64, it.begin + j * BK, it.hk, it.b);
+      }
+  }
   ptx::grid_dep_wait();
-  ptx::grid_dep_launch();
 
   if (warp == kProducerWarp) {
     // -------------------------------------------------------------- producer --
     // All 32 lanes walk the items (an item without keys gets its empty result from this warp);
     // lane 0 publishes the others and issues the loads.
     uint32_t g = 0, pub = 0;
-    bool ok = true;
+    bool ok = true, own = true;
     // draws items from the counter until one has keys, publishes it (or the end marker)
     auto publish_next = [&](ItemDesc* out) {
       ItemDesc it;
       it.n_tiles = -1;
       for (;;) {
-        int w = 0;
-        if (lane == 0) w = atomicAdd(a.sched, 1);
-        w = __shfl_sync(0xffffffffu, w, 0);
+        // the first item is the CTA's own number; the counter, where there is more, hands out the rest
+        int w = blockIdx.x;
+        if (!own) {
+          if (static_cast<int>(gridDim.x) >= n_items) break;
+          if (lane == 0) w = static_cast<int>(gridDim.x) + atomicAdd(a.sched, 1);
+          w = __shfl_sync(0xffffffffu, w, 0);
+        }
+        own = false;
         if (w >= n_items) break;
-        it = item_of(a, w);
+        it = item_of(a, w, a.kv_lens);
         if (it.n_tiles > 0) break;
+        it.n_tiles = -1;
+        if (it.split > 0) continue;  // (the combine kernel reads the splits that have rows, and the first)
         for (int h = 0; h < group; ++h) {
           const int hq = it.hk * group + h;
           if (a.nsplit == 1) {
@@ -206,7 +225,6 @@ __global__ void __launch_bounds__(kThreads, OCC)
             if (lane == 0) pp[D] = -INFINITY, pp[D + 1] = 0.f;
           }
         }
-        it.n_tiles = -1;
       }
       if (lane == 0) {
         const int slot = pub % NFIFO;
@@ -549,7 +567,8 @@ __global__ void __launch_bounds__(kThreads, OCC)
 }
 
 template <bool BF16, int D, int OCC, int GH>
-cudaError_t launch_g(int dtype, const DecodeArgs& a, cudaStream_t stream) {
+cudaError_t launch_g(int dtype, DecodeArgs a, cudaStream_t stream) {
+  if (!a.lens_hint) a.lens_hint = a.kv_lens;
   constexpr int kSmem = Cfg<D, OCC>::kSmemBytes;
   CUtensorMap tk, tv;
   if (!make_map(&tk, dtype, a.k, D, a.capacity, a.Hkv, a.B, a.ks) || !make_map(&tv, dtype, a.v, D, a.capacity, a.Hkv, a.B, a.vs))
@@ -563,21 +582,12 @@ cudaError_t launch_g(int dtype, const DecodeArgs& a, cudaStream_t stream) {
   const long long n_items = static_cast<long long>(a.B) * a.Hkv * a.nsplit;
   if (n_items > 0x7fffffffll || !a.sched) return cudaErrorInvalidValue;
   const int ctas = OCC * sm_count(device);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(n_items < ctas ? n_items : ctas));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  if (a.chained) {
-    cfg.attrs = attr, cfg.numAttrs = 1;
-  } else {
+  if (n_items > ctas && !a.chained) {
     e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);  // the work counter starts at zero for every launch
     if (e != cudaSuccess) return e;
   }
-  return cudaLaunchKernelEx(&cfg, kern, tk, tv, a, static_cast<int>(n_items));
+  return launch_early(kern, dim3(static_cast<unsigned>(n_items < ctas ? n_items : ctas)), dim3(kThreads), kSmem, stream, 1, tk, tv,
+                      a, static_cast<int>(n_items));
 }
 
 template <bool BF16, int D, int OCC>

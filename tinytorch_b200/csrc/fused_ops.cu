@@ -49,12 +49,16 @@ __device__ __forceinline__ void st_cs(void* p, const uint4& v) {
 
 // A group of `tpr` threads (a power of two, 32..256) owns one row; a CTA holds
 // kThreads / tpr rows.  Each thread keeps VPT 16-byte vectors of the row.
-template <typename T, int VPT>
+// FEW: so few rows that the kernel is a chain of latencies: the weight is fetched with the row instead of after the sum
+// (with many rows it comes from L1, and its registers would cost resident warps).
+template <typename T, int VPT, bool FEW>
 __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ input, T* __restrict__ residual,
                                                                 const T* __restrict__ weight, int64_t rows, int dim,
                                                                 int tpr, float eps) {
   constexpr int N = Pack<T>::N;
   __shared__ float s_part[kThreads / 32];
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rows_per_cta = kThreads / tpr;
   const int t_in_row = tid % tpr;
@@ -64,13 +68,14 @@ __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ 
   T* in_row = input + row * dim;
   T* res_row = residual + row * dim;
 
-  uint4 a[VPT], b[VPT];
+  uint4 a[VPT], b[VPT], wv[FEW ? VPT : 1];
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int idx = t_in_row + v * tpr;
     const bool ok = row_ok && idx < vecs;
     a[v] = ok ? ld_cs(in_row + idx * N) : make_uint4(0, 0, 0, 0);
     b[v] = ok ? ld_cs(res_row + idx * N) : make_uint4(0, 0, 0, 0);
+    if (FEW) wv[v] = ok ? __ldg(reinterpret_cast<const uint4*>(weight + idx * N)) : make_uint4(0, 0, 0, 0);
   }
   float sum_sq = 0.f;
 #pragma unroll
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ 
     if (!(row_ok && idx < vecs)) continue;
     float fr[N], fw[N];
     Pack<T>::unpack(b[v], fr);
-    Pack<T>::unpack(__ldg(reinterpret_cast<const uint4*>(weight + idx * N)), fw);
+    Pack<T>::unpack(FEW ? wv[FEW ? v : 0] : __ldg(reinterpret_cast<const uint4*>(weight + idx * N)), fw);
 #pragma unroll
     for (int i = 0; i < N; ++i) fr[i] = fr[i] * inv_rms * fw[i];
     st_cs(in_row + idx * N, Pack<T>::pack(fr));
@@ -117,6 +122,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) add_rms_norm_generic_kernel(T* input, T* residual, const T* weight, int64_t dim,
                                                                         float eps) {
   __shared__ float s_part[kThreads / 32];
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   T* in_row = input + static_cast<int64_t>(blockIdx.x) * dim;
   T* res_row = residual + static_cast<int64_t>(blockIdx.x) * dim;
@@ -160,6 +167,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) silu_mul_rows_kernel(T* __restrict__ out, const T* __restrict__ x,
                                                                  int vecs_per_row) {
   constexpr int N = Pack<T>::N;
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int64_t row = blockIdx.x;
   const int v0 = blockIdx.y * (kThreads * kSiluUnroll) + threadIdx.x;
   const T* gp = x + row * 2 * vecs_per_row * N;
@@ -183,6 +192,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads) silu_mul_kernel(T* __restrict__ out, const T* __restrict__ x, uint32_t total_vecs,
                                                             uint32_t vecs_per_row) {
   constexpr int N = Pack<T>::N;
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const uint32_t idx = blockIdx.x * kThreads + threadIdx.x;
   if (idx >= total_vecs) return;
   const uint32_t row = idx / vecs_per_row, col = idx - row * vecs_per_row;
@@ -192,6 +203,8 @@ __global__ void __launch_bounds__(kThreads) silu_mul_kernel(T* __restrict__ out,
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) silu_mul_generic_kernel(T* out, const T* x, int64_t n, int64_t d) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
   const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
   if (i >= n) return;
   const int64_t row = i / d, col = i - row * d;
@@ -284,26 +297,24 @@ cudaError_t rms_t(void* input, void* residual, const void* weight, int64_t rows,
   const int64_t vecs = dim / N;
   const bool vec_ok = dim % N == 0 && vecs <= kThreads * 8 && aligned16(in) && aligned16(res) && aligned16(w);
   if (!vec_ok) {
-    add_rms_norm_generic_kernel<T><<<static_cast<unsigned>(rows), kThreads, 0, stream>>>(in, res, w, dim, eps);
-    return cudaGetLastError();
+    return launch_early(add_rms_norm_generic_kernel<T>, dim3(static_cast<unsigned>(rows)), dim3(kThreads), 0, stream, 1, in, res,
+                        w, dim, eps);
   }
   // threads per row: the fewest (>= 32) that keep a thread at <= 8 vectors ... but prefer
-  // <= 4 so that enough loads are in flight without starving occupancy
+  // <= 4 so that enough loads are in flight without starving occupancy; with fewer rows than SMs as many as there are
+  // vectors, up to a whole CTA per row
+  const bool few = rows < 148;
   int tpr = 32;
-  while (tpr < kThreads && vecs > static_cast<int64_t>(tpr) * 4) tpr <<= 1;
+  while (tpr < kThreads && vecs > static_cast<int64_t>(tpr) * (few ? 1 : 4)) tpr <<= 1;
   const int vpt = static_cast<int>((vecs + tpr - 1) / tpr);
   const int rows_per_cta = kThreads / tpr;
   const unsigned grid = static_cast<unsigned>((rows + rows_per_cta - 1) / rows_per_cta);
   const int d = static_cast<int>(dim);
-  if (vpt <= 1)
-    add_rms_norm_kernel<T, 1><<<grid, kThreads, 0, stream>>>(in, res, w, rows, d, tpr, eps);
-  else if (vpt <= 2)
-    add_rms_norm_kernel<T, 2><<<grid, kThreads, 0, stream>>>(in, res, w, rows, d, tpr, eps);
-  else if (vpt <= 4)
-    add_rms_norm_kernel<T, 4><<<grid, kThreads, 0, stream>>>(in, res, w, rows, d, tpr, eps);
-  else
-    add_rms_norm_kernel<T, 8><<<grid, kThreads, 0, stream>>>(in, res, w, rows, d, tpr, eps);
-  return cudaGetLastError();
+  auto kern = vpt <= 1   ? (few ? add_rms_norm_kernel<T, 1, true> : add_rms_norm_kernel<T, 1, false>)
+              : vpt <= 2 ? (few ? add_rms_norm_kernel<T, 2, true> : add_rms_norm_kernel<T, 2, false>)
+              : vpt <= 4 ? (few ? add_rms_norm_kernel<T, 4, true> : add_rms_norm_kernel<T, 4, false>)
+                         : (few ? add_rms_norm_kernel<T, 8, true> : add_rms_norm_kernel<T, 8, false>);
+  return launch_early(kern, dim3(grid), dim3(kThreads), 0, stream, 1, in, res, w, rows, d, tpr, eps);
 }
 
 template <typename T>
@@ -314,17 +325,18 @@ cudaError_t silu_t(void* out, const void* x, int64_t rows, int64_t d, cudaStream
   const int64_t vpr = d / N, total = rows * vpr;
   const bool vec_ok = d % N == 0 && aligned16(o) && aligned16(xi);
   constexpr int kChunk = kThreads * kSiluUnroll;
-  if (vec_ok && vpr >= kThreads && (vpr + kChunk - 1) / kChunk <= 65535 && rows <= 0x7fffffff) {
+  // (a handful of rows: one vector per thread, four times the CTAs)
+  const bool few = rows * ((vpr + kChunk - 1) / kChunk) < 148;
+  if (vec_ok && !few && vpr >= kThreads && (vpr + kChunk - 1) / kChunk <= 65535 && rows <= 0x7fffffff) {
     dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>((vpr + kChunk - 1) / kChunk));
-    silu_mul_rows_kernel<T><<<grid, kThreads, 0, stream>>>(o, xi, static_cast<int>(vpr));
-  } else if (vec_ok && total < 0x7fffff00ll) {
-    silu_mul_kernel<T><<<static_cast<unsigned>((total + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
-        o, xi, static_cast<uint32_t>(total), static_cast<uint32_t>(vpr));
-  } else {
-    const int64_t n = rows * d;
-    silu_mul_generic_kernel<T><<<static_cast<unsigned>((n + kThreads - 1) / kThreads), kThreads, 0, stream>>>(o, xi, n, d);
+    return launch_early(silu_mul_rows_kernel<T>, grid, dim3(kThreads), 0, stream, 1, o, xi, static_cast<int>(vpr));
   }
-  return cudaGetLastError();
+  if (vec_ok && total < 0x7fffff00ll)
+    return launch_early(silu_mul_kernel<T>, dim3(static_cast<unsigned>((total + kThreads - 1) / kThreads)), dim3(kThreads), 0,
+                        stream, 1, o, xi, static_cast<uint32_t>(total), static_cast<uint32_t>(vpr));
+  const int64_t n = rows * d;
+  return launch_early(silu_mul_generic_kernel<T>, dim3(static_cast<unsigned>((n + kThreads - 1) / kThreads)), dim3(kThreads), 0,
+                      stream, 1, o, xi, n, d);
 }
 
 }  // namespace
