@@ -120,7 +120,6 @@ int take_mask(const void* ptr, int kind, const int64_t st[3], MaskArgs* m) {
 extern "C" {
 
 size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D) {
-  (void)Hkv;
   if (B <= 0 || Hq <= 0 || D <= 0) return 0;
   // fp16 / bf16 forward: one work counter for the persistent kernel's scheduler
   if (kind == TT_ATTN_KIND_FWD) return dtype == TT_ATTN_F32 ? 0 : 256;
@@ -128,7 +127,10 @@ size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int 
     // delta [B,Hq,Lq] fp32; the fp16 / bf16 path adds an fp32 dQ accumulator [B,Hq,Lq,D]
     const size_t rows = static_cast<size_t>(B) * Hq * (Lq > 0 ? Lq : 0);
     // and the persistent kernel's work counter
-    return round256(rows * sizeof(float)) + (dtype == TT_ATTN_F32 ? 0 : round256(rows * D * sizeof(float)) + 256);
+    if (dtype == TT_ATTN_F32) return round256(rows * sizeof(float));
+    // (and, where few key tiles are divided among several work items, their partial dK / dV)
+    return round256(rows * sizeof(float)) + round256(rows * D * sizeof(float)) +
+           round256(bwd_part_bytes(B, Hq, Hkv, Lq, Skv, D)) + 256;
   }
   if (kind == TT_ATTN_KIND_DECODE_APPEND) {
     // the decode scratch; on the grouped-query tensor-core path also the rotated q and the new lengths
@@ -229,7 +231,12 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   a.delta = static_cast<float*>(ws.ptr);
   a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) +
                                         round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * sizeof(float)));
-  a.sched = p->dtype == TT_ATTN_F32 ? nullptr : reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + need - 256);
+  if (p->dtype != TT_ATTN_F32) {
+    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + need - 256);
+    a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
+    a.dkv_part = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dq_accum) +
+                                          round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * p->D * sizeof(float)));
+  }
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_simt(p->dtype, p->D, a, stream)
                                           : launch_bwd_tc(p->dtype, p->D, a, p->device, stream);

@@ -51,9 +51,16 @@ constexpr int kCompute = 512;  // four compute warpgroups
 constexpr int kTmemCols = 512;
 constexpr int kHalfBytes = BM * 128;  // one 64-element column block of a 128-row tile
 
+// A work item, decoded once by the producer.
+struct Item {
+  int hk, b, kv0, kv_len, shift, part;
+  // the walk: n_steps query tiles from tile qt of query head h on; a head's tiles are [qt_begin, n_q_tiles)
+  int qt_begin, n_steps, h, qt;  // n_steps < 0: no more items
+};
+
 struct __align__(8) SmemCtl {
   uint64_t item_full[2], item_empty[2];  // work items, from the producer to the issuer and the compute threads
-  int item[2];
+  Item item[2];
   uint64_t kv_full, kv_empty;            // K / V of the current item
   uint64_t q_full, q_empty;              // Q / dO of the current step
   uint64_t vec_full[2];                  // per-query vectors of a step (buffer g & 1), written by the producer warp
@@ -79,6 +86,9 @@ struct Cfg128 {
   static constexpr int kSmem = 2 * TB + 2 * TB + kDsBytes + kDqStage + kVecBytes + 256;
   static_assert(kSmem <= 232448, "exceeds the shared memory a CTA may request");
 };
+
+// First of the n steps of a key tile that belongs to part p of `parts`.
+__device__ __forceinline__ int part_begin(int n, int p, int parts) { return parts == 1 ? p * n : n * p / parts; }
 
 template <bool BF16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -168,8 +178,9 @@ __device__ __forceinline__ void ds_chunk(const uint32_t (&p)[16], const uint32_t
 }
 
 // GEN: the general variant (a mask and / or a causal triangle that is not top-left
-// aligned); the fast variant compiles all of that out.
-template <bool BF16, bool GEN>
+// aligned); the fast variant compiles all of that out.  PARTS: a key tile's walk is
+// divided among a.parts work items (see bwd_parts).
+template <bool BF16, bool GEN, bool PARTS>
 __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -204,13 +215,12 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
   // drawn last are the short ones and the CTAs finish together.
   const int group = a.Hq / a.Hkv;
   const int n_kt = (a.Skv + BM - 1) / BM, n_heads = a.Hkv * a.B;
-  const int n_items = n_kt * n_heads;
+  const int n_items = n_kt * n_heads * (PARTS ? a.parts : 1);
   const int n_q_tiles = (a.Lq + BQ - 1) / BQ;
-  struct Item {
-    int hk, b, kv0, kv_len, shift, qt_begin, per_head, n_steps;
-  };
   auto decode_item = [&](int w) {
     Item it;
+    it.part = 0;
+    if (PARTS) it.part = w % a.parts, w /= a.parts;
     const int w0 = (n_heads - a.tail_heads) * n_kt;
     int bh, nt;
     if (w < w0) {
@@ -232,9 +242,18 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
     // BM == BQ: query tiles before the key tile see none of it (general: first tile with a row i >= kv0 - shift)
     it.qt_begin = a.causal ? (GEN ? (it.kv0 - it.shift > 0 ? (it.kv0 - it.shift) / BQ : 0) : nt) : 0;
-    it.per_head = (it.kv0 < kv_len && it.qt_begin < n_q_tiles) ? n_q_tiles - it.qt_begin : 0;
-    it.n_steps = it.per_head * group;
+    const int per_head = (it.kv0 < kv_len && it.qt_begin < n_q_tiles) ? n_q_tiles - it.qt_begin : 0;
+    it.n_steps = per_head * group, it.h = it.hk * group, it.qt = it.qt_begin;
+    if (PARTS && per_head > 0) {
+      const int n0 = part_begin(it.n_steps, it.part, a.parts);
+      it.n_steps = part_begin(it.n_steps, it.part + 1, a.parts) - n0;
+      it.h += n0 / per_head, it.qt += n0 % per_head;
+    }
     return it;
+  };
+  // the next query tile of the walk
+  auto advance = [&](int& h, int& qt, int qt_begin) {
+    if (++qt == n_q_tiles) qt = qt_begin, ++h;
   };
 
   if (warp == C::kProdWarp && lane == 0) {
@@ -288,17 +307,16 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     uint32_t gq = 0;  // steps of earlier items
     bool dep_waited = false;
     // per-query vectors of running step g into buffer g & 1
-    auto fetch_vec = [&](const Item& it, int n, uint32_t g) {
+    auto fetch_vec = [&](const Item& it, uint32_t g) {
       if (!dep_waited) {
         // This kernel is launched early behind the delta pre-pass: barriers, TMEM and the first loads need
         // only the inputs; delta is first read here.
         ptx::grid_dep_wait();
         dep_waited = true;
       }
-      const int h = it.hk * group + n / it.per_head;
-      const int q0 = (it.qt_begin + n % it.per_head) * BQ;
+      const int q0 = it.qt * BQ;
       float lv[4], dl[4];
-      const int64_t base = (static_cast<int64_t>(it.b) * a.Hq + h) * a.Lq + q0;
+      const int64_t base = (static_cast<int64_t>(it.b) * a.Hq + it.h) * a.Lq + q0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int row = j * 32 + lane;
@@ -327,6 +345,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       w = __shfl_sync(0xffffffffu, w, 0);
       const bool redraw = w >= 0;  // (nothing is drawn behind the end of the list)
       Item it = {};
+      it.n_steps = -1;
       if (w >= 0) {
         it = decode_item(w);
         if (it.n_steps == 0) {
@@ -334,7 +353,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
           for (int t = 0; t < 2; ++t) {
             void* base = t == 0 ? a.dv : a.dk;
             const Str3& st = t == 0 ? a.dvs : a.dks;
-            if (!base) continue;
+            if (!base || PARTS) continue;  // (of a divided key tile the last kernel knows which parts exist)
             T* out = reinterpret_cast<T*>(base) + it.b * st.b + it.hk * st.h;
             for (int e = lane; e < BM * (D / 8); e += 32) {
               const int row = it.kv0 + e / (D / 8);
@@ -352,7 +371,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         const int slot = i & 1;
         ok = ptx::mbar_wait(&ctl->item_empty[slot], ((i >> 1) & 1) ^ 1, abort_flag);
         if (ok) {
-          ctl->item[slot] = w;
+          ctl->item[slot] = it;
           ptx::mbar_arrive(&ctl->item_full[slot]);
         }
         // every MMA of the item before has completed
@@ -368,15 +387,14 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok || w < 0) break;
-      for (int n = 0; n < it.n_steps; ++n) {
+      for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
         if (redraw && n + 1 == it.n_steps && lane == 0) drawn = atomicAdd(a.sched, 1);
         const uint32_t g = gq + n;
-        const int h = it.hk * group + n / it.per_head;
-        const int q0 = (it.qt_begin + n % it.per_head) * BQ;
+        const int h = it.h, q0 = it.qt * BQ;
         // The vectors (two buffers) are fetched a step ahead of the tiles (one stage): the wait passed for the
         // tiles of step g - 1 says that step g - 2, the last to read this buffer, is over.
         const bool vec_first = g > 0;
-        if (vec_first) fetch_vec(it, n, g);
+        if (vec_first) fetch_vec(it, g);
         if (lane == 0) {
           // the MMAs that read Q / dO of the step before have completed
           ok = ptx::mbar_wait(&ctl->q_empty, (g & 1) ^ 1, abort_flag);
@@ -391,7 +409,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        if (!vec_first) fetch_vec(it, n, g);
+        if (!vec_first) fetch_vec(it, g);
       }
       if (!ok) break;
       gq += it.n_steps;
@@ -417,17 +435,15 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     const uint32_t dolo_mn = ptx::smem_desc_lo(ptx::smem_u32(sdO), kHalfBytes);
     const uint32_t dslo_mn = ptx::smem_desc_lo(ptx::smem_u32(sdS), kHalfBytes);
     uint32_t fi = 0;  // items taken from the queue
-    // the next item, or false: none is left or a wait ran out
-    auto fetch = [&](Item& it) {
+    // the steps of the next item, or false: none is left or a wait ran out
+    auto fetch = [&](int& n_steps) {
       const int slot = fi & 1;
       if (!uwait(&ctl->item_full[slot], (fi >> 1) & 1)) return false;
-      const int w = ctl->item[slot];
+      n_steps = ctl->item[slot].n_steps;
       __syncwarp();  // every lane has read the slot
       if (leader) ptx::mbar_arrive(&ctl->item_empty[slot]);
       ++fi;
-      if (w < 0) return false;
-      it = decode_item(w);
-      return true;
+      return n_steps >= 0;
     };
     // dP^T = V dO^T of running step g into region B
     auto issue_dp = [&]() {
@@ -446,7 +462,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       }
       if (leader) ptx::mma_commit(&ctl->sp_full);
     };
-    Item cur = {}, nxt = {};
+    int cur = 0, nxt = 0;  // steps of the current and the next item
     uint32_t g = 0, k = 0;
     bool have = fetch(cur);
     bool ok = have && uwait(&ctl->kv_full, 0) && uwait(&ctl->q_full, 0);
@@ -457,8 +473,8 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     }
     while (have && ok) {
       bool have_next = false;
-      for (int n = 0; n < cur.n_steps && ok; ++n, ++g) {
-        const bool last = n + 1 == cur.n_steps;
+      for (int n = 0; n < cur && ok; ++n, ++g) {
+        const bool last = n + 1 == cur;
         // dV and dK contract over the 128 queries, 16 per k-step (2048 bytes of B).  Warpgroup w forms
         // the queries of k-step 2w first and of k-step 2w+1 second, so the even k-steps run while the
         // odd ones are still being computed.
@@ -520,14 +536,13 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     for (uint32_t k = 0;; ++k) {
       const int slot = k & 1;
       if (ok) ok = ptx::mbar_wait(&ctl->item_full[slot], (k >> 1) & 1, abort_flag);
-      const int w = ok ? ctl->item[slot] : -1;
+      const Item it = ctl->item[slot];
       ptx::mbar_arrive(&ctl->item_empty[slot]);
       // a warpgroup leaves as one (its named barriers below count all 128 threads) when any of its waits ran out
       if (ptx::named_barrier_or(3 + wg, BM, !ok)) break;
-      if (w < 0) break;
-      const Item it = decode_item(w);
-      const int b = it.b, hk = it.hk, kv0 = it.kv0, kv_len = it.kv_len, shift = it.shift, qt_begin = it.qt_begin,
-                per_head = it.per_head, n_steps = it.n_steps;
+      if (it.n_steps < 0) break;
+      const int b = it.b, hk = it.hk, kv0 = it.kv0, kv_len = it.kv_len, shift = it.shift, n_steps = it.n_steps;
+      int h = it.h, qt = it.qt;  // query head and tile of the step
       const int kv_row = kv0 + r;
       const bool row_valid = kv_row < kv_len;
 
@@ -537,8 +552,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       // clipped by the tensor map)
       auto read_out_dq = [&](int n) {
         const uint32_t g = g0 + n;
-        const int h = hk * group + n / per_head;
-        const int q0 = (qt_begin + n % per_head) * BQ;
+        const int q0 = qt * BQ;
         if (ok) ok = ptx::mbar_wait(&ctl->dq_full, g & 1, abort_flag);
         ptx::tc_fence_after();
         uint32_t v[32];
@@ -561,9 +575,9 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         }
       };
 
-      for (int n = 0; n < n_steps; ++n) {
+      for (int n = 0; n < n_steps; ++n, advance(h, qt, it.qt_begin)) {
         const uint32_t g = g0 + n;
-        const int q0 = (qt_begin + n % per_head) * BQ;
+        const int q0 = qt * BQ;
         // per-query vectors of the step, written by the producer warp: [0,128) -lse * log2(e), [128,256) -delta * scale
         const float* vec = svec + (g & 1) * 2 * BQ;
         uint8_t* ds_tile = sdS;
@@ -583,7 +597,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
           uint32_t pk[8], dk[8];
           int64_t mo = 0;
           if constexpr (GEN)
-            mo = b * a.mask.sb + (hk * group + n / per_head) * a.mask.sh + static_cast<int64_t>(q0 + col) * a.mask.sl +
+            mo = b * a.mask.sb + h * a.mask.sh + static_cast<int64_t>(q0 + col) * a.mask.sl +
                  kv_row;
           int n_hidden = 0;
           if (masked) n_hidden = !row_valid ? 16 : (diag ? kv_row - (q0 + col + shift) : 0);
@@ -626,35 +640,61 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         ptx::tc_fence_after();
         const uint32_t src = (wg == 0 ? tdV : tdK) + lane_addr;
         uint8_t* stage = sdq + wg * (BQ * 128);
+        if constexpr (PARTS) {
+          // a part of the key tile's walk: fp32, 32 columns at a time, into its own place in the workspace
 #pragma unroll 1
-        for (int hf = 0; hf < HALVES; ++hf) {
-          if (r == 0) ptx::bulk_wait_read();  // the previous store / reduction has read the staging tile
-          ptx::named_barrier(3 + wg, BM);
-#pragma unroll
-          for (int c2 = 0; c2 < 2; ++c2) {
+          for (int cc = 0; cc < D / 32; ++cc) {
             uint32_t v[32];
-            ptx::tmem_ld32(src + hf * 64 + c2 * 32, v);
+            ptx::tmem_ld32(src + cc * 32, v);
+            if (r == 0) ptx::bulk_wait_read();
             ptx::tmem_wait_ld();
-            if (hf == HALVES - 1 && c2 == 1) {
-              // the accumulators may be overwritten by the next item's first products
+            if (cc == D / 32 - 1) {
               ptx::tc_fence_before();
               ptx::mbar_arrive(&ctl->acc_free);
             }
+            ptx::named_barrier(3 + wg, BM);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              uint4 w4;
-              w4.x = pack2<BF16>(__uint_as_float(v[j * 8 + 0]), __uint_as_float(v[j * 8 + 1]));
-              w4.y = pack2<BF16>(__uint_as_float(v[j * 8 + 2]), __uint_as_float(v[j * 8 + 3]));
-              w4.z = pack2<BF16>(__uint_as_float(v[j * 8 + 4]), __uint_as_float(v[j * 8 + 5]));
-              w4.w = pack2<BF16>(__uint_as_float(v[j * 8 + 6]), __uint_as_float(v[j * 8 + 7]));
-              *reinterpret_cast<uint4*>(stage + r * 128 + (((c2 * 4 + j) ^ (r & 7)) << 4)) = w4;
+            for (int ch = 0; ch < 8; ++ch)
+              *reinterpret_cast<uint4*>(stage + r * 128 + ((ch ^ (r & 7)) << 4)) =
+                  make_uint4(v[ch * 4 + 0], v[ch * 4 + 1], v[ch * 4 + 2], v[ch * 4 + 3]);
+            ptx::fence_proxy_async_smem();
+            ptx::named_barrier(3 + wg, BM);
+            if (r == 0 && ok && wanted) {
+              ptx::tma_store_4d(wg == 0 ? &tmdV : &tmdK, stage, cc * 32, kv0, b * a.Hkv + hk, it.part);
+              ptx::bulk_commit();
             }
           }
-          ptx::fence_proxy_async_smem();
-          ptx::named_barrier(3 + wg, BM);
-          if (r == 0 && ok && wanted) {
-            ptx::tma_store_4d(wg == 0 ? &tmdV : &tmdK, stage, hf * 64, kv0, hk, b);
-            ptx::bulk_commit();
+        } else {
+#pragma unroll 1
+          for (int hf = 0; hf < HALVES; ++hf) {
+            if (r == 0) ptx::bulk_wait_read();  // the previous store / reduction has read the staging tile
+            ptx::named_barrier(3 + wg, BM);
+#pragma unroll
+            for (int c2 = 0; c2 < 2; ++c2) {
+              uint32_t v[32];
+              ptx::tmem_ld32(src + hf * 64 + c2 * 32, v);
+              ptx::tmem_wait_ld();
+              if (hf == HALVES - 1 && c2 == 1) {
+                // the accumulators may be overwritten by the next item's first products
+                ptx::tc_fence_before();
+                ptx::mbar_arrive(&ctl->acc_free);
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                uint4 w4;
+                w4.x = pack2<BF16>(__uint_as_float(v[j * 8 + 0]), __uint_as_float(v[j * 8 + 1]));
+                w4.y = pack2<BF16>(__uint_as_float(v[j * 8 + 2]), __uint_as_float(v[j * 8 + 3]));
+                w4.z = pack2<BF16>(__uint_as_float(v[j * 8 + 4]), __uint_as_float(v[j * 8 + 5]));
+                w4.w = pack2<BF16>(__uint_as_float(v[j * 8 + 6]), __uint_as_float(v[j * 8 + 7]));
+                *reinterpret_cast<uint4*>(stage + r * 128 + (((c2 * 4 + j) ^ (r & 7)) << 4)) = w4;
+              }
+            }
+            ptx::fence_proxy_async_smem();
+            ptx::named_barrier(3 + wg, BM);
+            if (r == 0 && ok && wanted) {
+              ptx::tma_store_4d(wg == 0 ? &tmdV : &tmdK, stage, hf * 64, kv0, hk, b);
+              ptx::bulk_commit();
+            }
           }
         }
       }
@@ -693,7 +733,7 @@ struct __align__(8) Ctl64 {
   uint64_t p_done, ds_done;     // P^T / dS^T of a step have been formed
   uint64_t dq_full[2], dq_free[2];
   uint64_t acc_full, acc_free;
-  int item[2];
+  Item item[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -711,7 +751,7 @@ struct Cfg64 {
   static constexpr int kProdWarp = 20, kIssWarp = 21, kThreads = 768;
 };
 
-template <bool BF16, bool GEN>
+template <bool BF16, bool GEN, bool PARTS>
 __global__ void __launch_bounds__(Cfg64::kThreads, 1)
     bwd_tc64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -741,13 +781,12 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
   // items drawn last are the short ones and the CTAs finish together.
   const int group = a.Hq / a.Hkv;
   const int n_kt = (a.Skv + BM - 1) / BM, n_heads = a.Hkv * a.B;
-  const int n_items = n_kt * n_heads;
+  const int n_items = n_kt * n_heads * (PARTS ? a.parts : 1);
   const int n_q_tiles = (a.Lq + BQ - 1) / BQ;
-  struct Item {
-    int hk, b, kv0, kv_len, shift, qt_begin, per_head, n_steps;
-  };
   auto decode_item = [&](int w) {
     Item it;
+    it.part = 0;
+    if (PARTS) it.part = w % a.parts, w /= a.parts;
     const int w0 = (n_heads - a.tail_heads) * n_kt;
     int bh, nt;
     if (w < w0) {
@@ -769,9 +808,18 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
     it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
     // BM == BQ: query tiles before the key tile see none of it (general: first tile with a row i >= kv0 - shift)
     it.qt_begin = a.causal ? (GEN ? (it.kv0 - it.shift > 0 ? (it.kv0 - it.shift) / BQ : 0) : nt) : 0;
-    it.per_head = (it.kv0 < kv_len && it.qt_begin < n_q_tiles) ? n_q_tiles - it.qt_begin : 0;
-    it.n_steps = it.per_head * group;
+    const int per_head = (it.kv0 < kv_len && it.qt_begin < n_q_tiles) ? n_q_tiles - it.qt_begin : 0;
+    it.n_steps = per_head * group, it.h = it.hk * group, it.qt = it.qt_begin;
+    if (PARTS && per_head > 0) {
+      const int n0 = part_begin(it.n_steps, it.part, a.parts);
+      it.n_steps = part_begin(it.n_steps, it.part + 1, a.parts) - n0;
+      it.h += n0 / per_head, it.qt += n0 % per_head;
+    }
     return it;
+  };
+  // the next query tile of the walk
+  auto advance = [&](int& h, int& qt, int qt_begin) {
+    if (++qt == n_q_tiles) qt = qt_begin, ++h;
   };
 
   if (warp == C::kProdWarp && lane == 0) {
@@ -846,6 +894,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
         w = __shfl_sync(0xffffffffu, w, 0);
         bool redraw = w >= 0;  // (nothing is drawn behind the end of the list)
         Item it = {};
+        it.n_steps = -1;
         if (w >= 0) {
           it = decode_item(w);
           if (it.n_steps == 0) {
@@ -853,7 +902,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
             for (int t = 0; t < 2; ++t) {
               void* base = t == 0 ? a.dv : a.dk;
               const Str3& st = t == 0 ? a.dvs : a.dks;
-              if (!base) continue;
+              if (!base || PARTS) continue;  // (of a divided key tile the last kernel knows which parts exist)
               T* out = reinterpret_cast<T*>(base) + it.b * st.b + it.hk * st.h;
               for (int e = lane; e < BM * (D / 8); e += 32) {
                 const int row = it.kv0 + e / (D / 8);
@@ -871,7 +920,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
           const int slot = i & 1;
           ok = ptx::mbar_wait(&ctl->item_empty[slot], ((i >> 1) & 1) ^ 1, abort_flag);
           if (ok) {
-            ctl->item[slot] = w;
+            ctl->item[slot] = it;
             ptx::mbar_arrive(&ctl->item_full[slot]);
           }
           // the MMAs that read this stage (two items ago) have completed
@@ -884,12 +933,11 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok || w < 0) break;
-        for (int n = 0; n < it.n_steps; ++n) {
+        for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
           if (redraw && n + 1 == it.n_steps && lane == 0) drawn = atomicAdd(a.sched, 1);
           const uint32_t g = gq + n;
           const int st = g % NQ;
-          const int h = it.hk * group + n / it.per_head;
-          const int q0 = (it.qt_begin + n % it.per_head) * BQ;
+          const int h = it.h, q0 = it.qt * BQ;
           if (lane == 0) {
             ok = ptx::mbar_wait(&ctl->q_empty[st], ((g / NQ) & 1) ^ 1, abort_flag);
             if (ok) {
@@ -953,17 +1001,15 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
       const uint32_t idesc_acc = ptx::make_idesc_f16(BM, D, fmt, 0, 1);  // dV, dK: A from TMEM, B MN-major
       const uint32_t idesc_dq = ptx::make_idesc_f16(BQ, D, fmt, 1, 1);   // dQ: both operands MN-major
       uint32_t fi = 0;  // items taken from the queue
-      // the next item, or false: none is left or a wait ran out
-      auto fetch = [&](Item& it) {
+      // the steps of the next item, or false: none is left or a wait ran out
+      auto fetch = [&](int& n_steps) {
         const int slot = fi & 1;
         if (!uwait(&ctl->item_full[slot], (fi >> 1) & 1)) return false;
-        const int w = ctl->item[slot];
+        n_steps = ctl->item[slot].n_steps;
         __syncwarp();  // every lane has read the slot
         if (leader) ptx::mbar_arrive(&ctl->item_empty[slot]);
         ++fi;
-        if (w < 0) return false;
-        it = decode_item(w);
-        return true;
+        return n_steps >= 0;
       };
       // K and V of the k-th item of this CTA are in shared memory
       auto kv_ready = [&](uint32_t k) { return uwait(&ctl->kv_full[k & 1], (k >> 1) & 1); };
@@ -991,14 +1037,14 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
         if (leader) ptx::mma_commit(&ctl->dp_full);
         return true;
       };
-      Item cur = {}, nxt = {};
+      int cur = 0, nxt = 0;  // steps of the current and the next item
       uint32_t g = 0, k = 0;
       bool have = fetch(cur);
       bool ok = have && kv_ready(0) && issue_s(0, 0) && issue_dp(0, 0);
       while (have && ok) {
         bool have_next = false;
-        for (int n = 0; n < cur.n_steps && ok; ++n, ++g) {
-          const bool last = n + 1 == cur.n_steps;
+        for (int n = 0; n < cur && ok; ++n, ++g) {
+          const bool last = n + 1 == cur;
           const uint32_t qlo_mn = ptx::smem_desc_lo(ptx::smem_u32(sQ + (g % NQ) * TB), kHalfBytes);
           const uint32_t dolo_mn = ptx::smem_desc_lo(ptx::smem_u32(sdO + (g & 1) * TB), kHalfBytes);
           // P^T is ready: dV += P^T dO, contraction over the queries, 16 per k-step (2048 bytes of B)
@@ -1063,30 +1109,35 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
     for (uint32_t k = 0;; ++k) {
       const int slot = k & 1;
       wwait(&ctl->item_full[slot], (k >> 1) & 1);
-      const int w = ok ? ctl->item[slot] : -1;
+      Item it = ctl->item[slot];
       ptx::mbar_arrive(&ctl->item_empty[slot]);
-      if (w < 0) break;
-      const Item it = decode_item(w);
-      for (int n = 0; n < it.n_steps; ++n, ++g) {
+      if (!ok || it.n_steps < 0) break;
+      for (int n = 0; n < it.n_steps; ++n, ++g, advance(it.h, it.qt, it.qt_begin)) {
         if (n + 1 == it.n_steps) {
           // dV, then dK: complete once the last step's products are (before its dQ); through the warp's staging
           // box (as [32 key rows][64 elements]) and a TMA store: coalesced, rows beyond Skv clipped
           wwait(&ctl->acc_full, k & 1);
           ptx::tc_fence_after();
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            if (lane == 0) ptx::bulk_wait_read();  // the previous store / reduction has read the box
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {  // 32 columns at a time: dV's two pieces, then dK's, whose columns follow
+            const bool is_v = c < 2, half = (c & 1) != 0;
+            uint32_t v[32];
+            ptx::tmem_ld32(tdV + lane_addr + c * 32, v);
+            // the previous store / reduction has read the box (16 bits: both pieces of a tensor go into one)
+            if (lane == 0 && (PARTS || !half)) ptx::bulk_wait_read();
+            ptx::tmem_wait_ld();
+            if (c == 3) {
+              // the accumulators may be overwritten by the next item's first products
+              ptx::tc_fence_before();
+              ptx::mbar_arrive(&ctl->acc_free);
+            }
             __syncwarp();
+            if (PARTS) {  // a part of the key tile's walk: fp32, into its own place in the workspace
 #pragma unroll
-            for (int cc = 0; cc < D / 32; ++cc) {
-              uint32_t v[32];
-              ptx::tmem_ld32((t == 0 ? tdV : tdK) + lane_addr + cc * 32, v);
-              ptx::tmem_wait_ld();
-              if (t == 1 && cc == D / 32 - 1) {
-                // the accumulators may be overwritten by the next item's first products
-                ptx::tc_fence_before();
-                ptx::mbar_arrive(&ctl->acc_free);
-              }
+              for (int ch = 0; ch < 8; ++ch)
+                *reinterpret_cast<uint4*>(box + lane * 128 + ((ch ^ (lane & 7)) << 4)) =
+                    make_uint4(v[ch * 4 + 0], v[ch * 4 + 1], v[ch * 4 + 2], v[ch * 4 + 3]);
+            } else {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 uint4 w4;
@@ -1094,19 +1145,22 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
                 w4.y = pack2<BF16>(__uint_as_float(v[j * 8 + 2]), __uint_as_float(v[j * 8 + 3]));
                 w4.z = pack2<BF16>(__uint_as_float(v[j * 8 + 4]), __uint_as_float(v[j * 8 + 5]));
                 w4.w = pack2<BF16>(__uint_as_float(v[j * 8 + 6]), __uint_as_float(v[j * 8 + 7]));
-                *reinterpret_cast<uint4*>(box + lane * 128 + (((cc * 4 + j) ^ (lane & 7)) << 4)) = w4;
+                *reinterpret_cast<uint4*>(box + lane * 128 + ((((c & 1) * 4 + j) ^ (lane & 7)) << 4)) = w4;
               }
             }
+            if (!PARTS && !half) continue;
             ptx::fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && ok && (t == 0 ? a.dv != nullptr : a.dk != nullptr) && it.kv0 + wj * 32 < a.Skv) {
-              ptx::tma_store_4d(t == 0 ? &tmdV : &tmdK, box, 0, it.kv0 + wj * 32, it.hk, it.b);
+            if (lane == 0 && ok && (is_v ? a.dv != nullptr : a.dk != nullptr) && it.kv0 + wj * 32 < a.Skv) {
+              if (PARTS)
+                ptx::tma_store_4d(is_v ? &tmdV : &tmdK, box, (c & 1) * 32, it.kv0 + wj * 32, it.b * a.Hkv + it.hk, it.part);
+              else
+                ptx::tma_store_4d(is_v ? &tmdV : &tmdK, box, 0, it.kv0 + wj * 32, it.hk, it.b);
               ptx::bulk_commit();
             }
           }
         }
-        const int h = it.hk * group + n / it.per_head;
-        const int q0 = (it.qt_begin + n % it.per_head) * BQ + wj * 32;
+        const int h = it.h, q0 = it.qt * BQ + wj * 32;
         wwait(&ctl->dq_full[g & 1], (g >> 1) & 1);
         ptx::tc_fence_after();
 #pragma unroll
@@ -1148,14 +1202,12 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
     for (uint32_t k = 0;; ++k) {
       const int slot = k & 1;
       if (ok) ok = ptx::mbar_wait(&ctl->item_full[slot], (k >> 1) & 1, abort_flag);
-      const int w = ok ? ctl->item[slot] : -1;
+      Item it = ctl->item[slot];
       ptx::mbar_arrive(&ctl->item_empty[slot]);
-      if (w < 0) break;
-      const Item it = decode_item(w);
+      if (!ok || it.n_steps < 0) break;
       const int kv_row = it.kv0 + r;
-      for (int n = 0; n < it.n_steps; ++n, ++g) {
-        const int hq = it.hk * group + n / it.per_head;
-        const int q0 = (it.qt_begin + n % it.per_head) * BQ;
+      for (int n = 0; n < it.n_steps; ++n, ++g, advance(it.h, it.qt, it.qt_begin)) {
+        const int hq = it.h, q0 = it.qt * BQ;
         const float* vec = svec + (g & 1) * 2 * BQ;
         // some (query, key) pairs of this step are hidden: the diagonal step, a ragged last key tile
         const bool diag = a.causal && q0 + it.shift < it.kv0 + BM;
@@ -1223,24 +1275,60 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
   if (tid == 0 && ctl->abort_flag && a.status) atomicOr(a.status, kStatusWaitExpired);
 }
 
-// dq_accum (fp32, dense [B,Hq,Lq,D]) -> dq (tensor dtype, strided)
+// 8 elements of a row, fp32 -> tensor dtype
+template <typename T>
+__device__ __forceinline__ void store8(T* dst, const float4& x, const float4& y) {
+  T out[8] = {from_f32<T>(x.x), from_f32<T>(x.y), from_f32<T>(x.z), from_f32<T>(x.w),
+              from_f32<T>(y.x), from_f32<T>(y.y), from_f32<T>(y.z), from_f32<T>(y.w)};
+  *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(out);
+}
+
+// dq_accum (fp32, dense [B,Hq,Lq,D]) -> dq (tensor dtype, strided), and where key tiles were divided the sum of their
+// parts' dK / dV, in part order.
 template <typename T, int D>
 __global__ void __launch_bounds__(256) dq_convert_kernel(const BwdArgs a) {
   ptx::grid_dep_wait();  // launched early: the accumulator is complete from here on
-  const int64_t total = static_cast<int64_t>(a.B) * a.Hq * a.Lq * (D / 8);
-  for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x, first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t total = a.dq ? static_cast<int64_t>(a.B) * a.Hq * a.Lq * (D / 8) : 0;
+  for (int64_t idx = first; idx < total; idx += step) {
     const int c8 = static_cast<int>(idx % (D / 8));
     const int64_t rowi = idx / (D / 8);
     const int i = static_cast<int>(rowi % a.Lq);
     const int h = static_cast<int>((rowi / a.Lq) % a.Hq);
     const int b = static_cast<int>(rowi / (static_cast<int64_t>(a.Lq) * a.Hq));
     const float4* src = reinterpret_cast<const float4*>(a.dq_accum + rowi * D + c8 * 8);
-    const float4 x = src[0], y = src[1];
-    T out[8] = {from_f32<T>(x.x), from_f32<T>(x.y), from_f32<T>(x.z), from_f32<T>(x.w),
-                from_f32<T>(y.x), from_f32<T>(y.y), from_f32<T>(y.z), from_f32<T>(y.w)};
-    T* dst = reinterpret_cast<T*>(a.dq) + b * a.dqs.b + h * a.dqs.h + static_cast<int64_t>(i) * a.dqs.s + c8 * 8;
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(out);
+    store8(reinterpret_cast<T*>(a.dq) + b * a.dqs.b + h * a.dqs.h + static_cast<int64_t>(i) * a.dqs.s + c8 * 8, src[0], src[1]);
+  }
+  if (a.parts <= 1) return;
+  const int64_t rows = static_cast<int64_t>(a.B) * a.Hkv * a.Skv, per_part = rows * D;
+  const int n_q_tiles = (a.Lq + BQ - 1) / BQ, group = a.Hq / a.Hkv;
+  for (int64_t idx = first; idx < 2 * rows * (D / 8); idx += step) {
+    const int t = idx >= rows * (D / 8);  // 0: dK, 1: dV
+    T* base = reinterpret_cast<T*>(t ? a.dv : a.dk);
+    if (!base) continue;
+    const Str3& st = t ? a.dvs : a.dks;
+    const int64_t e = idx - t * rows * (D / 8), rowi = e / (D / 8);
+    const int c8 = static_cast<int>(e % (D / 8)), j = static_cast<int>(rowi % a.Skv);
+    const int h = static_cast<int>((rowi / a.Skv) % a.Hkv), b = static_cast<int>(rowi / (static_cast<int64_t>(a.Skv) * a.Hkv));
+    // the steps of this row's key tile, as the main kernel counts them: a part without any has left nothing
+    const int kv0 = j / BM * BM;
+    int kv_len = a.Skv;
+    if (a.kv_lens) {
+      const int l = a.kv_lens[b];
+      kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
+    }
+    const int shift = causal_shift(a.causal, kv_len, a.Lq);
+    const int qt0 = a.causal ? (kv0 - shift > 0 ? (kv0 - shift) / BQ : 0) : 0;
+    const int n_all = kv0 < kv_len && qt0 < n_q_tiles ? (n_q_tiles - qt0) * group : 0;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    const float* src = a.dkv_part + t * a.parts * per_part + rowi * D + c8 * 8;
+    for (int p = 0; p < a.parts; ++p) {
+      if (part_begin(n_all, p, a.parts) == part_begin(n_all, p + 1, a.parts)) continue;
+      const float4 u = reinterpret_cast<const float4*>(src + p * per_part)[0], v = reinterpret_cast<const float4*>(src + p * per_part)[1];
+      x.x += u.x, x.y += u.y, x.z += u.z, x.w += u.w;
+      y.x += v.x, y.y += v.y, y.z += v.z, y.w += v.w;
+    }
+    store8(base + b * st.b + h * st.h + static_cast<int64_t>(j) * st.s + c8 * 8, x, y);
   }
 }
 
@@ -1255,19 +1343,24 @@ cudaError_t launch_t(const BwdArgs& a, int dtype, int device, cudaStream_t strea
     return cudaErrorInvalidValue;
   // dK / dV leave through TMA stores (boxes of 64 columns x 32 or 128 rows); an absent output gets a map that is never used
   constexpr int kOutRows = D == 64 ? 32 : 128;
-  if (!make_map(&tdk, dtype, a.dk ? a.dk : a.k, D, a.Skv, a.Hkv, a.B, a.dk ? a.dks : a.ks, kOutRows) ||
+  if (a.parts > 1) {
+    float* dv_part = a.dkv_part + static_cast<int64_t>(a.parts) * a.B * a.Hkv * a.Skv * D;
+    if (!make_map_f32(&tdk, a.dkv_part, D, a.Skv, a.B * a.Hkv, a.parts, kOutRows) ||
+        !make_map_f32(&tdv, dv_part, D, a.Skv, a.B * a.Hkv, a.parts, kOutRows))
+      return cudaErrorInvalidValue;
+  } else if (!make_map(&tdk, dtype, a.dk ? a.dk : a.k, D, a.Skv, a.Hkv, a.B, a.dk ? a.dks : a.ks, kOutRows) ||
       !make_map(&tdv, dtype, a.dv ? a.dv : a.v, D, a.Skv, a.Hkv, a.B, a.dv ? a.dvs : a.vs, kOutRows))
     return cudaErrorInvalidValue;
   cudaError_t e;  // (dq_accum has been cleared by the delta pre-pass)
   void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdArgs);
-  if constexpr (D == 64) kern = bwd_tc64_kernel<BF16, GEN>;
-  else kern = bwd_tc_kernel<BF16, GEN>;
+  if constexpr (D == 64) kern = a.parts > 1 ? bwd_tc64_kernel<BF16, GEN, true> : bwd_tc64_kernel<BF16, GEN, false>;
+  else kern = a.parts > 1 ? bwd_tc_kernel<BF16, GEN, true> : bwd_tc_kernel<BF16, GEN, false>;
   constexpr int kSmemBytes = D == 64 ? Cfg64::kSmem : Cfg128::kSmem;
   constexpr int kBlock = D == 64 ? Cfg64::kThreads : Cfg128::kThreads;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return e;
   const int n_kt = (a.Skv + BM - 1) / BM;
-  const long long n_items = static_cast<long long>(n_kt) * a.Hkv * a.B;
+  const long long n_items = static_cast<long long>(n_kt) * a.Hkv * a.B * a.parts;
   if (n_items > 0x7fffffffll) return cudaErrorInvalidValue;
   const int sms = sm_count(device);
   dim3 grid(static_cast<unsigned>(n_items < sms ? n_items : sms));  // persistent: one CTA per SM
@@ -1276,28 +1369,17 @@ cudaError_t launch_t(const BwdArgs& a, int dtype, int device, cudaStream_t strea
   ka.tail_heads = 0;
   if (a.causal) {
     const long long heads = static_cast<long long>(a.Hkv) * a.B;
-    const long long want = (2ll * sm_count(device) + n_kt - 1) / n_kt;
+    const long long want = (2ll * sm_count(device) + n_kt * a.parts - 1) / (n_kt * a.parts);
     ka.tail_heads = static_cast<int>(want < heads ? want : heads);
   }
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kBlock);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = stream;
-  cfg.attrs = attr, cfg.numAttrs = 1;  // early launch behind the delta pre-pass
-  e = cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, tdq, tdk, tdv, ka);
-  if (e != cudaSuccess || !a.dq) return e;
-  const int64_t total = static_cast<int64_t>(a.B) * a.Hq * a.Lq * (D / 8);
-  const int blocks = static_cast<int>((total + 255) / 256 < 8 * sm_count(device) ? (total + 255) / 256 : 8 * sm_count(device));
-  cudaLaunchConfig_t cv = {};
-  cv.gridDim = dim3(blocks);
-  cv.blockDim = dim3(256);
-  cv.stream = stream;
-  cv.attrs = attr, cv.numAttrs = 1;
-  return cudaLaunchKernelEx(&cv, dq_convert_kernel<T, D>, a);
+  // early, behind the delta pre-pass; the conversion kernel likewise behind this one
+  e = launch_early(kern, grid, dim3(kBlock), kSmemBytes, stream, 1, tq, tk, tv, tdo, tdq, tdk, tdv, ka);
+  if (e != cudaSuccess || (!a.dq && a.parts <= 1)) return e;
+  const int64_t total = static_cast<int64_t>(a.B) * D / 8 *
+                        ((a.dq ? static_cast<int64_t>(a.Hq) * a.Lq : 0) + (a.parts > 1 ? 2ll * a.Hkv * a.Skv : 0));
+  const int64_t most = 8 * sm_count(device);
+  const int blocks = static_cast<int>((total + 255) / 256 < most ? (total + 255) / 256 : most);
+  return launch_early(dq_convert_kernel<T, D>, dim3(blocks), dim3(256), 0, stream, 1, a);
 }
 
 }  // namespace
@@ -1310,6 +1392,41 @@ cudaError_t launch_g(int dtype, int D, const BwdArgs& a, int device, cudaStream_
   if (D == 64)
     return bf ? launch_t<64, true, GEN>(a, dtype, device, stream) : launch_t<64, false, GEN>(a, dtype, device, stream);
   return cudaErrorInvalidValue;
+}
+
+// A work item walks the query tiles that see its key tile, one after the other, so that with few key tiles the time is
+// that of the longest walk while most SMs are idle (3000 rows, 8 kv heads of 4 query heads: 192 walks of up to 96 steps
+// on 148 SMs, 65 steps' worth of work each).  The walk of a key tile can be divided among up to 8 items, each of which
+// leaves its share of dK and dV as fp32 in the workspace; the conversion kernel adds them in order (so the result does
+// not depend on timing).  Chosen is the division with the least expected time (fitted to a sweep of 18 shapes; what it
+// picks is within 4 % of the best of them): steps of 2.9 us (D = 128) or 1.6 us, as many as the longest share has or an
+// SM gets under longest-first order (whole waves where all walks are equal), 1.2 more for each item; and for divided
+// tiles 3 us, 0.5 us per share and the shares' way to memory and back (12 MB/us while L2 holds them, else 5.5).
+// Measured, us: 32/8 heads x 3000 D128 causal 305 -> 256; 2 x 2660, 16/4 heads D64 160 -> 122; 8000, 4/2 heads D128 370 ->
+// 207; 600, 2 x 8/2 heads D64 51 -> 29; undivided 2048, 8 x 16 heads D64 causal 252 (divided in two: 350).
+int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal) {
+  constexpr double kSms = 148, kItem = 1.2;
+  const double tiles = static_cast<double>((Skv + BM - 1) / BM) * Hkv * B, step_us = D == 128 ? 2.9 : 1.6;
+  const int group = Hq / Hkv, n = (Lq + BQ - 1) / BQ * group;
+  if (tiles > 4 * kSms) return 1;
+  int best = 1;
+  double best_us = 1e30;
+  for (int p = 1; p <= 8 && p <= n; ++p) {
+    const double share = (n + p - 1) / p + kItem, items = tiles * p;
+    const double all = tiles * (0.5 * (n + group) + kItem * p) / kSms * 1.05;  // causal: half of the pairs, a little uneven
+    const double steps = causal ? (share > all ? share : all) : static_cast<int>((items + kSms - 1) / kSms) * share;
+    const double bytes = items * BM * D * 8.0;
+    const double us = steps * step_us + (p > 1 ? 3.0 + 0.5 * p + 2 * bytes / (bytes < 64e6 ? 12e6 : 5.5e6) : 0.0);
+    if (us < best_us) best = p, best_us = us;
+  }
+  return best;
+}
+
+size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
+  if (Hkv <= 0 || Skv <= 0 || Lq <= 0) return 0;
+  const int pc = bwd_parts(B, Hq, Hkv, Lq, Skv, D, true), pf = bwd_parts(B, Hq, Hkv, Lq, Skv, D, false);
+  const int p = pc > pf ? pc : pf;
+  return p > 1 ? static_cast<size_t>(2) * p * B * Hkv * Skv * D * sizeof(float) : 0;
 }
 
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream) {

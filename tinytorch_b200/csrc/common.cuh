@@ -64,6 +64,8 @@ struct BwdArgs {
   int tail_heads;     // tensor-core kernel: (batch, kv head) pairs at the end of the item order whose key tiles are
                       // ordered longest walk first across heads (set by its launcher)
   int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by its launcher
+  int parts;          // tensor-core kernel: work items per key tile (see bwd_parts); > 1: each leaves its dK / dV in ...
+  float* dkv_part;    // ... workspace [dK, dV][parts][B * Hkv][Skv][D] fp32
   void* dq;
   void* dk;
   void* dv;
@@ -113,7 +115,10 @@ cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, cudaStream_t str
 cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
 // rowsum(dO o O) into a.delta only (first step of every backward)
 cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
-// fp16 / bf16 backward on the tensor cores; needs a.delta and a.dq_accum
+// Work items per key tile of the tensor-core backward, and the workspace they need beside dq_accum (0 for one item)
+int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal);
+size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
+// fp16 / bf16 backward on the tensor cores; needs a.delta, a.dq_accum and what a.parts asks for
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t stream);
 // grouped-query decode on the tensor cores (decode_tc.cu): 16-bit tensors, 2..16 query heads per kv head

@@ -322,42 +322,67 @@ __device__ __forceinline__ int splits_of(const DecodeArgs& a, int b, bool append
 
 constexpr int kMaxSplit = 64;
 
-// One CTA per (head, batch): fold the per-split partials into O and LSE.  A thread per split fetches maximum and sum,
-// then a thread per channel adds the weighted partials, eight loads in flight.
+// One CTA per (head, batch): fold the per-split partials into O and LSE.  The first warp fetches the splits' maxima and
+// sums (two per lane) and turns them into weights; then kGroups groups of D threads, a thread per channel, each add
+// every kGroups-th partial, eight loads in flight.
 template <typename T, int D, bool APPEND>
-__global__ void __launch_bounds__(D) decode_combine_kernel(const DecodeArgs a) {
-  __shared__ float s_w[kMaxSplit], s_l[kMaxSplit];
-  const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
+__global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeArgs a) {
+  constexpr int kGroups = 256 / D;
+  __shared__ float s_w[kMaxSplit], s_acc[256], s_inv, s_lse;
+  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, d = tid % D, grp = tid / D;
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();  // (launched early after the scan: its partials are complete from here on)
   const int n = splits_of(a, b, APPEND);
   const float* pp = a.partial + (static_cast<int64_t>(b) * a.Hq + h) * a.nsplit * (D + 2);
-  for (int s = d; s < n; s += D) s_w[s] = pp[s * (D + 2) + D], s_l[s] = pp[s * (D + 2) + D + 1];
-  __syncthreads();
-  float mn = -INFINITY;
-  for (int s = 0; s < n; ++s) mn = fmaxf(mn, s_w[s]);
-  float lt = 0.f, at = 0.f;
-  for (int s0 = 0; s0 < n; s0 += 8) {
-    float p[8];
+  // (the channels' first loads are on their way while the weights are computed)
+  float p[8];
+  auto fetch = [&](int s0) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) p[u] = s0 + u < n ? pp[(s0 + u) * (D + 2) + d] : 0.f;
+    for (int u = 0; u < 8; ++u) p[u] = s0 + u * kGroups < n ? pp[(s0 + u * kGroups) * (D + 2) + d] : 0.f;
+  };
+  fetch(grp);
+  if (tid < 32) {
+    float m[2], l[2];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      if (s0 + u >= n) break;
-      const float ms = s_w[s0 + u];
-      const float w = (ms == -INFINITY) ? 0.f : exp2f(ms - mn);
-      lt += s_l[s0 + u] * w;
-      at += p[u] * w;
+    for (int k = 0; k < 2; ++k) {
+      const int s = tid + 32 * k;
+      m[k] = s < n ? pp[s * (D + 2) + D] : -INFINITY, l[k] = s < n ? pp[s * (D + 2) + D + 1] : 0.f;
     }
+    float mn = fmaxf(m[0], m[1]);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    float lt = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float w = m[k] == -INFINITY ? 0.f : exp2f(m[k] - mn);
+      s_w[tid + 32 * k] = w;
+      lt = fmaf(l[k], w, lt);
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
+    if (tid == 0) s_inv = lt > 0.f ? 1.f / lt : 0.f, s_lse = lt > 0.f ? (mn + log2f(lt)) * kLn2 : -INFINITY;
   }
-  const float inv = lt > 0.f ? 1.f / lt : 0.f;
-  reinterpret_cast<T*>(a.o)[b * a.os.b + h * a.os.h + d] = from_f32<T>(at * inv);
-  if (a.lse && d == 0) a.lse[static_cast<int64_t>(b) * a.Hq + h] = lt > 0.f ? (mn + log2f(lt)) * kLn2 : -INFINITY;
+  __syncthreads();
+  float at = 0.f;
+  for (int s0 = grp; s0 < n; s0 += 8 * kGroups) {
+    if (s0 != grp) fetch(s0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s0 + u * kGroups < n) at = fmaf(p[u], s_w[s0 + u * kGroups], at);
+  }
+  s_acc[tid] = at;
+  __syncthreads();
+  if (grp == 0) {
+#pragma unroll
+    for (int k = 1; k < kGroups; ++k) at += s_acc[k * D + d];
+    reinterpret_cast<T*>(a.o)[b * a.os.b + h * a.os.h + d] = from_f32<T>(at * s_inv);
+    if (a.lse && d == 0) a.lse[static_cast<int64_t>(b) * a.Hq + h] = s_lse;
+  }
 }
 
 template <typename T, int D, bool APPEND>
 cudaError_t combine_t(const DecodeArgs& a, cudaStream_t stream) {
-  return launch_early(decode_combine_kernel<T, D, APPEND>, dim3(a.Hq, a.B), dim3(D), 0, stream, 1, a);
+  return launch_early(decode_combine_kernel<T, D, APPEND>, dim3(a.Hq, a.B), dim3(256), 0, stream, 1, a);
 }
 
 template <typename T, int D, bool APPEND>
