@@ -17,7 +17,7 @@
 //   warps 8-11 row r of the CTA's half (TMEM lane r); a block is read with tcgen05.ld, gets the bias (fp32), is rounded
 //              to the tensor dtype and leaves through one of the warpgroup's two swizzled staging tiles and a TMA store (rows and
 //              columns beyond M, N are clipped by the tensor map; the K tail reads as zero)
-// Tiles are ordered in groups of four row-tiles so that CTAs running at the same time share slices of x and w in L2.
+// Tiles are ordered in groups of row-tiles so that CTAs running at the same time share slices of x and w in L2.
 // X_MN / W_MN: the operand is stored with the contraction as its slow dimension (x as [K, M], w as [K, N]) and is read
 // as an MN-major MMA operand, so that the gradients dX = dY W and dW = dY^T X need no transposed copies.
 // Every mbarrier wait is bounded; after an expired one the CTA still meets the cluster barrier at the end.
@@ -38,7 +38,6 @@ constexpr int kEpi = 128;  // threads of an epilogue warpgroup
 constexpr int kABytes = HM * BK * 2, kBBytes = HN * BK * 2;
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kOutBytes = HM * 128;  // staging: 128 rows x 64 columns of 16 bits
-constexpr int kGroupM = 4;           // row-tiles per L2 group
 
 struct __align__(8) SmemCtl {
   uint64_t full[NSTAGE], empty[NSTAGE];
@@ -53,6 +52,7 @@ static_assert(kSmemBytes <= 232448, "exceeds the shared memory a CTA may request
 struct LinArgs {
   const void* bias;  // [N] in the tensor dtype, or null
   int M, N, K;
+  int group_m;       // row-tiles per L2 group (see launch_t)
   int32_t* status;
 };
 
@@ -67,11 +67,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-__device__ __forceinline__ void tile_of(int t, int tiles_m, int tiles_n, int* m_tile, int* n_tile) {
-  const int per_group = kGroupM * tiles_n;
+__device__ __forceinline__ void tile_of(int t, int group_m, int tiles_m, int tiles_n, int* m_tile, int* n_tile) {
+  const int per_group = group_m * tiles_n;
   const int g = t / per_group, in_g = t - g * per_group;
-  const int first_m = g * kGroupM;
-  const int gm = tiles_m - first_m < kGroupM ? tiles_m - first_m : kGroupM;
+  const int first_m = g * group_m;
+  const int gm = tiles_m - first_m < group_m ? tiles_m - first_m : group_m;
   *m_tile = first_m + in_g % gm;
   *n_tile = in_g / gm;
 }
@@ -133,7 +133,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       uint32_t full0 = ptx::map_rank(ptx::smem_u32(&ctl->full[0]), 0);  // the leader's
       for (int t = first; t < n_tiles && ok; t += step) {
         int mt, nt;
-        tile_of(t, tiles_m, tiles_n, &mt, &nt);
+        tile_of(t, a.group_m, tiles_m, tiles_n, &mt, &nt);
         const int m0 = mt * BM + static_cast<int>(rank) * HM, n0 = nt * BN + static_cast<int>(rank) * HN;
         for (int kb = 0; kb < n_kb; ++kb) {
           if (!(ok = ptx::mbar_wait(&ctl->empty[s], ph, abort_flag))) break;
@@ -201,7 +201,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     int i = 0;
     for (int t = first; t < n_tiles; t += step, ++i) {
       int mt, nt;
-      tile_of(t, tiles_m, tiles_n, &mt, &nt);
+      tile_of(t, a.group_m, tiles_m, tiles_n, &mt, &nt);
       const int n0 = nt * BN, m0 = mt * BM + static_cast<int>(rank) * HM, buf = i & 1;
       {  // (threads that see an expired wait still meet the barriers)
         const int n = n0 + wg * 64 + (r >> 6) * 128 + (r & 63);  // blocks wg and wg + 2
@@ -271,8 +271,17 @@ cudaError_t launch_t(const LinearCall& c, int ctas) {
       !make_map_2d(&tw, c.dtype, c.w, W_MN ? c.N : c.K, W_MN ? c.K : c.N, c.ldw, W_MN ? BK : HN) ||
       !make_map_2d(&ty, c.dtype, c.y, c.N, c.M, c.ldy, HM))
     return cudaErrorInvalidValue;
+  // Row-tiles per L2 group.  The pairs running at one time work on one group: its rows of x are read from HBM once as long
+  // as they stay in L2 while w streams by, and w once per group.  So: as many row-tiles (a power of two) as take 60 MB of
+  // the 126; where w itself stays in L2 (up to 40 MB), 4, so that x does not push it out.  Under sustained load, us, with 4
+  // before: 4096 x 4096 -> 12288 342 -> 312, 16384 x 4096 -> 12288 1341 -> 1225, 8192 cubed 893 -> 861, 2000 x 4096 -> 28672
+  // 387 -> 362 (and 32 or 64 instead of 16 for the second: 1377, 1625).
+  const long long x_tile = 2ll * BM * c.K, w_bytes = 2ll * c.N * c.K;
+  int group_m = 4;
+  if (w_bytes > 40 << 20)
+    while (group_m < 64 && group_m * 2 * x_tile <= 60 << 20) group_m *= 2;
   return launch_early(kern, dim3(ctas), dim3(kThreads), kSmemBytes, c.stream, 1,
-                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, c.status});
+                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, group_m, c.status});
 }
 
 template <bool BF16>
