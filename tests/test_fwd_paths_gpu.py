@@ -1,5 +1,5 @@
-"""GPU: the prefill forward where its items are divided among clusters (few queries, many keys) and where the two query
-blocks of an item belong to different heads, against the CPU oracle.  Tolerances: those of test_fwd_gpu.py."""
+"""GPU: the prefill forward where a query block's keys are divided between the halves of a CTA and among clusters (few
+queries, many keys), and where the two query blocks of an item belong to different heads, against the CPU oracle.  Tolerances: those of test_fwd_gpu.py."""
 import numpy as np
 import pytest
 import torch
@@ -12,7 +12,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens", [
-    (1, 2, 2, 128, 768, False, None),                 # 6 key tiles: clusters of 2, three steps each
+    (1, 2, 2, 128, 768, False, None),                 # 6 key tiles, two blocks
+    (1, 3, 1, 100, 384, False, None),                 # an odd number of key tiles: the halves differ
+    (2, 20, 20, 600, 600, True, None),                # 200 blocks: CTAs with several items
+    (1, 2, 1, 64, 100, False, None),                  # one key tile: a half without any
     (1, 4, 1, 129, 1537, "bottom-right", None),       # clusters of 4, a block of one row
     (2, 3, 1, 40, 3100, "bottom-right", (3100, 700)),  # clusters of 8, an odd number of blocks, CTAs without keys
     (2, 2, 2, 300, 3072, False, (1, 0)),              # a sequence without keys, one with a single key

@@ -11,13 +11,12 @@
 // counter, heads in order and, within a head, the longest (latest causal) pair
 // first, so that the CTAs running at any moment share few heads' K/V in L2 and
 // the last items to be drawn are the shortest.
-// SPLIT: where the items leave most SMs idle (a chunk of new queries against a
-// long cache), the key tiles of an item are divided among the CTAs of a cluster,
-// one item per cluster; the unnormalised O, maxima and sums meet in distributed
-// shared memory at the end and every CTA of the cluster writes a share of the rows.
-// Measured (us, before -> now): 2 x 256 new queries against 8192 rows, 32/8 heads
-// 120 -> 75; 64 against 4096, 8/2 heads 60 -> 20; 32 against 15000, 8 heads, D = 64
-// 166 -> 29; grouped causal 8 x 2048, 32/8 heads 268 -> 262, 777, 32/8 heads 21 -> 19.
+// KEYS: where latency counts, i.e. with so few items that the longest walk over the key tiles sets the time, an item
+// is ONE query block and the two halves of the CTA take its key tiles alternately (even, odd): half the steps.  The two
+// accumulators are in the same TMEM lanes, so both warpgroups read both, each for half of the columns, and only maxima
+// and sums cross through shared memory.  With fewer blocks than SMs the key tiles are divided further among the CTAs of
+// a cluster, one item per cluster; their unnormalised O, maxima and sums meet in distributed shared memory at the end and
+// every CTA of the cluster writes a share of the rows.
 //   warp 8   producer : draws items and publishes them to the other warps; TMA
 //                       tiled loads (128-byte swizzle, one copy per CTA) of the item's
 //                       two Q tiles and of each K and V tile into a 2-stage ring.
@@ -42,6 +41,7 @@
 // the CTA unwind.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -100,13 +100,14 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 struct Item {
   int b, hk, h0, h1, row00, row01;  // head and first row of the two blocks
   int kv_len, shift;                // key j participates iff j <= i + shift (causal)
-  int j0, nt0, nt1, n_max;          // first key tile, and how many each block walks from there
+  int j0, nt0, nt1, n_max;          // first key tile, and how many each half walks from there (KEYS: in turn)
 };
 
 // GEN: the general variant of the kernel (a mask and / or a causal triangle that is
 // not top-left aligned); the fast variant compiles all of that out.
-template <bool GEN>
-__device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs, int rank = 0, int cluster = 1) {
+// KEYS: `per_head` items (query blocks) per (batch, kv head), `rank` of `cluster` shares of the key tiles; else pairs.
+template <bool GEN, bool KEYS>
+__device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_head, int rank = 0, int cluster = 1) {
   Item it;
   // Heads in order, the longest (latest causal) pair of a head first: the CTAs running at any moment share few
   // heads' K/V in L2.  Only the last items are ordered differently: over the final kTailWaves waves the pairs of
@@ -114,17 +115,17 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs
   // CTAs finish together (in head order the last head's longest pair, an eighth of a CTA's whole share of
   // 128 heads of 4096 rows, would be drawn when most CTAs are nearly done).  Those heads' K/V together fit L2.
   const int n_heads = a.B * a.Hkv, group = a.Hq / a.Hkv;
-  int tail_heads = (kTailWaves * static_cast<int>(gridDim.x) + n_pairs - 1) / n_pairs;
+  int tail_heads = (kTailWaves * static_cast<int>(gridDim.x) + per_head - 1) / per_head;
   if (tail_heads > n_heads) tail_heads = n_heads;
-  const int w0 = (n_heads - tail_heads) * n_pairs;
+  const int w0 = (n_heads - tail_heads) * per_head;
   int bh, mp;
   if (w < w0) {
-    bh = w / n_pairs;
-    mp = n_pairs - 1 - (w - bh * n_pairs);
+    bh = w / per_head;
+    mp = per_head - 1 - (w - bh * per_head);
   } else {
     const int x = w - w0, rank_in = x / tail_heads;
     bh = n_heads - tail_heads + (x - rank_in * tail_heads);
-    mp = n_pairs - 1 - rank_in;
+    mp = per_head - 1 - rank_in;
   }
   it.b = bh / a.Hkv;
   it.hk = bh - it.b * a.Hkv;
@@ -135,8 +136,8 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs
   }
   it.kv_len = kv_len;
   it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
-  const int x = mp * QT, qt0 = x / group, qt1 = (x + 1) / group;
-  it.h0 = it.hk * group + x - qt0 * group, it.h1 = it.hk * group + x + 1 - qt1 * group;
+  const int x = KEYS ? mp : mp * QT, qt0 = x / group, qt1 = KEYS ? qt0 : (x + 1) / group;
+  it.h0 = it.hk * group + x - qt0 * group, it.h1 = KEYS ? it.h0 : it.hk * group + x + 1 - qt1 * group;
   it.row00 = qt0 * BM, it.row01 = qt1 * BM;
   // key tiles that a block sees (0 for one wholly beyond Lq)
   auto tiles = [&](int row0) {
@@ -148,16 +149,17 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int n_pairs
     }
     return row0 < a.Lq ? (e + BN - 1) / BN : 0;
   };
-  int nt0 = tiles(it.row00), nt1 = tiles(it.row01);
   it.j0 = 0;
-  if (cluster > 1) {
-    // this CTA's share of the key tiles
-    const int n = nt0 > nt1 ? nt0 : nt1, lo = n * rank / cluster, hi = n * (rank + 1) / cluster;
-    it.j0 = lo;
-    nt0 = (nt0 < hi ? nt0 : hi) - lo, nt1 = (nt1 < hi ? nt1 : hi) - lo;
-    nt0 = nt0 > 0 ? nt0 : 0, nt1 = nt1 > 0 ? nt1 : 0;
+  if constexpr (KEYS) {
+    int n = tiles(it.row00);
+    if (cluster > 1) {
+      it.j0 = n * rank / cluster;
+      n = n * (rank + 1) / cluster - it.j0;
+    }
+    it.nt0 = (n + 1) / 2, it.nt1 = n / 2;
+  } else {
+    it.nt0 = tiles(it.row00), it.nt1 = tiles(it.row01);
   }
-  it.nt0 = nt0, it.nt1 = nt1;
   it.n_max = it.nt0 > it.nt1 ? it.nt0 : it.nt1;
   return it;
 }
@@ -205,7 +207,7 @@ __device__ __forceinline__ void add_mask_row(uint32_t (&s)[BN], const MaskArgs& 
   }
 }
 
-// SPLIT: the 256 rows of an item over the CS CTAs of the cluster.  `stats`: (reference, sum) of every row, `xo`: its
+// The 128 rows of an item over the CS CTAs of the cluster.  `stats`: (reference, sum) of every row, `xo`: its
 // unnormalised O, at the same place in the shared memory of each CTA.  D / 4 lanes read a row (a warp's reads are whole
 // 512-byte rows), 8 vectors are in flight per thread; this CTA's own share is read as ordinary shared memory.
 template <int D, bool BF16, int CS>
@@ -213,7 +215,7 @@ __device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, i
                                              uint32_t xo) {
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   constexpr int kPer = 128 / D;  // rows that a warp reads at a time
-  constexpr int kBatch = 8 / CS, kRows = QT * BM / CS;
+  constexpr int kBatch = 8 / CS, kRows = BM / CS;
   const int c4 = lane % (D / 4);
   uint32_t pstats[CS], pxo[CS];  // this CTA's first, then the others in turn
 #pragma unroll
@@ -235,8 +237,7 @@ __device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, i
     }
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
-      const int rr = rank * kRows + i + u * 8 * kPer, t = rr / BM;
-      const int row = (t == 0 ? it.row00 : it.row01) + (rr & (BM - 1)), head = t == 0 ? it.h0 : it.h1;
+      const int row = it.row00 + rank * kRows + i + u * 8 * kPer, head = it.h0;
       float m = -INFINITY, l = 0.f;
 #pragma unroll
       for (int r = 0; r < CS; ++r) m = fmaxf(m, ml[u][r].x);
@@ -258,7 +259,7 @@ __device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, i
   }
 }
 
-template <int D, bool BF16, bool GEN, bool SPLIT>
+template <int D, bool BF16, bool GEN, bool KEYS>
 __global__ void __launch_bounds__(kThreads, 1)
     fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -277,10 +278,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const int n_pairs = ((a.Lq + BM - 1) / BM * (a.Hq / a.Hkv) + QT - 1) / QT;
-  const int n_items = n_pairs * a.Hkv * a.B;
-  const int rank = SPLIT ? static_cast<int>(ptx::cluster_rank()) : 0;
-  auto item_of = [&](int w) { return SPLIT ? decode_item<GEN>(a, w, n_pairs, rank, cluster) : decode_item<GEN>(a, w, n_pairs); };
+  const int n_blocks = (a.Lq + BM - 1) / BM * (a.Hq / a.Hkv), per_head = KEYS ? n_blocks : (n_blocks + QT - 1) / QT;
+  const int n_items = per_head * a.Hkv * a.B;
+  const int rank = KEYS && cluster > 1 ? static_cast<int>(ptx::cluster_rank()) : 0;
+  auto item_of = [&](int w) { return KEYS ? decode_item<GEN, true>(a, w, per_head, rank, cluster) : decode_item<GEN, false>(a, w, per_head); };
 
   constexpr int HALVES = D / 64;  // 64-element (128-byte) column blocks per row
   constexpr int HALF_BYTES = BM * 128;
@@ -331,9 +332,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   // thread; the producer / issuer warpgroup needs little.
   if (warp >= 8) {
     // (D = 128: 224 + 224 + 56 registers per thread over the three warpgroups; D = 64, whose issuing loop
-    // carries the look-ahead at item boundaries: 216 + 216 + 72.  Both add up to the 168 x 384 registers
+    // carries the look-ahead at item boundaries, and KEYS: 216 + 216 + 72.  Both add up to the 168 x 384 registers
     // the CTA was launched with, so the increase below can always be served.)
-    ptx::setmaxnreg_dec<D == 128 ? 56 : 72>();
+    ptx::setmaxnreg_dec<D == 128 && !KEYS ? 56 : 72>();
     if (warp == 8) {
       // ---------------------------------------------------------- producer --
       if (lane == 0) {
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (uint32_t i = 0;; ++i) {
           // the first item is the CTA's own number; the counter, where one is needed, hands out the rest
           int w;
-          if (SPLIT)
+          if (KEYS && cluster > 1)
             w = i == 0 ? static_cast<int>(blockIdx.x) / cluster : -1;
           else
             w = i == 0 ? static_cast<int>(blockIdx.x) : (a.sched ? static_cast<int>(gridDim.x) + atomicAdd(a.sched, 1) : -1);
@@ -371,20 +372,42 @@ __global__ void __launch_bounds__(kThreads, 1)
             return true;
           };
           if (!(ok = load_q(0, qc0))) break;
-          for (int j = 0; j < it.n_max; ++j, ++g) {
-            const int st = g % NSTAGE;
-            const uint32_t ph = (g / NSTAGE) & 1;
-            if (!(ok = ptx::mbar_wait(&ctl->k_empty[st], ph ^ 1, abort_flag))) break;
-            ptx::mbar_arrive_expect_tx(&ctl->k_full[st], TB);
+          if constexpr (KEYS) {
+            // every tile goes to one half only; K a tile ahead of V, as the products consume them
+            const int n = it.nt0 + it.nt1;
+            auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* full, uint64_t* empty, int j) {
+              const uint32_t gj = g + j;
+              const int st = gj % NSTAGE;
+              if (!ptx::mbar_wait(&empty[st], ((gj / NSTAGE) & 1) ^ 1, abort_flag)) return false;
+              ptx::mbar_arrive_expect_tx(&full[st], TB);
 #pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf)
-              ptx::tma_load_4d(sK + st * TB + hf * HALF_BYTES, &tmK, &ctl->k_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
-            if (j == 0 && !(ok = load_q(1, qc1))) break;
-            if (!(ok = ptx::mbar_wait(&ctl->v_empty[st], ph ^ 1, abort_flag))) break;
-            ptx::mbar_arrive_expect_tx(&ctl->v_full[st], TB);
+              for (int hf = 0; hf < HALVES; ++hf)
+                ptx::tma_load_4d(dst + st * TB + hf * HALF_BYTES, map, &full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
+              return true;
+            };
+            ok = load(sK, &tmK, ctl->k_full, ctl->k_empty, 0);
+            for (int j = 0; j < n && ok; ++j) {
+              if (j + 1 < n) ok = load(sK, &tmK, ctl->k_full, ctl->k_empty, j + 1);
+              if (ok) ok = load(sV, &tmV, ctl->v_full, ctl->v_empty, j);
+            }
+            if (!ok) break;
+            g += n;
+          } else {
+            for (int j = 0; j < it.n_max; ++j, ++g) {
+              const int st = g % NSTAGE;
+              const uint32_t ph = (g / NSTAGE) & 1;
+              if (!(ok = ptx::mbar_wait(&ctl->k_empty[st], ph ^ 1, abort_flag))) break;
+              ptx::mbar_arrive_expect_tx(&ctl->k_full[st], TB);
 #pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf)
-              ptx::tma_load_4d(sV + st * TB + hf * HALF_BYTES, &tmV, &ctl->v_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
+              for (int hf = 0; hf < HALVES; ++hf)
+                ptx::tma_load_4d(sK + st * TB + hf * HALF_BYTES, &tmK, &ctl->k_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
+              if (j == 0 && !(ok = load_q(1, qc1))) break;
+              if (!(ok = ptx::mbar_wait(&ctl->v_empty[st], ph ^ 1, abort_flag))) break;
+              ptx::mbar_arrive_expect_tx(&ctl->v_full[st], TB);
+#pragma unroll
+              for (int hf = 0; hf < HALVES; ++hf)
+                ptx::tma_load_4d(sV + st * TB + hf * HALF_BYTES, &tmV, &ctl->v_full[st], hf * 64, (it.j0 + j) * BN, it.hk, it.b);
+            }
           }
           if (!ok) break;
         }
@@ -422,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
         auto wait_k = [&](uint32_t g) { return uwait(&ctl->k_full[g % NSTAGE], (g / NSTAGE) & 1); };
         auto issue_qk = [&](int t, uint32_t g) {
-          const uint32_t a0 = qlo + t * (TB >> 4), b0 = klo + (g % NSTAGE) * (TB >> 4), d = tmem + t * 128;
+          const uint32_t a0 = qlo + (KEYS ? 0 : t * (TB >> 4)), b0 = klo + (g % NSTAGE) * (TB >> 4), d = tmem + t * 128;
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks) {
             // K-major operands: 64-element halves HALF_BYTES apart, 32 bytes per k-step
@@ -467,6 +490,47 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (it.n_max == 0) continue;
           const int nt0 = it.nt0, nt1 = it.nt1, n_max = it.n_max;
           auto nt = [&](int t) { return t == 0 ? nt0 : nt1; };
+
+          if constexpr (KEYS) {
+            // half t takes the key tiles t, t + 2, ...: tile j of the item at ring position g0 + j, used once; the same
+            // order PV(0) QK(0)' PV(1) QK(1)' as below
+            const int n = nt0 + nt1;
+            auto qk = [&](int t, int j) {
+              issue_qk(t, g0 + j);
+              if (leader) ptx::mma_commit(&ctl->k_empty[(g0 + j) % NSTAGE]);
+              if (leader && j == n - 1) ptx::mma_commit(&ctl->q_empty[0]);
+            };
+            if (!(ok = uwait(&ctl->q_full[0], qc0 & 1))) break;
+            ++qc0;
+#pragma unroll
+            for (int t = 0; t < QT; ++t) {
+              if (t >= n) continue;
+              if (!(ok = wait_k(g0 + t))) break;
+              ptx::tc_fence_after();
+              qk(t, t);
+            }
+            for (int i2 = 0; i2 < nt0 && ok; ++i2) {
+#pragma unroll
+              for (int t = 0; t < QT; ++t) {
+                const int j = 2 * i2 + t;
+                if (j >= n) continue;
+                const uint32_t g = g0 + j;
+                bool okb = ptx::mbar_wait(&ctl->v_full[g % NSTAGE], (g / NSTAGE) & 1, abort_flag);
+                if (j + 2 < n && okb) okb = ptx::mbar_wait(&ctl->k_full[(g + 2) % NSTAGE], ((g + 2) / NSTAGE) & 1, abort_flag);
+                if (okb) okb = ptx::mbar_wait(&ctl->p_full[t], ((t == 0 ? c0 : c1) + i2) & 1, abort_flag);
+                if (!(ok = __all_sync(0xffffffffu, okb) != 0)) break;
+                ptx::tc_fence_after();
+                issue_pv(t, g, i2 == 0);
+                if (leader && i2 == nt(t) - 1) ptx::mma_commit(&ctl->o_full[t]);
+                if (leader) ptx::mma_commit(&ctl->v_empty[g % NSTAGE]);
+                if (j + 2 < n) qk(t, j + 2);
+              }
+            }
+            g0 += n;
+            c0 += nt0;
+            c1 += nt1;
+            continue;
+          }
 
           if (nt0 > 0 && !pre0 && !(ok = first_qk(0, qc0, g0, nt0))) break;
           pre0 = false;
@@ -527,7 +591,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else {
-    ptx::setmaxnreg_inc<D == 128 ? 224 : 216>();
+    ptx::setmaxnreg_inc<D == 128 && !KEYS ? 224 : 216>();
     // ------------------------------------------------------------- softmax --
     const int t = warp >> 2;          // query tile of this warpgroup
     const int r_in = tid & (BM - 1);  // row within the tile = TMEM lane
@@ -541,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const float2 c2 = make_float2(cm, cm);
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
     uint32_t cnt = 0;  // softmax iterations completed (s_full phase)
-    uint32_t ec = 0;   // items with work completed (o_full phase)
+    uint32_t ec = 0, e1 = 0;  // items with work completed (o_full phase; KEYS: of tile 0, of tile 1)
     bool ok = true;
     uint32_t s[BN];
 
@@ -551,7 +615,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (uint32_t i = 0;; ++i) {
       const int slot = i & 1;
       ok = ptx::mbar_wait(&ctl->item_full[slot], (i >> 1) & 1, abort_flag);
-      if (ptx::named_barrier_or(1 + t, BM, !ok)) break;
+      // (KEYS: both warpgroups, which also meet after the walk)
+      if (KEYS ? ptx::named_barrier_or(3, QT * BM, !ok) : ptx::named_barrier_or(1 + t, BM, !ok)) break;
       const int w = ctl->item[slot];
       ptx::mbar_arrive(&ctl->item_empty[slot]);
       if (w < 0) break;
@@ -563,9 +628,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       T* orow = reinterpret_cast<T*>(a.o) + it.b * a.os.b + head * a.os.h + static_cast<int64_t>(row) * a.os.s;
       float* lse_row = a.lse ? a.lse + (static_cast<int64_t>(it.b) * a.Hq + head) * a.Lq + row : nullptr;
 
-      if (!SPLIT && n_t == 0) {
+      if (KEYS ? cluster == 1 && it.n_max == 0 : n_t == 0) {
         // no participating key (or tile beyond Lq): O = 0, LSE = -inf
-        if (row < a.Lq) {
+        if (row < a.Lq && (!KEYS || t == 0)) {
 #pragma unroll
           for (int e = 0; e < D; e += 8) *reinterpret_cast<uint4*>(orow + e) = make_uint4(0, 0, 0, 0);
           if (lse_row) *lse_row = -INFINITY;
@@ -583,7 +648,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int cc = 0; cc < 4; ++cc) ptx::tmem_ld32p(tS + cc * 32, s + cc * 32);
         ptx::tmem_wait_ld();
 
-        const int col0 = (it.j0 + j) * BN;
+        const int col0 = (it.j0 + (KEYS ? 2 * j + t : j)) * BN;
         if constexpr (GEN) {
           if (a.mask.ptr && row < a.Lq)
             add_mask_row<T>(s, a.mask, it.b * a.mask.sb + head * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
@@ -676,25 +741,76 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       cnt += n_t;
 
-      if constexpr (SPLIT) {
-        // The unnormalised O (over the K / V stages), reference and sum (over the Q tiles) of this CTA's key tiles go
-        // to shared memory once every MMA of the CTA is complete; the rows are put together below.
-        if (ok && it.nt0 > 0) ok = ptx::mbar_wait(&ctl->o_full[0], 0, abort_flag);
-        if (ok && it.nt1 > 0) ok = ptx::mbar_wait(&ctl->o_full[1], 0, abort_flag);
-        __syncwarp();
+      if constexpr (KEYS) {
+        // Both halves of the walk: wait for both accumulators (tile 0's phase ec, tile 1's e1), exchange references and
+        // sums (over the unused second Q tile), then warpgroup t puts columns [64 t, 64 t + 64) together (D = 64:
+        // warpgroup 0 all of them).
+        if (ok && it.nt0 > 0) ok = ptx::mbar_wait(&ctl->o_full[0], ec & 1, abort_flag);
+        if (ok && it.nt1 > 0) ok = ptx::mbar_wait(&ctl->o_full[1], e1 & 1, abort_flag);
+        ec += it.nt0 > 0, e1 += it.nt1 > 0;
+        float2* stat = reinterpret_cast<float2*>(sQ + TB);
+        stat[t * BM + r_in] = make_float2(n_t > 0 ? m_ref : -INFINITY, l2.x + l2.y);
+        if (ptx::named_barrier_or(3, QT * BM, !ok)) break;
         ptx::tc_fence_after();
-        float* xo = reinterpret_cast<float*>(sK) + (t * BM + r_in) * D;
-        reinterpret_cast<float2*>(sQ)[t * BM + r_in] = make_float2(n_t > 0 ? m_ref : -INFINITY, l2.x + l2.y);
-        if (n_t > 0) {
+        const float2 sa = stat[r_in], sb = stat[BM + r_in];
+        const float m = fmaxf(sa.x, sb.x);
+        // (a half without key tiles, or a row that none of its keys takes part in, has reference -inf)
+        const float wa = sa.x == -INFINITY ? 0.f : ptx::ex2(sa.x - m), wb = sb.x == -INFINITY ? 0.f : ptx::ex2(sb.x - m);
+        const float l = sa.y * wa + sb.y * wb;
+        const bool mine = D == 128 || t == 0;
+        const int c0 = D == 128 ? t * 64 : 0;
+        if (mine) {
+          const uint32_t ta = tmem + 256 + lane_addr + c0;
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) ptx::tmem_ld32p(tO + cc * 32, s + cc * 32);
+          for (int cc = 0; cc < 2; ++cc) {
+            if (it.nt0 > 0) ptx::tmem_ld32p(ta + cc * 32, s + cc * 32);
+            if (it.nt1 > 0) ptx::tmem_ld32p(ta + D + cc * 32, s + 64 + cc * 32);
+          }
           ptx::tmem_wait_ld();
+          const float inv = cluster > 1 ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+          const float ua = wa * inv, ub = wb * inv;
 #pragma unroll
-          for (int ch = 0; ch < D / 4; ++ch)  // (16-byte pieces of a row permuted by the row: no bank conflicts)
-            *reinterpret_cast<uint4*>(xo + ((ch ^ r_in) & (D / 4 - 1)) * 4) =
-                make_uint4(s[ch * 4], s[ch * 4 + 1], s[ch * 4 + 2], s[ch * 4 + 3]);
+          for (int e = 0; e < 64; ++e) {
+            const float x = it.nt0 > 0 ? __uint_as_float(s[e]) * ua : 0.f;
+            s[e] = __float_as_uint(it.nt1 > 0 ? fmaf(__uint_as_float(s[64 + e]), ub, x) : x);
+          }
         }
-        break;
+        ptx::tc_fence_before();
+        ptx::named_barrier(3, QT * BM);  // both accumulators and the statistics have been read
+        if (cluster > 1) {
+          // unnormalised O (over the K / V stages: every MMA of the CTA is complete), reference and sum for the others
+          if (t == 0) stat[2 * BM + r_in] = make_float2(m, l);
+          if (mine) {
+            float* xo = reinterpret_cast<float*>(sK) + r_in * D;
+#pragma unroll
+            for (int ch = 0; ch < 16; ++ch)  // (16-byte pieces of a row permuted by the row: no bank conflicts)
+              *reinterpret_cast<uint4*>(xo + (((c0 >> 2) + ch) ^ (r_in & (D / 4 - 1))) * 4) =
+                  make_uint4(s[ch * 4], s[ch * 4 + 1], s[ch * 4 + 2], s[ch * 4 + 3]);
+          }
+          break;
+        }
+        if (mine) {
+          uint8_t* stage = sO + t * kStageBytes;
+          if (r_in == 0) ptx::bulk_wait_read();  // previous store out of this block has been read
+          ptx::named_barrier(1 + t, BM);
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch) {
+            uint4 wv;
+            wv.x = pack2<BF16>(__uint_as_float(s[ch * 8 + 0]), __uint_as_float(s[ch * 8 + 1]));
+            wv.y = pack2<BF16>(__uint_as_float(s[ch * 8 + 2]), __uint_as_float(s[ch * 8 + 3]));
+            wv.z = pack2<BF16>(__uint_as_float(s[ch * 8 + 4]), __uint_as_float(s[ch * 8 + 5]));
+            wv.w = pack2<BF16>(__uint_as_float(s[ch * 8 + 6]), __uint_as_float(s[ch * 8 + 7]));
+            *reinterpret_cast<uint4*>(stage + r_in * 128 + ((ch ^ (r_in & 7)) << 4)) = wv;
+          }
+          ptx::fence_proxy_async_smem();
+          ptx::named_barrier(1 + t, BM);
+          if (r_in == 0) {
+            ptx::tma_store_4d(&tmO, stage, c0, tile_row0, head, it.b);
+            ptx::bulk_commit();
+          }
+        }
+        if (t == 0 && row < a.Lq && lse_row) *lse_row = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+        continue;
       }
 
       // epilogue: O / l -> global, LSE.  The issuer may already be computing the
@@ -738,17 +854,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (r_in == 0) ptx::bulk_wait_all();
   }
 
-  if constexpr (SPLIT) {
+  if (KEYS && cluster > 1) {
     __syncwarp();
     ptx::cluster_sync();
     if (warp < 8 && *abort_flag == 0) {
       const Item it = item_of(blockIdx.x / cluster);
+      const uint32_t stats = ptx::smem_u32(sQ + TB) + 2 * BM * 8, xo = ptx::smem_u32(sK);
       if (cluster == 2)
-        combine_rows<D, BF16, 2>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+        combine_rows<D, BF16, 2>(a, it, rank, warp, lane, stats, xo);
       else if (cluster == 4)
-        combine_rows<D, BF16, 4>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+        combine_rows<D, BF16, 4>(a, it, rank, warp, lane, stats, xo);
       else
-        combine_rows<D, BF16, 8>(a, it, rank, warp, lane, ptx::smem_u32(sQ), ptx::smem_u32(sK));
+        combine_rows<D, BF16, 8>(a, it, rank, warp, lane, stats, xo);
     }
     __syncwarp();
     ptx::cluster_sync();  // no CTA leaves while another still reads its shared memory
@@ -764,13 +881,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ------------------------------------------------------------------ host ----
-template <int D, bool BF16, bool GEN, bool SPLIT>
+template <int D, bool BF16, bool GEN, bool KEYS>
 cudaError_t launch_k(const FwdArgs& a, int dtype, int grid, int cluster, cudaStream_t stream) {
   CUtensorMap tq, tk, tv, to;
   if (!make_map(&tq, dtype, a.q, D, a.Lq, a.Hq, a.B, a.qs) || !make_map(&tk, dtype, a.k, D, a.Skv, a.Hkv, a.B, a.ks) ||
       !make_map(&tv, dtype, a.v, D, a.Skv, a.Hkv, a.B, a.vs) || !make_map(&to, dtype, a.o, D, a.Lq, a.Hq, a.B, a.os))
     return cudaErrorInvalidValue;
-  auto kern = fwd_tc_kernel<D, BF16, GEN, SPLIT>;
+  auto kern = fwd_tc_kernel<D, BF16, GEN, KEYS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D>());
   if (e != cudaSuccess) return e;
   return launch_early(kern, dim3(grid), dim3(kThreads), smem_bytes<D>(), stream, cluster, tq, tk, tv, to, a, cluster);
@@ -779,7 +896,7 @@ cudaError_t launch_k(const FwdArgs& a, int dtype, int grid, int cluster, cudaStr
 // CTAs of clusters of this size that can be resident at once, one to an SM (a cluster lives inside one GPC, and GPCs
 // differ in size).  Asked once per device.
 template <int D, bool BF16, bool GEN>
-int split_slots(int device, int cluster) {
+int cluster_slots(int device, int cluster) {
   static std::atomic<int> known[64][3];
   if (device < 0 || device >= 64) return 0;
   std::atomic<int>& k = known[device][cluster == 2 ? 0 : (cluster == 4 ? 1 : 2)];
@@ -806,28 +923,70 @@ int split_slots(int device, int cluster) {
   return n;
 }
 
+// How the work is divided (see the head of the file): what is expected to take the least time, by a model fitted to a sweep
+// of 20 shapes (what it picks is within 2 us of the best of pairs, blocks, and clusters of 2, 4 and 8 for each).  Pairs: 6.5
+// us and the longest walk, or an SM's share of all walks, 4.5 us for every item besides its steps.  Single blocks: half the
+// steps, a little longer ones, 9 us, and 7 us an item.  A cluster adds 5 us.  Measured, us, pairs -> chosen: 2 x 256 queries
+// against 8192 keys, 32/8 heads 117 -> 66; 64 against 4096, 8/2 heads 64 -> 18; 32 against 15000, 8 heads D = 64 186 -> 22;
+// causal 1024, 16 heads 20.4 -> 16.1; causal 4096, 8 heads 61 -> 41; causal 8 x 512, 32/8 heads 35 (blocks: 58).
+struct Plan {
+  bool keys;
+  int cluster;
+};
+template <int D, bool BF16, bool GEN>
+Plan plan_of(const FwdArgs& a, int device) {
+  const int group = a.Hq / a.Hkv, n_qt = (a.Lq + BM - 1) / BM, sms = sm_count(device);
+  const long long heads = static_cast<long long>(a.B) * a.Hkv, blocks = heads * group * n_qt, pairs = heads * ((group * n_qt + 1) / 2);
+  if (blocks > 8ll * sms) return Plan{false, 1};
+  const int n_all = (a.Skv + BN - 1) / BN;
+  auto tiles = [&](int qt) {  // key tiles of query tile qt, every cache row taken as valid
+    if (!a.causal) return n_all;
+    const long long c = (qt + 1ll) * BM + (a.causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT ? a.Skv - a.Lq : 0);
+    const long long t = c > 0 ? (c + BN - 1) / BN : 0;
+    return t < n_all ? static_cast<int>(t) : n_all;
+  };
+  constexpr double kPairStep = D == 128 ? 1.65 : 1.35, kKeysStep = D == 128 ? 1.75 : 1.35, kPairItem = 4.5, kKeysItem = 7.0;
+  double pair_all = kPairItem * pairs, keys_all = kKeysItem * blocks;
+  for (int qt = 0; qt < n_qt; ++qt) {
+    const int n = tiles(qt);
+    keys_all += kKeysStep * heads * group * ((n + 1) / 2);
+    pair_all += kPairStep * heads * 0.5 * group * n;
+  }
+  const int last = tiles(n_qt - 1);
+  auto share = [&](double all, long long items, double one) {  // of an SM; walks of one length come in whole rounds
+    return 2.0 + (a.causal ? all / sms : static_cast<double>((items + sms - 1) / sms) * one);
+  };
+  const double pair_one = 6.5 + kPairStep * last, keys_one = 9.0 + kKeysStep * ((last + 1) / 2);
+  const double pair_us = std::max(pair_one, share(pair_all, pairs, kPairItem + kPairStep * last));
+  const double keys_us = blocks <= sms ? keys_one
+                                       : std::max(keys_one, share(keys_all, blocks, kKeysItem + kKeysStep * ((last + 1) / 2)));
+  Plan best{keys_us < pair_us, 1};
+  double best_us = std::min(keys_us, pair_us);
+  for (int cs = 2; cs <= 8; cs *= 2) {
+    if (blocks * cs > sms || blocks * cs > cluster_slots<D, BF16, GEN>(device, cs)) break;
+    const double us = 14.0 + kKeysStep * (((last + cs - 1) / cs + 1) / 2);
+    if (us < best_us) best = Plan{true, cs}, best_us = us;
+  }
+  return best;
+}
+
 template <int D, bool BF16, bool GEN>
 cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
-  const long long n_pairs = ((a.Lq + BM - 1ll) / BM * (a.Hq / a.Hkv) + QT - 1) / QT, n_items = n_pairs * a.Hkv * a.B;
+  const long long n_blocks = (a.Lq + BM - 1ll) / BM * (a.Hq / a.Hkv), heads = static_cast<long long>(a.Hkv) * a.B;
+  const Plan p = plan_of<D, BF16, GEN>(a, device);
+  const long long n_items = (p.keys ? n_blocks : (n_blocks + QT - 1) / QT) * heads;
   if (n_items > 0x7fffffffll) return cudaErrorInvalidValue;
   const int sms = sm_count(device);
-  // Keys divided over clusters: the largest cluster whose CTAs are all resident at once and walk at least three key
-  // tiles each (a step takes 1.6 us; the exchange and the cluster barriers about five).
-  const int n_tiles = ((a.causal == TT_ATTN_CAUSAL_TOP_LEFT && a.Lq < a.Skv ? a.Lq : a.Skv) + BN - 1) / BN;
-  for (int cs = 8; cs >= 2; cs >>= 1)
-    if (n_tiles >= 3 * cs && n_items * cs <= sms && n_items * cs <= split_slots<D, BF16, GEN>(device, cs)) {
-      a.sched = nullptr;
-      return launch_k<D, BF16, GEN, true>(a, dtype, static_cast<int>(n_items) * cs, cs, stream);
-    }
-  const int grid = static_cast<int>(n_items < sms ? n_items : sms);
-  if (n_items > grid) {
+  const int grid = p.cluster > 1 ? static_cast<int>(n_items) * p.cluster : static_cast<int>(n_items < sms ? n_items : sms);
+  if (p.cluster == 1 && n_items > grid) {
     // the counter that hands out what comes after the CTAs' first items must start at zero for every launch
     cudaError_t e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);
     if (e != cudaSuccess) return e;
   } else {
     a.sched = nullptr;
   }
-  return launch_k<D, BF16, GEN, false>(a, dtype, grid, 1, stream);
+  return p.keys ? launch_k<D, BF16, GEN, true>(a, dtype, grid, p.cluster, stream)
+                : launch_k<D, BF16, GEN, false>(a, dtype, grid, 1, stream);
 }
 
 }  // namespace
