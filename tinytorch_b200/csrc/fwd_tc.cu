@@ -64,13 +64,20 @@ constexpr int kItemConsumers = 1 + QT * BM;  // issuer thread + every softmax th
 #endif
 constexpr int kTailWaves = TT_FWD_TAIL_WAVES;  // waves of work items at the end that are ordered longest first across heads
 
-struct __align__(8) SmemCtl {
+// One work item, decoded once by the producer.
+struct Item {
+  int b, hk, h[QT], row0[QT];  // head and first row of the two blocks
+  int kv_len, shift;           // key j participates iff j <= i + shift (causal)
+  int j0, nt[QT];              // first key tile, and how many each half walks from there (KEYS: in turn)
+  int n_max;                   // the longer walk; -1: no more items
+};
+
+struct __align__(16) SmemCtl {
   uint64_t q_full[QT], q_empty[QT];  // per query tile: tile 0 of the next item is loaded while tile 1 still works
   uint64_t k_full[NSTAGE], k_empty[NSTAGE], v_full[NSTAGE], v_empty[NSTAGE];
   uint64_t s_full[QT], p_full[QT], o_full[QT];
   uint64_t item_full[2], item_empty[2];
-  int item[2];
-  int item_nt0[2];  // key tiles of query tile 0 of the published item (the issuer's look-ahead needs only this)
+  Item item[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -82,7 +89,7 @@ constexpr int tile_bytes() {
 constexpr int kStageBytes = BM * 128;  // per warpgroup: one 64-column block of an O tile
 template <int D>
 constexpr int smem_bytes() {
-  return (QT + 2 * NSTAGE) * tile_bytes<D>() + QT * kStageBytes + 1024 /*alignment slack*/ + 256 /*SmemCtl*/;
+  return (QT + 2 * NSTAGE) * tile_bytes<D>() + QT * kStageBytes + 1024 /*alignment slack*/ + 512 /*SmemCtl*/;
 }
 
 template <bool BF16>
@@ -95,13 +102,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&t);
   }
 }
-
-// One work item, decoded identically by every role.
-struct Item {
-  int b, hk, h0, h1, row00, row01;  // head and first row of the two blocks
-  int kv_len, shift;                // key j participates iff j <= i + shift (causal)
-  int j0, nt0, nt1, n_max;          // first key tile, and how many each half walks from there (KEYS: in turn)
-};
 
 // GEN: the general variant of the kernel (a mask and / or a causal triangle that is
 // not top-left aligned); the fast variant compiles all of that out.
@@ -137,8 +137,8 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_hea
   it.kv_len = kv_len;
   it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
   const int x = KEYS ? mp : mp * QT, qt0 = x / group, qt1 = KEYS ? qt0 : (x + 1) / group;
-  it.h0 = it.hk * group + x - qt0 * group, it.h1 = KEYS ? it.h0 : it.hk * group + x + 1 - qt1 * group;
-  it.row00 = qt0 * BM, it.row01 = qt1 * BM;
+  it.h[0] = it.hk * group + x - qt0 * group, it.h[1] = KEYS ? it.h[0] : it.hk * group + x + 1 - qt1 * group;
+  it.row0[0] = qt0 * BM, it.row0[1] = qt1 * BM;
   // key tiles that a block sees (0 for one wholly beyond Lq)
   auto tiles = [&](int row0) {
     int e = kv_len;
@@ -151,16 +151,16 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_hea
   };
   it.j0 = 0;
   if constexpr (KEYS) {
-    int n = tiles(it.row00);
+    int n = tiles(it.row0[0]);
     if (cluster > 1) {
       it.j0 = n * rank / cluster;
       n = n * (rank + 1) / cluster - it.j0;
     }
-    it.nt0 = (n + 1) / 2, it.nt1 = n / 2;
+    it.nt[0] = (n + 1) / 2, it.nt[1] = n / 2;
   } else {
-    it.nt0 = tiles(it.row00), it.nt1 = tiles(it.row01);
+    it.nt[0] = tiles(it.row0[0]), it.nt[1] = tiles(it.row0[1]);
   }
-  it.n_max = it.nt0 > it.nt1 ? it.nt0 : it.nt1;
+  it.n_max = it.nt[0] > it.nt[1] ? it.nt[0] : it.nt[1];
   return it;
 }
 
@@ -237,7 +237,7 @@ __device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, i
     }
 #pragma unroll
     for (int u = 0; u < kBatch; ++u) {
-      const int row = it.row00 + rank * kRows + i + u * 8 * kPer, head = it.h0;
+      const int row = it.row0[0] + rank * kRows + i + u * 8 * kPer, head = it.h[0];
       float m = -INFINITY, l = 0.f;
 #pragma unroll
       for (int r = 0; r < CS; ++r) m = fmaxf(m, ml[u][r].x);
@@ -350,10 +350,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (w >= n_items) w = -1;
           const int slot = i & 1;
           Item it{};
+          it.n_max = -1;
           if (w >= 0) it = item_of(w);
           if (!ptx::mbar_wait(&ctl->item_empty[slot], ((i >> 1) & 1) ^ 1, abort_flag)) break;
-          ctl->item[slot] = w;
-          ctl->item_nt0[slot] = w >= 0 ? it.nt0 : 0;
+          ctl->item[slot] = it;
           ptx::mbar_arrive(&ctl->item_full[slot]);
           if (w < 0) break;
           if (it.n_max == 0) continue;
@@ -361,20 +361,20 @@ __global__ void __launch_bounds__(kThreads, 1)
           // a Q tile is loaded only if it has key tiles to walk; tile 0 goes first and, with the first K tile,
           // ahead of tile 1: the issuer starts tile 0 of this item while tile 1 of the previous one still works
           auto load_q = [&](int t, uint32_t& qc) {
-            if ((t == 0 ? it.nt0 : it.nt1) == 0) return true;
+            if ((t == 0 ? it.nt[0] : it.nt[1]) == 0) return true;
             if (!ptx::mbar_wait(&ctl->q_empty[t], (qc & 1) ^ 1, abort_flag)) return false;
             ptx::mbar_arrive_expect_tx(&ctl->q_full[t], TB);
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf)
               ptx::tma_load_4d(sQ + t * TB + hf * HALF_BYTES, &tmQ, &ctl->q_full[t], hf * 64,
-                              t == 0 ? it.row00 : it.row01, t == 0 ? it.h0 : it.h1, it.b);
+                              t == 0 ? it.row0[0] : it.row0[1], t == 0 ? it.h[0] : it.h[1], it.b);
             ++qc;
             return true;
           };
           if (!(ok = load_q(0, qc0))) break;
           if constexpr (KEYS) {
             // every tile goes to one half only; K a tile ahead of V, as the products consume them
-            const int n = it.nt0 + it.nt1;
+            const int n = it.nt[0] + it.nt[1];
             auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* full, uint64_t* empty, int j) {
               const uint32_t gj = g + j;
               const int st = gj % NSTAGE;
@@ -482,13 +482,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (uint32_t i = 0; ok; ++i) {
           const int slot = i & 1;
           if (!uwait(&ctl->item_full[slot], (i >> 1) & 1)) break;
-          const int w = ctl->item[slot];
+          const int nt0 = ctl->item[slot].nt[0], nt1 = ctl->item[slot].nt[1], n_max = ctl->item[slot].n_max;
           __syncwarp();  // every lane has read the slot before it is handed back
           if (leader) ptx::mbar_arrive(&ctl->item_empty[slot]);
-          if (w < 0) break;
-          const Item it = item_of(w);
-          if (it.n_max == 0) continue;
-          const int nt0 = it.nt0, nt1 = it.nt1, n_max = it.n_max;
+          if (n_max < 0) break;
+          if (n_max == 0) continue;
           auto nt = [&](int t) { return t == 0 ? nt0 : nt1; };
 
           if constexpr (KEYS) {
@@ -545,7 +543,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (pre0 || nt0 == 0) return;
             const int nslot = (i + 1) & 1;
             if (!utest(&ctl->item_full[nslot], ((i + 1) >> 1) & 1)) return;
-            const int nt0n = ctl->item_nt0[nslot];
+            const int nt0n = ctl->item[nslot].n_max < 0 ? 0 : ctl->item[nslot].nt[0];
             const uint32_t gn = g0 + n_max;
             if (nt0n <= 0 || !utest(&ctl->q_full[0], qc0 & 1) || !utest(&ctl->k_full[gn % NSTAGE], (gn / NSTAGE) & 1))
               return;
@@ -617,18 +615,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       ok = ptx::mbar_wait(&ctl->item_full[slot], (i >> 1) & 1, abort_flag);
       // (KEYS: both warpgroups, which also meet after the walk)
       if (KEYS ? ptx::named_barrier_or(3, QT * BM, !ok) : ptx::named_barrier_or(1 + t, BM, !ok)) break;
-      const int w = ctl->item[slot];
-      ptx::mbar_arrive(&ctl->item_empty[slot]);
-      if (w < 0) break;
-      const Item it = item_of(w);
-      const int n_t = t == 0 ? it.nt0 : it.nt1;
-      const int tile_row0 = t == 0 ? it.row00 : it.row01, head = t == 0 ? it.h0 : it.h1;
+      const volatile Item* pub = &ctl->item[slot];
+      const int b = pub->b, kv_len = pub->kv_len, shift = pub->shift, j0 = pub->j0, n_max = pub->n_max;
+      const int n_t = pub->nt[t], tile_row0 = pub->row0[t], head = pub->h[t];
+      if (!KEYS) ptx::mbar_arrive(&ctl->item_empty[slot]);  // (KEYS: read again after the walk, and then handed back)
+      if (n_max < 0) break;
       const int row = tile_row0 + r_in;  // global query row of this thread
-      const int kv_len = it.kv_len;
-      T* orow = reinterpret_cast<T*>(a.o) + it.b * a.os.b + head * a.os.h + static_cast<int64_t>(row) * a.os.s;
-      float* lse_row = a.lse ? a.lse + (static_cast<int64_t>(it.b) * a.Hq + head) * a.Lq + row : nullptr;
+      T* orow = reinterpret_cast<T*>(a.o) + b * a.os.b + head * a.os.h + static_cast<int64_t>(row) * a.os.s;
+      float* lse_row = a.lse ? a.lse + (static_cast<int64_t>(b) * a.Hq + head) * a.Lq + row : nullptr;
 
-      if (KEYS ? cluster == 1 && it.n_max == 0 : n_t == 0) {
+      if (KEYS ? cluster == 1 && n_max == 0 : n_t == 0) {
+        if (KEYS) ptx::mbar_arrive(&ctl->item_empty[slot]);
         // no participating key (or tile beyond Lq): O = 0, LSE = -inf
         if (row < a.Lq && (!KEYS || t == 0)) {
 #pragma unroll
@@ -648,16 +645,16 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int cc = 0; cc < 4; ++cc) ptx::tmem_ld32p(tS + cc * 32, s + cc * 32);
         ptx::tmem_wait_ld();
 
-        const int col0 = (it.j0 + (KEYS ? 2 * j + t : j)) * BN;
+        const int col0 = (j0 + (KEYS ? 2 * j + t : j)) * BN;
         if constexpr (GEN) {
           if (a.mask.ptr && row < a.Lq)
-            add_mask_row<T>(s, a.mask, it.b * a.mask.sb + head * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
+            add_mask_row<T>(s, a.mask, b * a.mask.sb + head * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
         }
-        const bool mask_tile = (col0 + BN > kv_len) || (a.causal && col0 + BN - 1 > tile_row0 + it.shift);
+        const bool mask_tile = (col0 + BN > kv_len) || (a.causal && col0 + BN - 1 > tile_row0 + shift);
         if (mask_tile) {
           // Highest valid column of this row within the tile.
           int lim = kv_len - 1 - col0;
-          if (a.causal && row + it.shift - col0 < lim) lim = row + it.shift - col0;
+          if (a.causal && row + shift - col0 < lim) lim = row + shift - col0;
 #pragma unroll
           for (int e = 0; e < BN; ++e)
             if (e > lim) s[e] = 0xff800000u;  // -inf
@@ -745,9 +742,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Both halves of the walk: wait for both accumulators (tile 0's phase ec, tile 1's e1), exchange references and
         // sums (over the unused second Q tile), then warpgroup t puts columns [64 t, 64 t + 64) together (D = 64:
         // warpgroup 0 all of them).
-        if (ok && it.nt0 > 0) ok = ptx::mbar_wait(&ctl->o_full[0], ec & 1, abort_flag);
-        if (ok && it.nt1 > 0) ok = ptx::mbar_wait(&ctl->o_full[1], e1 & 1, abort_flag);
-        ec += it.nt0 > 0, e1 += it.nt1 > 0;
+        const int nt0 = pub->nt[0], nt1 = pub->nt[1];
+        ptx::mbar_arrive(&ctl->item_empty[slot]);
+        if (ok && nt0 > 0) ok = ptx::mbar_wait(&ctl->o_full[0], ec & 1, abort_flag);
+        if (ok && nt1 > 0) ok = ptx::mbar_wait(&ctl->o_full[1], e1 & 1, abort_flag);
+        ec += nt0 > 0, e1 += nt1 > 0;
         float2* stat = reinterpret_cast<float2*>(sQ + TB);
         stat[t * BM + r_in] = make_float2(n_t > 0 ? m_ref : -INFINITY, l2.x + l2.y);
         if (ptx::named_barrier_or(3, QT * BM, !ok)) break;
@@ -759,53 +758,56 @@ __global__ void __launch_bounds__(kThreads, 1)
         const float l = sa.y * wa + sb.y * wb;
         const bool mine = D == 128 || t == 0;
         const int c0 = D == 128 ? t * 64 : 0;
+        uint8_t* stage = sO + t * kStageBytes;
         if (mine) {
-          const uint32_t ta = tmem + 256 + lane_addr + c0;
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            if (it.nt0 > 0) ptx::tmem_ld32p(ta + cc * 32, s + cc * 32);
-            if (it.nt1 > 0) ptx::tmem_ld32p(ta + D + cc * 32, s + 64 + cc * 32);
+          if (cluster == 1) {
+            if (r_in == 0) ptx::bulk_wait_read();  // previous store out of this block has been read
+            ptx::named_barrier(1 + t, BM);
           }
-          ptx::tmem_wait_ld();
           const float inv = cluster > 1 ? 1.f : (l > 0.f ? 1.f / l : 0.f);
           const float ua = wa * inv, ub = wb * inv;
+          const uint32_t ta = tmem + 256 + lane_addr + c0;
+#pragma unroll 1
+          for (int cc = 0; cc < 2; ++cc) {  // 32 columns at a time
+            if (nt0 > 0) ptx::tmem_ld32p(ta + cc * 32, s);
+            if (nt1 > 0) ptx::tmem_ld32p(ta + D + cc * 32, s + 32);
+            ptx::tmem_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 64; ++e) {
-            const float x = it.nt0 > 0 ? __uint_as_float(s[e]) * ua : 0.f;
-            s[e] = __float_as_uint(it.nt1 > 0 ? fmaf(__uint_as_float(s[64 + e]), ub, x) : x);
+            for (int e = 0; e < 32; ++e) {
+              const float x = nt0 > 0 ? __uint_as_float(s[e]) * ua : 0.f;
+              s[e] = __float_as_uint(nt1 > 0 ? fmaf(__uint_as_float(s[32 + e]), ub, x) : x);
+            }
+            if (cluster == 1) {
+#pragma unroll
+              for (int ch = 0; ch < 4; ++ch) {
+                uint4 wv;
+                wv.x = pack2<BF16>(__uint_as_float(s[ch * 8 + 0]), __uint_as_float(s[ch * 8 + 1]));
+                wv.y = pack2<BF16>(__uint_as_float(s[ch * 8 + 2]), __uint_as_float(s[ch * 8 + 3]));
+                wv.z = pack2<BF16>(__uint_as_float(s[ch * 8 + 4]), __uint_as_float(s[ch * 8 + 5]));
+                wv.w = pack2<BF16>(__uint_as_float(s[ch * 8 + 6]), __uint_as_float(s[ch * 8 + 7]));
+                *reinterpret_cast<uint4*>(stage + r_in * 128 + (((cc * 4 + ch) ^ (r_in & 7)) << 4)) = wv;
+              }
+            } else {
+              // unnormalised O for the other CTAs, over the K / V stages (every MMA of the CTA is complete)
+              float* xo = reinterpret_cast<float*>(sK) + r_in * D;
+#pragma unroll
+              for (int ch = 0; ch < 8; ++ch)  // (16-byte pieces of a row permuted by the row: no bank conflicts)
+                *reinterpret_cast<uint4*>(xo + (((c0 >> 2) + cc * 8 + ch) ^ (r_in & (D / 4 - 1))) * 4) =
+                    make_uint4(s[ch * 4], s[ch * 4 + 1], s[ch * 4 + 2], s[ch * 4 + 3]);
+            }
           }
         }
         ptx::tc_fence_before();
         ptx::named_barrier(3, QT * BM);  // both accumulators and the statistics have been read
         if (cluster > 1) {
-          // unnormalised O (over the K / V stages: every MMA of the CTA is complete), reference and sum for the others
           if (t == 0) stat[2 * BM + r_in] = make_float2(m, l);
-          if (mine) {
-            float* xo = reinterpret_cast<float*>(sK) + r_in * D;
-#pragma unroll
-            for (int ch = 0; ch < 16; ++ch)  // (16-byte pieces of a row permuted by the row: no bank conflicts)
-              *reinterpret_cast<uint4*>(xo + (((c0 >> 2) + ch) ^ (r_in & (D / 4 - 1))) * 4) =
-                  make_uint4(s[ch * 4], s[ch * 4 + 1], s[ch * 4 + 2], s[ch * 4 + 3]);
-          }
           break;
         }
         if (mine) {
-          uint8_t* stage = sO + t * kStageBytes;
-          if (r_in == 0) ptx::bulk_wait_read();  // previous store out of this block has been read
-          ptx::named_barrier(1 + t, BM);
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch) {
-            uint4 wv;
-            wv.x = pack2<BF16>(__uint_as_float(s[ch * 8 + 0]), __uint_as_float(s[ch * 8 + 1]));
-            wv.y = pack2<BF16>(__uint_as_float(s[ch * 8 + 2]), __uint_as_float(s[ch * 8 + 3]));
-            wv.z = pack2<BF16>(__uint_as_float(s[ch * 8 + 4]), __uint_as_float(s[ch * 8 + 5]));
-            wv.w = pack2<BF16>(__uint_as_float(s[ch * 8 + 6]), __uint_as_float(s[ch * 8 + 7]));
-            *reinterpret_cast<uint4*>(stage + r_in * 128 + ((ch ^ (r_in & 7)) << 4)) = wv;
-          }
           ptx::fence_proxy_async_smem();
           ptx::named_barrier(1 + t, BM);
           if (r_in == 0) {
-            ptx::tma_store_4d(&tmO, stage, c0, tile_row0, head, it.b);
+            ptx::tma_store_4d(&tmO, stage, c0, tile_row0, head, b);
             ptx::bulk_commit();
           }
         }
@@ -845,7 +847,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::fence_proxy_async_smem();
         ptx::named_barrier(1 + t, BM);
         if (r_in == 0 && ok) {
-          ptx::tma_store_4d(&tmO, stage, hf * 64, tile_row0, head, it.b);
+          ptx::tma_store_4d(&tmO, stage, hf * 64, tile_row0, head, b);
           ptx::bulk_commit();
         }
       }
