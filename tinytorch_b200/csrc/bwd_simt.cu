@@ -33,17 +33,20 @@ constexpr int kThreads = 256;  // of the delta kernel
 // reductions need zeros to start from), which saves a separate memset of that size.
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) bwd_delta_kernel(const BwdArgs a) {
-  ptx::grid_dep_launch();  // the tensor-core backward kernel may set itself up and start on Q, K, V, dO meanwhile
+  // Launched early itself.  The main kernel may come up, and start on Q, K, V and dO without waiting for this grid, once
+  // every CTA here has seen everything before it complete.
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
+  if (a.sched && blockIdx.x == 0 && threadIdx.x == 0) *a.sched = 0;  // the main kernel's work counter
   constexpr int N = 16 / sizeof(T);  // elements per thread
   constexpr int TPR = D / N;         // threads per row (8, 16 or 32)
-  const int64_t row = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) / TPR;
+  // (a device holds fewer than 2^31 rows of 64 elements)
+  const uint32_t row = blockIdx.x * (kThreads / TPR) + threadIdx.x / TPR;
   const int part = threadIdx.x % TPR;
-  const int64_t total = static_cast<int64_t>(a.B) * a.Hq * a.Lq;
+  const uint32_t total = static_cast<uint32_t>(a.B) * a.Hq * a.Lq;
   float s = 0.f;
   if (row < total) {
-    const int i = static_cast<int>(row % a.Lq);
-    const int h = static_cast<int>((row / a.Lq) % a.Hq);
-    const int b = static_cast<int>(row / (static_cast<int64_t>(a.Lq) * a.Hq));
+    const uint32_t i = row % a.Lq, bh = row / a.Lq, h = bh % a.Hq, b = bh / a.Hq;
     const T* o = reinterpret_cast<const T*>(a.o) + b * a.os.b + h * a.os.h + static_cast<int64_t>(i) * a.os.s + part * N;
     const T* g =
         reinterpret_cast<const T*>(a.d_o) + b * a.dos.b + h * a.dos.h + static_cast<int64_t>(i) * a.dos.s + part * N;
@@ -53,7 +56,7 @@ __global__ void __launch_bounds__(kThreads) bwd_delta_kernel(const BwdArgs a) {
 #pragma unroll
     for (int e = 0; e < N; ++e) s = fmaf(to_f32<T>(op[e]), to_f32<T>(gp[e]), s);
     if (a.zero_dq_accum) {
-      float4* z = reinterpret_cast<float4*>(a.dq_accum + row * D + part * N);
+      float4* z = reinterpret_cast<float4*>(a.dq_accum + static_cast<int64_t>(row) * D + part * N);
 #pragma unroll
       for (int e = 0; e < N / 4; ++e) z[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -260,8 +263,9 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
 template <typename T, int D>
 cudaError_t launch_delta_t(const BwdArgs& a, cudaStream_t stream) {
   const int64_t rows = static_cast<int64_t>(a.B) * a.Hq * a.Lq;
-  bwd_delta_kernel<T, D><<<static_cast<unsigned>((rows * (D * sizeof(T) / 16) + kThreads - 1) / kThreads), kThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  if (rows > 0x7fffffffll) return cudaErrorInvalidValue;
+  return launch_early(bwd_delta_kernel<T, D>, dim3(static_cast<unsigned>((rows * (D * sizeof(T) / 16) + kThreads - 1) / kThreads)), dim3(kThreads), 0,
+                      stream, 1, a);
 }
 
 template <int D, bool MASK>

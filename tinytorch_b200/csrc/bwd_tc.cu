@@ -338,7 +338,13 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     };
     // The next item is drawn while the last step of this one is fed (lane 0 holds it in `drawn`), so that the
     // latency of the atomic does not sit between two items.
-    int drawn = lane == 0 ? atomicAdd(a.sched, 1) : 0;
+    // The first item is the CTA's own number; the counter, which the delta pre-pass has zeroed, hands out the rest.
+    int drawn = blockIdx.x;
+    auto draw = [&]() {
+      if (!dep_waited) ptx::grid_dep_wait();
+      dep_waited = true;
+      if (lane == 0) drawn = static_cast<int>(gridDim.x) + atomicAdd(a.sched, 1);
+    };
     for (uint32_t i = 0;;) {  // i: items published so far
       int w = drawn;
       if (w >= n_items) w = -1;
@@ -362,7 +368,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
                     make_uint4(0, 0, 0, 0);
             }
           }
-          if (lane == 0) drawn = atomicAdd(a.sched, 1);
+          draw();
           continue;
         }
       }
@@ -388,7 +394,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok || w < 0) break;
       for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
-        if (redraw && n + 1 == it.n_steps && lane == 0) drawn = atomicAdd(a.sched, 1);
+        if (redraw && n + 1 == it.n_steps) draw();
         const uint32_t g = gq + n;
         const int h = it.h, q0 = it.qt * BQ;
         // The vectors (two buffers) are fetched a step ahead of the tiles (one stage): the wait passed for the
@@ -887,7 +893,13 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
       bool dep_waited = false;
       // The next item is drawn while the last step of this one is fed (lane 0 holds it in `drawn`), so that the
       // latency of the atomic does not sit between two items.
-      int drawn = lane == 0 ? atomicAdd(a.sched, 1) : 0;
+      // The first item is the CTA's own number; the counter, which the delta pre-pass has zeroed, hands out the rest.
+      int drawn = blockIdx.x;
+      auto draw = [&]() {
+        if (!dep_waited) ptx::grid_dep_wait();
+        dep_waited = true;
+        if (lane == 0) drawn = static_cast<int>(gridDim.x) + atomicAdd(a.sched, 1);
+      };
       for (uint32_t i = 0;;) {  // i: items published so far
         int w = drawn;
         if (w >= n_items) w = -1;
@@ -911,7 +923,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
                       make_uint4(0, 0, 0, 0);
               }
             }
-            if (lane == 0) drawn = atomicAdd(a.sched, 1);
+            draw();
             continue;
           }
         }
@@ -934,7 +946,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok || w < 0) break;
         for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
-          if (redraw && n + 1 == it.n_steps && lane == 0) drawn = atomicAdd(a.sched, 1);
+          if (redraw && n + 1 == it.n_steps) draw();
           const uint32_t g = gq + n;
           const int st = g % NQ;
           const int h = it.h, q0 = it.qt * BQ;
@@ -1290,14 +1302,29 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const BwdArgs a) {
   ptx::grid_dep_wait();  // launched early: the accumulator is complete from here on
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x, first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t total = a.dq ? static_cast<int64_t>(a.B) * a.Hq * a.Lq * (D / 8) : 0;
-  for (int64_t idx = first; idx < total; idx += step) {
-    const int c8 = static_cast<int>(idx % (D / 8));
-    const int64_t rowi = idx / (D / 8);
-    const int i = static_cast<int>(rowi % a.Lq);
-    const int h = static_cast<int>((rowi / a.Lq) % a.Hq);
-    const int b = static_cast<int>(rowi / (static_cast<int64_t>(a.Lq) * a.Hq));
-    const float4* src = reinterpret_cast<const float4*>(a.dq_accum + rowi * D + c8 * 8);
-    store8(reinterpret_cast<T*>(a.dq) + b * a.dqs.b + h * a.dqs.h + static_cast<int64_t>(i) * a.dqs.s + c8 * 8, src[0], src[1]);
+  T* dq = reinterpret_cast<T*>(a.dq);
+  const bool dense = a.dqs.s == D && a.dqs.h == static_cast<int64_t>(a.Lq) * D && a.dqs.b == a.dqs.h * a.Hq;
+  constexpr int U = 4;  // 128 bytes in flight per thread
+  for (int64_t idx = first; idx < total; idx += U * step) {
+    float4 x[U], y[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (idx + u * step < total) {
+        const float4* src = reinterpret_cast<const float4*>(a.dq_accum + (idx + u * step) * 8);
+        x[u] = __ldcs(src), y[u] = __ldcs(src + 1);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = idx + u * step;
+      if (e >= total) break;
+      if (dense) {
+        store8(dq + e * 8, x[u], y[u]);
+      } else {
+        const uint32_t rowi = static_cast<uint32_t>(e / (D / 8)), c8 = static_cast<uint32_t>(e % (D / 8));
+        const uint32_t i = rowi % a.Lq, bh = rowi / a.Lq, h = bh % a.Hq, b = bh / a.Hq;
+        store8(dq + b * a.dqs.b + h * a.dqs.h + static_cast<int64_t>(i) * a.dqs.s + c8 * 8, x[u], y[u]);
+      }
+    }
   }
   if (a.parts <= 1) return;
   const int64_t rows = static_cast<int64_t>(a.B) * a.Hkv * a.Skv, per_part = rows * D;
@@ -1307,9 +1334,9 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const BwdArgs a) {
     T* base = reinterpret_cast<T*>(t ? a.dv : a.dk);
     if (!base) continue;
     const Str3& st = t ? a.dvs : a.dks;
-    const int64_t e = idx - t * rows * (D / 8), rowi = e / (D / 8);
-    const int c8 = static_cast<int>(e % (D / 8)), j = static_cast<int>(rowi % a.Skv);
-    const int h = static_cast<int>((rowi / a.Skv) % a.Hkv), b = static_cast<int>(rowi / (static_cast<int64_t>(a.Skv) * a.Hkv));
+    const int64_t e = idx - t * rows * (D / 8);
+    const uint32_t rowi = static_cast<uint32_t>(e / (D / 8)), c8 = static_cast<uint32_t>(e % (D / 8));
+    const int j = rowi % a.Skv, bh = rowi / a.Skv, h = bh % a.Hkv, b = bh / a.Hkv;
     // the steps of this row's key tile, as the main kernel counts them: a part without any has left nothing
     const int kv0 = j / BM * BM;
     int kv_len = a.Skv;
@@ -1321,7 +1348,7 @@ __global__ void __launch_bounds__(256) dq_convert_kernel(const BwdArgs a) {
     const int qt0 = a.causal ? (kv0 - shift > 0 ? (kv0 - shift) / BQ : 0) : 0;
     const int n_all = kv0 < kv_len && qt0 < n_q_tiles ? (n_q_tiles - qt0) * group : 0;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-    const float* src = a.dkv_part + t * a.parts * per_part + rowi * D + c8 * 8;
+    const float* src = a.dkv_part + t * a.parts * per_part + e * 8;
     for (int p = 0; p < a.parts; ++p) {
       if (part_begin(n_all, p, a.parts) == part_begin(n_all, p + 1, a.parts)) continue;
       const float4 u = reinterpret_cast<const float4*>(src + p * per_part)[0], v = reinterpret_cast<const float4*>(src + p * per_part)[1];
@@ -1432,11 +1459,7 @@ size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream) {
   BwdArgs pre = a;
   pre.zero_dq_accum = 1;
-  // The work counter starts at zero for every launch; cleared ahead of the pre-pass so that the kernel
-  // launched early behind the pre-pass already sees it.
-  cudaError_t e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);
-  if (e != cudaSuccess) return e;
-  e = launch_bwd_delta(dtype, D, pre, stream);
+  cudaError_t e = launch_bwd_delta(dtype, D, pre, stream);
   if (e != cudaSuccess) return e;
   const bool general = a.mask.ptr != nullptr || a.causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT;
   return general ? launch_g<true>(dtype, D, a, device, stream) : launch_g<false>(dtype, D, a, device, stream);

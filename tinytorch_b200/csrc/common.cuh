@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../include/tt_attn.h"
+#include "ptx.cuh"
 
 namespace ttattn {
 
@@ -63,7 +64,7 @@ struct BwdArgs {
   int zero_dq_accum;  // set by the tensor-core launcher: the delta kernel also clears dq_accum
   int tail_heads;     // tensor-core kernel: (batch, kv head) pairs at the end of the item order whose key tiles are
                       // ordered longest walk first across heads (set by its launcher)
-  int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by its launcher
+  int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by the delta pre-pass
   int parts;          // tensor-core kernel: work items per key tile (see bwd_parts); > 1: each leaves its dK / dV in ...
   float* dkv_part;    // ... workspace [dK, dV][parts][B * Hkv][Skv][D] fp32
   void* dq;
@@ -181,6 +182,17 @@ cudaError_t launch_early(void (*kern)(P...), dim3 grid, dim3 block, int smem, cu
   cfg.stream = stream;
   cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// Zeroes a work counter ahead of the kernel that draws from it: 1 us between two kernels that are launched early, where a
+// memset, which waits for the one and is waited for by the other, takes 3.3.
+static __global__ void zero_word_kernel(int* word) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
+  if (threadIdx.x == 0) *word = 0;
+}
+inline cudaError_t launch_zero_word(int* word, cudaStream_t stream) {
+  return launch_early(zero_word_kernel, dim3(1), dim3(32), 0, stream, 1, word);
 }
 
 template <typename T>

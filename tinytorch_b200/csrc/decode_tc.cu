@@ -583,7 +583,7 @@ cudaError_t launch_g(int dtype, DecodeArgs a, cudaStream_t stream) {
   if (n_items > 0x7fffffffll || !a.sched) return cudaErrorInvalidValue;
   const int ctas = OCC * sm_count(device);
   if (n_items > ctas && !a.chained) {
-    e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);  // the work counter starts at zero for every launch
+    e = launch_zero_word(a.sched, stream);  // the work counter starts at zero for every launch
     if (e != cudaSuccess) return e;
   }
   return launch_early(kern, dim3(static_cast<unsigned>(n_items < ctas ? n_items : ctas)), dim3(kThreads), kSmem, stream, 1, tk, tv,

@@ -982,7 +982,7 @@ cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
   const int grid = p.cluster > 1 ? static_cast<int>(n_items) * p.cluster : static_cast<int>(n_items < sms ? n_items : sms);
   if (p.cluster == 1 && n_items > grid) {
     // the counter that hands out what comes after the CTAs' first items must start at zero for every launch
-    cudaError_t e = cudaMemsetAsync(a.sched, 0, sizeof(int), stream);
+    cudaError_t e = launch_zero_word(a.sched, stream);
     if (e != cudaSuccess) return e;
   } else {
     a.sched = nullptr;
