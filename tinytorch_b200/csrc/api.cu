@@ -424,8 +424,9 @@ int tt_linear(const tt_linear_params* p) {
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   const LinearCall c{p->dtype, p->x, p->w, p->bias, p->y, static_cast<int>(p->M), static_cast<int>(p->N),
                      static_cast<int>(p->K), ldx, ldw, ldy, x_t, w_t, p->status, p->device, stream};
-  cudaError_t e = launch_linear_tc(c);
-  if (e == cudaSuccess && x_sum) e = launch_column_sums(p->dtype, p->x, x_sum, p->K, p->M, ldx, p->device, stream);
+  bool persistent = false;
+  cudaError_t e = launch_linear_tc(c, &persistent);
+  if (e == cudaSuccess && x_sum) e = launch_column_sums(p->dtype, p->x, x_sum, p->K, p->M, ldx, persistent, stream);
   return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
 }
 

@@ -150,12 +150,13 @@ struct LinearCall {
   int device;
   cudaStream_t stream;
 };
-cudaError_t launch_linear_tc(const LinearCall& c);
+cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  // *persistent: linear_tc_kernel was taken
 // ... for outputs with too few tiles to occupy the machine: contraction split over clusters (linear_split.cu)
 double linear_split_us(const LinearCall& c);  // what it is expected to take
 cudaError_t launch_linear_split(const LinearCall& c);
 // out[n] = sum over the rows of x[rows, n] (fused_ops.cu); n and ldx are multiples of 8
-cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, int device,
+// `beside`: the kernel launched just before is a linear_tc_kernel, beside which this one may run
+cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, bool beside,
                                cudaStream_t stream);
 
 // one CTA waiting `limit_ns` on an mbarrier nobody arrives on (selftest.cu)

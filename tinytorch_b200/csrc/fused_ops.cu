@@ -212,34 +212,34 @@ __global__ void __launch_bounds__(kThreads) silu_mul_generic_kernel(T* out, cons
   out[i] = from_f32<T>(silu_mul1(g, u));
 }
 
-// out[c] = sum over the rows of x[rows, n] (row stride ld) in fp32, rounded once.  HBM bound: a CTA reads 256-byte
-// segments of its share of the rows (16 threads across, 16 rows at a time, 8 loads per thread in flight), the CTAs of a
-// cluster share the rows of one block of 128 columns and are summed in rank order through distributed shared memory:
-// no scratch memory, no second kernel, and the same result every time.  (Before: a copy to fp32 and a library
-// reduction, 185 us for 4096 x 12288; now 17-19 us.)
-constexpr int kSumCols = 128, kSumRows = 16;
+// out[c] = sum over the rows of x[rows, n] (row stride ld) in fp32, rounded once.  A CTA is one warp: 16 lanes across (128
+// columns, 256 bytes of a row), two rows at a time, 16 loads per lane in flight; the CTAs of a cluster share the rows of
+// a block of columns and are summed in rank order through distributed shared memory: no scratch memory, no second
+// kernel, and the same result every time.  `beside`: the kernel before in the stream is the gradient product that reads
+// the same x; it leaves 1.8 KB of shared memory and most of HBM's bandwidth unused, and 1.5 KB, 1 of them the system's, are all that a CTA
+// here asks for, so it runs beside it instead of behind it (32 us of a pass over 4096 x 12288, and 185 us as a copy to
+// fp32 and a library reduction).
+constexpr int kSumCols = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads) column_sums_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows,
-                                                               int64_t n, int64_t ld, int cluster) {
+__global__ void __launch_bounds__(32) column_sums_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t rows, int64_t n,
+                                                         int64_t ld, int cluster, bool beside) {
   constexpr int N = Pack<T>::N;
   static_assert(N == 8, "16-bit types");
   ptx::grid_dep_launch();
-  ptx::grid_dep_wait();
-  __shared__ float s_sum[kSumRows][kSumCols + 4];
-  __shared__ __align__(16) float s_total[kSumCols];
-  const int rank = blockIdx.x % cluster;
-  const int64_t col = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + (threadIdx.x % 16) * N;
-  const int rl = threadIdx.x / 16;
+  if (!beside) ptx::grid_dep_wait();
+  __shared__ __align__(16) float s_sum[kSumCols];
+  const int rank = blockIdx.x % cluster, lane = threadIdx.x;
+  const int64_t col = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + (lane % 16) * N;
   const int64_t per = (rows + cluster - 1) / cluster, r0 = rank * per, r1 = r0 + per < rows ? r0 + per : rows;
   float acc[N] = {};
   if (col < n) {
-    constexpr int U = 8;
-    for (int64_t r = r0 + rl; r < r1; r += U * kSumRows) {
+    constexpr int U = 16;
+    for (int64_t r = r0 + lane / 16; r < r1; r += 2 * U) {
       uint4 v[U];
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        v[u] = r + u * kSumRows < r1 ? *reinterpret_cast<const uint4*>(x + (r + u * kSumRows) * ld + col) : make_uint4(0, 0, 0, 0);
+        v[u] = r + 2 * u < r1 ? __ldcg(reinterpret_cast<const uint4*>(x + (r + 2 * u) * ld + col)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         float f[N];
@@ -250,39 +250,42 @@ __global__ void __launch_bounds__(kThreads) column_sums_kernel(const T* __restri
     }
   }
 #pragma unroll
-  for (int i = 0; i < N; ++i) s_sum[rl][(threadIdx.x % 16) * N + i] = acc[i];
-  __syncthreads();
-  if (threadIdx.x < kSumCols) {
-    float t = 0.f;
+  for (int i = 0; i < N; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+  if (lane < 16) {
 #pragma unroll
-    for (int r = 0; r < kSumRows; ++r) t += s_sum[r][threadIdx.x];
-    s_total[threadIdx.x] = t;
+    for (int i = 0; i < N; ++i) s_sum[lane * N + i] = acc[i];
   }
   if (cluster > 1)
     ptx::cluster_sync();
   else
-    __syncthreads();
-  if (rank == 0 && threadIdx.x < kSumCols / 4) {
-    const int64_t c0 = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + threadIdx.x * 4;
+    __syncwarp();
+  if (rank == 0) {
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x / cluster) * kSumCols + lane * 4;
     if (c0 < n) {
       float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int r = 0; r < cluster; ++r) {
-        const float4 p = ptx::ld_cluster_f4(ptx::map_rank(ptx::smem_u32(s_total + threadIdx.x * 4), r));
+        const float4 p = ptx::ld_cluster_f4(ptx::map_rank(ptx::smem_u32(s_sum + lane * 4), r));
         t.x += p.x, t.y += p.y, t.z += p.z, t.w += p.w;
       }
       out[c0] = from_f32<T>(t.x), out[c0 + 1] = from_f32<T>(t.y), out[c0 + 2] = from_f32<T>(t.z), out[c0 + 3] = from_f32<T>(t.w);
     }
   }
   if (cluster > 1) ptx::cluster_sync();  // no CTA leaves while rank 0 still reads its sums
+  // what comes after this grid waits for its end only: it does not end before the grid beside it
+  if (beside && blockIdx.x == 0) ptx::grid_dep_wait();
 }
 
 template <typename T>
-cudaError_t sums_t(const void* x, void* out, int64_t rows, int64_t n, int64_t ld, cudaStream_t stream) {
+cudaError_t sums_t(const void* x, void* out, int64_t rows, int64_t n, int64_t ld, bool beside, cudaStream_t stream) {
   // the rows of a column block are divided while a CTA keeps at least 64 of them
   int cluster = 1;
   while (cluster < 8 && rows >= cluster * 2 * 64) cluster *= 2;
-  return launch_early(column_sums_kernel<T>, dim3(static_cast<unsigned>((n + kSumCols - 1) / kSumCols) * cluster), dim3(kThreads), 0, stream, cluster,
-                      static_cast<const T*>(x), static_cast<T*>(out), rows, n, ld, cluster);
+  auto kern = column_sums_kernel<T>;
+  // (the SM's shared memory stays divided as the kernel beside needs it)
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  if (e != cudaSuccess) return e;
+  return launch_early(kern, dim3(static_cast<unsigned>((n + kSumCols - 1) / kSumCols) * cluster), dim3(32), 0, stream, cluster,
+                      static_cast<const T*>(x), static_cast<T*>(out), rows, n, ld, cluster, beside);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -348,11 +351,10 @@ cudaError_t launch_fused_add_rms_norm(int dtype, void* input, void* residual, co
   return rms_t<__nv_bfloat16>(input, residual, weight, rows, dim, eps, stream);
 }
 
-cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, int device,
+cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, bool beside,
                                cudaStream_t stream) {
-  (void)device;
-  return dtype == TT_ATTN_F16 ? sums_t<__half>(x, out, rows, n, ldx, stream)
-                              : sums_t<__nv_bfloat16>(x, out, rows, n, ldx, stream);
+  return dtype == TT_ATTN_F16 ? sums_t<__half>(x, out, rows, n, ldx, beside, stream)
+                              : sums_t<__nv_bfloat16>(x, out, rows, n, ldx, beside, stream);
 }
 
 cudaError_t launch_silu_mul(int dtype, void* out, const void* x, int64_t rows, int64_t d, cudaStream_t stream) {

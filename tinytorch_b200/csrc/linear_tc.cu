@@ -120,8 +120,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   ptx::cluster_sync();  // the barriers of both CTAs are initialised
   ptx::tc_fence_after();
   const uint32_t tmem = ctl->tmem_base;
-  ptx::grid_dep_launch();  // (the next kernel may come up: this grid has its TMEM)
   ptx::grid_dep_wait();    // everything below reads or writes global memory
+  // The next kernel may come up: this grid has its TMEM.  (After the wait, so that column_sums_kernel, which reads only x,
+  // may run beside this one: once all CTAs here have come this far, everything before is complete.)
+  ptx::grid_dep_launch();
   const bool usable = *abort_flag == 0;
 
   if (warp == 0) {
@@ -292,7 +294,8 @@ cudaError_t launch_bf(const LinearCall& c, int ctas) {
 
 }  // namespace
 
-cudaError_t launch_linear_tc(const LinearCall& c) {
+cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent) {
+  if (persistent) *persistent = false;
   if (c.dtype != TT_ATTN_BF16 && c.dtype != TT_ATTN_F16) return cudaErrorInvalidValue;
   // The persistent pairs where they are expected to be the faster: whole rounds of 256 x 256 tiles at 0.29 us per 64 of
   // the contraction (or an epilogue each, where the contraction is short), 4.5 us for ramp and drain.  Few rows leave
@@ -302,6 +305,7 @@ cudaError_t launch_linear_tc(const LinearCall& c) {
   const double round_us = 0.29 * ((c.K + BK - 1) / BK);
   const double pair_us = 4.5 + static_cast<double>((tiles + pairs - 1) / pairs) * (round_us > 1.6 ? round_us : 1.6);
   if (tiles < 2 * pairs && (c.M <= HM || linear_split_us(c) < pair_us)) return launch_linear_split(c);
+  if (persistent) *persistent = true;
   const int ctas = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
   return c.dtype == TT_ATTN_BF16 ? launch_bf<true>(c, ctas) : launch_bf<false>(c, ctas);
 }
