@@ -19,6 +19,7 @@ namespace ttattn {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int64_t kKeepBytes = 64 << 20;  // half of L2: larger tensors are streamed past it
 
 template <typename T>
 struct Pack {
@@ -42,16 +43,27 @@ __device__ __forceinline__ uint4 ld_cs(const void* p) {
   asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
 }
+// KEEP: the tensors fit L2, where the next operator finds them
+template <bool KEEP>
+__device__ __forceinline__ uint4 ld_vec(const void* p) {
+  if constexpr (KEEP) return *reinterpret_cast<const uint4*>(p);
+  else return ld_cs(p);
+}
 __device__ __forceinline__ void st_cs(void* p, const uint4& v) {
   asm volatile("st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");
+}
+template <bool KEEP>
+__device__ __forceinline__ void st_vec(void* p, const uint4& v) {
+  if constexpr (KEEP) *reinterpret_cast<uint4*>(p) = v;
+  else st_cs(p, v);
 }
 
 // A group of `tpr` threads (a power of two, 32..256) owns one row; a CTA holds
 // kThreads / tpr rows.  Each thread keeps VPT 16-byte vectors of the row.
 // FEW: so few rows that the kernel is a chain of latencies: the weight is fetched with the row instead of after the sum
 // (with many rows it comes from L1, and its registers would cost resident warps).
-template <typename T, int VPT, bool FEW>
+template <typename T, int VPT, bool FEW, bool KEEP>
 __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ input, T* __restrict__ residual,
                                                                 const T* __restrict__ weight, int64_t rows, int dim,
                                                                 int tpr, float eps) {
@@ -73,8 +85,8 @@ __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ 
   for (int v = 0; v < VPT; ++v) {
     const int idx = t_in_row + v * tpr;
     const bool ok = row_ok && idx < vecs;
-    a[v] = ok ? ld_cs(in_row + idx * N) : make_uint4(0, 0, 0, 0);
-    b[v] = ok ? ld_cs(res_row + idx * N) : make_uint4(0, 0, 0, 0);
+    a[v] = ok ? ld_vec<KEEP>(in_row + idx * N) : make_uint4(0, 0, 0, 0);
+    b[v] = ok ? ld_vec<KEEP>(res_row + idx * N) : make_uint4(0, 0, 0, 0);
     if (FEW) wv[v] = ok ? __ldg(reinterpret_cast<const uint4*>(weight + idx * N)) : make_uint4(0, 0, 0, 0);
   }
   float sum_sq = 0.f;
@@ -90,7 +102,7 @@ __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ 
       sum_sq = fmaf(fa[i], fa[i], sum_sq);  // of the unrounded sum, as the reference does
     }
     b[v] = Pack<T>::pack(fa);  // residual, rounded to T; the scaling below uses this rounded value
-    if (row_ok && idx < vecs) st_cs(res_row + idx * N, b[v]);
+    if (row_ok && idx < vecs) st_vec<KEEP>(res_row + idx * N, b[v]);
   }
   // sum over the thread group: warp shuffles, then the group's warps through shared memory
 #pragma unroll
@@ -112,7 +124,7 @@ __global__ void __launch_bounds__(kThreads) add_rms_norm_kernel(T* __restrict__ 
     Pack<T>::unpack(FEW ? wv[FEW ? v : 0] : __ldg(reinterpret_cast<const uint4*>(weight + idx * N)), fw);
 #pragma unroll
     for (int i = 0; i < N; ++i) fr[i] = fr[i] * inv_rms * fw[i];
-    st_cs(in_row + idx * N, Pack<T>::pack(fr));
+    st_vec<KEEP>(in_row + idx * N, Pack<T>::pack(fr));
   }
 }
 
@@ -163,7 +175,7 @@ __device__ __forceinline__ uint4 silu_vec(const uint4& g, const uint4& u) {
 
 // x [rows, 2d] -> out [rows, d], long rows: CTA (row, chunk) handles kThreads * kSiluUnroll
 // vectors of one row, so that no index needs a division.  vecs_per_row = d / N.
-template <typename T>
+template <typename T, bool KEEP>
 __global__ void __launch_bounds__(kThreads) silu_mul_rows_kernel(T* __restrict__ out, const T* __restrict__ x,
                                                                  int vecs_per_row) {
   constexpr int N = Pack<T>::N;
@@ -178,12 +190,12 @@ __global__ void __launch_bounds__(kThreads) silu_mul_rows_kernel(T* __restrict__
 #pragma unroll
   for (int k = 0; k < kSiluUnroll; ++k) {
     const int v = v0 + k * kThreads;
-    if (v < vecs_per_row) g[k] = ld_cs(gp + v * N), u[k] = ld_cs(up + v * N);
+    if (v < vecs_per_row) g[k] = ld_vec<KEEP>(gp + v * N), u[k] = ld_vec<KEEP>(up + v * N);
   }
 #pragma unroll
   for (int k = 0; k < kSiluUnroll; ++k) {
     const int v = v0 + k * kThreads;
-    if (v < vecs_per_row) st_cs(op + v * N, silu_vec<T>(g[k], u[k]));
+    if (v < vecs_per_row) st_vec<KEEP>(op + v * N, silu_vec<T>(g[k], u[k]));
   }
 }
 
@@ -198,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) silu_mul_kernel(T* __restrict__ out,
   if (idx >= total_vecs) return;
   const uint32_t row = idx / vecs_per_row, col = idx - row * vecs_per_row;
   const T* gp = x + (static_cast<int64_t>(row) * 2 * vecs_per_row + col) * N;
-  st_cs(out + static_cast<int64_t>(idx) * N, silu_vec<T>(ld_cs(gp), ld_cs(gp + static_cast<int64_t>(vecs_per_row) * N)));
+  st_vec<true>(out + static_cast<int64_t>(idx) * N, silu_vec<T>(ld_vec<true>(gp), ld_vec<true>(gp + static_cast<int64_t>(vecs_per_row) * N)));
 }
 
 template <typename T>
@@ -313,10 +325,11 @@ cudaError_t rms_t(void* input, void* residual, const void* weight, int64_t rows,
   const int rows_per_cta = kThreads / tpr;
   const unsigned grid = static_cast<unsigned>((rows + rows_per_cta - 1) / rows_per_cta);
   const int d = static_cast<int>(dim);
-  auto kern = vpt <= 1   ? (few ? add_rms_norm_kernel<T, 1, true> : add_rms_norm_kernel<T, 1, false>)
-              : vpt <= 2 ? (few ? add_rms_norm_kernel<T, 2, true> : add_rms_norm_kernel<T, 2, false>)
-              : vpt <= 4 ? (few ? add_rms_norm_kernel<T, 4, true> : add_rms_norm_kernel<T, 4, false>)
-                         : (few ? add_rms_norm_kernel<T, 8, true> : add_rms_norm_kernel<T, 8, false>);
+  const bool keep = 2 * rows * dim * static_cast<int64_t>(sizeof(T)) <= kKeepBytes;
+#define TT_RMS(V) \
+  (few ? add_rms_norm_kernel<T, V, true, true> : keep ? add_rms_norm_kernel<T, V, false, true> : add_rms_norm_kernel<T, V, false, false>)
+  auto kern = vpt <= 1 ? TT_RMS(1) : vpt <= 2 ? TT_RMS(2) : vpt <= 4 ? TT_RMS(4) : TT_RMS(8);
+#undef TT_RMS
   return launch_early(kern, dim3(grid), dim3(kThreads), 0, stream, 1, in, res, w, rows, d, tpr, eps);
 }
 
@@ -332,7 +345,9 @@ cudaError_t silu_t(void* out, const void* x, int64_t rows, int64_t d, cudaStream
   const bool few = rows * ((vpr + kChunk - 1) / kChunk) < 148;
   if (vec_ok && !few && vpr >= kThreads && (vpr + kChunk - 1) / kChunk <= 65535 && rows <= 0x7fffffff) {
     dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>((vpr + kChunk - 1) / kChunk));
-    return launch_early(silu_mul_rows_kernel<T>, grid, dim3(kThreads), 0, stream, 1, o, xi, static_cast<int>(vpr));
+    const bool keep = 3 * rows * d * static_cast<int64_t>(sizeof(T)) <= kKeepBytes;
+    return launch_early(keep ? silu_mul_rows_kernel<T, true> : silu_mul_rows_kernel<T, false>, grid, dim3(kThreads), 0, stream, 1, o,
+                        xi, static_cast<int>(vpr));
   }
   if (vec_ok && total < 0x7fffff00ll)
     return launch_early(silu_mul_kernel<T>, dim3(static_cast<unsigned>((total + kThreads - 1) / kThreads)), dim3(kThreads), 0,
