@@ -113,6 +113,8 @@ int take_mask(const void* ptr, int kind, const int64_t st[3], MaskArgs* m) {
   if (kind < 0 || kind > TT_ATTN_MASK_ADD_F32) return TT_ATTN_ERR_DTYPE;
   if (st[0] < 0 || st[1] < 0 || st[2] < 0) return TT_ATTN_ERR_SHAPE;
   m->ptr = ptr, m->kind = kind, m->sb = st[0], m->sh = st[1], m->sl = st[2];
+  const int64_t esz = kind == TT_ATTN_MASK_BOOL ? 1 : (kind == TT_ATTN_MASK_ADD_F32 ? 4 : 2);
+  m->wide = ((reinterpret_cast<uintptr_t>(ptr) | (m->sb * esz) | (m->sh * esz) | (m->sl * esz)) & 15) == 0;
   return TT_ATTN_OK;
 }
 }  // namespace
@@ -122,7 +124,8 @@ extern "C" {
 size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (B <= 0 || Hq <= 0 || D <= 0) return 0;
   // fp16 / bf16 forward: one work counter for the persistent kernel's scheduler
-  if (kind == TT_ATTN_KIND_FWD) return dtype == TT_ATTN_F32 ? 0 : 256;
+  // (and the lengths that a padding mask comes to)
+  if (kind == TT_ATTN_KIND_FWD) return dtype == TT_ATTN_F32 ? 0 : round256(scratch_words(B) * sizeof(int));
   if (kind == TT_ATTN_KIND_BWD) {
     // delta [B,Hq,Lq] fp32; the fp16 / bf16 path adds an fp32 dQ accumulator [B,Hq,Lq,D]
     const size_t rows = static_cast<size_t>(B) * Hq * (Lq > 0 ? Lq : 0);
@@ -130,7 +133,7 @@ size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int 
     if (dtype == TT_ATTN_F32) return round256(rows * sizeof(float));
     // (and, where few key tiles are divided among several work items, their partial dK / dV)
     return round256(rows * sizeof(float)) + round256(rows * D * sizeof(float)) +
-           round256(bwd_part_bytes(B, Hq, Hkv, Lq, Skv, D)) + 256;
+           round256(bwd_part_bytes(B, Hq, Hkv, Lq, Skv, D)) + round256(scratch_words(B) * sizeof(int));
   }
   if (kind == TT_ATTN_KIND_DECODE_APPEND) {
     // the decode scratch; on the grouped-query tensor-core path also the rotated q and the new lengths
@@ -232,7 +235,7 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) +
                                         round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * sizeof(float)));
   if (p->dtype != TT_ATTN_F32) {
-    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + need - 256);
+    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + need - round256(scratch_words(p->B) * sizeof(int)));
     a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
     a.dkv_part = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dq_accum) +
                                           round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * p->D * sizeof(float)));

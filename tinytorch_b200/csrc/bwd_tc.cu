@@ -56,6 +56,7 @@ struct Item {
   int hk, b, kv0, kv_len, shift, part;
   // the walk: n_steps query tiles from tile qt of query head h on; a head's tiles are [qt_begin, n_q_tiles)
   int qt_begin, n_steps, h, qt;  // n_steps < 0: no more items
+  int mask;                      // whether the mask has to be looked at
 };
 
 struct __align__(8) SmemCtl {
@@ -101,13 +102,52 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
+// The mask of 16 queries and this thread's key, as stored: adjacent threads read adjacent keys.  Fetched before the scores
+// arrive, all loads in flight together (one by one inside the arithmetic they made a step ten times as long): B5 H32/16
+// L1620 D64 with an additive bf16 mask 3447 -> 602 us, without a mask 340; D128, 2 x 16/4 heads x 2048: 398, 272.  `off`:
+// mask offset of (first query, this key); n_q: how many of the queries exist (0: nothing is read); a mask that is
+// the same for all rows is read once.
+__device__ __forceinline__ void fetch_mask(const MaskArgs& m, int64_t off, int n_q, uint32_t (&w)[16]) {
+  auto fetch = [&](auto* p) {
+    if (m.sl == 0) {
+      w[0] = n_q > 0 ? static_cast<uint32_t>(*p) : 0u;
+#pragma unroll
+      for (int i = 1; i < 16; ++i) w[i] = w[0];
+    } else {
+      if (n_q >= 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i, p += m.sl) w[i] = static_cast<uint32_t>(*p);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i, p += m.sl) w[i] = i < n_q ? static_cast<uint32_t>(*p) : 0u;
+      }
+    }
+  };
+  if (m.kind == TT_ATTN_MASK_BOOL) fetch(reinterpret_cast<const uint8_t*>(m.ptr) + off);
+  else if (m.kind == TT_ATTN_MASK_ADD_F32) fetch(reinterpret_cast<const uint32_t*>(m.ptr) + off);
+  else fetch(reinterpret_cast<const uint16_t*>(m.ptr) + off);
+}
+
+// By a whole warp: the mask of a step's queries and key tile on its way to L2, ahead of the threads that fetch it.
+__device__ __forceinline__ void prefetch_mask(const BwdArgs& a, int b, int h, int q0, int kv0, int lane) {
+  const MaskArgs& m = a.mask;
+  if (m.sl == 0) return;
+  const int esz = m.kind == TT_ATTN_MASK_BOOL ? 1 : (m.kind == TT_ATTN_MASK_ADD_F32 ? 4 : 2);
+  const int bytes = (a.Skv - kv0 < BM ? a.Skv - kv0 : BM) * esz;
+  const char* p = reinterpret_cast<const char*>(m.ptr) + (b * m.sb + h * m.sh + kv0) * esz;
+  for (int i = lane; i < BQ && q0 + i < a.Lq; i += 32) {
+    const char* row = p + static_cast<int64_t>(q0 + i) * m.sl * esz;
+    for (int at = 0; at < bytes; at += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(row + at)));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(row + bytes - 1)));
+  }
+}
+
 // P of 16 queries for this thread's key row: in place of s (S^T, fp32 bits) and as packed 16-bit pairs in pk.
-// lse2: -lse * log2(e) of the 16 queries; q_first: index of the first query; mo: offset of (first query, this
-// key) in the mask; n_hidden: how many of the 16 queries, from the first on, do not see this key (causal
-// triangle; all 16 for a key beyond kv_len).
+// lse2: -lse * log2(e) of the 16 queries; mw: the mask, if use_mask; n_hidden: how many of the 16 queries, from the first
+// on, do not see this key (causal triangle; all 16 for a key beyond kv_len).
 template <bool BF16, bool GEN, typename T>
 __device__ __forceinline__ void p_chunk(const BwdArgs& a, uint32_t (&s)[16], const float* lse2, float2 c2v,
-                                        int n_hidden, int kv_row, int q_first, int64_t mo, uint32_t (&pk)[8]) {
+                                        int n_hidden, bool use_mask, const uint32_t (&mw)[16], uint32_t (&pk)[8]) {
   // exponents c*s - lse2, in packed fp32 pairs
 #pragma unroll
   for (int i = 0; i < 16; i += 4) {
@@ -115,19 +155,23 @@ __device__ __forceinline__ void p_chunk(const BwdArgs& a, uint32_t (&s)[16], con
     float2 x0 = ptx::fma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), c2v, make_float2(l4.x, l4.y));
     float2 x1 =
         ptx::fma2(make_float2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), c2v, make_float2(l4.z, l4.w));
-    if constexpr (GEN) {
-      if (a.mask.ptr && kv_row < a.Skv) {
-        // the mask element of (query, this thread's key): adjacent threads read adjacent keys
-        const int q = q_first + i;
-        const int64_t m = mo + static_cast<int64_t>(i) * a.mask.sl;
-        if (q + 0 < a.Lq) x0.x += mask_bias2<T>(a.mask, m);
-        if (q + 1 < a.Lq) x0.y += mask_bias2<T>(a.mask, m + a.mask.sl);
-        if (q + 2 < a.Lq) x1.x += mask_bias2<T>(a.mask, m + 2 * a.mask.sl);
-        if (q + 3 < a.Lq) x1.y += mask_bias2<T>(a.mask, m + 3 * a.mask.sl);
-      }
-    }
     s[i] = __float_as_uint(x0.x), s[i + 1] = __float_as_uint(x0.y);
     s[i + 2] = __float_as_uint(x1.x), s[i + 3] = __float_as_uint(x1.y);
+  }
+  if constexpr (GEN) {
+    if (use_mask) {
+      if (a.mask.kind == TT_ATTN_MASK_BOOL) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] = mw[i] ? s[i] : 0xff800000u;
+      } else if (a.mask.kind == TT_ATTN_MASK_ADD_F32) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) + __uint_as_float(mw[i]) * kLog2e);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          s[i] = __float_as_uint(__uint_as_float(s[i]) + to_f32<T>(*reinterpret_cast<const T*>(&mw[i])) * kLog2e);
+      }
+    }
   }
   // Hidden pairs get P = 0 through the exponent.  (Kept apart from the arithmetic before and after, which then
   // is the same straight-line code for every step; only the diagonal step and a ragged last key tile come here.)
@@ -239,6 +283,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
     }
     it.kv_len = kv_len;
+    it.mask = GEN && a.mask.ptr && !(a.mask_pure && a.mask_pure[it.b]);
     it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
     // BM == BQ: query tiles before the key tile see none of it (general: first tile with a row i >= kv0 - shift)
     it.qt_begin = a.causal ? (GEN ? (it.kv0 - it.shift > 0 ? (it.kv0 - it.shift) / BQ : 0) : nt) : 0;
@@ -340,6 +385,10 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
     // latency of the atomic does not sit between two items.
     // The first item is the CTA's own number; the counter, which the delta pre-pass has zeroed, hands out the rest.
     int drawn = blockIdx.x;
+    if (GEN && a.mask_pure) {  // (the lengths come from the pre-pass)
+      ptx::grid_dep_wait();
+      dep_waited = true;
+    }
     auto draw = [&]() {
       if (!dep_waited) ptx::grid_dep_wait();
       dep_waited = true;
@@ -395,6 +444,7 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
       if (!ok || w < 0) break;
       for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
         if (redraw && n + 1 == it.n_steps) draw();
+        if (GEN && it.mask) prefetch_mask(a, it.b, it.h, it.qt * BQ, it.kv0, lane);
         const uint32_t g = gq + n;
         const int h = it.h, q0 = it.qt * BQ;
         // The vectors (two buffers) are fetched a step ahead of the tiles (one stage): the wait passed for the
@@ -581,6 +631,16 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         }
       };
 
+      // the mask of a step is fetched a step ahead, while dQ is read out
+      uint32_t mw[2][16];
+      auto fetch = [&](int h, int qt) {
+#pragma unroll
+        for (int sc = 0; sc < 2; ++sc) {
+          const int q = qt * BQ + wg * 32 + sc * 16;
+          fetch_mask(a.mask, b * a.mask.sb + h * a.mask.sh + q * a.mask.sl + kv_row, kv_row < a.Skv ? a.Lq - q : 0, mw[sc]);
+        }
+      };
+      if (GEN && it.mask) fetch(h, qt);
       for (int n = 0; n < n_steps; ++n, advance(h, qt, it.qt_begin)) {
         const uint32_t g = g0 + n;
         const int q0 = qt * BQ;
@@ -601,13 +661,9 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
           ptx::tmem_ld16(tB + lane_addr + col, dp);
           ptx::tmem_wait_ld();
           uint32_t pk[8], dk[8];
-          int64_t mo = 0;
-          if constexpr (GEN)
-            mo = b * a.mask.sb + h * a.mask.sh + static_cast<int64_t>(q0 + col) * a.mask.sl +
-                 kv_row;
           int n_hidden = 0;
           if (masked) n_hidden = !row_valid ? 16 : (diag ? kv_row - (q0 + col + shift) : 0);
-          p_chunk<BF16, GEN, T>(a, s, vec + col, c2v, n_hidden, kv_row, q0 + col, mo, pk);
+          p_chunk<BF16, GEN, T>(a, s, vec + col, c2v, n_hidden, GEN && it.mask, mw[sc], pk);
           ds_chunk<BF16>(s, dp, vec + BQ + col, sc2, dk);
           // Warpgroup w keeps its 16-bit results in columns [32w, 32w+16) of the
           // region, i.e. over the first 16 columns it loaded itself, never over
@@ -633,6 +689,11 @@ __global__ void __launch_bounds__(Cfg128::kThreads, 1)
         ptx::fence_proxy_async_smem();
         ptx::tc_fence_before();
         ptx::mbar_arrive(&ctl->pds_full);
+        if (GEN && it.mask && n + 1 < n_steps) {
+          int h1 = h, qt1 = qt;
+          advance(h1, qt1, it.qt_begin);
+          fetch(h1, qt1);
+        }
         read_out_dq(n);
       }
       g0 += n_steps;
@@ -811,6 +872,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
       kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
     }
     it.kv_len = kv_len;
+    it.mask = GEN && a.mask.ptr && !(a.mask_pure && a.mask_pure[it.b]);
     it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
     // BM == BQ: query tiles before the key tile see none of it (general: first tile with a row i >= kv0 - shift)
     it.qt_begin = a.causal ? (GEN ? (it.kv0 - it.shift > 0 ? (it.kv0 - it.shift) / BQ : 0) : nt) : 0;
@@ -895,6 +957,10 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
       // latency of the atomic does not sit between two items.
       // The first item is the CTA's own number; the counter, which the delta pre-pass has zeroed, hands out the rest.
       int drawn = blockIdx.x;
+      if (GEN && a.mask_pure) {  // (the lengths come from the pre-pass)
+        ptx::grid_dep_wait();
+        dep_waited = true;
+      }
       auto draw = [&]() {
         if (!dep_waited) ptx::grid_dep_wait();
         dep_waited = true;
@@ -947,6 +1013,7 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
         if (!ok || w < 0) break;
         for (int n = 0; n < it.n_steps; ++n, advance(it.h, it.qt, it.qt_begin)) {
           if (redraw && n + 1 == it.n_steps) draw();
+          if (GEN && it.mask) prefetch_mask(a, it.b, it.h, it.qt * BQ, it.kv0, lane);
           const uint32_t g = gq + n;
           const int st = g % NQ;
           const int h = it.h, q0 = it.qt * BQ;
@@ -1218,12 +1285,18 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
       ptx::mbar_arrive(&ctl->item_empty[slot]);
       if (!ok || it.n_steps < 0) break;
       const int kv_row = it.kv0 + r;
+      uint32_t mw[2][16];
+      auto fetch = [&](int sc, int h, int qt) {
+        const int q = qt * BQ + wg * 32 + sc * 16;
+        fetch_mask(a.mask, it.b * a.mask.sb + h * a.mask.sh + q * a.mask.sl + kv_row, kv_row < a.Skv ? a.Lq - q : 0, mw[sc]);
+      };
       for (int n = 0; n < it.n_steps; ++n, ++g, advance(it.h, it.qt, it.qt_begin)) {
         const int hq = it.h, q0 = it.qt * BQ;
         const float* vec = svec + (g & 1) * 2 * BQ;
         // some (query, key) pairs of this step are hidden: the diagonal step, a ragged last key tile
         const bool diag = a.causal && q0 + it.shift < it.kv0 + BM;
         const bool masked = diag || it.kv0 + BM > it.kv_len;
+        if (GEN && it.mask) fetch(0, hq, it.qt), fetch(1, hq, it.qt);
         if (ok) ok = ptx::mbar_wait(&ctl->vec_full[g & 1], (g >> 1) & 1, abort_flag);
         // phase 1: P^T from S^T; P stays in registers for phase 2
         if (ok) ok = ptx::mbar_wait(&ctl->s_full, g & 1, abort_flag);
@@ -1235,12 +1308,9 @@ __global__ void __launch_bounds__(Cfg64::kThreads, 1)
           ptx::tmem_ld16(tA + lane_addr + col, p[sc]);
           ptx::tmem_wait_ld();
           uint32_t pk[8];
-          int64_t mo = 0;
-          if constexpr (GEN)
-            mo = it.b * a.mask.sb + hq * a.mask.sh + static_cast<int64_t>(q0 + col) * a.mask.sl + kv_row;
           int n_hidden = 0;
           if (masked) n_hidden = kv_row >= it.kv_len ? 16 : (diag ? kv_row - (q0 + col + it.shift) : 0);
-          p_chunk<BF16, GEN, T>(a, p[sc], vec + col, c2v, n_hidden, kv_row, q0 + col, mo, pk);
+          p_chunk<BF16, GEN, T>(a, p[sc], vec + col, c2v, n_hidden, GEN && it.mask, mw[sc], pk);
           // Warpgroup w keeps its 16-bit results in columns [32w, 32w+16) of the region, i.e. over the first 16
           // columns it loaded itself, never over columns another warpgroup still has to read.
           ptx::tmem_st8(tA + lane_addr + wg * 32 + sc * 8, pk);
@@ -1456,9 +1526,13 @@ size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   return p > 1 ? static_cast<size_t>(2) * p * B * Hkv * Skv * D * sizeof(float) : 0;
 }
 
-cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream) {
-  BwdArgs pre = a;
+cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& call, int device, cudaStream_t stream) {
+  BwdArgs a = call, pre = call;
   pre.zero_dq_accum = 1;
+  if (is_padding_mask(a.mask, a.causal)) {
+    pre.mask_pure = a.mask_pure = a.sched + 1 + a.B;  // (to the pre-pass: that it is to find the lengths)
+    a.kv_lens = a.sched + 1;
+  }
   cudaError_t e = launch_bwd_delta(dtype, D, pre, stream);
   if (e != cudaSuccess) return e;
   const bool general = a.mask.ptr != nullptr || a.causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT;

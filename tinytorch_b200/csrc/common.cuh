@@ -33,6 +33,7 @@ struct MaskArgs {
   const void* ptr;  // null: no mask
   int kind;         // tt_attn_mask_kind
   int64_t sb, sh, sl;
+  bool wide;        // every row starts on a 16-byte boundary
 };
 
 // Arguments common to the prefill kernels (SIMT and tensor-core).
@@ -49,7 +50,8 @@ struct FwdArgs {
   const int32_t* kv_lens;
   int32_t* status;
   MaskArgs mask;
-  int* sched;  // tensor-core path: work counter in scratch memory, zeroed by the launcher
+  int* sched;  // tensor-core path: scratch memory of scratch_words(B) integers, the first of them the work counter
+  const int32_t* mask_pure;  // tensor-core path, with masked_lens: whether the mask is all true up to the length
 };
 
 struct BwdArgs {
@@ -77,6 +79,7 @@ struct BwdArgs {
   const int32_t* kv_lens;
   int32_t* status;
   MaskArgs mask;
+  const int32_t* mask_pure;  // as in FwdArgs
 };
 
 struct DecodeArgs {
@@ -194,6 +197,46 @@ static __global__ void zero_word_kernel(int* word) {
 }
 inline cudaError_t launch_zero_word(int* word, cudaStream_t stream) {
   return launch_early(zero_word_kernel, dim3(1), dim3(32), 0, stream, 1, word);
+}
+
+// Scratch integers of the tensor-core kernels: the work counter and, for a padding mask, a length and a flag per sequence.
+constexpr size_t scratch_words(int B) { return 1 + 2 * static_cast<size_t>(B); }
+
+// A boolean mask that is the same for all heads and rows is most often padding: true up to a length.  Its sequences are
+// then worth no more than that many keys, and within them the mask need not be looked at.  (Not under the bottom-right
+// alignment, which is taken from the number of cache rows.)
+inline bool is_padding_mask(const MaskArgs& m, int causal) {
+  return m.ptr && m.kind == TT_ATTN_MASK_BOOL && m.sh == 0 && m.sl == 0 && causal != TT_ATTN_CAUSAL_BOTTOM_RIGHT;
+}
+// By all threads of a CTA: lens[b] = 1 + the last key that takes part, pure[b] = whether all before it do.
+__device__ __forceinline__ void masked_lens(const MaskArgs& m, const int32_t* kv_lens, int Skv, int b, int32_t* lens,
+                                            int32_t* pure) {
+  __shared__ int s_last, s_count;
+  if (threadIdx.x == 0) s_last = 0, s_count = 0;
+  __syncthreads();
+  int len = Skv;
+  if (kv_lens) {
+    const int l = kv_lens[b];
+    len = l < 0 ? 0 : (l < Skv ? l : Skv);
+  }
+  const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + b * m.sb;
+  const int lead = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 15), n = (lead + len + 15) / 16;
+  int last = 0, count = 0;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {  // the aligned vectors that hold the row
+    const uint4 v = reinterpret_cast<const uint4*>(p - lead)[j];
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int key = j * 16 + i - lead;
+      if (key >= 0 && key < len && ((w[i / 4] >> (i % 4 * 8)) & 0xffu)) last = key + 1, ++count;
+    }
+  }
+  last = __reduce_max_sync(0xffffffffu, last);
+  count = __reduce_add_sync(0xffffffffu, count);
+  if (threadIdx.x % 32 == 0 && count > 0) atomicMax(&s_last, last), atomicAdd(&s_count, count);
+  __syncthreads();
+  if (threadIdx.x == 0) lens[b] = s_last, pure[b] = s_count == s_last;
+  __syncthreads();
 }
 
 template <typename T>

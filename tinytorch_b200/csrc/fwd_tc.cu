@@ -70,6 +70,7 @@ struct Item {
   int kv_len, shift;           // key j participates iff j <= i + shift (causal)
   int j0, nt[QT];              // first key tile, and how many each half walks from there (KEYS: in turn)
   int n_max;                   // the longer walk; -1: no more items
+  int mask;                    // whether the mask has to be looked at
 };
 
 struct __align__(16) SmemCtl {
@@ -87,9 +88,12 @@ constexpr int tile_bytes() {
   return BM * D * 2;
 }
 constexpr int kStageBytes = BM * 128;  // per warpgroup: one 64-column block of an O tile
-template <int D>
+// a second buffer for mask rows (see MaskRows), where there is room for it
+template <int D, int GEN>
+constexpr int kMaskExtra = D == 64 && GEN == 2 ? QT * kStageBytes : 0;
+template <int D, int GEN>
 constexpr int smem_bytes() {
-  return (QT + 2 * NSTAGE) * tile_bytes<D>() + QT * kStageBytes + 1024 /*alignment slack*/ + 512 /*SmemCtl*/;
+  return (QT + 2 * NSTAGE) * tile_bytes<D>() + QT * kStageBytes + kMaskExtra<D, GEN> + 1024 /*alignment slack*/ + 512 /*SmemCtl*/;
 }
 
 template <bool BF16>
@@ -103,10 +107,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-// GEN: the general variant of the kernel (a mask and / or a causal triangle that is
-// not top-left aligned); the fast variant compiles all of that out.
+// GEN: 1: the variant for a causal triangle that is not top-left aligned, 2: that and a mask; the fast variant (0) compiles
+// all of that out.
 // KEYS: `per_head` items (query blocks) per (batch, kv head), `rank` of `cluster` shares of the key tiles; else pairs.
-template <bool GEN, bool KEYS>
+template <int GEN, bool KEYS>
 __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_head, int rank = 0, int cluster = 1) {
   Item it;
   // Heads in order, the longest (latest causal) pair of a head first: the CTAs running at any moment share few
@@ -135,6 +139,7 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_hea
     kv_len = l < 0 ? 0 : (l < a.Skv ? l : a.Skv);
   }
   it.kv_len = kv_len;
+  it.mask = GEN == 2 && !(a.mask_pure && a.mask_pure[it.b]);
   it.shift = GEN ? causal_shift(a.causal, kv_len, a.Lq) : 0;  // key j participates iff j <= i + shift
   const int x = KEYS ? mp : mp * QT, qt0 = x / group, qt1 = KEYS ? qt0 : (x + 1) / group;
   it.h[0] = it.hk * group + x - qt0 * group, it.h[1] = KEYS ? it.h[0] : it.hk * group + x + 1 - qt1 * group;
@@ -164,46 +169,117 @@ __device__ __forceinline__ Item decode_item(const FwdArgs& a, int w, int per_hea
   return it;
 }
 
-// s[e] <- c * s[e] + mask(row, col0 + e) * log2(e) for the 128 scores of one
-// query row; `off` is the mask's element offset of (row, col0) and n_valid the
-// number of keys that exist from col0 on.  16-byte loads when the row segment is
-// whole and aligned, element loads otherwise.
+// The mask of one warp's 32 query rows, 128 bytes of a row at a time (128 keys of a boolean mask, 64 of a 16-bit or 32 of
+// an fp32 one) through 4 KB of shared memory.  A thread owns a whole row of scores, but 32 rows read by 32 threads are 32
+// cache lines per load, and rows of an odd length are not even aligned: 13 times the time without a mask.  The warp copies
+// row by row instead, the aligned 16-byte pieces that hold the segment, eight lanes a row (cp.async: nothing waits for them
+// until the scores have arrived; the pieces of a row are rotated by its number against bank conflicts), and each thread
+// reads its row back and shifts it into place; a ninth piece, of a row that is not aligned, waits in registers.  A mask that
+// is the same for all rows is one row.  B5 H32/16 L1620 D64 with an additive bf16 mask: 2193 -> 440 us, without a
+// mask 167.
 template <typename T>
-__device__ __forceinline__ void add_mask_row(uint32_t (&s)[BN], const MaskArgs& m, int64_t off, int n_valid, float c) {
-  const int esz = m.kind == TT_ATTN_MASK_BOOL ? 1 : (m.kind == TT_ATTN_MASK_ADD_F32 ? 4 : 2);
-  const uint8_t* base = reinterpret_cast<const uint8_t*>(m.ptr) + off * esz;
-  const bool fast = n_valid >= BN && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
+struct MaskRows {
+  const uint8_t* base;  // the warp's first row
+  int rows;             // rows that exist
+
+  static __device__ __forceinline__ const uint8_t* down16(const uint8_t* p) {
+    return reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15));
+  }
+
+  __device__ __forceinline__ void stage(const FwdArgs& a, int esz, int lane, int at, uint32_t buf, uint4& tail) const {
+    const int64_t pitch = a.mask.sl * esz;
+    const int left = a.Skv * esz - at;  // bytes of a row that exist from there on
+    const int piece = lane & 7, r0 = lane >> 3;
+    const uint8_t* p = base + r0 * pitch + at;
+    const uint32_t dst = buf + r0 * 128;
+    if (rows >= 32 && left >= 128 + 15) {
 #pragma unroll
-  for (int ch = 0; ch < BN / 16; ++ch) {
-    float bias[16];
-    if (fast) {
-      if (m.kind == TT_ATTN_MASK_BOOL) {
-        const uint4 v = *reinterpret_cast<const uint4*>(base + ch * 16);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      for (int i = 0; i < 32; i += 4, p += 4 * pitch)
+        ptx::cp_async16(dst + i * 128 + (((piece + r0 + i) & 7) << 4), down16(p) + piece * 16, 16);
+    } else {
+      const uint8_t* any = reinterpret_cast<const uint8_t*>(a.mask.ptr);  // a valid address, for copies of nothing
+#pragma unroll 1
+      for (int i = 0; i < 32; i += 4, p += 4 * pitch) {
+        const uint8_t* src = down16(p) + piece * 16;
+        const int n = r0 + i < rows ? static_cast<int>(p + left - src) : 0;
+        if (pitch != 0 || r0 == 0) ptx::cp_async16(dst + i * 128 + (((piece + r0 + i) & 7) << 4), n > 0 ? src : any, n > 16 ? 16 : (n > 0 ? n : 0));
+        if (pitch == 0) break;
+      }
+    }
+    if (!a.mask.wide) {
+      const uint8_t* mine = base + lane * pitch + at;
+      const uint8_t* src = down16(mine) + 128;
+      tail = make_uint4(0, 0, 0, 0);
+      if ((lane < rows || pitch == 0) && src < mine + left && down16(mine) != mine) tail = *reinterpret_cast<const uint4*>(src);
+    }
+  }
+
+  // this lane's segment, 8 words at a time: use(first word, words)
+  template <typename F>
+  __device__ __forceinline__ void read(const FwdArgs& a, int esz, int lane, uint32_t buf, const uint4& tail, F use) const {
+    ptx::cp_async_wait();
+    __syncwarp();
+    const int64_t pitch = a.mask.sl * esz;
+    uint32_t r = pitch == 0 ? 0 : lane;
+    asm volatile("" : "+r"(r));  // (the addresses are computed here, not kept in registers)
+    const uint32_t row = buf + r * 128;
+    auto piece = [&](int i) { return ptx::ld_shared4(row + (((i + r) & 7) << 4)); };
+    uint4 p[4];  // the pieces of a chunk and the next
+    p[0] = piece(0), p[1] = piece(1);
+    if (a.mask.wide) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) bias[i] = ((w[i >> 2] >> ((i & 3) * 8)) & 0xffu) ? 0.f : -INFINITY;
-      } else if (m.kind == TT_ATTN_MASK_ADD_F32) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 v = *reinterpret_cast<const float4*>(base + ch * 64 + q * 16);
-          bias[q * 4 + 0] = v.x * kLog2e, bias[q * 4 + 1] = v.y * kLog2e;
-          bias[q * 4 + 2] = v.z * kLog2e, bias[q * 4 + 3] = v.w * kLog2e;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const uint4 v = *reinterpret_cast<const uint4*>(base + ch * 32 + q * 16);
-          const T* t = reinterpret_cast<const T*>(&v);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) bias[q * 8 + i] = to_f32<T>(t[i]) * kLog2e;
-        }
+      for (int c = 0; c < 4; ++c) {
+        const uint4 x = p[(c & 1) * 2], y = p[(c & 1) * 2 + 1];
+        if (c < 3) p[(~c & 1) * 2] = piece(2 * c + 2), p[(~c & 1) * 2 + 1] = piece(2 * c + 3);
+        const uint32_t w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        use(c * 8, w);
       }
     } else {
+      const uint32_t mis = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(base) + lane * pitch) & 15;
+      const bool by2 = mis & 8, by1 = mis & 4;
+      const uint32_t sh = (mis & 3) * 8;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) bias[i] = (ch * 16 + i < n_valid) ? mask_bias2<T>(m, off + ch * 16 + i) : 0.f;
+      for (int c = 0; c < 4; ++c) {
+        const uint4 x = p[(c & 1) * 2], y = p[(c & 1) * 2 + 1];
+        if (c < 3) p[(~c & 1) * 2] = piece(2 * c + 2), p[(~c & 1) * 2 + 1] = piece(2 * c + 3);
+        const uint4 z = c < 3 ? p[(~c & 1) * 2] : tail;
+        uint32_t w[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+#pragma unroll
+        for (int i = 0; i < 10; ++i) w[i] = by2 ? w[i + 2] : w[i];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) w[i] = by1 ? w[i + 1] : w[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], sh);
+        use(c * 8, w);
+      }
     }
+    __syncwarp();  // the buffer may be filled again
+  }
+};
+
+// s[e] <- c * s[e] + mask for the keys of 8 words, the first of them key e0 of the tile
+template <typename T, int KIND>
+__device__ __forceinline__ void add_mask(uint32_t (&s)[BN], int e0, const uint32_t* w, float c) {
+  const float2 c2 = make_float2(c, c);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) s[ch * 16 + i] = __float_as_uint(fmaf(__uint_as_float(s[ch * 16 + i]), c, bias[i]));
+  for (int k = 0; k < 8; ++k) {
+    if constexpr (KIND == TT_ATTN_MASK_BOOL) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = e0 + k * 4 + i;
+        s[e] = (w[k] >> (8 * i)) & 0xffu ? __float_as_uint(__uint_as_float(s[e]) * c) : 0xff800000u;
+      }
+    } else if constexpr (KIND == TT_ATTN_MASK_ADD_F32) {
+      s[e0 + k] = __float_as_uint(fmaf(__uint_as_float(s[e0 + k]), c, __uint_as_float(w[k])));
+    } else {
+      const int e = e0 + k * 2;
+      const T* t = reinterpret_cast<const T*>(&w[k]);
+      const float2 m = std::is_same<T, __nv_bfloat16>::value
+                           ? make_float2(__uint_as_float(__byte_perm(w[k], 0, 0x1044)), __uint_as_float(w[k] & 0xffff0000u))
+                           : make_float2(to_f32<T>(t[0]), to_f32<T>(t[1]));
+      const float2 x = ptx::fma2(make_float2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), c2, m);
+      s[e] = __float_as_uint(x.x), s[e + 1] = __float_as_uint(x.y);
+    }
   }
 }
 
@@ -259,7 +335,7 @@ __device__ __forceinline__ void combine_rows(const FwdArgs& a, const Item& it, i
   }
 }
 
-template <int D, bool BF16, bool GEN, bool KEYS>
+template <int D, bool BF16, int GEN, bool KEYS>
 __global__ void __launch_bounds__(kThreads, 1)
     fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -272,7 +348,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* sK = smem + QT * TB;          // NSTAGE tiles
   uint8_t* sV = sK + NSTAGE * TB;        // NSTAGE tiles
   uint8_t* sO = sV + NSTAGE * TB;        // QT staging blocks for the O stores
-  SmemCtl* ctl = reinterpret_cast<SmemCtl*>(sO + QT * kStageBytes);
+  SmemCtl* ctl = reinterpret_cast<SmemCtl*>(sO + QT * kStageBytes + kMaskExtra<D, GEN>);
   volatile int* abort_flag = &ctl->abort_flag;
 
   const int tid = threadIdx.x;
@@ -597,10 +673,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tS = tmem + t * 128 + lane_addr;
     const uint32_t tO = tmem + 256 + t * D + lane_addr;
     // > 0 so that a masked (-inf) score stays -inf when it is scaled
-    const float c = fmaxf(fabsf(a.scale) * kLog2e, 1e-30f);
-    // with a mask the scores are scaled when the mask is added, and the rest of the loop multiplies by 1
-    const float cm = (GEN && a.mask.ptr) ? 1.f : c;
-    const float2 c2 = make_float2(cm, cm);
+    const float c = fmaxf(fabsf(a.scale) * kLog2e, 1e-30f), cs = fmaxf(fabsf(a.scale), 1e-30f);
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
     uint32_t cnt = 0;  // softmax iterations completed (s_full phase)
     uint32_t ec = 0, e1 = 0;  // items with work completed (o_full phase; KEYS: of tile 0, of tile 1)
@@ -618,6 +691,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const volatile Item* pub = &ctl->item[slot];
       const int b = pub->b, kv_len = pub->kv_len, shift = pub->shift, j0 = pub->j0, n_max = pub->n_max;
       const int n_t = pub->nt[t], tile_row0 = pub->row0[t], head = pub->h[t];
+      const bool use_mask = GEN == 2 && pub->mask;
       if (!KEYS) ptx::mbar_arrive(&ctl->item_empty[slot]);  // (KEYS: read again after the walk, and then handed back)
       if (n_max < 0) break;
       const int row = tile_row0 + r_in;  // global query row of this thread
@@ -635,6 +709,32 @@ __global__ void __launch_bounds__(kThreads, 1)
         continue;
       }
 
+      // with a mask the scores are scaled when the mask is added, and the rest of the loop multiplies by log2(e)
+      const float cm = use_mask ? kLog2e : c;
+      const float2 c2 = make_float2(cm, cm);
+      MaskRows<T> mk = {};
+      const int esz = a.mask.kind == TT_ATTN_MASK_BOOL ? 1 : (a.mask.kind == TT_ATTN_MASK_ADD_F32 ? 4 : 2);
+      // segments of the tile alternate between the buffers, of which D = 128 has one
+      constexpr int kBufs = kMaskExtra<D, GEN> > 0 ? 2 : 1;
+      const uint32_t mbuf = ptx::smem_u32(sO + t * kStageBytes + (warp & 3) * 32 * 128);
+      auto buffer = [&](int seg) { return mbuf + seg % kBufs * (QT * kStageBytes); };
+      uint4 mtail[kBufs];
+      auto stage_mask = [&](int j, int seg) {
+        mk.stage(a, esz, lane, (j0 + (KEYS ? 2 * j + t : j)) * BN * esz + seg * 128, buffer(seg), mtail[seg % kBufs]);
+      };
+      if constexpr (GEN == 2) {
+        if (use_mask && n_t > 0) {
+          // (through this warp's rows of the staging block of O, out of which the item before may still be stored)
+          const int row0 = tile_row0 + (warp & 3) * 32;
+          mk.base = reinterpret_cast<const uint8_t*>(a.mask.ptr) + (b * a.mask.sb + head * a.mask.sh + row0 * a.mask.sl) * esz;
+          mk.rows = a.mask.sl == 0 ? 1 : a.Lq - row0;
+          if (r_in == 0) ptx::bulk_wait_read();
+          ptx::named_barrier(1 + t, BM);
+          stage_mask(0, 0);
+          if (kBufs > 1 && esz > 1) stage_mask(0, 1);
+        }
+      }
+
       float m_ref = -INFINITY;  // reference max, in scaled log2 units
       float2 l2 = make_float2(0.f, 0.f);
       for (int j = 0; j < n_t && ok; ++j) {
@@ -646,9 +746,27 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::tmem_wait_ld();
 
         const int col0 = (j0 + (KEYS ? 2 * j + t : j)) * BN;
-        if constexpr (GEN) {
-          if (a.mask.ptr && row < a.Lq)
-            add_mask_row<T>(s, a.mask, b * a.mask.sb + head * a.mask.sh + row * a.mask.sl + col0, a.Skv - col0, c);
+        if constexpr (GEN == 2) {
+          if (use_mask) {
+            auto read = [&](int seg, auto use) {
+              mk.read(a, esz, lane, buffer(seg), mtail[seg % kBufs], use);
+              if (seg + kBufs < esz) stage_mask(j, seg + kBufs);
+            };
+            if (esz == 1) {
+              read(0, [&](int k, const uint32_t* w) { add_mask<T, TT_ATTN_MASK_BOOL>(s, k * 4, w, cs); });
+            } else if (esz == 2) {
+              read(0, [&](int k, const uint32_t* w) { add_mask<T, TT_ATTN_MASK_ADD>(s, k * 2, w, cs); });
+              read(1, [&](int k, const uint32_t* w) { add_mask<T, TT_ATTN_MASK_ADD>(s, 64 + k * 2, w, cs); });
+            } else {
+#pragma unroll
+              for (int seg = 0; seg < 4; ++seg)
+                read(seg, [&](int k, const uint32_t* w) { add_mask<T, TT_ATTN_MASK_ADD_F32>(s, seg * 32 + k, w, cs); });
+            }
+            if (j + 1 < n_t) {
+              stage_mask(j + 1, 0);
+              if (kBufs > 1 && esz > 1) stage_mask(j + 1, 1);
+            }
+          }
         }
         const bool mask_tile = (col0 + BN > kv_len) || (a.causal && col0 + BN - 1 > tile_row0 + shift);
         if (mask_tile) {
@@ -883,21 +1001,21 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ------------------------------------------------------------------ host ----
-template <int D, bool BF16, bool GEN, bool KEYS>
+template <int D, bool BF16, int GEN, bool KEYS>
 cudaError_t launch_k(const FwdArgs& a, int dtype, int grid, int cluster, cudaStream_t stream) {
   CUtensorMap tq, tk, tv, to;
   if (!make_map(&tq, dtype, a.q, D, a.Lq, a.Hq, a.B, a.qs) || !make_map(&tk, dtype, a.k, D, a.Skv, a.Hkv, a.B, a.ks) ||
       !make_map(&tv, dtype, a.v, D, a.Skv, a.Hkv, a.B, a.vs) || !make_map(&to, dtype, a.o, D, a.Lq, a.Hq, a.B, a.os))
     return cudaErrorInvalidValue;
   auto kern = fwd_tc_kernel<D, BF16, GEN, KEYS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D>());
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D, GEN>());
   if (e != cudaSuccess) return e;
-  return launch_early(kern, dim3(grid), dim3(kThreads), smem_bytes<D>(), stream, cluster, tq, tk, tv, to, a, cluster);
+  return launch_early(kern, dim3(grid), dim3(kThreads), smem_bytes<D, GEN>(), stream, cluster, tq, tk, tv, to, a, cluster);
 }
 
 // CTAs of clusters of this size that can be resident at once, one to an SM (a cluster lives inside one GPC, and GPCs
 // differ in size).  Asked once per device.
-template <int D, bool BF16, bool GEN>
+template <int D, bool BF16, int GEN>
 int cluster_slots(int device, int cluster) {
   static std::atomic<int> known[64][3];
   if (device < 0 || device >= 64) return 0;
@@ -911,10 +1029,10 @@ int cluster_slots(int device, int cluster) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count(device) / cluster * cluster);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_bytes<D>();
+    cfg.dynamicSmemBytes = smem_bytes<D, GEN>();
     cfg.attrs = attr, cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D>()) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<D, GEN>()) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
       cudaGetLastError();
       clusters = 0;
@@ -935,7 +1053,7 @@ struct Plan {
   bool keys;
   int cluster;
 };
-template <int D, bool BF16, bool GEN>
+template <int D, bool BF16, int GEN>
 Plan plan_of(const FwdArgs& a, int device) {
   const int group = a.Hq / a.Hkv, n_qt = (a.Lq + BM - 1) / BM, sms = sm_count(device);
   const long long heads = static_cast<long long>(a.B) * a.Hkv, blocks = heads * group * n_qt, pairs = heads * ((group * n_qt + 1) / 2);
@@ -972,7 +1090,15 @@ Plan plan_of(const FwdArgs& a, int device) {
   return best;
 }
 
-template <int D, bool BF16, bool GEN>
+// ahead of the main kernel: the lengths that a padding mask comes to, and the work counter
+__global__ void __launch_bounds__(256) lens_kernel(const FwdArgs a, int* sched, int32_t* lens, int32_t* pure) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sched = 0;
+  masked_lens(a.mask, a.kv_lens, a.Skv, blockIdx.x, lens, pure);
+}
+
+template <int D, bool BF16, int GEN>
 cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
   const long long n_blocks = (a.Lq + BM - 1ll) / BM * (a.Hq / a.Hkv), heads = static_cast<long long>(a.Hkv) * a.B;
   const Plan p = plan_of<D, BF16, GEN>(a, device);
@@ -980,20 +1106,25 @@ cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
   if (n_items > 0x7fffffffll) return cudaErrorInvalidValue;
   const int sms = sm_count(device);
   const int grid = p.cluster > 1 ? static_cast<int>(n_items) * p.cluster : static_cast<int>(n_items < sms ? n_items : sms);
-  if (p.cluster == 1 && n_items > grid) {
+  const bool counter = p.cluster == 1 && n_items > grid;
+  if (GEN == 2 && is_padding_mask(a.mask, a.causal)) {
+    int* lens = a.sched + 1;
+    cudaError_t e = launch_early(lens_kernel, dim3(a.B), dim3(256), 0, stream, 1, a, a.sched, lens, lens + a.B);
+    if (e != cudaSuccess) return e;
+    a.kv_lens = lens, a.mask_pure = lens + a.B;
+  } else if (counter) {
     // the counter that hands out what comes after the CTAs' first items must start at zero for every launch
     cudaError_t e = launch_zero_word(a.sched, stream);
     if (e != cudaSuccess) return e;
-  } else {
-    a.sched = nullptr;
   }
+  if (!counter) a.sched = nullptr;
   return p.keys ? launch_k<D, BF16, GEN, true>(a, dtype, grid, p.cluster, stream)
                 : launch_k<D, BF16, GEN, false>(a, dtype, grid, 1, stream);
 }
 
 }  // namespace
 
-template <bool GEN>
+template <int GEN>
 cudaError_t launch_g(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream) {
   const bool bf = dtype == TT_ATTN_BF16;
   if (D == 128)
@@ -1005,8 +1136,10 @@ cudaError_t launch_g(int dtype, int D, const FwdArgs& a, int device, cudaStream_
 
 cudaError_t launch_fwd_tc(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream) {
   // the general variant only where it is needed: the fast one carries none of its code
-  const bool general = a.mask.ptr != nullptr || a.causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT;
-  return general ? launch_g<true>(dtype, D, a, device, stream) : launch_g<false>(dtype, D, a, device, stream);
+  const bool general = a.causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT;
+  return a.mask.ptr ? launch_g<2>(dtype, D, a, device, stream)
+         : general  ? launch_g<1>(dtype, D, a, device, stream)
+                    : launch_g<0>(dtype, D, a, device, stream);
 }
 
 }  // namespace ttattn
