@@ -1,0 +1,47 @@
+"""GPU: the fp32 forward where the key tiles of a query tile are divided among the CTAs of a cluster (few query tiles), against
+the CPU oracle: 2, 4 and 8 shares, shares without key tiles, sequences without keys, masks, ragged ends.
+Tolerance: that of test_fwd_gpu.py for fp32."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import rel_err
+from gpu_util import TOL_REL_FP32, make, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens,mask", [
+    (1, 2, 1, 70, 256, False, None, False),             # 4 key tiles in 2 shares
+    (1, 2, 2, 64, 1030, False, None, False),            # 17 in 8
+    (2, 3, 3, 500, 500, True, None, False),             # 1 .. 8 tiles in 4 shares: early query tiles leave some empty
+    (3, 2, 1, 100, 700, "bottom-right", (700, 30, 0), False),
+    (2, 2, 1, 65, 600, False, (600, 1), True),
+    (1, 1, 1, 1, 65, False, None, False),               # not divided
+])
+def test_divided_keys_fp32(oracle, D, B, Hq, Hkv, L, S, causal, lens, mask):
+    from tinytorch_b200 import op
+    q, qn = make((B, Hq, L, D), torch.float32, 61)
+    k, kn = make((B, Hkv, S, D), torch.float32, 62)
+    v, vn = make((B, Hkv, S, D), torch.float32, 63)
+    ln = np.array(lens if lens else (S,) * B, dtype=np.int32)
+    j, i = np.arange(S)[None, None, None, :], np.arange(L)[None, None, :, None]
+    seen = j < ln[:, None, None, None]
+    if causal:
+        seen = seen & (j <= i + (ln[:, None, None, None] - L if causal == "bottom-right" else 0))
+    seen = np.broadcast_to(seen, (B, 1, L, S)).copy()
+    t = None
+    if mask:
+        m = np.random.default_rng(64).random((B, 1, L, S)) < 0.5
+        t = torch.from_numpy(m).cuda()
+        seen &= m
+    o, lse = op.sdpAttentionFwd(q, k, v, isCausal=causal, kvLens=torch.from_numpy(ln).cuda() if lens else None, attnMask=t)
+    torch.cuda.synchronize()
+    some = np.broadcast_to(seen.any(-1), (B, Hq, L))  # rows that see a key
+    bias = np.where(seen, 0.0, -1e30).astype(np.float32)
+    want_o, want_l = oracle.fwd(qn, kn, vn, bias=bias)
+    got_o, got_l = to_np(o), to_np(lse)
+    assert rel_err(got_o[some], want_o[some]) <= TOL_REL_FP32
+    assert np.abs(got_l[some] - want_l[some]).max() <= 1e-4
+    assert (got_o[~some] == 0).all() and np.isneginf(got_l[~some]).all()

@@ -12,6 +12,13 @@
 // (simt_tile.cuh); the next K tile is copied in under the P V product and the next V tile under Q K^T; 3 CTAs of
 // D = 64 and 2 of D = 128 share an SM.  B4 H16 S2048 D64 causal: 1587 -> 958 us (21.7 -> 35.9 TFLOP/s) against scalar
 // shared-memory loads (eight per sixteen FMAs); ncu: FMA pipe 58 % busy, 2.7 warps per scheduler, the rest latency.
+//
+// Few query tiles leave most SMs idle for the time of the longest walk over the keys, 4 us (D = 64) or 8 us per key tile.
+// The key tiles are then divided among the CTAs of a cluster (SPLIT); their unnormalised O, maxima and sums meet in
+// distributed shared memory and every CTA writes a share of the rows.  3 heads x 890 D128 causal: 116 -> 44 us; 2 x 3
+// heads x 2221 D64 causal: 295 -> 156.
+#include <algorithm>
+
 #include "simt_tile.cuh"
 
 namespace ttattn {
@@ -23,8 +30,10 @@ constexpr int kThreads = 128, TY = kThreads / 16, R = TS / TY;
 template <int D>
 constexpr int kSmemBytes = (3 * kTileFloats<D> + kScoreFloats) * static_cast<int>(sizeof(float));
 
-template <int D, bool MASK>
-__global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_kernel(const FwdArgs a) {
+template <int D, bool MASK, bool SPLIT>
+__global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_kernel(const FwdArgs a, int cluster) {
+  ptx::grid_dep_launch();
+  ptx::grid_dep_wait();  // launched early: everything below reads or writes global memory
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
   float* Ks = Qs + kTileFloats<D>;
@@ -32,7 +41,8 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
   float* Ps = Vs + kTileFloats<D>;
 
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int mt = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // under a causal mask the last is longest
+  const int n_mt = SPLIT ? gridDim.x / cluster : gridDim.x, rank = SPLIT ? blockIdx.x % cluster : 0;
+  const int mt = n_mt - 1 - static_cast<int>(SPLIT ? blockIdx.x / cluster : blockIdx.x);  // under a causal mask the last is longest
   const int h = blockIdx.y, b = blockIdx.z, hk = h / (a.Hq / a.Hkv);
   const int row0 = mt * TS;
   const float* q = reinterpret_cast<const float*>(a.q) + b * a.qs.b + h * a.qs.h;
@@ -47,15 +57,16 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
   const int shift = causal_shift(a.causal, kv_len, a.Lq);
   int kv_end = kv_len;
   if (a.causal && row0 + TS + shift < kv_end) kv_end = row0 + TS + shift > 0 ? row0 + TS + shift : 0;
-  const int n_tiles = (kv_end + TS - 1) / TS;
+  const int all_tiles = (kv_end + TS - 1) / TS;
+  const int t0 = SPLIT ? all_tiles * rank / cluster : 0, n_tiles = SPLIT ? all_tiles * (rank + 1) / cluster : all_tiles;
   const float c = a.scale * kLog2e;
   const int64_t mask_base = b * a.mask.sb + h * a.mask.sh;
 
-  if (n_tiles > 0) {
+  if (n_tiles > t0) {
     load_tile<D, kThreads>(Qs, q, a.qs.s, row0, a.Lq, tid);
-    load_tile<D, kThreads>(Ks, k, a.ks.s, 0, kv_len, tid);
+    load_tile<D, kThreads>(Ks, k, a.ks.s, t0 * TS, kv_len, tid);
     copies_commit();
-    load_tile<D, kThreads>(Vs, v, a.vs.s, 0, kv_len, tid);
+    load_tile<D, kThreads>(Vs, v, a.vs.s, t0 * TS, kv_len, tid);
     copies_commit();
   }
 
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
     for (int j = 0; j < D / 32; ++j) acc[i][j] = make_float2(0.f, 0.f);
   }
 
-  for (int t = 0; t < n_tiles; ++t) {
+  for (int t = t0; t < n_tiles; ++t) {
     const int col0 = t * TS;
     copies_wait<1>();  // Q and K of this tile; V may still be on its way
     __syncthreads();
@@ -128,31 +139,104 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
   }
 
   float* o = reinterpret_cast<float*>(a.o) + b * a.os.b + h * a.os.h;
+  float* lse = a.lse ? a.lse + (static_cast<int64_t>(b) * a.Hq + h) * a.Lq : nullptr;
+  if constexpr (SPLIT) {
+    // this CTA's share, where the others find it: O over the Q tile, (maximum, sum) over the scores
+    constexpr int kMost = 8;  // CTAs per cluster
+    float* share = Ps;
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    float ls = l[i];
+    for (int i = 0; i < R; ++i) {
+      float ls = l[i];
 #pragma unroll
-    for (int of = 8; of >= 1; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
-    const int row = row0 + ty + TY * i;
-    if (row >= a.Lq) continue;
-    const float inv = ls > 0.f ? 1.f / ls : 0.f;
+      for (int of = 8; of >= 1; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
+      const int r = ty + TY * i;
 #pragma unroll
-    for (int j = 0; j < D / 64; ++j)
-      *reinterpret_cast<float4*>(o + static_cast<int64_t>(row) * a.os.s + tx * 4 + j * 64) =
-          make_float4(acc[i][2 * j].x * inv, acc[i][2 * j].y * inv, acc[i][2 * j + 1].x * inv, acc[i][2 * j + 1].y * inv);
-    if (a.lse && tx == 0)
-      a.lse[(static_cast<int64_t>(b) * a.Hq + h) * a.Lq + row] = ls > 0.f ? (m[i] + log2f(ls)) * kLn2 : -INFINITY;
+      for (int j = 0; j < D / 64; ++j)
+        *reinterpret_cast<float4*>(Qs + r * D + tx * 4 + j * 64) = make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
+      if (tx == 0) share[2 * r] = m[i], share[2 * r + 1] = ls;
+    }
+    ptx::cluster_sync();
+    const int rows = TS / cluster, first = rank * rows;
+    float* weight = Ps + 2 * TS;  // [row][CTA]
+    if (tid < rows) {
+      float2 st[kMost];
+      float mx = -INFINITY, ls = 0.f;
+#pragma unroll
+      for (int r = 0; r < kMost; ++r)
+        if (r < cluster) {
+          st[r] = ptx::ld_cluster_f2(ptx::map_rank(ptx::smem_u32(share + 2 * (first + tid)), r));
+          mx = fmaxf(mx, st[r].x);
+        }
+      const float ref = mx == -INFINITY ? 0.f : mx;
+#pragma unroll
+      for (int r = 0; r < kMost; ++r)
+        if (r < cluster) ls += st[r].y * exp2f(st[r].x - ref);
+      const float inv = ls > 0.f ? 1.f / ls : 0.f;
+#pragma unroll
+      for (int r = 0; r < kMost; ++r)
+        if (r < cluster) weight[tid * kMost + r] = exp2f(st[r].x - ref) * inv;
+      if (lse && row0 + first + tid < a.Lq) lse[row0 + first + tid] = ls > 0.f ? (mx + log2f(ls)) * kLn2 : -INFINITY;
+    }
+    __syncthreads();
+    for (int e = tid; e < rows * (D / 4); e += kThreads) {
+      const int r = e / (D / 4), d = e % (D / 4) * 4;
+      if (row0 + first + r >= a.Lq) break;
+      float4 x[kMost], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int p = 0; p < kMost; ++p)
+        if (p < cluster) x[p] = ptx::ld_cluster_f4(ptx::map_rank(ptx::smem_u32(Qs + (first + r) * D + d), p));
+#pragma unroll
+      for (int p = 0; p < kMost; ++p)
+        if (p < cluster) {
+          const float w = weight[r * kMost + p];
+          sum.x = fmaf(x[p].x, w, sum.x), sum.y = fmaf(x[p].y, w, sum.y), sum.z = fmaf(x[p].z, w, sum.z), sum.w = fmaf(x[p].w, w, sum.w);
+        }
+      *reinterpret_cast<float4*>(o + static_cast<int64_t>(row0 + first + r) * a.os.s + d) = sum;
+    }
+    ptx::cluster_sync();  // no CTA leaves while another still reads its share
+  } else {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float ls = l[i];
+#pragma unroll
+      for (int of = 8; of >= 1; of >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, of);
+      const int row = row0 + ty + TY * i;
+      if (row >= a.Lq) continue;
+      const float inv = ls > 0.f ? 1.f / ls : 0.f;
+#pragma unroll
+      for (int j = 0; j < D / 64; ++j)
+        *reinterpret_cast<float4*>(o + static_cast<int64_t>(row) * a.os.s + tx * 4 + j * 64) =
+            make_float4(acc[i][2 * j].x * inv, acc[i][2 * j].y * inv, acc[i][2 * j + 1].x * inv, acc[i][2 * j + 1].y * inv);
+      if (lse && tx == 0) lse[row] = ls > 0.f ? (m[i] + log2f(ls)) * kLn2 : -INFINITY;
+    }
   }
+}
+
+// CTAs per cluster, by how many query tiles there are (under a causal mask half: their walks are half as long on average),
+// and only while the longest walk gets shorter.  From a sweep of 24 shapes with 1, 2, 4 and 8 (within 5 % of the best of them for each).
+// D = 64, where three CTAs share an SM, is divided further than D = 128, where one already takes most of what the SM gives.
+// Measured, us, undivided -> chosen: D64, 64 rows on 4000 keys, 2 heads 330 -> 54; 1024, 4 heads 88 -> 52; causal 2048, 8
+// heads 304 -> 164; 128, 2 x 4 heads 15.1 -> 11.6.  D128, 512, 8 heads 69 -> 40; causal 2048, 8 heads 382 -> 320.  One step
+// further in these: -, 50, 174, 11.6, 45, 336.
+int split_of(const FwdArgs& a, int D) {
+  const int n_mt = (a.Lq + TS - 1) / TS, tiles = (a.Skv + TS - 1) / TS;
+  const bool triangle = a.causal == TT_ATTN_CAUSAL_TOP_LEFT;
+  const int longest = triangle ? std::min(tiles, n_mt) : tiles;
+  const long long ctas = static_cast<long long>(n_mt) * a.Hq * a.B, full = triangle ? (ctas + 1) / 2 : ctas;
+  const int at_most[3] = {D == 64 ? 256 : 128, D == 64 ? 128 : 32, D == 64 ? 18 : 16};  // for 2, 4, 8 CTAs
+  int cluster = 1;
+  auto walk = [&](int c) { return (longest + c - 1) / c; };
+  for (int i = 0; i < 3 && full <= at_most[i] && walk(2 * cluster) < walk(cluster); ++i) cluster *= 2;
+  return cluster;
 }
 
 template <int D, bool MASK>
 cudaError_t launch_t(const FwdArgs& a, cudaStream_t stream) {
-  auto kern = fwd_simt_kernel<D, MASK>;
+  const int cluster = split_of(a, D);
+  auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true> : fwd_simt_kernel<D, MASK, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<D>);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.Lq + TS - 1) / TS, a.Hq, a.B);
-  kern<<<grid, kThreads, kSmemBytes<D>, stream>>>(a);
-  return cudaGetLastError();
+  return launch_early(kern, dim3((a.Lq + TS - 1) / TS * cluster, a.Hq, a.B), dim3(kThreads), kSmemBytes<D>, stream, cluster, a, cluster);
 }
 
 }  // namespace
