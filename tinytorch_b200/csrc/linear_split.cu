@@ -50,7 +50,7 @@ struct SplitArgs {
   int64_t ldy;
   int M, N, K;
   int mt;      // rows of x per tile: the N dimension of the MMA, a multiple of 16 (X_MN: of 64)
-  int tiles_m;
+  int tiles_m, tiles_n;
   int stages, cluster;
   uint32_t tmem_cols;
   int32_t* status;
@@ -100,7 +100,11 @@ __global__ void __launch_bounds__(kThreads)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = a.cluster > 1 ? ptx::cluster_rank() : 0;
   const int tile = blockIdx.x / a.cluster;
-  const int m0 = (tile % a.tiles_m) * a.mt, n0 = (tile / a.tiles_m) * BW;
+  // Neighbouring CTAs share the larger operand, which then comes from HBM once (M = 13787, N = 264, K = 9848 with the rows of x
+  // fastest: every column tile read x again, 169 us; TIME with the columns fastest).
+  const bool columns = a.M > a.N;
+  const int tm = columns ? tile / a.tiles_n : tile % a.tiles_m, tn = columns ? tile % a.tiles_n : tile / a.tiles_m;
+  const int m0 = tm * a.mt, n0 = tn * BW;
   // this CTA's share of the contraction
   const int n_kb = (a.K + BK - 1) / BK, per = (n_kb + a.cluster - 1) / a.cluster;
   const int kb0 = static_cast<int>(rank) * per;
@@ -262,7 +266,7 @@ struct Plan {
 // 1024 to 2000 x 1024 x 1024 and 64 x 4096 x 28672 (B200; within 1.5 us of the measured time for the plans near the
 // best, and the plan it picks within 8 % of the best of the sweep):
 //   2.8 us     launch, set-up, first tile, cluster barriers, last store
-//   + the slower of  the weight from HBM (6.0 TB/s, or less where the stages in flight do not cover 1.7 us)  and
+//   + the slower of  weight and x from HBM (6.0 TB/s, or less where the stages in flight do not cover 1.7 us)  and
 //     an SM's share of the tiles through its L2 port (135 B/ns)
 //   + 10 ns per row of x: the partial tile through shared memory;  + 12.5 ns more where the cluster sums it
 //   + 2.5 us and the partial tile again for every further wave of CTAs (half where CTAs that share an SM overlap)
@@ -277,7 +281,7 @@ Plan plan_split(int M, int N, int K, bool x_t, int device) {
   Plan best{};
   best.us = 1e30;
   const int n_kb = (K + BK - 1) / BK, tiles_n = (N + BW - 1) / BW;
-  const double w_bytes = 2.0 * N * K;
+  const double bytes = 2.0 * K * (static_cast<double>(N) + M);
   int last_mt = 0;
   const int unit = x_t ? 64 : 16;
   for (int tm = (M + 255) / 256; tm <= (M + unit - 1) / unit; tm += tm < 16 ? 1 : tm / 8) {
@@ -302,7 +306,7 @@ Plan plan_split(int M, int N, int K, bool x_t, int device) {
       const long long slots = cluster_slots(device, p.cluster, per_sm), waves = (ctas + slots - 1) / slots;
       const double sm_us = static_cast<double>(waves) * per_sm * ((n_kb + p.cluster - 1) / p.cluster) * stage / 135e3;
       const double in_flight = static_cast<double>(ctas < slots ? ctas : slots) * p.stages * kWBytes / 1.7;
-      const double hbm_us = w_bytes / (in_flight < 6.0e6 ? in_flight : 6.0e6);
+      const double hbm_us = bytes / (in_flight < 6.0e6 ? in_flight : 6.0e6);
       p.us = 2.8 + (sm_us > hbm_us ? sm_us : hbm_us) + 0.010 * mt + (p.cluster > 1 ? 0.0125 * mt : 0.0) +
              static_cast<double>(waves - 1) * (2.5 + 0.010 * mt) * (per_sm == 1 ? 1.0 : 0.5);
       p.smem = p.stages * stage + static_cast<int>(sizeof(SmemCtl));
@@ -323,7 +327,7 @@ cudaError_t launch_t(const LinearCall& c, const Plan& p) {
     return cudaErrorInvalidValue;
   uint32_t cols = 32;
   while (static_cast<int>(cols) < p.mt) cols *= 2;
-  const SplitArgs a{c.bias, c.y, c.ldy, c.M, c.N, c.K, p.mt, p.tiles_m, p.stages, p.cluster, cols, c.status};
+  const SplitArgs a{c.bias, c.y, c.ldy, c.M, c.N, c.K, p.mt, p.tiles_m, p.tiles / p.tiles_m, p.stages, p.cluster, cols, c.status};
   return launch_early(kern, dim3(static_cast<unsigned>(p.tiles) * p.cluster), dim3(kThreads), p.smem, c.stream, p.cluster,
                       tw, tx, a);
 }
