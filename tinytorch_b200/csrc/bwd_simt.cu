@@ -18,7 +18,10 @@
 // Bound by the FMA pipes: seven products where five would do if dQ left through atomics, whose order is not
 // deterministic.  16 x TY threads per tile (simt_tile.cuh): 8 rows per thread for D = 64; 4 for D = 128, where 8
 // would need more accumulators than there are registers.  B4 H16 S2048 D64 causal: 4986 -> 2807 us (24 -> 43 TFLOP/s),
-// B2 H4 S128 D64: 63 -> 23 us; ncu: FMA pipe 63 % busy.
+// B2 H4 S128 D64: 63 -> 23 us; ncu: FMA pipe 63 % busy.  Where tiles are few, or a key tile's walk is long because several
+// query heads share it, the CTAs of a cluster share a walk (SPLIT, split_of) and add their accumulators in rank order.
+#include <algorithm>
+
 #include "simt_tile.cuh"
 
 namespace ttattn {
@@ -86,15 +89,7 @@ __device__ __forceinline__ void tile_p_ds(const BwdArgs& a, const float* Qs, con
   constexpr int TY = Cfg<D>::TY, R = Cfg<D>::R;
   const float c = a.scale * kLog2e;
   float bias[MASK ? R : 1][4];
-  if constexpr (MASK) {
-#pragma unroll
-    for (int i = 0; i < R; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int row = row0 + ty + TY * i, col = col0 + tx + 16 * j;
-        bias[i][j] = row < a.Lq && col < kv_len ? mask_bias2<float>(a.mask, mask_base + row * a.mask.sl + col) : 0.f;
-      }
-  }
+  if constexpr (MASK) load_mask<TY>(a.mask, mask_base, row0 + ty, a.Lq, col0 + tx, kv_len, bias);
   float p[R][4], dp[R][4];
   product_nt<D, TY>(Qs, Ks, ty, tx, p);
   const bool edge = row0 + TS > a.Lq || col0 + TS > kv_len || (a.causal && col0 + TS - 1 > row0 + shift);
@@ -132,6 +127,37 @@ __device__ __forceinline__ void load_vectors(const BwdArgs& a, float* lse2_s, fl
   }
 }
 
+// SPLIT: the sum of the cluster's accumulators, in rank order; each CTA stores a share of the rows.  `share`: this CTA's own
+// accumulator in shared memory, [TS][D], where the others find it (complete before the cluster barrier ahead of this).
+template <int D>
+__device__ __forceinline__ void keep_rows(float* share, int step, int first, int tx, const float2 (&acc)[Cfg<D>::R][D / 32]) {
+#pragma unroll
+  for (int i = 0; i < Cfg<D>::R; ++i)
+#pragma unroll
+    for (int c = 0; c < D / 64; ++c)
+      *reinterpret_cast<float4*>(share + (first + step * i) * D + tx * 4 + c * 64) =
+          make_float4(acc[i][2 * c].x, acc[i][2 * c].y, acc[i][2 * c + 1].x, acc[i][2 * c + 1].y);
+}
+template <int D>
+__device__ __forceinline__ void sum_rows(float* out, const Str3& st, int row0, int n_rows, const float* share, int rank, int cluster,
+                                         int tid) {
+  constexpr int kMost = 8;
+  const int rows = TS / cluster, first = rank * rows;
+  for (int e = tid; e < rows * (D / 4); e += Cfg<D>::NT) {
+    const int r = first + e / (D / 4), d = e % (D / 4) * 4;
+    if (row0 + r >= n_rows) break;
+    const uint32_t at = ptx::smem_u32(share + r * D + d);
+    float4 x[kMost], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < kMost; ++p)
+      if (p < cluster) x[p] = ptx::ld_cluster_f4(ptx::map_rank(at, p));
+#pragma unroll
+    for (int p = 0; p < kMost; ++p)
+      if (p < cluster) sum.x += x[p].x, sum.y += x[p].y, sum.z += x[p].z, sum.w += x[p].w;
+    *reinterpret_cast<float4*>(out + static_cast<int64_t>(row0 + r) * st.s + d) = sum;
+  }
+}
+
 template <int D>
 __device__ __forceinline__ void store_rows(float* out, const Str3& st, int row0, int step, int n_rows, int first, int tx,
                                            const float2 (&acc)[Cfg<D>::R][D / 32]) {
@@ -146,8 +172,9 @@ __device__ __forceinline__ void store_rows(float* out, const Str3& st, int row0,
   }
 }
 
-template <int D, bool MASK>
-__global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(const BwdArgs a, int key_tiles, int key_ctas) {
+template <int D, bool MASK, bool SPLIT>
+__global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(const BwdArgs a, int key_tiles, int key_ctas,
+                                                                               int cluster) {
   using C = Cfg<D>;
   constexpr int TY = C::TY, R = C::R, NT = C::NT;
   extern __shared__ __align__(16) float sm[];
@@ -160,7 +187,9 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
   float* lse2_s = dSs + kScoreFloats;
   float* delta_s = lse2_s + TS;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const bool keys = static_cast<int>(blockIdx.x) < key_ctas;
+  // SPLIT: the CTAs of a cluster share the walk of one tile
+  const int item = SPLIT ? blockIdx.x / cluster : blockIdx.x, rank = SPLIT ? blockIdx.x % cluster : 0;
+  const bool keys = item < key_ctas;
   const int group = a.Hq / a.Hkv;
 
   float2 acc0[R][D / 32], acc1[R][D / 32];
@@ -177,7 +206,7 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
 
   if (keys) {
     // ------------------------------------------------------------- dK, dV of a key tile --
-    const int nt = blockIdx.x % key_tiles, bh = blockIdx.x / key_tiles;  // (the first key tile is seen by most queries)
+    const int nt = item % key_tiles, bh = item / key_tiles;  // (the first key tile is seen by most queries)
     const int hk = bh % a.Hkv, b = bh / a.Hkv, col0 = nt * TS;
     int kv_len = a.Skv;
     if (a.kv_lens) {
@@ -190,40 +219,53 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
     load_tile<D, NT>(Ks, kb + b * a.ks.b + hk * a.ks.h, a.ks.s, col0, a.Skv, tid);
     load_tile<D, NT>(Vs, vb + b * a.vs.b + hk * a.vs.h, a.vs.s, col0, a.Skv, tid);
     bool first = true;
-    if (col0 < kv_len) {
-      for (int g = 0; g < group; ++g) {
-        const int h = hk * group + g;
-        const float* q = qb + b * a.qs.b + h * a.qs.h;
-        const float* dO = gb + b * a.dos.b + h * a.dos.h;
-        const int64_t base = (static_cast<int64_t>(b) * a.Hq + h) * a.Lq;
-        for (int qt = qt0; qt < q_tiles; ++qt) {
-          const int row0 = qt * TS;
-          __syncthreads();  // the tiles of the step before have been read
-          load_tile<D, NT>(Qs, q, a.qs.s, row0, a.Lq, tid);
-          load_tile<D, NT>(dOs, dO, a.dos.s, row0, a.Lq, tid);
-          copies_commit();
-          if (first) ptx::grid_dep_wait();  // launched early behind the delta pre-pass
-          first = false;
-          load_vectors(a, lse2_s, delta_s, base, row0, tid);
-          copies_wait<0>();
-          __syncthreads();
-          tile_p_ds<D, MASK, true>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift,
-                                   b * a.mask.sb + h * a.mask.sh, ty, tx);
-          __syncthreads();
-          product_tn<D, TY>(Ps, dOs, ty, tx, acc0);
-          product_tn<D, TY>(dSs, Qs, ty, tx, acc1);
-        }
+    // the walk: query tiles qt0.. of the group's heads, one after the other; this CTA's share of it
+    const int per_head = col0 < kv_len && qt0 < q_tiles ? q_tiles - qt0 : 0, steps = per_head * group;
+    int n = SPLIT ? steps * rank / cluster : 0;
+    const int n_end = SPLIT ? steps * (rank + 1) / cluster : steps;
+    while (n < n_end) {
+      const int g = n / per_head, h = hk * group + g, end = min(n_end, (g + 1) * per_head);
+      const float* q = qb + b * a.qs.b + h * a.qs.h;
+      const float* dO = gb + b * a.dos.b + h * a.dos.h;
+      const int64_t base = (static_cast<int64_t>(b) * a.Hq + h) * a.Lq;
+      for (; n < end; ++n) {
+        const int row0 = (qt0 + n - g * per_head) * TS;
+        __syncthreads();  // the tiles of the step before have been read
+        load_tile<D, NT>(Qs, q, a.qs.s, row0, a.Lq, tid);
+        load_tile<D, NT>(dOs, dO, a.dos.s, row0, a.Lq, tid);
+        copies_commit();
+        if (first) ptx::grid_dep_wait();  // launched early behind the delta pre-pass
+        first = false;
+        load_vectors(a, lse2_s, delta_s, base, row0, tid);
+        copies_wait<0>();
+        __syncthreads();
+        tile_p_ds<D, MASK, true>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift,
+                                 b * a.mask.sb + h * a.mask.sh, ty, tx);
+        __syncthreads();
+        product_tn<D, TY>(Ps, dOs, ty, tx, acc0);
+        product_tn<D, TY>(dSs, Qs, ty, tx, acc1);
       }
     }
+    copies_commit();
     copies_wait<0>();
     if (first) ptx::grid_dep_wait();
-    if (a.dv)
-      store_rows<D>(reinterpret_cast<float*>(a.dv) + b * a.dvs.b + hk * a.dvs.h, a.dvs, col0, 1, a.Skv, ty * R, tx, acc0);
-    if (a.dk)
-      store_rows<D>(reinterpret_cast<float*>(a.dk) + b * a.dks.b + hk * a.dks.h, a.dks, col0, 1, a.Skv, ty * R, tx, acc1);
+    if constexpr (SPLIT) {
+      __syncthreads();  // the tiles have been read
+      keep_rows<D>(Qs, 1, ty * R, tx, acc0);
+      keep_rows<D>(Ks, 1, ty * R, tx, acc1);
+      ptx::cluster_sync();
+      if (a.dv) sum_rows<D>(reinterpret_cast<float*>(a.dv) + b * a.dvs.b + hk * a.dvs.h, a.dvs, col0, a.Skv, Qs, rank, cluster, tid);
+      if (a.dk) sum_rows<D>(reinterpret_cast<float*>(a.dk) + b * a.dks.b + hk * a.dks.h, a.dks, col0, a.Skv, Ks, rank, cluster, tid);
+      ptx::cluster_sync();  // no CTA leaves while another still reads its share
+    } else {
+      if (a.dv)
+        store_rows<D>(reinterpret_cast<float*>(a.dv) + b * a.dvs.b + hk * a.dvs.h, a.dvs, col0, 1, a.Skv, ty * R, tx, acc0);
+      if (a.dk)
+        store_rows<D>(reinterpret_cast<float*>(a.dk) + b * a.dks.b + hk * a.dks.h, a.dks, col0, 1, a.Skv, ty * R, tx, acc1);
+    }
   } else {
     // ----------------------------------------------------------------- dQ of a query tile --
-    const int x = blockIdx.x - key_ctas;
+    const int x = item - key_ctas;
     const int mt = q_tiles - 1 - x % q_tiles, bh = x / q_tiles;  // (under a causal mask the last tile is longest)
     const int h = bh % a.Hq, b = bh / a.Hq, hk = h / group, row0 = mt * TS;
     int kv_len = a.Skv;
@@ -234,19 +276,20 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
     const int shift = causal_shift(a.causal, kv_len, a.Lq);
     int kv_end = kv_len;
     if (a.causal && row0 + TS + shift < kv_end) kv_end = row0 + TS + shift > 0 ? row0 + TS + shift : 0;
-    const int n_tiles = (kv_end + TS - 1) / TS;
+    const int all_tiles = (kv_end + TS - 1) / TS;
+    const int t0 = SPLIT ? all_tiles * rank / cluster : 0, n_tiles = SPLIT ? all_tiles * (rank + 1) / cluster : all_tiles;
     const float* k = kb + b * a.ks.b + hk * a.ks.h;
     const float* v = vb + b * a.vs.b + hk * a.vs.h;
     load_tile<D, NT>(Qs, qb + b * a.qs.b + h * a.qs.h, a.qs.s, row0, a.Lq, tid);
     load_tile<D, NT>(dOs, gb + b * a.dos.b + h * a.dos.h, a.dos.s, row0, a.Lq, tid);
-    if (n_tiles > 0) {
-      load_tile<D, NT>(Ks, k, a.ks.s, 0, a.Skv, tid);
-      load_tile<D, NT>(Vs, v, a.vs.s, 0, a.Skv, tid);
+    if (n_tiles > t0) {
+      load_tile<D, NT>(Ks, k, a.ks.s, t0 * TS, a.Skv, tid);
+      load_tile<D, NT>(Vs, v, a.vs.s, t0 * TS, a.Skv, tid);
     }
     copies_commit();
     ptx::grid_dep_wait();  // launched early behind the delta pre-pass
     load_vectors(a, lse2_s, delta_s, (static_cast<int64_t>(b) * a.Hq + h) * a.Lq, row0, tid);
-    for (int t = 0; t < n_tiles; ++t) {
+    for (int t = t0; t < n_tiles; ++t) {
       const int col0 = t * TS;
       copies_wait<0>();
       __syncthreads();
@@ -260,7 +303,16 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
       copies_commit();
     }
     copies_wait<0>();
-    store_rows<D>(reinterpret_cast<float*>(a.dq) + b * a.dqs.b + h * a.dqs.h, a.dqs, row0, TY, a.Lq, ty, tx, acc0);
+    float* dq = reinterpret_cast<float*>(a.dq) + b * a.dqs.b + h * a.dqs.h;
+    if constexpr (SPLIT) {
+      __syncthreads();
+      keep_rows<D>(Ks, TY, ty, tx, acc0);
+      ptx::cluster_sync();
+      sum_rows<D>(dq, a.dqs, row0, a.Lq, Ks, rank, cluster, tid);
+      ptx::cluster_sync();
+    } else {
+      store_rows<D>(dq, a.dqs, row0, TY, a.Lq, ty, tx, acc0);
+    }
   }
 }
 
@@ -272,18 +324,42 @@ cudaError_t launch_delta_t(const BwdArgs& a, cudaStream_t stream) {
                       stream, 1, a);
 }
 
+// CTAs per cluster: with few tiles the longest walk sets the time, with many the SMs' throughput, and every CTA has its fixed
+// part.  The cheapest of 1, 2, 4 and 8 by a model fitted to 22 shapes (what it picks is on average within 3 % of the best):
+// a step 12.6 us (D = 64) or 14.7 in a CTA alone, 5 or 13.8 of an SM's throughput (a query tile's three products count three
+// quarters), 6 or 14.6 us of an SM per CTA.  Measured, us, undivided -> chosen: causal, 2 query heads on one, 3000, D64 1224
+// -> 246; 8/2 heads x 700, D128 634 -> 165; 4 heads x 1500, D64 327 -> 152; 2 x 4 heads x 128, D64 20.5 -> 15.2; undivided
+// 4 x 16 heads x 512, D64 237 (two shares: 250).
+int split_of(const BwdArgs& a, int D) {
+  const double step = D == 64 ? 12.6 : 14.7, busy = D == 64 ? 5.0 : 13.8, fixed = D == 64 ? 6.0 : 14.6, tail = D == 64 ? 0.62 : 0.23;
+  const double kt = (a.Skv + TS - 1) / TS, qt = (a.Lq + TS - 1) / TS, heads = static_cast<double>(a.B) * a.Hq;
+  const int longest = a.Hq / a.Hkv * static_cast<int>(qt);
+  const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.5 * (kt + 1) / kt : 1.0;  // of all (query, key) tiles
+  const double work = 1.75 * heads * kt * qt * seen * busy, ctas = heads * qt + static_cast<double>(a.B) * a.Hkv * kt;
+  int best = 1;
+  double best_us = 1e30;
+  for (int c = 1, lg = 0; c <= 8; c *= 2, ++lg) {
+    const double walk = (longest + c - 1) / c * step;
+    // (clusters of 8 do not fill every GPC)
+    const double us = std::max(walk + 1.5 * lg, (work + ctas * c * fixed) / 148 * (c == 8 ? 1.1 : 1.0) + tail * walk);
+    if (us < best_us) best = c, best_us = us;
+  }
+  return best;
+}
+
 template <int D, bool MASK>
 cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
   cudaError_t e = launch_delta_t<float, D>(a, stream);
   if (e != cudaSuccess) return e;
-  auto kern = bwd_simt_kernel<D, MASK>;
+  const int cluster = split_of(a, D);
+  auto kern = cluster > 1 ? bwd_simt_kernel<D, MASK, true> : bwd_simt_kernel<D, MASK, false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes);
   if (e != cudaSuccess) return e;
   const long long key_tiles = (a.Skv + TS - 1) / TS, q_tiles = (a.Lq + TS - 1) / TS;
   const long long key_ctas = a.dk || a.dv ? key_tiles * a.Hkv * a.B : 0, q_ctas = a.dq ? q_tiles * a.Hq * a.B : 0;
-  if (key_ctas + q_ctas > 0x7fffffffll) return cudaErrorInvalidValue;
-  return launch_early(kern, dim3(static_cast<unsigned>(key_ctas + q_ctas)), dim3(Cfg<D>::NT), Cfg<D>::kSmemBytes, stream, 1,
-                      a, static_cast<int>(key_tiles), static_cast<int>(key_ctas));
+  if ((key_ctas + q_ctas) * cluster > 0x7fffffffll) return cudaErrorInvalidValue;
+  return launch_early(kern, dim3(static_cast<unsigned>((key_ctas + q_ctas) * cluster)), dim3(Cfg<D>::NT), Cfg<D>::kSmemBytes, stream,
+                      cluster, a, static_cast<int>(key_tiles), static_cast<int>(key_ctas), cluster);
 }
 
 }  // namespace

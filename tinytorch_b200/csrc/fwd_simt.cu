@@ -84,15 +84,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
     copies_wait<1>();  // Q and K of this tile; V may still be on its way
     __syncthreads();
     float bias[MASK ? R : 1][4];
-    if constexpr (MASK) {
-#pragma unroll
-      for (int i = 0; i < R; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int row = row0 + ty + TY * i, col = col0 + tx + 16 * j;
-          bias[i][j] = row < a.Lq && col < kv_len ? mask_bias2<float>(a.mask, mask_base + row * a.mask.sl + col) : 0.f;
-        }
-    }
+    if constexpr (MASK) load_mask<TY>(a.mask, mask_base, row0 + ty, a.Lq, col0 + tx, kv_len, bias);
     float s[R][4];
     product_nt<D, TY>(Qs, Ks, ty, tx, s);
     __syncthreads();  // K of this tile has been read

@@ -128,5 +128,20 @@ __device__ __forceinline__ void product_tn(const float* P, const float* X, int t
   }
 }
 
+// The mask elements (times log2 e) of this thread's scores: rows row, row + TY, .., columns col, col + 16, ..; 0 outside.
+template <int TY, int R>
+__device__ __forceinline__ void load_mask(const MaskArgs& m, int64_t base, int row, int n_rows, int col, int n_cols,
+                                          float (&bias)[R][4]) {
+  auto load = [&](auto* p, auto value) {  // (one loop per kind: nothing is decided per element)
+    p += base + row * m.sl + col;
+#pragma unroll
+    for (int i = 0; i < R; ++i, p += TY * m.sl)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bias[i][j] = row + TY * i < n_rows && col + 16 * j < n_cols ? value(p[16 * j]) : 0.f;
+  };
+  if (m.kind == TT_ATTN_MASK_BOOL) load(reinterpret_cast<const uint8_t*>(m.ptr), [](uint8_t x) { return x ? 0.f : -INFINITY; });
+  else load(reinterpret_cast<const float*>(m.ptr), [](float x) { return x * kLog2e; });
+}
+
 }  // namespace simt
 }  // namespace ttattn
