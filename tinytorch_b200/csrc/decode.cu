@@ -428,6 +428,14 @@ void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int
   DecodeArgs probe{};
   probe.Hq = Hq, probe.Hkv = Hkv;
   if (!decode_tc_applies(dtype, D, probe)) {
+    // a cache whose rows of K are at most 64 KB per head (less where several query heads multiply the work) is scanned in
+    // one piece: the second kernel costs more than the longer scan (bf16 D64, 3 x 8 heads x 469: 6.9 -> 4.3 us a call; D128,
+    // 4 heads x 500, which is over: 4.7 us of GPU time divided, 7.1 in one piece)
+    const int group = Hkv > 0 && Hq > 2 * Hkv ? Hq / Hkv / 2 : 1;
+    if (static_cast<long long>(capacity) * D * (dtype == TT_ATTN_F32 ? 4 : 2) * group <= 65536) {
+      *chunk = (capacity + 63) / 64 * 64, *nsplit = 1;
+      return;
+    }
     decode_plan(B, Hkv, capacity, nsplit, chunk);
     return;
   }
@@ -436,6 +444,9 @@ void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int
   while (ck > 512 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < want) ck >>= 1;
   while (ck > 128 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 74) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 127) / 128 * 128;
+  // three tiles in one piece take less than the second kernel (2 x 16/4 heads x 191, D64: 7.9 -> 6.0 us a call; append, 17 x 8/4
+  // heads x 135, D128: 11.6 -> 9.0; at 512 rows 8.9 -> 9.4)
+  if (capacity <= 384) ck = 384;
   *chunk = ck;
   *nsplit = capacity <= ck ? 1 : (capacity + ck - 1) / ck;
 }
