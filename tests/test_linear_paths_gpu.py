@@ -55,3 +55,23 @@ def test_strided_rows_and_repeat():
     y1, y2 = fused.linear(x, w), fused.linear(x, w)
     assert torch.equal(y1, y2)
     _check(y1, x.double(), w.double().t(), None, torch.bfloat16)
+
+
+@pytest.mark.parametrize("M,N", [
+    (2309, 4608),   # the lower half of the last row of tiles lies wholly beyond M
+    (2560, 4616),   # of the last column of tiles only the first block of 64 columns exists
+    (2560, 4744),   # ... the first two and a part of the third
+    (2309, 4744),
+])
+def test_blocks_beyond_the_edge_between_full_tiles(M, N):
+    """The persistent pairs with tiles of which some blocks store nothing, followed by tiles of which all do, and a
+    contraction so short that the next tile is complete before a store has left shared memory: every element, and the
+    same bits each time."""
+    from tinytorch_b200 import fused
+    g = torch.Generator("cuda").manual_seed(M + N)
+    for K in (8, 64):
+        x, w = (torch.randn(s, device="cuda", generator=g).bfloat16() for s in ((M, K), (N, K)))
+        y = fused.linear(x, w)
+        _check(y, x.double(), w.double().t(), None, torch.bfloat16)
+        for _ in range(20):
+            assert torch.equal(fused.linear(x, w), y)

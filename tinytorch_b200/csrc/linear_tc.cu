@@ -243,8 +243,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ptx::fence_proxy_async_smem();
         // (also: every thread has read the bias before the next tile's is written)
         ptx::named_barrier(1 + wg, kEpi);
-        if (r == 0 && ok && n0 + c * 64 < a.N && m0 < a.M) {
-          ptx::tma_store_4d(&tmY, stage, n0 + c * 64, m0, 0, 0);
+        if (r == 0) {
+          if (ok && n0 + c * 64 < a.N && m0 < a.M) ptx::tma_store_4d(&tmY, stage, n0 + c * 64, m0, 0, 0);
+          // also where nothing was stored (a block beyond M or N): the wait above counts groups, one per block
           ptx::bulk_commit();
         }
       }
