@@ -65,3 +65,20 @@ def test_padding_masks(oracle, dt, D, holes, L, S):
     mask = torch.from_numpy(m[:, None, None, :]).cuda()
     bias = np.broadcast_to(np.where(m, np.float32(0), NEG)[:, None, None, :], (len(lens), 1, L, S))
     _run(oracle, dt, D, len(lens), 2, 1, L, S, mask, bias, keep=[b for b in range(len(lens)) if m[b].any()])
+
+
+@pytest.mark.parametrize("kind", ["bool", "add"])
+def test_masks_that_start_at_any_byte(oracle, kind):
+    """Views of one mask that start at every byte (bool) or element (16 bit) of a 16-byte piece, with rows and keys beyond the
+    last tile: copies of nothing, too, come from an aligned address."""
+    L, S = 33, 130
+    rng = np.random.default_rng(56)
+    for skip in range(16 if kind == "bool" else 8):
+        if kind == "bool":
+            m = rng.random((1, 2, L, S + skip)) < 0.7
+            m[..., skip] = True
+            mask, bias = torch.from_numpy(m).cuda(), np.where(m, np.float32(0), NEG)
+        else:
+            mask = torch.from_numpy(rng.standard_normal((1, 2, L, S + skip)).astype(np.float32)).bfloat16().cuda()
+            bias = mask.float().cpu().numpy()
+        _run(oracle, "bf16", 64, 1, 2, 2, L, S, mask[..., skip:], np.ascontiguousarray(bias[..., skip:]))

@@ -197,7 +197,7 @@ struct MaskRows {
       for (int i = 0; i < 32; i += 4, p += 4 * pitch)
         ptx::cp_async16(dst + i * 128 + (((piece + r0 + i) & 7) << 4), down16(p) + piece * 16, 16);
     } else {
-      const uint8_t* any = reinterpret_cast<const uint8_t*>(a.mask.ptr);  // a valid address, for copies of nothing
+      const uint8_t* any = down16(reinterpret_cast<const uint8_t*>(a.mask.ptr));  // valid and aligned, for copies of nothing
 #pragma unroll 1
       for (int i = 0; i < 32; i += 4, p += 4 * pitch) {
         const uint8_t* src = down16(p) + piece * 16;
