@@ -77,7 +77,7 @@ def build_native():
     import sysconfig
     from torch.utils import cpp_extension
     src, out = os.path.join(CSRC, "binding.cpp"), os.path.join(OUT, "_native.so")
-    if os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), _headers_mtime()):
+    if os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), os.path.getmtime(__file__), _headers_mtime()):
         return out
     os.makedirs(OUT, exist_ok=True)
     cuda = os.path.dirname(os.path.dirname(NVCC))
@@ -87,7 +87,9 @@ def build_native():
         cmd += ["-isystem", i]
     for p in cpp_extension.library_paths():
         cmd += ["-L" + p]
-    cmd += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl"]
+    # the process's libstdc++, by name: a compiler that finds only the archive would put a second one into the module, whose
+    # streams crash on the locale of the first (an error message with a number in it ended the process)
+    cmd += ["-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl", "-l:libstdc++.so.6"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("building the torch binding failed:\n%s\n%s" % (r.stdout, r.stderr))
