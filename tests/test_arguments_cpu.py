@@ -1,0 +1,78 @@
+"""CPU: arguments that do not belong together are refused before anything is launched.
+
+The tensors are fake CUDA tensors (no memory behind them), so a call that is let through fails on the missing driver, with
+another error than the ValueError asked for here."""
+import os
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from conftest import ROOT
+from tinytorch_b200 import function, op
+
+
+@pytest.fixture(autouse=True)
+def fake():
+    if not os.path.exists(os.path.join(ROOT, "tinytorch_b200", "lib", "_native.so")):
+        from tinytorch_b200.build import build, build_native
+        build()
+        build_native()
+    with FakeTensorMode():
+        yield
+
+
+def t(*shape, dtype=torch.bfloat16, device="cuda"):
+    return torch.empty(shape, dtype=dtype, device=device)
+
+
+Q, KV, CACHE, NEW = (3, 8, 40, 64), (3, 4, 50, 64), (3, 4, 128, 64), (3, 4, 1, 64)
+SMALLER = [dict(k=(2, 4, 50, 64)), dict(v=(2, 4, 50, 64)), dict(v=(3, 2, 50, 64)), dict(v=(3, 4, 49, 64)), dict(v=(3, 4, 50, 32)),
+           dict(k=(3, 4, 50, 32))]
+
+
+@pytest.mark.parametrize("wrong", SMALLER)
+def test_keys_and_values_smaller_than_what_is_read(wrong):
+    args = [t(*Q), t(*wrong.get("k", KV)), t(*wrong.get("v", KV))]
+    for call in (op.sdpAttentionFwd, function.sdpAttention):
+        with pytest.raises(ValueError):
+            call(*args)
+
+
+@pytest.mark.parametrize("wrong", [dict(k=(4, 4, 50, 64)), dict(v=(4, 4, 50, 64)), dict(v=(3, 5, 50, 64)), dict(v=(3, 4, 51, 64))] + SMALLER)
+def test_gradients_of_keys_and_values_of_other_shapes(wrong):
+    """Larger ones too: the kernels would leave a part of the gradient unwritten."""
+    q, k, v = (x.requires_grad_() for x in (t(*Q), t(*wrong.get("k", KV)), t(*wrong.get("v", KV))))
+    with pytest.raises(ValueError):
+        function.sdpAttention(q, k, v)
+    with pytest.raises(ValueError):
+        op.sdpAttentionBwd(t(*Q), q.detach(), k.detach(), v.detach(), t(*Q), t(*Q[:3], dtype=torch.float32))
+
+
+@pytest.mark.parametrize("name,x", [
+    ("dO", dict(shape=(3, 8, 39, 64))), ("dO", dict(shape=Q, dtype=torch.float16)), ("o", dict(shape=(3, 7, 40, 64))),
+    ("o", dict(shape=Q, dtype=torch.float32)), ("lse", dict(shape=(3, 8, 39), dtype=torch.float32)),
+    ("lse", dict(shape=(3, 8, 40), dtype=torch.bfloat16)), ("lse", dict(shape=(3, 8, 40), dtype=torch.float32, device="cpu")),
+])
+def test_backward_operands(name, x):
+    args = dict(dO=t(*Q), q=t(*Q), k=t(*KV), v=t(*KV), o=t(*Q), lse=t(*Q[:3], dtype=torch.float32))
+    shape = x.pop("shape")
+    args[name] = t(*shape, **x)
+    with pytest.raises(ValueError):
+        op.sdpAttentionBwd(**args)
+
+
+@pytest.mark.parametrize("wrong", [
+    dict(k=((2, 4, 128, 64), torch.bfloat16)), dict(v=((3, 4, 127, 64), torch.bfloat16)), dict(v=((3, 3, 128, 64), torch.bfloat16)),
+    dict(k=(CACHE, torch.float16)), dict(v=(CACHE, torch.float32)), dict(new=(NEW, torch.float16)),
+])
+def test_decode_caches(wrong):
+    q = t(3, 8, 1, 64)
+    k, v, new = (t(*wrong.get(n, (s, torch.bfloat16))[0], dtype=wrong.get(n, (s, torch.bfloat16))[1])
+                 for n, s in (("k", CACHE), ("v", CACHE), ("new", NEW)))
+    lens = t(3, dtype=torch.int32)
+    if "new" not in wrong:
+        with pytest.raises(ValueError):
+            op.sdpAttentionDecode(q, k, v, lens)
+    with pytest.raises(ValueError):
+        op.sdpAttentionDecodeAppend(q, new, t(*NEW), k, v, lens)

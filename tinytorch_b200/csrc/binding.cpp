@@ -49,15 +49,20 @@ struct Api {
 } api;
 PyObject* attn_error = nullptr;  // _capi.AttnError
 
+// Called with or without the GIL (the backward nodes run in the engine's threads).
 [[noreturn]] void raise(PyObject* type, const char* fmt, ...) {
+  const PyGILState_STATE st = PyGILState_Ensure();
+  python_error err;
   va_list ap;
   va_start(ap, fmt);
   PyErr_FormatV(type, fmt, ap);
   va_end(ap);
-  throw python_error();
+  err.persist();
+  PyGILState_Release(st);
+  throw err;
 }
 
-// Called with or without the GIL (the backward nodes run in the engine's threads).
+// As above.
 void check(int rc) {
   if (rc == TT_ATTN_OK) return;
   std::string text = api.strerror(rc);
@@ -113,6 +118,23 @@ void check_attn_tensor(const Tensor& t, const char* name) {
   if (t.dim() != 4) raise(PyExc_ValueError, "%s must be [B, H, S, D]", name);
   if (t.stride(3) != 1) raise(PyExc_ValueError, "%s: innermost dimension must be contiguous", name);
   if (dtype_of(t.scalar_type()) < 0) raise(PyExc_ValueError, "%s: dtype %s not supported", name, c10::toString(t.scalar_type()));
+}
+
+// The C ABI sees the sizes of q (and the key heads and rows of k) only; every other operand has to have at least what a
+// kernel will take from it, in q's dtype and on its device.
+void check_operand(const Tensor& t, const char* name, const Tensor& q, int64_t B, int64_t H, int64_t S) {
+  if (t.scalar_type() != q.scalar_type() || t.device() != q.device())
+    raise(PyExc_ValueError, "%s must have the dtype and device of q", name);
+  if (t.size(0) < B || t.size(1) < H || t.size(2) < S || t.size(3) < q.size(3))
+    raise(PyExc_ValueError, "%s is smaller than [%lld, %lld, %lld, %lld], which q and the keys ask for", name, (long long)B,
+          (long long)H, (long long)S, (long long)q.size(3));
+}
+// `grads`: gradients of the same shapes are to be written, every element of them
+void check_kv(const Tensor& q, const Tensor& k, const Tensor& v, bool grads) {
+  check_operand(k, "k", q, q.size(0), 1, 0);
+  check_operand(v, "v", q, q.size(0), k.size(1), k.size(2));
+  if (grads && (k.size(0) != q.size(0) || k.size(3) != q.size(3) || v.sizes() != k.sizes()))
+    raise(PyExc_ValueError, "gradients need k and v of one shape, with the batch and head dimension of q");
 }
 
 tt_attn_strides strides_of(const Tensor& t) { return {t.stride(0), t.stride(1), t.stride(2)}; }
@@ -238,6 +260,15 @@ BwdResult attn_bwd(const Tensor& dO, const Tensor& q, const Tensor& k, const Ten
   return r;
 }
 
+void check_bwd(const Tensor& dO, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse) {
+  check_kv(q, k, v, true);
+  check_operand(dO, "dO", q, q.size(0), q.size(1), q.size(2));
+  check_operand(o, "o", q, q.size(0), q.size(1), q.size(2));
+  if (lse.scalar_type() != at::kFloat || lse.device() != q.device() || !lse.is_contiguous() ||
+      lse.numel() < q.size(0) * q.size(1) * q.size(2))
+    raise(PyExc_ValueError, "lse must be a contiguous float32 tensor [B, Hq, L] on the device of q");
+}
+
 // What FuncSDPAttention::backward (src/Function/FuncNNLayer.h:267) leaves unimplemented: the forward saves (O, LSE)
 // and hands dQ, dK, dV to autograd.  The mask and the lengths receive no gradient.
 struct AttentionBackward : public torch::autograd::Node {
@@ -258,6 +289,7 @@ struct AttentionBackward : public torch::autograd::Node {
     at::NoGradGuard no_grad;
     const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this());
     if (dO.stride(3) != 1) dO = dO.contiguous();
+    check_bwd(dO, qt, kt, vt, ot, lse);
     const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), task_should_compute_output(2)};
     BwdResult r = attn_bwd(dO, qt, kt, vt, ot, lse, mode, scale, kv_lens, needs, mask);
     for (int i = 0; i < 3; ++i) out[i] = std::move(r.g[i]);
@@ -265,13 +297,17 @@ struct AttentionBackward : public torch::autograd::Node {
   }
 };
 
-void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
+void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v, bool grads) {
   check_attn_tensor(q, "q");
   check_attn_tensor(k, "k");
   check_attn_tensor(v, "v");
   if (!(q.scalar_type() == k.scalar_type() && k.scalar_type() == v.scalar_type() && q.device() == k.device() &&
         k.device() == v.device()))
     raise(PyExc_ValueError, "q, k, v must share dtype and device");
+  check_kv(q, k, v, grads);
+}
+bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
+  return at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
 }
 
 // ------------------------------------------------------------------------------------------------- linear --
@@ -399,7 +435,8 @@ PyObject* py_sdp_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 7);
   const Tensor &q = tensor_of(a[0], "q"), &k = tensor_of(a[1], "k"), &v = tensor_of(a[2], "v");
-  check_qkv(q, k, v);
+  const bool grad = wants_grad(q, k, v);
+  check_qkv(q, k, v, grad);
   const int mode = int_arg(a[3]);
   const Tensor kv_lens = optional_of(a[4], "kvLens");
   const float scale = scale_or_default(scale_arg(a[5]), q.size(3));
@@ -407,7 +444,6 @@ PyObject* py_sdp_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   FwdResult r;
   {
     NoGil nogil;
-    const bool grad = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
     r = attn_fwd(q, k, v, mode, scale, kv_lens, grad, Tensor(), mask);
     if (grad) {
       auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
@@ -427,7 +463,7 @@ PyObject* py_attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 9);
   const Tensor &q = tensor_of(a[0], "q"), &k = tensor_of(a[1], "k"), &v = tensor_of(a[2], "v");
-  check_qkv(q, k, v);
+  check_qkv(q, k, v, false);
   const int mode = int_arg(a[3]);
   const float scale = scale_or_default(scale_arg(a[4]), q.size(3));
   const Tensor kv_lens = optional_of(a[5], "kvLens"), status = optional_of(a[7], "status");
@@ -453,6 +489,7 @@ PyObject* py_attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   check_attn_tensor(k, "k");
   check_attn_tensor(v, "v");
   check_attn_tensor(o, "o");
+  check_bwd(dO, q, k, v, o, lse);
   const int mode = int_arg(a[6]);
   const float scale = scale_or_default(scale_arg(a[7]), q.size(3));
   const Tensor kv_lens = optional_of(a[8], "kvLens");
@@ -476,6 +513,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   check_attn_tensor(k, "kCache");
   check_attn_tensor(v, "vCache");
   if (q.size(2) != 1) raise(PyExc_ValueError, "decode takes exactly one query per sequence");
+  check_kv(q, k, v, false);
   const Tensor kv_lens = optional_of(a[3], "kvLens"), ws = optional_of(a[6], "workspace");
   const float scale = scale_or_default(scale_arg(a[4]), q.size(3));
   const bool need_lse = bool_arg(a[5]);
@@ -517,6 +555,9 @@ PyObject* py_decode_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::DimVector row = {B, Hkv, 1, D};
   if (q.size(2) != 1 || kn.sizes() != at::IntArrayRef(row) || vn.sizes() != at::IntArrayRef(row))
     raise(PyExc_ValueError, "decode-append takes one query and one new key / value row per sequence");
+  check_kv(q, kc, vc, false);
+  check_operand(kn, "kNew", q, B, Hkv, 1);
+  check_operand(vn, "vNew", q, B, Hkv, 1);
   const Tensor kv_lens = optional_of(a[5], "kvLens");
   if (!kv_lens.defined() || kv_lens.scalar_type() != at::kInt) raise(PyExc_ValueError, "kvLens (int32 [B]) is required");
   const Tensor cos = optional_of(a[6], "ropeCos"), sin = optional_of(a[7], "ropeSin"), status = optional_of(a[11], "status");
