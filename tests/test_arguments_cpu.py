@@ -76,3 +76,33 @@ def test_decode_caches(wrong):
             op.sdpAttentionDecode(q, k, v, lens)
     with pytest.raises(ValueError):
         op.sdpAttentionDecodeAppend(q, new, t(*NEW), k, v, lens)
+
+
+@pytest.mark.parametrize("lens", [dict(dtype=torch.int64), dict(n=2), dict(dtype=torch.float32), dict(step=2), dict(device="cpu")])
+def test_lengths(lens):
+    """An int64 tensor would be read as pairs of int32 words, a strided or short one beyond its end."""
+    n, step = lens.get("n", 3), lens.get("step", 1)
+    x = t(n * step, dtype=lens.get("dtype", torch.int32), device=lens.get("device", "cuda"))[::step]
+    q1, k, v, new = t(3, 8, 1, 64), t(*CACHE), t(*CACHE), t(*NEW)
+    for call in (lambda: op.sdpAttentionFwd(t(*Q), k, v, kvLens=x), lambda: function.sdpAttention(t(*Q), k, v, kvLens=x),
+                 lambda: op.sdpAttentionBwd(t(*Q), t(*Q), k, v, t(*Q), t(*Q[:3], dtype=torch.float32), kvLens=x),
+                 lambda: op.sdpAttentionDecode(q1, k, v, x), lambda: op.sdpAttentionDecodeAppend(q1, new, new, k, v, x)):
+        with pytest.raises(ValueError):
+            call()
+
+
+def test_status_word_workspace_and_rotary_tables():
+    q1, k, v, new, lens = t(3, 8, 1, 64), t(*CACHE), t(*CACHE), t(*NEW), t(3, dtype=torch.int32)
+    for status in (t(1, dtype=torch.int64), t(0, dtype=torch.int32), t(1, dtype=torch.int32, device="cpu")):
+        with pytest.raises(ValueError):
+            op.sdpAttentionFwd(t(*Q), k, v, status=status)
+        with pytest.raises(ValueError):
+            op.sdpAttentionDecodeAppend(q1, new, new, k, v, lens, status=status)
+    for ws in (t(4096, dtype=torch.uint8, device="cpu"), t(64, 64, dtype=torch.uint8)[:, :32]):
+        with pytest.raises(ValueError):
+            op.sdpAttentionDecode(q1, k, v, lens, workspace=ws)
+    table = t(128, 32, dtype=torch.float32)
+    for cos, sin in ((table, t(128, 32, dtype=torch.float64)), (table, t(128, 32, dtype=torch.float32, device="cpu")),
+                     (t(128, 32, dtype=torch.float32, device="cpu"), table)):
+        with pytest.raises(ValueError):
+            op.sdpAttentionDecodeAppend(q1, new, new, k, v, lens, cos, sin)

@@ -18,3 +18,11 @@ def test_caches_and_keys_for_more_sequences_than_q(Hkv):
     q = make((2, 8, 40, 64), torch.bfloat16, 74)[0]
     want, _ = op.sdpAttentionFwd(q, k[:2].contiguous(), v[:2, :Hkv, :300].contiguous())
     assert torch.equal(op.sdpAttentionFwd(q, k, v)[0], want)
+
+
+def test_lengths_in_pinned_memory():
+    from tinytorch_b200 import op
+    q, k, v = (make((3, 4, 150, 64), torch.bfloat16, s)[0] for s in (75, 76, 77))
+    lens = torch.tensor([150, 20, 3], dtype=torch.int32)
+    got, _ = op.sdpAttentionFwd(q, k, v, kvLens=lens.pin_memory())
+    assert torch.equal(got, op.sdpAttentionFwd(q, k, v, kvLens=lens.cuda())[0])

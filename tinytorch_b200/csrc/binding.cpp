@@ -203,7 +203,17 @@ void set_mask(P* p, const Mask& m) {
   for (int i = 0; i < 3; ++i) p->mask_strides[i] = m.strides[i];
 }
 
-const int32_t* lens_ptr(const Tensor& t) { return t.defined() ? static_cast<const int32_t*>(t.data_ptr()) : nullptr; }
+// Integers that a kernel reads or writes: lengths [B], a status word.  Pinned host memory is reachable as well.
+void check_ints(const Tensor& t, const char* name, int64_t n, const Tensor& q) {
+  if (!t.defined()) return;
+  if (t.scalar_type() != at::kInt || !t.is_contiguous() || t.numel() < n || !(t.is_cuda() ? t.device() == q.device() : t.is_pinned()))
+    raise(PyExc_ValueError, "%s must be a contiguous int32 tensor of %lld elements or more on the device of q", name, (long long)n);
+}
+void check_ints(const Tensor& kv_lens, const Tensor& status, const Tensor& q) {
+  check_ints(kv_lens, "kvLens", q.size(0), q);
+  check_ints(status, "status", 1, q);
+}
+int32_t* ints_ptr(const Tensor& t) { return t.defined() ? static_cast<int32_t*>(t.data_ptr()) : nullptr; }
 
 // --------------------------------------------------------------------------------------------- attention --
 struct FwdResult {
@@ -212,6 +222,7 @@ struct FwdResult {
 
 FwdResult attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, int mode, float scale, const Tensor& kv_lens,
                    bool need_lse, const Tensor& status, const Mask& mask) {
+  check_ints(kv_lens, status, q);
   FwdResult r;
   const int64_t B = q.size(0), Hq = q.size(1), L = q.size(2), D = q.size(3);
   tt_attn_fwd_params p{};
@@ -223,9 +234,9 @@ FwdResult attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, int mode, 
   p.q = q.data_ptr(), p.k = k.data_ptr(), p.v = v.data_ptr(), p.o = r.o.data_ptr();
   p.lse = need_lse ? static_cast<float*>(r.lse.data_ptr()) : nullptr;
   p.q_strides = strides_of(q), p.k_strides = strides_of(k), p.v_strides = strides_of(v), p.o_strides = strides_of(r.o);
-  p.is_causal = mode, p.scale = scale, p.kv_lens = lens_ptr(kv_lens);
+  p.is_causal = mode, p.scale = scale, p.kv_lens = ints_ptr(kv_lens);
   p.alloc = &hook;
-  p.status = status.defined() ? static_cast<int32_t*>(status.data_ptr()) : nullptr;
+  p.status = ints_ptr(status);
   set_mask(&p, mask);
   check(api.fwd(&p));
   return r;
@@ -237,6 +248,7 @@ struct BwdResult {
 
 BwdResult attn_bwd(const Tensor& dO, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse,
                    int mode, float scale, const Tensor& kv_lens, const bool (&needs)[3], const Mask& mask) {
+  check_ints(kv_lens, Tensor(), q);
   BwdResult r;
   const Tensor* like[3] = {&q, &k, &v};
   for (int i = 0; i < 3; ++i)
@@ -253,7 +265,7 @@ BwdResult attn_bwd(const Tensor& dO, const Tensor& q, const Tensor& k, const Ten
   tt_attn_strides* st[3] = {&p.dq_strides, &p.dk_strides, &p.dv_strides};
   for (int i = 0; i < 3; ++i)
     if (needs[i]) *out[i] = r.g[i].data_ptr(), *st[i] = strides_of(r.g[i]);
-  p.is_causal = mode, p.scale = scale, p.kv_lens = lens_ptr(kv_lens);
+  p.is_causal = mode, p.scale = scale, p.kv_lens = ints_ptr(kv_lens);
   p.alloc = &hook;
   set_mask(&p, mask);
   check(api.bwd(&p));
@@ -317,6 +329,7 @@ int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.siz
 // y[M, N] (dense memory) = x[M, K] w[N, K]^T + bias; x_t / w_t: the operand is given as [K, M] / [K, N]
 void linear_raw(const Tensor& x, bool x_t, const Tensor& w, bool w_t, const Tensor& bias, const Tensor& y, const Tensor& status,
                 const Tensor& x_sum) {
+  check_ints(status, "status", 1, x);
   tt_linear_params p{};
   set_common(&p, x);
   p.dtype = dtype_of(x.scalar_type());
@@ -324,7 +337,7 @@ void linear_raw(const Tensor& x, bool x_t, const Tensor& w, bool w_t, const Tens
   p.x = x.data_ptr(), p.w = w.data_ptr(), p.y = y.data_ptr();
   p.bias = bias.defined() ? bias.data_ptr() : nullptr;
   p.ldx = row_stride(x), p.ldw = row_stride(w), p.ldy = p.N;
-  p.status = status.defined() ? static_cast<int32_t*>(status.data_ptr()) : nullptr;
+  p.status = ints_ptr(status);
   p.x_t = x_t, p.w_t = w_t;
   p.x_sum = x_sum.defined() ? x_sum.data_ptr() : nullptr;
   check(api.linear(&p));
@@ -515,6 +528,9 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (q.size(2) != 1) raise(PyExc_ValueError, "decode takes exactly one query per sequence");
   check_kv(q, k, v, false);
   const Tensor kv_lens = optional_of(a[3], "kvLens"), ws = optional_of(a[6], "workspace");
+  check_ints(kv_lens, Tensor(), q);
+  if (ws.defined() && (ws.device() != q.device() || !ws.is_contiguous()))
+    raise(PyExc_ValueError, "workspace must be a contiguous tensor on the device of q");
   const float scale = scale_or_default(scale_arg(a[4]), q.size(3));
   const bool need_lse = bool_arg(a[5]);
   Tensor o, lse;
@@ -530,7 +546,7 @@ PyObject* py_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.q = q.data_ptr(), p.k = k.data_ptr(), p.v = v.data_ptr(), p.o = o.data_ptr();
     p.lse = need_lse ? static_cast<float*>(lse.data_ptr()) : nullptr;
     p.q_strides = strides_of(q), p.k_strides = strides_of(k), p.v_strides = strides_of(v), p.o_strides = strides_of(o);
-    p.scale = scale, p.kv_lens = lens_ptr(kv_lens);
+    p.scale = scale, p.kv_lens = ints_ptr(kv_lens);
     p.alloc = &hook;
     if (ws.defined()) p.workspace = ws.data_ptr(), p.workspace_bytes = ws.numel() * ws.element_size();
     check(api.decode(&p));
@@ -559,11 +575,13 @@ PyObject* py_decode_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   check_operand(kn, "kNew", q, B, Hkv, 1);
   check_operand(vn, "vNew", q, B, Hkv, 1);
   const Tensor kv_lens = optional_of(a[5], "kvLens");
-  if (!kv_lens.defined() || kv_lens.scalar_type() != at::kInt) raise(PyExc_ValueError, "kvLens (int32 [B]) is required");
+  if (!kv_lens.defined() || !kv_lens.is_cuda()) raise(PyExc_ValueError, "kvLens (int32 [B] on the device of q) is required");
   const Tensor cos = optional_of(a[6], "ropeCos"), sin = optional_of(a[7], "ropeSin"), status = optional_of(a[11], "status");
+  check_ints(kv_lens, status, q);
   if (cos.defined() && (!sin.defined() || cos.scalar_type() != at::kFloat || cos.sizes() != sin.sizes() || cos.dim() != 2 ||
-                        cos.size(1) != D / 2 || !cos.is_contiguous() || !sin.is_contiguous()))
-    raise(PyExc_ValueError, "rope tables must be contiguous fp32 [positions, D/2]");
+                        cos.size(1) != D / 2 || !cos.is_contiguous() || !sin.is_contiguous() || sin.scalar_type() != at::kFloat ||
+                        cos.device() != q.device() || sin.device() != q.device()))
+    raise(PyExc_ValueError, "rope tables must be contiguous fp32 [positions, D/2] on the device of q");
   const bool interleaved = bool_arg(a[8]), need_lse = bool_arg(a[10]);
   const float scale = scale_or_default(scale_arg(a[9]), D);
   Tensor o, lse, new_lens;
@@ -581,14 +599,14 @@ PyObject* py_decode_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.lse = need_lse ? static_cast<float*>(lse.data_ptr()) : nullptr;
     p.q_strides = strides_of(q), p.k_new_strides = strides_of(kn), p.v_new_strides = strides_of(vn);
     p.k_strides = strides_of(kc), p.v_strides = strides_of(vc), p.o_strides = strides_of(o);
-    p.scale = scale, p.kv_lens = lens_ptr(kv_lens), p.new_lens = static_cast<int32_t*>(new_lens.data_ptr());
+    p.scale = scale, p.kv_lens = ints_ptr(kv_lens), p.new_lens = static_cast<int32_t*>(new_lens.data_ptr());
     if (cos.defined()) {
       p.rope_cos = static_cast<const float*>(cos.data_ptr()), p.rope_sin = static_cast<const float*>(sin.data_ptr());
       p.rope_positions = cos.size(0);
     }
     p.rope_interleaved = interleaved ? 1 : 0;
     p.alloc = &hook;
-    p.status = status.defined() ? static_cast<int32_t*>(status.data_ptr()) : nullptr;
+    p.status = ints_ptr(status);
     check(api.decode_append(&p));
   }
   return tuple_of({&o, &lse, &new_lens});
