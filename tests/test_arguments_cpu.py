@@ -9,7 +9,7 @@ import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
 from conftest import ROOT
-from tinytorch_b200 import function, op
+from tinytorch_b200 import fused, function, op
 
 
 @pytest.fixture(autouse=True)
@@ -106,3 +106,22 @@ def test_status_word_workspace_and_rotary_tables():
                      (t(128, 32, dtype=torch.float32, device="cpu"), table)):
         with pytest.raises(ValueError):
             op.sdpAttentionDecodeAppend(q1, new, new, k, v, lens, cos, sin)
+
+
+def test_projection_operands():
+    x, w = t(6, 64), t(16, 64)
+    for call in (fused.linear, fused._linear_raw):
+        with pytest.raises(ValueError):
+            call(x, w, t(16, device="cpu"))
+        with pytest.raises(AssertionError):
+            call(x, w, t(8))
+    for a, b in ((t(2, 6, 64), w), (x, t(16, 32)), (x, t(16, 64, dtype=torch.float16)), (t(64, 6).t(), w), (x, t(16, 64, device="cpu"))):
+        with pytest.raises(ValueError):
+            fused._linear_raw(a, b, None)
+    with pytest.raises(ValueError):
+        fused._linear_raw(x, w, None, t(1, dtype=torch.int64))
+
+
+def test_norm_operands_on_another_device():
+    with pytest.raises(ValueError):
+        fused.fusedAddRmsNorm(t(4, 64), t(4, 64), t(64, device="cuda:1"), 1e-5)

@@ -26,3 +26,14 @@ def test_lengths_in_pinned_memory():
     lens = torch.tensor([150, 20, 3], dtype=torch.int32)
     got, _ = op.sdpAttentionFwd(q, k, v, kvLens=lens.pin_memory())
     assert torch.equal(got, op.sdpAttentionFwd(q, k, v, kvLens=lens.cuda())[0])
+
+
+def test_bias_with_a_stride():
+    from tinytorch_b200 import fused
+    x, w = make((40, 64), torch.bfloat16, 78)[0], make((24, 64), torch.bfloat16, 79)[0]
+    b = make((24, 3), torch.bfloat16, 80)[0]
+    for call in (fused.linear, fused._linear_raw):
+        assert torch.equal(call(x, w, b[:, 1]), call(x, w, b[:, 1].contiguous()))
+    leaf = b[:, 1].requires_grad_()
+    fused.linear(x, w, leaf).float().sum().backward()
+    assert torch.equal(leaf.grad, torch.full_like(leaf, 40))

@@ -329,7 +329,6 @@ int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.siz
 // y[M, N] (dense memory) = x[M, K] w[N, K]^T + bias; x_t / w_t: the operand is given as [K, M] / [K, N]
 void linear_raw(const Tensor& x, bool x_t, const Tensor& w, bool w_t, const Tensor& bias, const Tensor& y, const Tensor& status,
                 const Tensor& x_sum) {
-  check_ints(status, "status", 1, x);
   tt_linear_params p{};
   set_common(&p, x);
   p.dtype = dtype_of(x.scalar_type());
@@ -378,14 +377,22 @@ struct LinearBackward : public torch::autograd::Node {
   }
 };
 
+// [N] values in the dtype and on the device of x, contiguous
+Tensor bias_of(const Tensor& bias, const Tensor& x, int64_t N) {
+  if (!bias.defined()) return bias;
+  if (bias.dim() != 1 || bias.size(0) != N || bias.scalar_type() != x.scalar_type())
+    raise(PyExc_AssertionError, "bias must be [N] (OpLinalg.cpp:261-263)");
+  if (bias.device() != x.device()) raise(PyExc_ValueError, "bias must be on the device of input");
+  return bias.contiguous();
+}
+
 Tensor linear_autograd(const Tensor& x, const Tensor& w, const Tensor& bias) {
   if (!x.is_cuda() || (x.scalar_type() != at::kHalf && x.scalar_type() != at::kBFloat16))
     raise(PyExc_ValueError, "linear needs CUDA float16 / bfloat16 tensors (float32 stays on the library gemm; no CPU path)");
   if (w.dim() != 2 || w.scalar_type() != x.scalar_type() || w.device() != x.device())
     raise(PyExc_ValueError, "weight must be [N, K] with the dtype and device of input");
   if (x.size(-1) != w.size(1)) raise(PyExc_AssertionError, "matmul error: shape not aligned (OpLinalg.cpp:251-254)");
-  if (bias.defined() && (bias.dim() != 1 || bias.size(0) != w.size(0) || bias.scalar_type() != x.scalar_type()))
-    raise(PyExc_AssertionError, "bias must be [N] (OpLinalg.cpp:261-263)");
+  const Tensor b = bias_of(bias, x, w.size(0));
   NoGil nogil;
   const bool grad = at::GradMode::is_enabled() &&
                     (x.requires_grad() || w.requires_grad() || (bias.defined() && bias.requires_grad()));
@@ -397,7 +404,7 @@ Tensor linear_autograd(const Tensor& x, const Tensor& w, const Tensor& bias) {
     at::DimVector shape(x.sizes().begin(), x.sizes().end());
     shape.back() = w.size(0);
     y = empty(shape, x.scalar_type(), x.device());
-    linear_raw(x2, false, wc, false, bias, y, Tensor(), Tensor());
+    linear_raw(x2, false, wc, false, b, y, Tensor(), Tensor());
   }
   if (grad) {
     auto node = std::shared_ptr<LinearBackward>(new LinearBackward(), torch::autograd::deleteNode);
@@ -646,8 +653,8 @@ PyObject* py_add_rms_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   expect(n, 4);
   const Tensor &input = tensor_of(a[0], "input"), &residual = tensor_of(a[1], "residual"), &weight = tensor_of(a[2], "weight");
   for (const Tensor* t : {&input, &residual, &weight})
-    if (!t->is_cuda() || t->scalar_type() != input.scalar_type() || dtype_of(t->scalar_type()) < 0)
-      raise(PyExc_ValueError, "fusedAddRmsNorm needs CUDA tensors of one dtype (float32 / float16 / bfloat16)");
+    if (!t->is_cuda() || t->device() != input.device() || t->scalar_type() != input.scalar_type() || dtype_of(t->scalar_type()) < 0)
+      raise(PyExc_ValueError, "fusedAddRmsNorm needs tensors of one dtype (float32 / float16 / bfloat16) on one CUDA device");
   if (input.sizes() != residual.sizes())
     raise(PyExc_AssertionError, "input and residual must have the same shape (OpFusedCpu.h:44)");
   if (!(input.is_contiguous() && residual.is_contiguous() && weight.is_contiguous()))
@@ -683,7 +690,12 @@ PyObject* py_linear_raw(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 4);
   const Tensor &x = tensor_of(a[0], "x"), &w = tensor_of(a[1], "w");
-  const Tensor bias = optional_of(a[2], "bias"), status = optional_of(a[3], "status");
+  const Tensor status = optional_of(a[3], "status");
+  if (x.dim() != 2 || w.dim() != 2 || x.size(1) != w.size(1) || w.scalar_type() != x.scalar_type() || !x.is_cuda() ||
+      w.device() != x.device() || (x.size(1) > 1 && (x.stride(1) != 1 || w.stride(1) != 1)))
+    raise(PyExc_ValueError, "x [M, K] and w [N, K] must be CUDA matrices of one dtype and device with contiguous columns");
+  const Tensor bias = bias_of(optional_of(a[2], "bias"), x, w.size(0));
+  check_ints(status, "status", 1, x);
   Tensor y;
   {
     NoGil nogil;
