@@ -117,6 +117,13 @@ int take_mask(const void* ptr, int kind, const int64_t st[3], MaskArgs* m) {
   m->wide = ((reinterpret_cast<uintptr_t>(ptr) | (m->sb * esz) | (m->sh * esz) | (m->sl * esz)) & 15) == 0;
   return TT_ATTN_OK;
 }
+// The fused decode step on the tensor-core path, beside the scan's scratch: the rotated q and the new lengths.
+size_t append_bytes(int dtype, int B, int Hq, int Hkv, int D) {
+  DecodeArgs probe{};
+  probe.Hq = Hq, probe.Hkv = Hkv;
+  if (!decode_tc_applies(dtype, D, probe)) return 0;
+  return round256(static_cast<size_t>(B) * Hq * D * elem_size(dtype)) + round256(static_cast<size_t>(B) * 4);
+}
 }  // namespace
 
 extern "C" {
@@ -138,21 +145,13 @@ size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int 
   if (kind == TT_ATTN_KIND_DECODE_APPEND) {
     // the decode scratch; on the grouped-query tensor-core path also the rotated q and the new lengths
     const size_t base = tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE, dtype, B, Hq, Hkv, Lq, Skv, D);
-    DecodeArgs probe{};
-    probe.Hq = Hq, probe.Hkv = Hkv;
-    if (Skv <= 0 || !decode_tc_applies(dtype, D, probe)) return base;
-    return base + round256(static_cast<size_t>(B) * Hq * D * elem_size(dtype)) + round256(static_cast<size_t>(B) * 4);
+    return base + (Skv > 0 ? append_bytes(dtype, B, Hq, Hkv, D) : 0);
   }
   if (kind == TT_ATTN_KIND_DECODE) {
     if (Skv <= 0) return 0;
     int nsplit, chunk;
     decode_plan_for(dtype, D, B, Hq, Hkv, Skv, &nsplit, &chunk);
-    // per-split partials, and for the tensor-core path (several query heads per kv head) a work counter
-    DecodeArgs probe{};
-    probe.Hq = Hq, probe.Hkv = Hkv;
-    const size_t counter = decode_tc_applies(dtype, D, probe) ? 256 : 0;
-    if (nsplit == 1) return counter;
-    return round256(static_cast<size_t>(B) * Hq * nsplit * (D + 2) * sizeof(float)) + counter;
+    return decode_scratch_bytes(dtype, D, B, Hq, Hkv, nsplit);
   }
   return 0;
 }
@@ -264,12 +263,11 @@ int tt_attn_decode(const tt_attn_decode_params* p) {
   a.B = p->B, a.Hq = p->Hq, a.Hkv = p->Hkv, a.capacity = p->capacity;
   a.scale = p->scale;
   a.kv_lens = p->kv_lens;
-  decode_plan_for(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity, &a.nsplit, &a.chunk);
+  const size_t need = decode_plan_within(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity,
+                                         p->workspace ? p->workspace_bytes : SIZE_MAX, &a.nsplit, &a.chunk);
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   Workspace ws;
-  const size_t need =
-      tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE, p->dtype, p->B, p->Hq, p->Hkv, 1, p->capacity, p->D);
   if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
   a.partial = static_cast<float*>(ws.ptr);
   // the tensor-core path's work counter sits in the last 256 bytes (unused by the scan kernel)
@@ -310,14 +308,13 @@ int tt_attn_decode_append(const tt_attn_decode_append_params* p) {
   a.rope_cos = p->rope_cos, a.rope_sin = p->rope_sin;
   a.rope_positions = p->rope_positions, a.rope_interleaved = p->rope_interleaved;
   a.status = p->status;
-  decode_plan_for(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity, &a.nsplit, &a.chunk);
+  const size_t more = append_bytes(p->dtype, p->B, p->Hq, p->Hkv, p->D);
+  const size_t room = !p->workspace ? SIZE_MAX : (p->workspace_bytes > more ? p->workspace_bytes - more : 0);
+  const size_t base = decode_plan_within(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity, room, &a.nsplit, &a.chunk);
+  const size_t need = base + more;
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   Workspace ws;
-  const size_t base =
-      tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE, p->dtype, p->B, p->Hq, p->Hkv, 1, p->capacity, p->D);
-  const size_t need =
-      tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE_APPEND, p->dtype, p->B, p->Hq, p->Hkv, 1, p->capacity, p->D);
   if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
   a.partial = static_cast<float*>(ws.ptr);
   a.sched = base >= 256 ? reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + base - 256) : nullptr;
@@ -348,9 +345,8 @@ int tt_attn_decode_static(const tt_attn_decode_params* p) {
   a.scale = p->scale;
   a.kv_lens = p->kv_lens;
   a.status = p->status;
-  decode_plan_for(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity, &a.nsplit, &a.chunk);
-  const size_t need =
-      tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE, p->dtype, p->B, p->Hq, p->Hkv, 1, p->capacity, p->D);
+  const size_t need = decode_plan_within(p->dtype, p->D, p->B, p->Hq, p->Hkv, p->capacity, TT_ATTN_STATIC_SCRATCH_BYTES,
+                                         &a.nsplit, &a.chunk);
   if (need > TT_ATTN_STATIC_SCRATCH_BYTES) return TT_ATTN_ERR_TOO_LARGE;
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;

@@ -169,6 +169,9 @@ cudaError_t launch_wait_expiry(int32_t* status, uint64_t limit_ns, unsigned long
 void decode_plan(int B, int Hkv, int capacity, int* nsplit, int* chunk);
 // ... for the tensor-core path (several query heads per kv head): longer chunks, see decode.cu
 void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int* nsplit, int* chunk);
+size_t decode_scratch_bytes(int dtype, int D, int B, int Hq, int Hkv, int nsplit);  // what a plan's partial results take
+// ... in `room` bytes of scratch: longer chunks, up to those of a large batch, where the partial results would not fit
+size_t decode_plan_within(int dtype, int D, int B, int Hq, int Hkv, int capacity, size_t room, int* nsplit, int* chunk);
 
 // Launches a kernel that calls ptx::grid_dep_wait() before it touches global memory: it may come up, and set itself up,
 // while the kernel before it in the stream ends (or, if that one allows it, still runs).  `cluster`: CTAs per cluster.

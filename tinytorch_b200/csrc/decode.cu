@@ -403,8 +403,9 @@ cudaError_t launch_t(const DecodeArgs& a, cudaStream_t stream) {
 // Splits of the scan: 512-row chunks keep CTAs short enough that mixed sequence lengths balance across the SMs; shorter
 // ones (down to 64 rows, one pass of a CTA) where a small batch would leave SMs without a CTA and every CTA with a long
 // serial scan (one sequence of 1024 rows and 8 heads: 16 CTAs of 512 rows, or 128 of 64); at most 64 per sequence.
+constexpr int kScanChunk = 512, kTcChunk = 2048;  // rows of a chunk in a large batch
 void decode_plan(int B, int Hkv, int capacity, int* nsplit, int* chunk) {
-  int ck = 512;
+  int ck = kScanChunk;
   while (ck > 64 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 148) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 63) / 64 * 64;
   *chunk = ck;
@@ -439,7 +440,7 @@ void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int
     decode_plan(B, Hkv, capacity, nsplit, chunk);
     return;
   }
-  int ck = 2048;
+  int ck = kTcChunk;
   const long long want = D == 64 ? 592 : 296;  // two items per resident CTA (D = 64 runs two CTAs per SM)
   while (ck > 512 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < want) ck >>= 1;
   while (ck > 128 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 74) ck >>= 1;
@@ -449,6 +450,28 @@ void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int
   if (capacity <= 384) ck = 384;
   *chunk = ck;
   *nsplit = capacity <= ck ? 1 : (capacity + ck - 1) / ck;
+}
+
+// Per-split partials, and for the tensor-core path (several query heads per kv head) a work counter.
+size_t decode_scratch_bytes(int dtype, int D, int B, int Hq, int Hkv, int nsplit) {
+  DecodeArgs probe{};
+  probe.Hq = Hq, probe.Hkv = Hkv;
+  const size_t partials = nsplit > 1 ? static_cast<size_t>(B) * Hq * nsplit * (D + 2) * sizeof(float) : 0;
+  return (partials + 255) / 256 * 256 + (decode_tc_applies(dtype, D, probe) ? 256 : 0);
+}
+
+// A small batch is divided further than a large one and can need more scratch.  A caller who sized a buffer for the large
+// one, or the fixed array of the allocation-free entry point, gets the large batch's chunks then, whose need falls with B.
+size_t decode_plan_within(int dtype, int D, int B, int Hq, int Hkv, int capacity, size_t room, int* nsplit, int* chunk) {
+  decode_plan_for(dtype, D, B, Hq, Hkv, capacity, nsplit, chunk);
+  DecodeArgs probe{};
+  probe.Hq = Hq, probe.Hkv = Hkv;
+  const int longest = decode_tc_applies(dtype, D, probe) ? kTcChunk : kScanChunk;
+  while (*chunk < longest && decode_scratch_bytes(dtype, D, B, Hq, Hkv, *nsplit) > room) {
+    *chunk = *chunk * 2 < longest ? *chunk * 2 : longest;
+    *nsplit = capacity <= *chunk ? 1 : (capacity + *chunk - 1) / *chunk;
+  }
+  return decode_scratch_bytes(dtype, D, B, Hq, Hkv, *nsplit);
 }
 
 cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t stream) {
