@@ -85,3 +85,59 @@ def test_static_scratch_takes_every_batch_below_its_largest():
         p.scale, p.device, p.stream = D ** -0.5, torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream
         _capi.check(_capi.lib().tt_attn_decode_static(C.byref(p)))
         _close(got, op.sdpAttentionDecode(q, k, v)[0], torch.float32)
+
+
+def _prefill(name, cls, q, k, v, o, ws, causal=0, mask=None, **ptrs):
+    """tt_attn_fwd / tt_attn_bwd with a scratch buffer of the caller's."""
+    from tinytorch_b200 import _capi
+    p = cls()
+    p.struct_size, p.dtype = C.sizeof(p), {torch.bfloat16: _capi.BF16, torch.float16: _capi.F16}[q.dtype]
+    p.B, p.Hq, p.Hkv, p.Lq, p.Skv, p.D = q.shape[0], q.shape[1], k.shape[1], q.shape[2], k.shape[2], q.shape[3]
+    p.q, p.k, p.v, p.o = (t.data_ptr() for t in (q, k, v, o))
+    for n, t in ptrs.items():
+        setattr(p, n, t.data_ptr())
+    p.is_causal, p.scale = causal, q.shape[3] ** -0.5
+    p.device, p.stream = torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    if mask is not None:  # [B, 1, 1, S]
+        p.mask, p.mask_kind = mask.data_ptr(), _capi.MASK_BOOL
+        p.mask_strides[0] = mask.stride(0)
+    _capi.check(getattr(_capi.lib(), name)(C.byref(p)))
+
+
+def test_backward_buffer_of_the_largest_batch():
+    from tinytorch_b200 import _capi, op
+    H, L, D, most, dt = 8, 2048, 128, 2, torch.bfloat16
+    need = [op.workspaceBytes(_capi.KIND_BWD, dt, b, H, H, L, L, D) for b in range(1, most + 1)]
+    assert need[0] > need[1]
+    q, k, v, do = (make((most, H, L, D), dt, 95 + i)[0] for i in range(4))
+    ws = torch.empty(need[-1] + 64, dtype=torch.uint8, device="cuda").fill_(171)
+    for b in (1, 2):
+        o, lse = op.sdpAttentionFwd(q[:b], k[:b], v[:b], isCausal=True)
+        grads = [torch.empty_like(q[:b]) for _ in range(3)]
+        _prefill("tt_attn_bwd", _capi.BwdParams, q[:b], k[:b], v[:b], o, ws[:need[-1]], causal=1, lse=lse, d_o=do[:b],
+                 dq=grads[0], dk=grads[1], dv=grads[2])
+        for got, want in zip(grads, op.sdpAttentionBwd(do[:b], q[:b], k[:b], v[:b], o, lse, isCausal=True)):
+            _close(got, want, dt)
+    assert bool((ws[need[-1]:] == 171).all())
+
+
+def test_work_counter_alone_is_enough_for_a_large_batch():
+    """256 bytes (and the backward's accumulators), at a batch whose mask lengths take more: with a padding mask and without."""
+    from tinytorch_b200 import _capi, op
+    B, H, L, D, dt = 40, 2, 130, 64, torch.float16
+    q, k, v, do = (make((B, H, L, D), dt, 61 + i)[0] for i in range(4))
+    n = torch.arange(B, device="cuda") * 3 + 5
+    mask = (torch.arange(L, device="cuda")[None] < n[:, None])[:, None, None]
+    lse = torch.empty((B, H, L), device="cuda")
+    base = sum((B * H * L * 4 * x + 255) // 256 * 256 for x in (1, D))
+    for m in (None, mask):
+        o, grads = torch.empty_like(q), [torch.empty_like(q) for _ in range(3)]
+        _prefill("tt_attn_fwd", _capi.FwdParams, q, k, v, o, torch.empty(256, dtype=torch.uint8, device="cuda"), mask=m, lse=lse)
+        want, wl = op.sdpAttentionFwd(q, k, v, attnMask=m)
+        _close(o, want, dt)
+        assert float((lse - wl).abs().max()) <= 1e-4
+        _prefill("tt_attn_bwd", _capi.BwdParams, q, k, v, want, torch.empty(base + 256, dtype=torch.uint8, device="cuda"), mask=m,
+                 lse=wl, d_o=do, dq=grads[0], dk=grads[1], dv=grads[2])
+        for got, w in zip(grads, op.sdpAttentionBwd(do, q, k, v, want, wl, attnMask=m)):
+            _close(got, w, dt)

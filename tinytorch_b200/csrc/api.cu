@@ -117,6 +117,12 @@ int take_mask(const void* ptr, int kind, const int64_t st[3], MaskArgs* m) {
   m->wide = ((reinterpret_cast<uintptr_t>(ptr) | (m->sb * esz) | (m->sh * esz) | (m->sl * esz)) & 15) == 0;
   return TT_ATTN_OK;
 }
+// Whether the lengths that a padding mask comes to have a place in the scratch memory (of `room` bytes, `used` of them taken);
+// a caller who knows of the work counter only, or whose mask is of another kind, needs 256 bytes.
+bool mask_lens_fit(const MaskArgs& m, int causal, int B, size_t room, size_t used) {
+  return is_padding_mask(m, causal) && room >= used + round256(scratch_words(B) * sizeof(int));
+}
+
 // The fused decode step on the tensor-core path, beside the scan's scratch: the rotated q and the new lengths.
 size_t append_bytes(int dtype, int B, int Hq, int Hkv, int D) {
   DecodeArgs probe{};
@@ -130,8 +136,8 @@ extern "C" {
 
 size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (B <= 0 || Hq <= 0 || D <= 0) return 0;
-  // fp16 / bf16 forward: one work counter for the persistent kernel's scheduler
-  // (and the lengths that a padding mask comes to)
+  // fp16 / bf16 forward: one work counter for the persistent kernel's scheduler, and the lengths that a padding mask
+  // comes to (a call without such a mask takes 256 bytes of it)
   if (kind == TT_ATTN_KIND_FWD) return dtype == TT_ATTN_F32 ? 0 : round256(scratch_words(B) * sizeof(int));
   if (kind == TT_ATTN_KIND_BWD) {
     // delta [B,Hq,Lq] fp32; the fp16 / bf16 path adds an fp32 dQ accumulator [B,Hq,Lq,D]
@@ -183,9 +189,12 @@ int tt_attn_fwd(const tt_attn_fwd_params* p) {
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   Workspace ws;
-  const size_t need = tt_attn_workspace_bytes(TT_ATTN_KIND_FWD, p->dtype, p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D);
+  const size_t room = p->workspace ? p->workspace_bytes : SIZE_MAX;
+  const bool lens = p->dtype != TT_ATTN_F32 && mask_lens_fit(a.mask, a.causal, p->B, room, 0);
+  const size_t need = p->dtype == TT_ATTN_F32 ? 0 : (lens ? round256(scratch_words(p->B) * sizeof(int)) : 256);
   if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
   a.sched = static_cast<int*>(ws.ptr);
+  a.mask_lens = lens ? a.sched + 1 : nullptr;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_fwd_simt(p->dtype, p->D, a, stream)
                                           : launch_fwd_tc(p->dtype, p->D, a, p->device, stream);
@@ -228,16 +237,27 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   Workspace ws;
-  const size_t need = tt_attn_workspace_bytes(TT_ATTN_KIND_BWD, p->dtype, p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D);
+  // delta | dQ accumulator | shares of dK / dV | work counter and, if they fit, a padding mask's lengths
+  const size_t rows = static_cast<size_t>(p->B) * p->Hq * p->Lq, delta = round256(rows * sizeof(float));
+  const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
+  size_t need = delta, part = 0;
+  bool lens = false;
+  if (p->dtype != TT_ATTN_F32) {
+    // a buffer that is too small for the division (a small batch is divided further than a large one): fewer shares
+    a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
+    while (a.parts > 1 && delta + accum + round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D)) + 256 > room) --a.parts;
+    part = round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D));
+    need = delta + accum + part;
+    lens = mask_lens_fit(a.mask, a.causal, p->B, room, need);
+    need += lens ? round256(scratch_words(p->B) * sizeof(int)) : 256;
+  }
   if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
   a.delta = static_cast<float*>(ws.ptr);
-  a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) +
-                                        round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * sizeof(float)));
   if (p->dtype != TT_ATTN_F32) {
-    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + need - round256(scratch_words(p->B) * sizeof(int)));
-    a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
-    a.dkv_part = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dq_accum) +
-                                          round256(static_cast<size_t>(p->B) * p->Hq * p->Lq * p->D * sizeof(float)));
+    a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
+    a.dkv_part = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta + accum);
+    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + delta + accum + part);
+    a.mask_lens = lens ? a.sched + 1 : nullptr;
   }
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
   cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_simt(p->dtype, p->D, a, stream)

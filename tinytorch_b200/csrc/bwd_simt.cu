@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kThreads) bwd_delta_kernel(const BwdArgs a) {
   ptx::grid_dep_launch();
   if (a.sched && blockIdx.x == 0 && threadIdx.x == 0) *a.sched = 0;  // the main kernel's work counter
   if (a.mask_pure) {  // ... and the lengths that a padding mask comes to
-    int* lens = a.sched + 1;
+    int32_t* lens = a.mask_lens;
     for (int b = blockIdx.x; b < a.B; b += gridDim.x) masked_lens(a.mask, a.kv_lens, a.Skv, b, lens, lens + a.B);
   }
   constexpr int N = 16 / sizeof(T);  // elements per thread

@@ -1519,19 +1519,22 @@ int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal) {
   return best;
 }
 
+size_t bwd_part_bytes_of(int parts, int B, int Hkv, int Skv, int D) {
+  return parts > 1 ? static_cast<size_t>(2) * parts * B * Hkv * Skv * D * sizeof(float) : 0;
+}
+
 size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (Hkv <= 0 || Skv <= 0 || Lq <= 0) return 0;
   const int pc = bwd_parts(B, Hq, Hkv, Lq, Skv, D, true), pf = bwd_parts(B, Hq, Hkv, Lq, Skv, D, false);
-  const int p = pc > pf ? pc : pf;
-  return p > 1 ? static_cast<size_t>(2) * p * B * Hkv * Skv * D * sizeof(float) : 0;
+  return bwd_part_bytes_of(pc > pf ? pc : pf, B, Hkv, Skv, D);
 }
 
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& call, int device, cudaStream_t stream) {
   BwdArgs a = call, pre = call;
   pre.zero_dq_accum = 1;
-  if (is_padding_mask(a.mask, a.causal)) {
-    pre.mask_pure = a.mask_pure = a.sched + 1 + a.B;  // (to the pre-pass: that it is to find the lengths)
-    a.kv_lens = a.sched + 1;
+  if (a.mask_lens) {
+    pre.mask_pure = a.mask_pure = a.mask_lens + a.B;  // (to the pre-pass: that it is to find the lengths)
+    a.kv_lens = a.mask_lens;
   }
   cudaError_t e = launch_bwd_delta(dtype, D, pre, stream);
   if (e != cudaSuccess) return e;

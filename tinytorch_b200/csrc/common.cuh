@@ -50,8 +50,9 @@ struct FwdArgs {
   const int32_t* kv_lens;
   int32_t* status;
   MaskArgs mask;
-  int* sched;  // tensor-core path: scratch memory of scratch_words(B) integers, the first of them the work counter
-  const int32_t* mask_pure;  // tensor-core path, with masked_lens: whether the mask is all true up to the length
+  int* sched;  // tensor-core path: work counter in scratch memory
+  int32_t* mask_lens;        // tensor-core path: scratch of 2 B integers for masked_lens, or null: a padding mask is read in full
+  const int32_t* mask_pure;  // with masked_lens: whether the mask is all true up to the length
 };
 
 struct BwdArgs {
@@ -79,6 +80,7 @@ struct BwdArgs {
   const int32_t* kv_lens;
   int32_t* status;
   MaskArgs mask;
+  int32_t* mask_lens;        // as in FwdArgs
   const int32_t* mask_pure;  // as in FwdArgs
 };
 
@@ -122,6 +124,7 @@ cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t st
 // Work items per key tile of the tensor-core backward, and the workspace they need beside dq_accum (0 for one item)
 int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal);
 size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
+size_t bwd_part_bytes_of(int parts, int B, int Hkv, int Skv, int D);
 // fp16 / bf16 backward on the tensor cores; needs a.delta, a.dq_accum and what a.parts asks for
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t stream);
@@ -202,7 +205,8 @@ inline cudaError_t launch_zero_word(int* word, cudaStream_t stream) {
   return launch_early(zero_word_kernel, dim3(1), dim3(32), 0, stream, 1, word);
 }
 
-// Scratch integers of the tensor-core kernels: the work counter and, for a padding mask, a length and a flag per sequence.
+// Scratch integers of the tensor-core prefill kernels: the work counter and, for a padding mask, a length and a flag per
+// sequence.  (The counter alone: 256 bytes, as every scratch block is rounded up to.)
 constexpr size_t scratch_words(int B) { return 1 + 2 * static_cast<size_t>(B); }
 
 // A boolean mask that is the same for all heads and rows is most often padding: true up to a length.  Its sequences are

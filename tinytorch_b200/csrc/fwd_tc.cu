@@ -1107,8 +1107,8 @@ cudaError_t launch_t(FwdArgs a, int dtype, int device, cudaStream_t stream) {
   const int sms = sm_count(device);
   const int grid = p.cluster > 1 ? static_cast<int>(n_items) * p.cluster : static_cast<int>(n_items < sms ? n_items : sms);
   const bool counter = p.cluster == 1 && n_items > grid;
-  if (GEN == 2 && is_padding_mask(a.mask, a.causal)) {
-    int* lens = a.sched + 1;
+  if (GEN == 2 && a.mask_lens) {
+    int32_t* lens = a.mask_lens;
     cudaError_t e = launch_early(lens_kernel, dim3(a.B), dim3(256), 0, stream, 1, a, a.sched, lens, lens + a.B);
     if (e != cudaSuccess) return e;
     a.kv_lens = lens, a.mask_pure = lens + a.B;
