@@ -5,7 +5,8 @@
 // ctypes, calling back into Python for scratch memory and going through Python autograd functions took 16-50 us per
 // operator (150-220 us for a forward and backward pass) while the kernels of such a call run for 2-20 us.
 //
-// The Python layer (op.py, function.py, fused.py) keeps the public signatures and hands its arguments on.  The GIL is
+// The Python layer (op.py, function.py, fused.py) keeps the public signatures and hands its arguments on; its autograd
+// functions take the calls that need more than reverse mode (needs_python_function).  The GIL is
 // released around every launch.  Scratch memory comes from torch's caching allocator on the current stream, the
 // stand-in for the reference's getCUDACachedAllocator(device) (src/Tensor/Allocator.cpp:117-139).
 #define PY_SSIZE_T_CLEAN
@@ -22,6 +23,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <cmath>
 #include <cstdarg>
@@ -349,6 +351,27 @@ Tensor rows_of(const Tensor& t) {  // [.., C] as [rows, C] with contiguous colum
 }
 
 // function::FuncLinear::backward (src/Function/FuncNNLayer.h:20-34)
+struct LinearGrads {
+  Tensor g[3];
+};
+LinearGrads linear_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, at::IntArrayRef dx_shape, const bool (&needs)[3]) {
+  LinearGrads r;
+  const Tensor g2 = rows_of(dy);
+  // the products contract over the slow dimension of W, and of dY and X: read as they are stored
+  if (needs[0]) {  // dX[M,K] = dY[M,N] W[N,K]
+    r.g[0] = empty(dx_shape, g2.scalar_type(), g2.device());
+    linear_raw(g2, false, w, true, Tensor(), r.g[0], Tensor(), Tensor());
+  }
+  if (needs[2]) r.g[2] = empty({g2.size(1)}, g2.scalar_type(), g2.device());
+  if (needs[1]) {  // dW[N,K] = dY[M,N]^T X[M,K], with db[N] = sum of dY over its rows
+    r.g[1] = empty({g2.size(1), x2.size(1)}, g2.scalar_type(), g2.device());
+    linear_raw(g2, true, x2, true, Tensor(), r.g[1], Tensor(), r.g[2]);
+  } else if (needs[2]) {
+    r.g[2] = g2.to(at::kFloat).sum(0).to(g2.scalar_type());
+  }
+  return r;
+}
+
 struct LinearBackward : public torch::autograd::Node {
   SavedVariable x2, w;
   at::DimVector in_shape;
@@ -359,20 +382,9 @@ struct LinearBackward : public torch::autograd::Node {
     variable_list out(3);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
-    const Tensor g2 = rows_of(grads[0]), xt = x2.unpack(), wt = w.unpack();
-    // the products contract over the slow dimension of W, and of dY and X: read as they are stored
-    if (task_should_compute_output(0)) {  // dX[M,K] = dY[M,N] W[N,K]
-      out[0] = empty(in_shape, g2.scalar_type(), g2.device());
-      linear_raw(g2, false, wt, true, Tensor(), out[0], Tensor(), Tensor());
-    }
-    const bool need_db = has_bias && task_should_compute_output(2);
-    if (need_db) out[2] = empty({g2.size(1)}, g2.scalar_type(), g2.device());
-    if (task_should_compute_output(1)) {  // dW[N,K] = dY[M,N]^T X[M,K], with db[N] = sum of dY over its rows
-      out[1] = empty({g2.size(1), xt.size(1)}, g2.scalar_type(), g2.device());
-      linear_raw(g2, true, xt, true, Tensor(), out[1], Tensor(), out[2]);
-    } else if (need_db) {
-      out[2] = g2.to(at::kFloat).sum(0).to(g2.scalar_type());
-    }
+    const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), has_bias && task_should_compute_output(2)};
+    LinearGrads r = linear_bwd(grads[0], x2.unpack(), w.unpack(), in_shape, needs);
+    for (int i = 0; i < 3; ++i) out[i] = std::move(r.g[i]);
     return out;
   }
 };
@@ -419,6 +431,15 @@ Tensor linear_autograd(const Tensor& x, const Tensor& w, const Tensor& bias) {
 }
 
 // ------------------------------------------------------------------------------------------ python methods --
+// The nodes here know reverse mode only.  A trace has to record the operator, forward-mode derivatives and functorch's
+// transforms have to reach torch, which refuses them: the Python autograd functions (function.py, fused.py) see to that.
+bool needs_python_function(std::initializer_list<const Tensor*> inputs) {
+  if (torch::jit::tracer::isTracing() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return true;
+  for (const Tensor* t : inputs)
+    if (t->defined() && t->_fw_grad(0).defined()) return true;
+  return false;
+}
 double scale_arg(PyObject* o) {  // NaN stands for "not given"
   if (o == Py_None) return std::nan("");
   const double d = PyFloat_AsDouble(o);
@@ -450,11 +471,13 @@ PyObject* tuple_of(std::initializer_list<const Tensor*> ts) {
   return r;
 }
 
-// sdp_attention(q, k, v, mode, kvLens, scale, mask) -> O, with an autograd node where one is needed
+// sdp_attention(q, k, v, mode, kvLens, scale, mask) -> O, with an autograd node where one is needed; NotImplemented where
+// the call is for the Python autograd function
 PyObject* py_sdp_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 7);
   const Tensor &q = tensor_of(a[0], "q"), &k = tensor_of(a[1], "k"), &v = tensor_of(a[2], "v");
+  if (needs_python_function({&q, &k, &v})) Py_RETURN_NOTIMPLEMENTED;
   const bool grad = wants_grad(q, k, v);
   check_qkv(q, k, v, grad);
   const int mode = int_arg(a[3]);
@@ -677,11 +700,34 @@ PyObject* py_add_rms_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// linear(input, weight, bias or None)
+// linear(input, weight, bias or None); NotImplemented as sdp_attention
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 3);
-  return wrap(linear_autograd(tensor_of(a[0], "input"), tensor_of(a[1], "weight"), optional_of(a[2], "bias")));
+  const Tensor &x = tensor_of(a[0], "input"), &w = tensor_of(a[1], "weight"), bias = optional_of(a[2], "bias");
+  if (needs_python_function({&x, &w, &bias})) Py_RETURN_NOTIMPLEMENTED;
+  return wrap(linear_autograd(x, w, bias));
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_bwd(dY [.., N], x2 [M, K], w [N, K], need_dx, need_dw, need_db) -> (dX [M, K], dW, db), None where not needed
+PyObject* py_linear_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 6);
+  const Tensor &dy = tensor_of(a[0], "dY"), &x2 = tensor_of(a[1], "x2"), &w = tensor_of(a[2], "w");
+  for (const Tensor* t : {&x2, &w})
+    if (t->dim() != 2 || (t->size(1) > 1 && t->stride(1) != 1) || t->scalar_type() != dy.scalar_type() || t->device() != dy.device())
+      raise(PyExc_ValueError, "x2 [M, K] and w [N, K] must be matrices of dY's dtype and device with contiguous columns");
+  if (!dy.is_cuda() || dy.dim() < 1 || dy.size(-1) != w.size(0) || x2.size(1) != w.size(1) || dy.numel() != x2.size(0) * w.size(0))
+    raise(PyExc_ValueError, "dY must be a CUDA tensor [.., N] with the rows of x2");
+  const bool needs[3] = {bool_arg(a[3]), bool_arg(a[4]), bool_arg(a[5])};
+  LinearGrads g;
+  {
+    NoGil nogil;
+    at::NoGradGuard no_grad;
+    g = linear_bwd(dy, x2, w, x2.sizes(), needs);
+  }
+  return tuple_of({&g.g[0], &g.g[1], &g.g[2]});
   END_HANDLE_TH_ERRORS
 }
 
@@ -748,6 +794,7 @@ PyMethodDef methods[] = {
     {"silu_mul", py_silu_mul, METH_O, nullptr},
     {"add_rms_norm", fast(py_add_rms_norm), METH_FASTCALL, nullptr},
     {"linear", fast(py_linear), METH_FASTCALL, nullptr},
+    {"linear_bwd", fast(py_linear_bwd), METH_FASTCALL, nullptr},
     {"linear_raw", fast(py_linear_raw), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 

@@ -21,17 +21,33 @@ src/Function/FuncNNLayer.h:249-256).  Differences, all forced by the fused path:
   * the mask receives no gradient; dropoutP must be 0 (dropout stays on the
     reference's generic-op composition, which this package does not contain).
 """
-from . import _capi
-from .op import _causal_mode
+import torch
+
+from . import _capi, op
 
 
-class FuncSDPAttention:
-    """The differentiable operator; its node (forward saves q, k, v, O and LSE, backward computes dQ, dK, dV) is
-    AttentionBackward in csrc/binding.cpp."""
+class FuncSDPAttention(torch.autograd.Function):
+    """The differentiable operator as a Python autograd function: what a trace records, and what torch refuses under
+    forward-mode differentiation and functorch's transforms.  Ordinary calls take the native node with the same kernels
+    (AttentionBackward in csrc/binding.cpp), which costs less host time."""
 
     @staticmethod
-    def apply(query, key, value, isCausal, kvLens, scale, attnMask=None):
-        return _capi.native().sdp_attention(query, key, value, _causal_mode(isCausal), kvLens, scale, attnMask)
+    def forward(ctx, query, key, value, isCausal, kvLens, scale, attnMask=None):
+        needs_grad = any(ctx.needs_input_grad[:3])
+        o, lse = op.sdpAttentionFwd(query, key, value, isCausal, scale, kvLens, needLse=needs_grad, attnMask=attnMask)
+        if needs_grad:
+            ctx.save_for_backward(query, key, value, o, lse)
+            ctx.isCausal, ctx.scale, ctx.kvLens, ctx.attnMask = isCausal, scale, kvLens, attnMask
+        return o
+
+    @staticmethod
+    def backward(ctx, grad):
+        query, key, value, o, lse = ctx.saved_tensors
+        if grad.stride(3) != 1:
+            grad = grad.contiguous()
+        dq, dk, dv = op.sdpAttentionBwd(grad, query, key, value, o, lse, ctx.isCausal, ctx.scale, ctx.kvLens,
+                                        needs=ctx.needs_input_grad[:3], attnMask=ctx.attnMask)
+        return dq, dk, dv, None, None, None, None
 
 
 def sdpAttention(query, key, value, isCausal=False, attnMask=None, dropoutP=0.0, scale=None, kvLens=None):
@@ -42,4 +58,8 @@ def sdpAttention(query, key, value, isCausal=False, attnMask=None, dropoutP=0.0,
         raise NotImplementedError("dropoutP > 0 is not on the fused path")
     if not isinstance(isCausal, str):
         isCausal = bool(isCausal)
-    return _capi.native().sdp_attention(query, key, value, _causal_mode(isCausal), kvLens, scale, attnMask)
+    o = _capi.native().sdp_attention(query, key, value, op._causal_mode(isCausal), kvLens, scale, attnMask)
+    if o is NotImplemented:
+        scale = op.default_scale(query.shape[-1]) if scale is None else float(scale)
+        o = FuncSDPAttention.apply(query, key, value, isCausal, kvLens, scale, None if attnMask is None else attnMask.detach())
+    return o

@@ -15,6 +15,8 @@ All go through the C ABI of libtt_attn.so (include/tt_fused.h) and launch on the
 current CUDA stream of the tensors' device.  None has a CPU implementation here, and - as
 in the reference (FuncFused.h:18,27) - siluMul and fusedAddRmsNorm have no backward.
 """
+import torch
+
 from . import _capi
 
 
@@ -33,15 +35,28 @@ def _linear_raw(x2, w, bias, status=None):
     return _capi.native().linear_raw(x2, w, bias, status)
 
 
-class FuncLinear:
-    """function::FuncLinear (src/Function/FuncNNLayer.h:14-35) on the tcgen05 kernel; its node is LinearBackward in
-    csrc/binding.cpp."""
+class FuncLinear(torch.autograd.Function):
+    """function::FuncLinear (src/Function/FuncNNLayer.h:14-35) on the tcgen05 kernels as a Python autograd function, for what
+    the native node (LinearBackward in csrc/binding.cpp) does not do; see function.FuncSDPAttention."""
 
     @staticmethod
-    def apply(input, weight, bias):
-        return _capi.native().linear(input, weight, bias)
+    def forward(ctx, input, weight, bias):
+        x2 = input.reshape(-1, input.shape[-1])
+        if x2.stride(1) != 1:
+            x2 = x2.contiguous()
+        w = weight if weight.stride(1) == 1 else weight.contiguous()
+        ctx.save_for_backward(x2, w)
+        ctx.in_shape = input.shape
+        return _linear_raw(x2, w, bias).reshape(input.shape[:-1] + (weight.shape[0],))
+
+    @staticmethod
+    def backward(ctx, grad):
+        x2, w = ctx.saved_tensors
+        dx, dw, db = _capi.native().linear_bwd(grad, x2, w, *ctx.needs_input_grad)
+        return dx if dx is None else dx.reshape(ctx.in_shape), dw, db
 
 
 def linear(input, weight, bias=None):
     """Drop-in for function::linear (src/Function/FuncNNLayer.h:270-272)."""
-    return _capi.native().linear(input, weight, bias)
+    y = _capi.native().linear(input, weight, bias)
+    return FuncLinear.apply(input, weight, bias) if y is NotImplemented else y
