@@ -67,3 +67,36 @@ def test_python_function_and_native_node_agree(which):
     assert torch.equal(y, z)
     # (two key tiles: dQ is a sum of two shares, whose order does not matter)
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, x, g), torch.autograd.grad(z, x, g)))
+
+
+def test_saved_tensors_pass_through_hooks():
+    """q, k, v, O and the row statistics: what a hook packs (here: to host memory) is what the backward pass uses."""
+    f, inputs = _ops()[0]
+    x = [t.requires_grad_() for t in inputs()]
+    g = torch.randn_like(x[0])
+    want = torch.autograd.grad(f(*x), x, g)
+    packed = []
+
+    def pack(t):
+        packed.append((t.dtype, tuple(t.shape)))
+        return t.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        y = f(*x)
+    assert len(packed) == 5 and (torch.float32, (2, 4, 130)) in packed
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, x, g), want))
+
+
+@pytest.mark.parametrize("kind", ["bool", "add"])
+def test_mask_and_lengths_pointed_elsewhere_before_the_backward(kind):
+    from tinytorch_b200 import function
+    x = [t.requires_grad_() for t in _attention()]
+    g = torch.randn_like(x[0])
+    mask = torch.rand(130, 130, device="cuda").lt(0.7) if kind == "bool" else torch.randn(130, 130, device="cuda").bfloat16()
+    lens = torch.tensor([130, 77], dtype=torch.int32, device="cuda")
+    call = lambda m, n: function.sdpAttention(*x, attnMask=m, kvLens=n)
+    want = torch.autograd.grad(call(mask.clone(), lens.clone()), x, g)
+    y = call(mask, lens)
+    mask.set_(torch.empty(1, dtype=mask.dtype, device="cuda"))
+    lens.set_(torch.empty(2, dtype=torch.int32, device="cuda").fill_(1))
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, x, g), want))

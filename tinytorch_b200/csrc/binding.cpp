@@ -160,8 +160,7 @@ void set_common(P* p, const Tensor& ref) {
 // attnMask of the reference (src/Function/FuncNNLayer.h:249-256): Bool -> keys that participate, otherwise added to
 // the scaled scores; any shape that broadcasts against [B, Hq, L, S] by trailing-dimension alignment.
 struct Mask {
-  Tensor keep;  // what `ptr` points into
-  const void* ptr = nullptr;
+  Tensor t;
   int kind = TT_ATTN_MASK_NONE;
   int64_t strides[3] = {0, 0, 0};
 };
@@ -193,15 +192,14 @@ Mask mask_of(const Tensor& mask, const Tensor& q, int64_t S) {
   }
   // keys must be contiguous in memory; a mask broadcast over keys is expanded
   if (m.size(3) != S || m.stride(3) != 1) m = m.expand({m.size(0), m.size(1), m.size(2), S}).contiguous();
-  r.ptr = m.data_ptr();
   for (int i = 0; i < 3; ++i) r.strides[i] = m.size(i) == 1 ? 0 : m.stride(i);
-  r.keep = std::move(m);
+  r.t = std::move(m);
   return r;
 }
 
 template <typename P>
 void set_mask(P* p, const Mask& m) {
-  p->mask = m.ptr, p->mask_kind = m.kind;
+  p->mask = m.t.defined() ? m.t.data_ptr() : nullptr, p->mask_kind = m.kind;
   for (int i = 0; i < 3; ++i) p->mask_strides[i] = m.strides[i];
 }
 
@@ -218,6 +216,8 @@ void check_ints(const Tensor& kv_lens, const Tensor& status, const Tensor& q) {
 int32_t* ints_ptr(const Tensor& t) { return t.defined() ? static_cast<int32_t*>(t.data_ptr()) : nullptr; }
 
 // --------------------------------------------------------------------------------------------- attention --
+Tensor same_memory(const Tensor& t) { return t.defined() ? t.variable_data() : Tensor(); }
+
 struct FwdResult {
   Tensor o, lse;
 };
@@ -284,28 +284,31 @@ void check_bwd(const Tensor& dO, const Tensor& q, const Tensor& k, const Tensor&
 }
 
 // What FuncSDPAttention::backward (src/Function/FuncNNLayer.h:267) leaves unimplemented: the forward saves (O, LSE)
-// and hands dQ, dK, dV to autograd.  The mask and the lengths receive no gradient.
+// and hands dQ, dK, dV to autograd.  What it saves goes through saved-tensor hooks, but for the mask and the lengths, which
+// receive no gradient.
 struct AttentionBackward : public torch::autograd::Node {
-  SavedVariable q, k, v, o;
-  Tensor lse, kv_lens;
+  SavedVariable q, k, v, o, lse;
+  Tensor kv_lens;  // as the mask: over the caller's memory, not the caller's tensor, which may be pointed elsewhere meanwhile
   Mask mask;
   int mode;
   float scale;
   std::string name() const override { return "FuncSDPAttentionBackward"; }
   void release_variables() override {
-    q.reset_data(), k.reset_data(), v.reset_data(), o.reset_data();
-    lse.reset(), kv_lens.reset(), mask = Mask();
+    std::lock_guard<std::mutex> lock(mutex_);
+    q.reset_data(), k.reset_data(), v.reset_data(), o.reset_data(), lse.reset_data();
+    kv_lens.reset(), mask = Mask();
   }
   variable_list apply(variable_list&& grads) override {
     variable_list out(3);
     Tensor dO = grads[0];
     if (!dO.defined()) return out;
+    std::lock_guard<std::mutex> lock(mutex_);
     at::NoGradGuard no_grad;
-    const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this());
+    const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this()), lt = lse.unpack();
     if (dO.stride(3) != 1) dO = dO.contiguous();
-    check_bwd(dO, qt, kt, vt, ot, lse);
+    check_bwd(dO, qt, kt, vt, ot, lt);
     const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), task_should_compute_output(2)};
-    BwdResult r = attn_bwd(dO, qt, kt, vt, ot, lse, mode, scale, kv_lens, needs, mask);
+    BwdResult r = attn_bwd(dO, qt, kt, vt, ot, lt, mode, scale, kv_lens, needs, mask);
     for (int i = 0; i < 3; ++i) out[i] = std::move(r.g[i]);
     return out;
   }
@@ -377,10 +380,14 @@ struct LinearBackward : public torch::autograd::Node {
   at::DimVector in_shape;
   bool has_bias;
   std::string name() const override { return "FuncLinearBackward"; }
-  void release_variables() override { x2.reset_data(), w.reset_data(); }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x2.reset_data(), w.reset_data();
+  }
   variable_list apply(variable_list&& grads) override {
     variable_list out(3);
     if (!grads[0].defined()) return out;
+    std::lock_guard<std::mutex> lock(mutex_);
     at::NoGradGuard no_grad;
     const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), has_bias && task_should_compute_output(2)};
     LinearGrads r = linear_bwd(grads[0], x2.unpack(), w.unpack(), in_shape, needs);
@@ -492,7 +499,8 @@ PyObject* py_sdp_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
       auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
       node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
       node->q = SavedVariable(q, false), node->k = SavedVariable(k, false), node->v = SavedVariable(v, false);
-      node->lse = r.lse, node->kv_lens = kv_lens, node->mask = mask, node->mode = mode, node->scale = scale;
+      node->lse = SavedVariable(r.lse, false), node->kv_lens = same_memory(kv_lens), node->mask = mask;
+      node->mask.t = same_memory(mask.t), node->mode = mode, node->scale = scale;
       torch::autograd::set_history(r.o, node);
       node->o = SavedVariable(r.o, true);
     }
