@@ -100,3 +100,21 @@ def test_mask_and_lengths_pointed_elsewhere_before_the_backward(kind):
     mask.set_(torch.empty(1, dtype=mask.dtype, device="cuda"))
     lens.set_(torch.empty(2, dtype=torch.int32, device="cuda").fill_(1))
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, x, g), want))
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_no_gradient_from_what_follows_is_a_gradient_of_zeros(which):
+    class Drop(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, grad):
+            return None
+
+    f, inputs = _ops()[which]
+    x = [t.requires_grad_() for t in inputs()]
+    Drop.apply(f(*x)).float().sum().backward()
+    for t in x:
+        assert t.grad is not None and not bool(t.grad.any())

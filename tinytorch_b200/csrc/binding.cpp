@@ -216,6 +216,11 @@ void check_ints(const Tensor& kv_lens, const Tensor& status, const Tensor& q) {
 int32_t* ints_ptr(const Tensor& t) { return t.defined() ? static_cast<int32_t*>(t.data_ptr()) : nullptr; }
 
 // --------------------------------------------------------------------------------------------- attention --
+// The output's gradient; zeros where what follows gave none, so that the inputs get gradients of zeros and not none.
+Tensor gradient_of(const torch::autograd::Node& node, const variable_list& grads) {
+  return grads[0].defined() ? grads[0] : node.input_metadata(0).zeros_like();
+}
+
 Tensor same_memory(const Tensor& t) { return t.defined() ? t.variable_data() : Tensor(); }
 
 struct FwdResult {
@@ -300,8 +305,7 @@ struct AttentionBackward : public torch::autograd::Node {
   }
   variable_list apply(variable_list&& grads) override {
     variable_list out(3);
-    Tensor dO = grads[0];
-    if (!dO.defined()) return out;
+    Tensor dO = gradient_of(*this, grads);
     std::lock_guard<std::mutex> lock(mutex_);
     at::NoGradGuard no_grad;
     const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = o.unpack(shared_from_this()), lt = lse.unpack();
@@ -386,11 +390,11 @@ struct LinearBackward : public torch::autograd::Node {
   }
   variable_list apply(variable_list&& grads) override {
     variable_list out(3);
-    if (!grads[0].defined()) return out;
+    const Tensor dY = gradient_of(*this, grads);
     std::lock_guard<std::mutex> lock(mutex_);
     at::NoGradGuard no_grad;
     const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), has_bias && task_should_compute_output(2)};
-    LinearGrads r = linear_bwd(grads[0], x2.unpack(), w.unpack(), in_shape, needs);
+    LinearGrads r = linear_bwd(dY, x2.unpack(), w.unpack(), in_shape, needs);
     for (int i = 0; i < 3; ++i) out[i] = std::move(r.g[i]);
     return out;
   }
