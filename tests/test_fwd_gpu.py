@@ -167,3 +167,13 @@ def test_config3_gqa_fp16_slices(oracle):
         wo, wl = oracle.fwd(qn, kn, vn, causal=True)
         assert np.abs(to_np(o[b:b + 1, hk * 4:hk * 4 + 4]) - wo).max() <= TOL_ABS_16BIT
         assert np.abs(to_np(lse[b:b + 1, hk * 4:hk * 4 + 4]) - wl).max() <= 2e-3
+
+
+def test_scale_that_is_not_a_number():
+    """... is not the default scale: the scores are NaN.  (The decode scan takes no score that is NaN for a key that takes part.)"""
+    from tinytorch_b200 import function, op
+    q, k, v = (make((1, 2, 70, 64), torch.float32, 95 + i)[0] for i in range(3))
+    nan = float("nan")
+    assert bool(torch.isnan(op.sdpAttentionFwd(q, k, v, scale=nan)[0]).all())
+    assert bool(torch.isnan(function.sdpAttention(q, k, v, scale=nan)).all())
+    assert not bool(op.sdpAttentionDecode(q[:, :, :1], k, v, scale=nan)[0].any())

@@ -27,6 +27,7 @@
 
 #include <cmath>
 #include <cstdarg>
+#include <optional>
 
 #include "../../include/tt_fused.h"
 
@@ -146,8 +147,8 @@ Tensor empty(at::IntArrayRef sizes, at::ScalarType dt, const at::Device& dev) {
 }
 
 // The reference's default scale 1/sqrt(D) (src/Function/FuncNNLayer.h:235) where the caller gave none.
-float scale_or_default(double scale, int64_t D) {
-  return std::isnan(scale) ? static_cast<float>(1.0 / std::sqrt(static_cast<double>(D))) : static_cast<float>(scale);
+float scale_or_default(const std::optional<double>& scale, int64_t D) {
+  return static_cast<float>(scale ? *scale : 1.0 / std::sqrt(static_cast<double>(D)));
 }
 
 template <typename P>
@@ -451,8 +452,8 @@ bool needs_python_function(std::initializer_list<const Tensor*> inputs) {
     if (t->defined() && t->_fw_grad(0).defined()) return true;
   return false;
 }
-double scale_arg(PyObject* o) {  // NaN stands for "not given"
-  if (o == Py_None) return std::nan("");
+std::optional<double> scale_arg(PyObject* o) {
+  if (o == Py_None) return std::nullopt;
   const double d = PyFloat_AsDouble(o);
   if (d == -1.0 && PyErr_Occurred()) throw python_error();
   return d;
