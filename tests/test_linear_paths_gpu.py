@@ -75,3 +75,18 @@ def test_blocks_beyond_the_edge_between_full_tiles(M, N):
         _check(y, x.double(), w.double().t(), None, torch.bfloat16)
         for _ in range(20):
             assert torch.equal(fused.linear(x, w), y)
+
+
+@pytest.mark.parametrize("first,width", [(3, 264), (0, 267), (8, 272), (1, 272)])
+def test_gradients_that_are_parts_of_larger_ones(first, width):
+    """dY at any offset and row stride, for every choice of gradients."""
+    from tinytorch_b200 import fused
+    g = torch.Generator("cuda").manual_seed(9)
+    M, K, N = 33, 72, 256
+    x, w, b = (torch.randn(s, device="cuda", generator=g).bfloat16().requires_grad_() for s in ((M, K), (N, K), (N,)))
+    dy = torch.randn(M, width, device="cuda", generator=g).bfloat16()[:, first:first + N]
+    y = fused.linear(x, w, b)
+    want = torch.autograd.grad(y, (x, w, b), dy.contiguous(), retain_graph=True)
+    for pick in ((0, 1, 2), (0,), (1,), (2,), (1, 2)):
+        got = torch.autograd.grad(y, [(x, w, b)[i] for i in pick], dy, retain_graph=True)
+        assert all(torch.equal(a, want[i]) for a, i in zip(got, pick))

@@ -358,13 +358,21 @@ Tensor rows_of(const Tensor& t) {  // [.., C] as [rows, C] with contiguous colum
   return r;
 }
 
+// ... that start on 16 bytes, as the kernels read them: a gradient may be a part of a larger one (the split of a projection,
+// a concatenation), at any offset and row stride, and is copied then
+Tensor aligned_rows_of(const Tensor& t) {
+  Tensor r = rows_of(t);
+  const bool aligned = reinterpret_cast<uintptr_t>(r.data_ptr()) % 16 == 0 && (r.size(0) <= 1 || r.stride(0) % 8 == 0);
+  return aligned ? r : r.clone(at::MemoryFormat::Contiguous);
+}
+
 // function::FuncLinear::backward (src/Function/FuncNNLayer.h:20-34)
 struct LinearGrads {
   Tensor g[3];
 };
 LinearGrads linear_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, at::IntArrayRef dx_shape, const bool (&needs)[3]) {
   LinearGrads r;
-  const Tensor g2 = rows_of(dy);
+  const Tensor g2 = aligned_rows_of(dy);
   // the products contract over the slow dimension of W, and of dY and X: read as they are stored
   if (needs[0]) {  // dX[M,K] = dY[M,N] W[N,K]
     r.g[0] = empty(dx_shape, g2.scalar_type(), g2.device());
