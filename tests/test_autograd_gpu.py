@@ -118,3 +118,15 @@ def test_no_gradient_from_what_follows_is_a_gradient_of_zeros(which):
     Drop.apply(f(*x)).float().sum().backward()
     for t in x:
         assert t.grad is not None and not bool(t.grad.any())
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("pick", [(2,), (1, 2), (0, 1, 2)])
+def test_the_bias_gradient_can_be_differentiated_again(native, pick):
+    from tinytorch_b200 import fused
+    x = [t.requires_grad_() for t in _projection()]
+    y = (fused.linear if native else fused.FuncLinear.apply)(*x)
+    dy, c = torch.randn_like(y).requires_grad_(), torch.randn_like(x[2])
+    got = torch.autograd.grad(y, [x[i] for i in pick], dy, create_graph=True)
+    assert torch.equal(torch.autograd.grad(got[-1], dy, c)[0], c.expand_as(dy))
+    assert all(torch.equal(a, b) for a, b in zip(got, torch.autograd.grad(fused.linear(*x), [x[i] for i in pick], dy.detach())))

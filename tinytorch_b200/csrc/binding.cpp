@@ -401,10 +401,16 @@ struct LinearBackward : public torch::autograd::Node {
     variable_list out(3);
     const Tensor dY = gradient_of(*this, grads);
     std::lock_guard<std::mutex> lock(mutex_);
+    bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), has_bias && task_should_compute_output(2)};
+    if (needs[2] && at::GradMode::is_enabled() && dY.requires_grad()) {
+      // create_graph: db is linear in dY and can be differentiated again (dX and dW cannot)
+      out[2] = dY.reshape({-1, dY.size(-1)}).to(at::kFloat).sum(0).to(dY.scalar_type());
+      needs[2] = false;
+    }
     at::NoGradGuard no_grad;
-    const bool needs[3] = {task_should_compute_output(0), task_should_compute_output(1), has_bias && task_should_compute_output(2)};
     LinearGrads r = linear_bwd(dY, x2.unpack(), w.unpack(), in_shape, needs);
-    for (int i = 0; i < 3; ++i) out[i] = std::move(r.g[i]);
+    for (int i = 0; i < 3; ++i)
+      if (needs[i]) out[i] = std::move(r.g[i]);
     return out;
   }
 };

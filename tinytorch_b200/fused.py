@@ -52,7 +52,11 @@ class FuncLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         x2, w = ctx.saved_tensors
-        dx, dw, db = _capi.native().linear_bwd(grad, x2, w, *ctx.needs_input_grad)
+        need_dx, need_dw, need_db = ctx.needs_input_grad
+        again = need_db and torch.is_grad_enabled() and grad.requires_grad  # create_graph: db can be differentiated again
+        dx, dw, db = _capi.native().linear_bwd(grad, x2, w, need_dx, need_dw, need_db and not again)
+        if again:
+            db = grad.reshape(-1, grad.shape[-1]).float().sum(0).to(grad.dtype)
         return dx if dx is None else dx.reshape(ctx.in_shape), dw, db
 
 
