@@ -76,7 +76,8 @@ typedef struct tt_silu_mul_params {
  *   dW[N,K] = dY^T X   x = dY (stored [contraction M, N]), w = X (stored [contraction M, K]),
  *                      x_t = w_t = 1; K (the contraction) may then be any size
  * x_sum (optional, with x_t): [M] receives the sums of x over the contraction, in the tensor
- * dtype (fp32 accumulation): db = sum of dY over its rows, beside dW. */
+ * dtype (fp32 accumulation): db = sum of dY over its rows, beside dW; with w and y both NULL
+ * the sums alone. */
 typedef struct tt_linear_params {
   uint32_t struct_size;
   int32_t dtype;

@@ -129,3 +129,15 @@ def test_python_ops_refuse_cpu_tensors():
         F.siluMul(torch.zeros(2, 8))
     with pytest.raises(ValueError):
         F.fusedAddRmsNorm(torch.zeros(2, 8), torch.zeros(2, 8), torch.zeros(8), 1e-5)
+
+
+def test_column_sums_alone_are_asked_for_with_both_operands_absent():
+    lib = _capi.lib()
+    p = _capi.LinearParams()
+    p.struct_size = C.sizeof(p)
+    p.dtype, p.M, p.N, p.K, p.x, p.x_sum = 2, 64, 8, 33, 0x1000, 0x2000
+    assert lib.tt_linear(C.byref(p)) == -3    # x_sum goes with x_t
+    p.x_t, p.y = 1, 0x3000
+    assert lib.tt_linear(C.byref(p)) == -1    # y without w
+    p.y, p.x = None, 0x1004
+    assert lib.tt_linear(C.byref(p)) == -5    # x is still looked at

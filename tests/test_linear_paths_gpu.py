@@ -90,3 +90,28 @@ def test_gradients_that_are_parts_of_larger_ones(first, width):
     for pick in ((0, 1, 2), (0,), (1,), (2,), (1, 2)):
         got = torch.autograd.grad(y, [(x, w, b)[i] for i in pick], dy, retain_graph=True)
         assert all(torch.equal(a, want[i]) for a, i in zip(got, pick))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N", [(1, 8), (2, 128), (63, 136), (129, 256), (4097, 1000)])
+def test_bias_gradient_alone(dtype, M, N):
+    """The column sums without a product beside them: the same sums as with one, every row counted."""
+    from tinytorch_b200 import fused
+    g = torch.Generator("cuda").manual_seed(M + N)
+    x, w = (torch.randn(s, device="cuda", generator=g).to(dtype) for s in ((M, 64), (N, 64)))
+    b = torch.randn(N, device="cuda", generator=g).to(dtype).requires_grad_()
+    dy = torch.randn(M, N, device="cuda", generator=g).to(dtype)
+    db, = torch.autograd.grad(fused.linear(x, w, b), b, dy)
+    _check(db[:, None], dy.double().t(), torch.ones(M, 1, device="cuda", dtype=torch.float64), None, dtype)
+    w.requires_grad_()
+    assert torch.equal(db, torch.autograd.grad(fused.linear(x, w, b), (w, b), dy)[1])
+
+
+def test_gradients_of_no_rows():
+    from tinytorch_b200 import fused
+    x, w, b = (torch.randn(s, device="cuda").bfloat16().requires_grad_() for s in ((3, 0, 64), (40, 64), (40,)))
+    for pick in ((x, w, b), (b,)):
+        y = fused.linear(x, w, b)
+        assert y.shape == (3, 0, 40)
+        for t, d in zip(pick, torch.autograd.grad(y, pick, torch.empty_like(y))):
+            assert d.shape == t.shape and not bool(d.any())

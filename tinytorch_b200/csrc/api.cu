@@ -428,19 +428,25 @@ int tt_linear(const tt_linear_params* p) {
   if (p->M < 0 || p->N <= 0 || p->K <= 0 || p->M > 0x7fffffff || p->N > 0x7fffffff || p->K > 0x7fffffff)
     return TT_ATTN_ERR_SHAPE;
   if (p->M == 0) return TT_ATTN_OK;
-  if (!p->x || !p->w || !p->y) return TT_ATTN_ERR_NULL;
   const bool x_t = ext && p->x_t != 0, w_t = ext && p->w_t != 0;
   void* x_sum = ext ? p->x_sum : nullptr;
+  const bool sums_only = x_sum && !p->w && !p->y;
+  if (!p->x || (!sums_only && (!p->w || !p->y))) return TT_ATTN_ERR_NULL;
   if (x_sum && !x_t) return TT_ATTN_ERR_SHAPE;
   const int64_t x_cols = x_t ? p->M : p->K, w_cols = w_t ? p->N : p->K;  // the contiguous dimensions
   const int64_t ldx = p->ldx ? p->ldx : x_cols, ldw = p->ldw ? p->ldw : w_cols, ldy = p->ldy ? p->ldy : p->N;
   if (ldx < x_cols || ldw < w_cols || ldy < p->N) return TT_ATTN_ERR_SHAPE;
-  if (x_cols % 8 || w_cols % 8 || p->N % 8 || ldx % 8 || ldw % 8 || ldy % 8 || !aligned16(p->x) || !aligned16(p->w) ||
+  // (sums alone: w and y, and what describes them, are not looked at any further)
+  if (sums_only ? x_cols % 8 || ldx % 8 || !aligned16(p->x) || reinterpret_cast<uintptr_t>(x_sum) % 2 : x_cols % 8 || w_cols % 8 || p->N % 8 || ldx % 8 || ldw % 8 || ldy % 8 || !aligned16(p->x) || !aligned16(p->w) ||
       !aligned16(p->y) || (p->bias && reinterpret_cast<uintptr_t>(p->bias) % 2) || reinterpret_cast<uintptr_t>(x_sum) % 2)
     return TT_ATTN_ERR_ALIGN;
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+  if (sums_only) {
+    cudaError_t e = launch_column_sums(p->dtype, p->x, x_sum, p->K, p->M, ldx, false, stream);
+    return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
+  }
   const LinearCall c{p->dtype, p->x, p->w, p->bias, p->y, static_cast<int>(p->M), static_cast<int>(p->N),
                      static_cast<int>(p->K), ldx, ldw, ldy, x_t, w_t, p->status, p->device, stream};
   bool persistent = false;

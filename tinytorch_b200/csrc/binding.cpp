@@ -336,14 +336,14 @@ bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
 // Row stride of a matrix with contiguous columns (a single row's stride may be anything).
 int64_t row_stride(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
 
-// y[M, N] (dense memory) = x[M, K] w[N, K]^T + bias; x_t / w_t: the operand is given as [K, M] / [K, N]
+// y[M, N] (dense memory) = x[M, K] w[N, K]^T + bias; x_t / w_t: the operand is given as [K, M] / [K, N]; without y only x_sum
 void linear_raw(const Tensor& x, bool x_t, const Tensor& w, bool w_t, const Tensor& bias, const Tensor& y, const Tensor& status,
                 const Tensor& x_sum) {
   tt_linear_params p{};
   set_common(&p, x);
   p.dtype = dtype_of(x.scalar_type());
   p.M = x.size(x_t ? 1 : 0), p.K = x.size(x_t ? 0 : 1), p.N = w.size(w_t ? 1 : 0);
-  p.x = x.data_ptr(), p.w = w.data_ptr(), p.y = y.data_ptr();
+  p.x = x.data_ptr(), p.w = y.defined() ? w.data_ptr() : nullptr, p.y = y.defined() ? y.data_ptr() : nullptr;
   p.bias = bias.defined() ? bias.data_ptr() : nullptr;
   p.ldx = row_stride(x), p.ldw = row_stride(w), p.ldy = p.N;
   p.status = ints_ptr(status);
@@ -373,6 +373,12 @@ struct LinearGrads {
 LinearGrads linear_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, at::IntArrayRef dx_shape, const bool (&needs)[3]) {
   LinearGrads r;
   const Tensor g2 = aligned_rows_of(dy);
+  if (g2.size(0) == 0) {  // sums of nothing
+    const at::IntArrayRef shapes[3] = {dx_shape, w.sizes(), w.sizes().slice(0, 1)};
+    for (int i = 0; i < 3; ++i)
+      if (needs[i]) r.g[i] = at::zeros(shapes[i], g2.options());
+    return r;
+  }
   // the products contract over the slow dimension of W, and of dY and X: read as they are stored
   if (needs[0]) {  // dX[M,K] = dY[M,N] W[N,K]
     r.g[0] = empty(dx_shape, g2.scalar_type(), g2.device());
@@ -383,7 +389,7 @@ LinearGrads linear_bwd(const Tensor& dy, const Tensor& x2, const Tensor& w, at::
     r.g[1] = empty({g2.size(1), x2.size(1)}, g2.scalar_type(), g2.device());
     linear_raw(g2, true, x2, true, Tensor(), r.g[1], Tensor(), r.g[2]);
   } else if (needs[2]) {
-    r.g[2] = g2.to(at::kFloat).sum(0).to(g2.scalar_type());
+    linear_raw(g2, true, x2, true, Tensor(), Tensor(), Tensor(), r.g[2]);  // (the sums alone)
   }
   return r;
 }
