@@ -13,9 +13,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens,mask", [
-    (1, 8, 1, 130, 130, True, None, None),         # walks of 8 .. 24 steps
-    (1, 2, 2, 500, 500, True, None, None),         # late key tiles and early query tiles: fewer steps than shares
-    (2, 4, 2, 65, 300, False, (300, 70), None),    # key tiles without keys
+    (1, 8, 1, 130, 130, True, None, None),         # walks of 8 .. 24 steps in 8 shares
+    (1, 2, 2, 500, 500, True, None, None),         # late key tiles and early query tiles: fewer steps than shares (8; D = 128: 4)
+    (2, 4, 2, 65, 300, False, (300, 70), None),    # key tiles without keys, 4 shares
+    (1, 2, 2, 100, 65, False, None, None),         # 2 shares
+    (8, 8, 8, 100, 100, True, None, None),         # not divided
     (1, 3, 1, 200, 129, False, None, "f32"),
     (2, 2, 1, 100, 190, False, None, "bool"),
 ])

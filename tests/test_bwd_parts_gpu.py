@@ -13,11 +13,11 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens", [
-    (1, 4, 1, 640, 640, True, None),                   # 20 .. 4 steps per key tile in 8 shares
-    (2, 3, 1, 300, 500, False, (500, 129)),            # 9 steps in up to 8 shares, key tiles without keys
+    (1, 4, 1, 640, 640, True, None),                   # 20 .. 4 steps per key tile in 7 shares
+    (2, 3, 1, 300, 500, False, (500, 129)),            # 9 steps in 5 shares, key tiles without keys
     (1, 2, 2, 1100, 1100, True, None),
     (1, 4, 2, 260, 700, "bottom-right", None),
-    (1, 2, 1, 200, 130, False, None),                  # a ragged second key tile
+    (1, 2, 1, 200, 130, False, None),                  # a ragged second key tile (D = 64: not divided)
 ])
 def test_divided_key_tiles(oracle, dt, D, B, Hq, Hkv, L, S, causal, lens):
     from tinytorch_b200 import op

@@ -13,12 +13,14 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens,mask", [
-    (1, 2, 1, 70, 256, False, None, False),             # 4 key tiles in 2 shares
+    (1, 2, 1, 70, 256, False, None, False),             # 4 key tiles in 4 shares
     (1, 2, 2, 64, 1030, False, None, False),            # 17 in 8
     (2, 3, 3, 500, 500, True, None, False),             # 1 .. 8 tiles in 4 shares: early query tiles leave some empty
     (3, 2, 1, 100, 700, "bottom-right", (700, 30, 0), False),
     (2, 2, 1, 65, 600, False, (600, 1), True),
-    (1, 1, 1, 1, 65, False, None, False),               # not divided
+    (1, 3, 3, 200, 128, False, None, False),            # 2 in 2
+    (16, 8, 4, 100, 300, False, None, False),           # 5 in 2 (D = 128: not divided)
+    (1, 1, 1, 1, 65, False, None, False),               # 2 in 2
 ])
 def test_divided_keys_fp32(oracle, D, B, Hq, Hkv, L, S, causal, lens, mask):
     from tinytorch_b200 import op

@@ -1,5 +1,6 @@
 """GPU: the prefill forward where a query block's keys are divided between the halves of a CTA and among clusters (few
-queries, many keys), and where the two query blocks of an item belong to different heads, against the CPU oracle.  Tolerances: those of test_fwd_gpu.py."""
+queries, many keys), beside the pairs of blocks that shorter walks get, and where the two query blocks of an item belong to
+different heads, against the CPU oracle.  The comments say what plan_of takes on 148 SMs.  Tolerances: those of test_fwd_gpu.py."""
 import numpy as np
 import pytest
 import torch
@@ -12,16 +13,20 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,Hq,Hkv,L,S,causal,lens", [
-    (1, 2, 2, 128, 768, False, None),                 # 6 key tiles, two blocks
-    (1, 3, 1, 100, 384, False, None),                 # an odd number of key tiles: the halves differ
-    (2, 20, 20, 600, 600, True, None),                # 200 blocks: CTAs with several items
-    (1, 2, 1, 64, 100, False, None),                  # one key tile: a half without any
-    (1, 4, 1, 129, 1537, "bottom-right", None),       # clusters of 4, a block of one row
+    (1, 2, 2, 128, 768, False, None),                 # halves, 6 key tiles
+    (1, 3, 1, 100, 384, False, None),                 # pairs, 3 key tiles
+    (2, 20, 20, 600, 600, True, None),                # pairs, 200 blocks
+    (1, 2, 1, 64, 100, False, None),                  # pairs, one key tile
+    (1, 4, 1, 129, 1537, "bottom-right", None),       # clusters of 8, a block of one row
     (2, 3, 1, 40, 3100, "bottom-right", (3100, 700)),  # clusters of 8, an odd number of blocks, CTAs without keys
-    (2, 2, 2, 300, 3072, False, (1, 0)),              # a sequence without keys, one with a single key
-    (3, 8, 2, 64, 1100, False, (1100, 128, 129)),
-    (1, 4, 4, 512, 900, True, None),                  # causal: too few tiles to divide
-    (1, 2, 1, 1024, 1024, True, None),                # ... and shares of a triangle
+    (2, 2, 2, 300, 3072, False, (1, 0)),              # clusters of 8: a sequence without keys, one with a single key
+    (3, 8, 2, 64, 1100, False, (1100, 128, 129)),      # halves (D = 128: clusters of 4): one key tile, a half without any
+    (1, 4, 4, 512, 900, True, None),                  # halves, 1 .. 4 key tiles
+    (1, 2, 1, 1024, 1024, True, None),                # halves (D = 128: clusters of 4): shares of a triangle
+    (1, 4, 4, 64, 520, False, None),                  # halves, an odd number of key tiles
+    (2, 40, 8, 129, 700, "bottom-right", (700, 131)),  # halves, 160 blocks: CTAs with a second item
+    (2, 20, 20, 100, 1930, False, (1930, 60)),        # clusters of 2, one CTA of which has no keys
+    (1, 20, 4, 64, 1700, False, None),                # clusters of 4
 ])
 def test_keys_divided_among_a_cluster(oracle, dt, D, B, Hq, Hkv, L, S, causal, lens):
     from tinytorch_b200 import op

@@ -43,8 +43,8 @@ def test_linear_shapes(fused, dt, M, N, K, bias):
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("M,N,K", [(2100, 4712, 200), (4096, 2560, 72), (2304, 4352, 1032)])
 def test_linear_tall_tiles(fused, dt, M, N, K):
-    # enough 256 x 256 tiles to fill the machine: the kernel takes 256-row tiles (two accumulators sharing a
-    # slice of w).  Ragged in every dimension; in the first shape the last tile's lower half lies wholly beyond M.
+    # enough 256 x 256 tiles to fill the machine: the persistent CTA pairs.
+    # Ragged in every dimension; in the first shape the last tile's lower half lies wholly beyond M.
     # The oracle runs on a band of rows from every part of the tile grid.
     from tinytorch_b200 import fused as F
     x, xn = make((M, K), DTYPES[dt], 631, std=0.5)
@@ -108,8 +108,7 @@ def test_full_size_projection_rows(fused):
 def test_autograd_matches_reference_gradients(fused):
     from tinytorch_b200 import fused as F
     g = np.load(os.path.join(GOLDEN, "ref_seeded_linear.npz"))
-    # pad the fixture (M=37, N=40, K=72) is fine for the forward; the backward contracts over M and N, which must be
-    # multiples of 8 for the kernel: use the leading 32 rows
+    # (the leading 32 of the fixture's 37 rows; any number of rows: test_linear_paths_gpu.py)
     x = torch.from_numpy(g["x"][:32]).cuda().bfloat16().requires_grad_(True)
     w = torch.from_numpy(g["w"]).cuda().bfloat16().requires_grad_(True)
     b = torch.from_numpy(g["b"]).cuda().bfloat16().requires_grad_(True)
