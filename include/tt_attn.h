@@ -43,7 +43,7 @@
  *    (src/Operation/OpTransformCpu.h:399-442) without materialising the copy.
  *  - All work is enqueued on `stream` of `device`; no entry point synchronises
  *    the host, allocates device memory itself, or aborts.  Scratch memory comes
- *    from `workspace` (>= tt_attn_workspace_bytes) or, when that is NULL, from
+ *    from `workspace` (see tt_attn_workspace_bytes) or, when that is NULL, from
  *    the allocator hook, which the TinyTorch shim backs with
  *    getCUDACachedAllocator(device) (src/Tensor/Allocator.cpp:117-139); blocks
  *    are handed back through the hook as soon as the last launch is enqueued,
@@ -267,16 +267,17 @@ TT_ATTN_API int tt_attn_decode_append(const tt_attn_decode_append_params* p);
  * it uses allocates or frees memory: the per-split partial results go to a fixed
  * TT_ATTN_STATIC_SCRATCH_BYTES array inside the library image (resident on every
  * GPU that loads the library, until the process exits).
- *  - A problem whose tt_attn_workspace_bytes(TT_ATTN_KIND_DECODE, ...) exceeds
- *    TT_ATTN_STATIC_SCRATCH_BYTES is refused with TT_ATTN_ERR_TOO_LARGE.
+ *  - A problem whose partial results do not fit TT_ATTN_STATIC_SCRATCH_BYTES, even with the long
+ *    pieces that a large batch is divided into, is refused with TT_ATTN_ERR_TOO_LARGE.
  *  - The first call on each device looks up the array's device address (once,
  *    with that device current); make that first call before starting any stream
  *    capture.
  *  - All calls on a device share the one array; calls that overlap in time on the
  *    same GPU race on it, so keep them on one stream or otherwise ordered.  It is
- *    never cleared as a whole: every launch writes what it later reads, and the one
- *    4-byte work counter that grouped-query shapes use is reset by a memset enqueued
- *    on the call's stream.
+ *    never cleared as a whole: a launch reads only the partial results it has written
+ *    (pieces without rows leave none), and the one 4-byte work counter that
+ *    grouped-query shapes with more pieces than CTAs use is reset by a small kernel
+ *    enqueued on the call's stream.
  * This entry point has no counterpart in the reference. */
 #define TT_ATTN_STATIC_SCRATCH_BYTES (24u << 20)
 TT_ATTN_API int tt_attn_decode_static(const tt_attn_decode_params* p);
@@ -289,9 +290,16 @@ TT_ATTN_API int tt_attn_decode_static(const tt_attn_decode_params* p);
 TT_ATTN_API int tt_attn_selftest_wait_expiry(int device, void* stream, uint64_t limit_ns, int32_t* status,
                                              unsigned long long* waited_ns);
 
-/* Scratch bytes the given call needs (0 if none; the fp16/bf16 forward needs a
- * 256-byte block for its work counter).  Skv is the cache capacity
- * for TT_ATTN_KIND_DECODE. */
+/* Scratch bytes with which the given call runs at its best (0 if none).  Skv is the cache
+ * capacity for TT_ATTN_KIND_DECODE.  A buffer sized for a batch serves every smaller one,
+ * although a small batch, which is divided further, would like more:
+ *  - forward, fp16 / bf16: a work counter (256 bytes) and two words per sequence, which only a
+ *    padding mask uses; with 256 bytes such a mask is read in full;
+ *  - backward: rowsum(dO o O) and, fp16 / bf16, the fp32 dQ accumulator and the words above;
+ *    where key tiles are few also shares of dK / dV, as many as fit;
+ *  - decode: partial results of the pieces a cache is divided into, in longer pieces if need be,
+ *    and a work counter for several query heads per key head.
+ * TT_ATTN_ERR_WORKSPACE comes when not even the least of this fits. */
 TT_ATTN_API size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D);
 
 TT_ATTN_API const char* tt_attn_strerror(int status);

@@ -341,7 +341,7 @@ int split_of(const BwdArgs& a, int D) {
   for (int c = 1, lg = 0; c <= 8; c *= 2, ++lg) {
     const double walk = (longest + c - 1) / c * step;
     // (clusters of 8 do not fill every GPC)
-    const double us = std::max(walk + 1.5 * lg, (work + ctas * c * fixed) / 148 * (c == 8 ? 1.1 : 1.0) + tail * walk);
+    const double us = std::max(walk + 1.5 * lg, (work + ctas * c * fixed) / kSms * (c == 8 ? 1.1 : 1.0) + tail * walk);
     if (us < best_us) best = c, best_us = us;
   }
   return best;

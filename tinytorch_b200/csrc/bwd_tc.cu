@@ -1502,7 +1502,7 @@ cudaError_t launch_g(int dtype, int D, const BwdArgs& a, int device, cudaStream_
 // Measured, us: 32/8 heads x 3000 D128 causal 305 -> 256; 2 x 2660, 16/4 heads D64 160 -> 122; 8000, 4/2 heads D128 370 ->
 // 207; 600, 2 x 8/2 heads D64 51 -> 29; undivided 2048, 8 x 16 heads D64 causal 252 (divided in two: 350).
 int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal) {
-  constexpr double kSms = 148, kItem = 1.2;
+  constexpr double kItem = 1.2;
   const double tiles = static_cast<double>((Skv + BM - 1) / BM) * Hkv * B, step_us = D == 128 ? 2.9 : 1.6;
   const int group = Hq / Hkv, n = (Lq + BQ - 1) / BQ * group;
   if (tiles > 4 * kSms) return 1;

@@ -13,6 +13,10 @@ namespace ttattn {
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
+// SMs of the part this library is written for: plans that the workspace query makes too, without a device at hand, divide by
+// it (the planners of the projections and of the prefill forward ask the device).
+constexpr int kSms = 148;
+
 // Status bits a kernel may OR into the caller's status word.
 constexpr int kStatusWaitExpired = 1;
 constexpr int kStatusBadSmemAlign = 2;   // dynamic shared memory did not start on a 1024-byte boundary
@@ -106,7 +110,7 @@ struct DecodeArgs {
   int rope_interleaved;            // pairs (2i, 2i+1) instead of (i, i + D/2)
   int32_t* new_lens;               // optional [B]: kv_lens[b] + 1
   int32_t* status;
-  int* sched;                      // tensor-core path: work counter in scratch memory, zeroed by the launcher
+  int* sched;                      // tensor-core path: work counter in scratch memory, zeroed ahead of the scan (see chained)
   void* q_rot;                     // append on the tensor-core path: scratch [B, Hq, D] for the rotated q
   int32_t* lens_scratch;           // ... and [B] for the lengths after the append
   int chained;                     // tensor-core path: the kernel before this one in the stream has zeroed the
@@ -279,15 +283,6 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) {
 // Query i sees key j under a causal mask iff j <= i + causal_shift(...).
 __host__ __device__ __forceinline__ int causal_shift(int causal, int kv_len, int Lq) {
   return causal == TT_ATTN_CAUSAL_BOTTOM_RIGHT ? kv_len - Lq : 0;
-}
-
-// What the mask adds to the scaled score of one (query, key) pair, in log2
-// units: 0 or -inf for a boolean mask.  `off` is the element offset of the pair.
-template <typename T>
-__device__ __forceinline__ float mask_bias2(const MaskArgs& m, int64_t off) {
-  if (m.kind == TT_ATTN_MASK_BOOL) return reinterpret_cast<const uint8_t*>(m.ptr)[off] ? 0.f : -INFINITY;
-  if (m.kind == TT_ATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(m.ptr)[off] * kLog2e;
-  return to_f32<T>(reinterpret_cast<const T*>(m.ptr)[off]) * kLog2e;
 }
 
 }  // namespace ttattn

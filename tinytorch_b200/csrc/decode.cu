@@ -406,7 +406,7 @@ cudaError_t launch_t(const DecodeArgs& a, cudaStream_t stream) {
 constexpr int kScanChunk = 512, kTcChunk = 2048;  // rows of a chunk in a large batch
 void decode_plan(int B, int Hkv, int capacity, int* nsplit, int* chunk) {
   int ck = kScanChunk;
-  while (ck > 64 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 148) ck >>= 1;
+  while (ck > 64 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < kSms) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 63) / 64 * 64;
   *chunk = ck;
   *nsplit = capacity <= ck ? 1 : (capacity + ck - 1) / ck;
@@ -441,9 +441,9 @@ void decode_plan_for(int dtype, int D, int B, int Hq, int Hkv, int capacity, int
     return;
   }
   int ck = kTcChunk;
-  const long long want = D == 64 ? 592 : 296;  // two items per resident CTA (D = 64 runs two CTAs per SM)
+  const long long want = (D == 64 ? 4 : 2) * kSms;  // two items per resident CTA (D = 64 runs two CTAs per SM)
   while (ck > 512 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < want) ck >>= 1;
-  while (ck > 128 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < 74) ck >>= 1;
+  while (ck > 128 && static_cast<long long>(B) * Hkv * ((capacity + ck - 1) / ck) < kSms / 2) ck >>= 1;
   if ((capacity + ck - 1) / ck > 64) ck = (((capacity + 63) / 64) + 127) / 128 * 128;
   // three tiles in one piece take less than the second kernel (2 x 16/4 heads x 191, D64: 7.9 -> 6.0 us a call; append, 17 x 8/4
   // heads x 135, D128: 11.6 -> 9.0; at 512 rows 8.9 -> 9.4)
@@ -569,11 +569,11 @@ cudaError_t launch_decode_append(int dtype, int D, const DecodeArgs& a, cudaStre
 // until the process exits, hence the modest size.
 //
 // The array is shared by every call on a device and keeps the previous call's
-// contents.  Each launch writes every (batch, head, split) slot before the combine
-// kernel reads it; the only word that must start at zero, the tensor-core path's
-// work counter in the last 256 bytes of what a call uses, is reset by a memset on
-// the call's stream.  Two calls that overlap on the GPU (different streams) would
-// race on the array.
+// contents.  The combine kernel reads the (batch, head, split) slots that have rows,
+// which the launch before it has written; the only word that must start at zero, the
+// tensor-core path's work counter in the last 256 bytes of what a call uses, is reset
+// by a kernel on the call's stream where the counter is drawn from at all.  Two calls
+// that overlap on the GPU (different streams) would race on the array.
 namespace {
 
 constexpr size_t kStaticScratchBytes = TT_ATTN_STATIC_SCRATCH_BYTES;

@@ -318,7 +318,7 @@ cudaError_t rms_t(void* input, void* residual, const void* weight, int64_t rows,
   // threads per row: the fewest (>= 32) that keep a thread at <= 8 vectors ... but prefer
   // <= 4 so that enough loads are in flight without starving occupancy; with fewer rows than SMs as many as there are
   // vectors, up to a whole CTA per row
-  const bool few = rows < 148;
+  const bool few = rows < kSms;
   int tpr = 32;
   while (tpr < kThreads && vecs > static_cast<int64_t>(tpr) * (few ? 1 : 4)) tpr <<= 1;
   const int vpt = static_cast<int>((vecs + tpr - 1) / tpr);
@@ -342,7 +342,7 @@ cudaError_t silu_t(void* out, const void* x, int64_t rows, int64_t d, cudaStream
   const bool vec_ok = d % N == 0 && aligned16(o) && aligned16(xi);
   constexpr int kChunk = kThreads * kSiluUnroll;
   // (a handful of rows: one vector per thread, four times the CTAs)
-  const bool few = rows * ((vpr + kChunk - 1) / kChunk) < 148;
+  const bool few = rows * ((vpr + kChunk - 1) / kChunk) < kSms;
   if (vec_ok && !few && vpr >= kThreads && (vpr + kChunk - 1) / kChunk <= 65535 && rows <= 0x7fffffff) {
     dim3 grid(static_cast<unsigned>(rows), static_cast<unsigned>((vpr + kChunk - 1) / kChunk));
     const bool keep = 3 * rows * d * static_cast<int64_t>(sizeof(T)) <= kKeepBytes;
