@@ -92,13 +92,13 @@ def fwd_bytes(w):
 # launch, from one ncu capture of a reduced case of each kernel; traffic grows in proportion to the units a launch
 # processes, so the figure reported for a full launch is this ratio times the launch's algorithmic bytes.
 NCU_TRAFFIC_RATIO = {
-    "fwd_tc_kernel": (254.1 / 269.5, "profiles/fwd_tc_kernel_prefill_bf16_S4096_D128.md"),
-    "bwd_tc64_kernel": (296.3 / 270.5, "profiles/bwd_tc64_kernel_train_fp16_S2048_D64.md"),
-    "decode_kernel": (1218.2 / 1213.0, "profiles/decode_kernel_bf16_cap8192_D128.md"),
-    "decode_tc_kernel": (1271.9 / 1248.0, "profiles/decode_tc_kernel_bf16_gqa4_cap8192_D128.md"),
-    "linear_tc_kernel": (87.4 / 100.7, "profiles/linear_tc_kernel_bf16_4096x4096x4096.md"),
-    "add_rms_norm_kernel": (478.5 / 536.9, "profiles/add_rms_norm_kernel_bf16_8192x8192.md"),
-    "silu_mul_kernel": (309.3 / 352.3, "profiles/silu_mul_rows_kernel_bf16_4096x28672.md"),
+    "fwd_tc_kernel": (252.5 / 269.5, "profiles/fwd_tc_kernel_prefill_bf16_S4096_D128.md"),
+    "bwd_tc64_kernel": (295.9 / 270.5, "profiles/bwd_tc64_kernel_train_fp16_S2048_D64.md"),
+    "decode_kernel": (1217.4 / 1213.0, "profiles/decode_kernel_bf16_cap8192_D128.md"),
+    "decode_tc_kernel": (1270.1 / 1248.0, "profiles/decode_tc_kernel_bf16_gqa4_cap8192_D128.md"),
+    "linear_tc_kernel": (93.1 / 100.7, "profiles/linear_tc_kernel_bf16_4096x4096x4096.md"),
+    "add_rms_norm_kernel": (478.3 / 536.9, "profiles/add_rms_norm_kernel_bf16_8192x8192.md"),
+    "silu_mul_kernel": (308.7 / 352.3, "profiles/silu_mul_rows_kernel_bf16_4096x28672.md"),
 }
 
 
