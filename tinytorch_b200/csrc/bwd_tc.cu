@@ -104,7 +104,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 // The mask of 16 queries and this thread's key, as stored: adjacent threads read adjacent keys.  Fetched before the scores
 // arrive, all loads in flight together (one by one inside the arithmetic they made a step ten times as long): B5 H32/16
-// L1620 D64 with an additive bf16 mask 3447 -> 602 us, without a mask 340; D128, 2 x 16/4 heads x 2048: 398, 272.  `off`:
+// L1620 D64 with an additive bf16 mask 3447 -> 620 us, without a mask 380; D128, 2 x 16/4 heads x 2048: 319, 213.  `off`:
 // mask offset of (first query, this key); n_q: how many of the queries exist (0: nothing is read); a mask that is
 // the same for all rows is read once.
 __device__ __forceinline__ void fetch_mask(const MaskArgs& m, int64_t off, int n_q, uint32_t (&w)[16]) {
