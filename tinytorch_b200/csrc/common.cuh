@@ -160,7 +160,13 @@ struct LinearCall {
   int device;
   cudaStream_t stream;
 };
-cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  // *persistent: linear_tc_kernel was taken
+// Cache lines that 128 bytes of a row cost: rows of `ld` 16-bit elements that are not a multiple of a line long touch two, and five
+// sectors instead of four where they are not a multiple of a sector (from the fits in linear_tile.cu and linear_split.cu).
+inline double row_lines(int64_t ld) { return ld % 16 ? 1.74 : (ld % 64 ? 1.17 : 1.0); }
+cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  // *persistent: the CTAs let the next kernel in once all before them is complete
+// ... with tiles made to measure (linear_tile.cu): single CTAs with 128 x `bn`, or pairs with 256 x 192
+double linear_tile_us(const LinearCall& c, bool pair, int bn);  // what it, or pairs with 256 x 256, are expected to take
+cudaError_t launch_linear_tile(const LinearCall& c, bool pair, int bn);
 // ... for outputs with too few tiles to occupy the machine: contraction split over clusters (linear_split.cu)
 double linear_split_us(const LinearCall& c);  // what it is expected to take
 cudaError_t launch_linear_split(const LinearCall& c);

@@ -295,18 +295,45 @@ cudaError_t launch_bf(const LinearCall& c, int ctas) {
 
 }  // namespace
 
+namespace {
+struct Plan {
+  enum { kSplit, kTiles, kPairs } kernel;
+  bool pair;  // kTiles: the shape
+  int bn;
+};
+
+// Which kernel and which tiles.  Pairs of 256 x 256 read the fewest bytes for a product and keep the tensor pipe busy: large
+// problems (two rounds of tiles) get them, and small ones a contraction divided over clusters where that is expected to be faster
+// (linear_split.cu; always up to 128 rows).  Between the two lie problems for which a shape of linear_tile.cu puts a tile on nearly
+// every SM; it is taken where it is expected to save 6 % and 0.25 us (10 % where x is MN-major), about the error of the models.  Of 251 problems with more
+// than 128 rows that the models were not fitted to the mean is 0.94 of the time before (1.04 of the best shape's), the worst 1.03.
+Plan plan_of(const LinearCall& c) {
+  const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + BN - 1) / BN);
+  if (tiles >= sm_count(c.device) / 2 * 2) return Plan{Plan::kPairs, false, 0};
+  if (c.M <= HM) return Plan{Plan::kSplit, false, 0};
+  Plan best{Plan::kPairs, false, 0};
+  double us = linear_tile_us(c, true, BN);
+  auto take = [&](const Plan& p, double t) {
+    if (t < us) best = p, us = t;
+  };
+  take(Plan{Plan::kSplit, false, 0}, linear_split_us(c));
+  us = us * (c.x_t ? 0.9 : 0.94) - 0.25;
+  if (!c.w_t) take(Plan{Plan::kTiles, true, 192}, linear_tile_us(c, true, 192));
+  // (an MN-major w comes in blocks of 64 columns)
+  for (int bn = 64; bn <= 256; bn += c.w_t ? 64 : 32) take(Plan{Plan::kTiles, false, bn}, linear_tile_us(c, false, bn));
+  return best;
+}
+}  // namespace
+
 cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent) {
   if (persistent) *persistent = false;
   if (c.dtype != TT_ATTN_BF16 && c.dtype != TT_ATTN_F16) return cudaErrorInvalidValue;
-  // The persistent pairs where they are expected to be the faster: whole rounds of 256 x 256 tiles at 0.29 us per 64 of
-  // the contraction (or an epilogue each, where the contraction is short), 4.5 us for ramp and drain.  Few rows leave
-  // most of a 256-row tile empty, and then the weight's way from HBM is what takes the time.
+  const Plan p = plan_of(c);
+  if (p.kernel == Plan::kSplit) return launch_linear_split(c);
+  if (persistent) *persistent = true;
+  if (p.kernel == Plan::kTiles) return launch_linear_tile(c, p.pair, p.bn);
   const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + BN - 1) / BN);
   const int pairs = sm_count(c.device) / 2;
-  const double round_us = 0.29 * ((c.K + BK - 1) / BK);
-  const double pair_us = 4.5 + static_cast<double>((tiles + pairs - 1) / pairs) * (round_us > 1.6 ? round_us : 1.6);
-  if (tiles < 2 * pairs && (c.M <= HM || linear_split_us(c) < pair_us)) return launch_linear_split(c);
-  if (persistent) *persistent = true;
   const int ctas = 2 * static_cast<int>(tiles < pairs ? tiles : pairs);
   return c.dtype == TT_ATTN_BF16 ? launch_bf<true>(c, ctas) : launch_bf<false>(c, ctas);
 }

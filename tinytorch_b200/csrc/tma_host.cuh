@@ -28,27 +28,28 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [B, H, S, D] tensor, box = 64 (D) x `box_rows` (S) x 1 x 1, 128-byte swizzle; rows
-// outside the tensor read as zero and are clipped on stores.
+// [B, H, S, D] tensor, box = `box_cols` (D; 64 with the 128-byte swizzle, or 32 with the 64-byte one) x `box_rows` (S)
+// x 1 x 1; rows outside the tensor read as zero and are clipped on stores.
 inline bool make_map(CUtensorMap* m, int dtype, const void* ptr, int D, int S, int H, int B, const Str3& st,
-                     int box_rows = 128) {
+                     int box_rows = 128, int box_cols = 64) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(H),
                         static_cast<cuuint64_t>(B)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(st.s) * 2, static_cast<cuuint64_t>(st.h) * 2,
                            static_cast<cuuint64_t>(st.b) * 2};
-  cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};
+  cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows), 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(m, dtype == TT_ATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                   const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
-// [rows, cols] matrix with row stride `ld` (elements), box = 64 columns x `box_rows` rows.
-inline bool make_map_2d(CUtensorMap* m, int dtype, const void* ptr, int cols, int rows, int64_t ld, int box_rows) {
-  return make_map(m, dtype, ptr, cols, rows, 1, 1, Str3{ld * rows, ld * rows, ld}, box_rows);
+// [rows, cols] matrix with row stride `ld` (elements), box = `box_cols` columns x `box_rows` rows.
+inline bool make_map_2d(CUtensorMap* m, int dtype, const void* ptr, int cols, int rows, int64_t ld, int box_rows, int box_cols = 64) {
+  return make_map(m, dtype, ptr, cols, rows, 1, 1, Str3{ld * rows, ld * rows, ld}, box_rows, box_cols);
 }
 
 // Dense fp32 [B, H, S, D] buffer, box = 32 floats (128 bytes) x `box_rows` rows, for TMA reductions.
