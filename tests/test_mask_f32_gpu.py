@@ -1,0 +1,49 @@
+"""GPU: masks of the fp32 kernels where their tiles are staged through shared memory: boolean rows at every byte offset,
+masks that are the same for all rows, additive ones; tiles ragged in both directions; rows without any key; with and without a divided walk.
+
+Reference: the composition in fp64.  Bound: that of the fp32 tests (1e-5 of the largest element)."""
+import pytest
+import torch
+
+from gpu_util import TOL_REL_FP32
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, k, v, g, mask):
+    q, k, v = (t.double().requires_grad_() for t in (q, k, v))
+    group = q.shape[1] // k.shape[1]
+    s = q @ k.repeat_interleave(group, 1).transpose(2, 3) * q.shape[3] ** -0.5
+    s = s.masked_fill(~mask, float("-inf")) if mask.dtype == torch.bool else s + mask.double()
+    p = torch.nan_to_num(s.softmax(-1))  # a row without any key: zeros
+    o = p @ v.repeat_interleave(group, 1)
+    return (o.detach(),) + torch.autograd.grad(o, (q, k, v), g.double())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("kind", ["bool", "row", "add", "lowest"])
+@pytest.mark.parametrize("B,Hq,Hkv,L,S,offset", [
+    (1, 2, 1, 65, 131, 0),      # rows of an odd length: every alignment in turn; a divided walk
+    (2, 2, 2, 64, 64, 3),       # ... and a mask that starts in the middle of a word
+    (1, 1, 1, 1, 5, 1),
+    (9, 8, 4, 130, 193, 2),     # more CTAs than SMs
+])
+def test_staged_masks(D, kind, B, Hq, Hkv, L, S, offset):
+    from tinytorch_b200 import op
+    gen = torch.Generator("cuda").manual_seed(D + L + S + offset)
+    q, k, v, g = (torch.randn(s, device="cuda", generator=gen) for s in ((B, Hq, L, D), (B, Hkv, S, D), (B, Hkv, S, D), (B, Hq, L, D)))
+    shape = (B, 1, 1, S) if kind == "row" else (1, Hq, L, S)
+    n = torch.Size(shape).numel()
+    if kind in ("bool", "row"):
+        mask = (torch.rand(n + offset, device="cuda", generator=gen) < 0.6)[offset:].view(shape)
+        if kind == "bool" and L > 2:
+            mask[0, :, 2] = False  # a row without any key
+    else:
+        mask = torch.randn(n + offset, device="cuda", generator=gen)[offset:].view(shape)
+        if kind == "lowest":
+            mask = torch.where(mask > 0.5, torch.finfo(torch.float32).min, 0.0)
+            mask[..., 0] = 0.0
+    o, lse = op.sdpAttentionFwd(q, k, v, attnMask=mask)
+    got = (o,) + tuple(op.sdpAttentionBwd(g, q, k, v, o, lse, attnMask=mask))
+    for a, b in zip(got, _reference(q, k, v, g, mask)):
+        assert float((a.double() - b).abs().max()) <= TOL_REL_FP32 * max(1.0, float(b.abs().max()))

@@ -79,17 +79,23 @@ struct Cfg {
   static constexpr int kSmemBytes = (4 * kTileFloats<D> + 2 * kScoreFloats + 2 * TS) * static_cast<int>(sizeof(float));
 };
 
-// The (query tile, key tile) pair in shared memory: P into Ps (if KEYS) and dS into dSs, [query][key] both.
-// `shift` is the causal alignment (key j participates iff j <= i + shift), `mask_base` the mask offset of (b, h).
+// The (query tile, key tile) pair in shared memory: P into Ps (if KEYS) and dS into dSs, [query][key] both.  With a mask, Ps
+// holds its elements before (see MaskTile).  `shift` is the causal alignment (key j participates iff j <= i + shift).
 template <int D, bool MASK, bool KEYS>
 __device__ __forceinline__ void tile_p_ds(const BwdArgs& a, const float* Qs, const float* Ks, const float* Vs,
                                           const float* dOs, const float* lse2_s, const float* delta_s, float* Ps,
-                                          float* dSs, int row0, int col0, int kv_len, int shift, int64_t mask_base,
-                                          int ty, int tx) {
+                                          float* dSs, int row0, int col0, int kv_len, int shift,
+                                          MaskTile<D, Cfg<D>::TY, Cfg<D>::NT, kPad>& mask) {
   constexpr int TY = Cfg<D>::TY, R = Cfg<D>::R;
   const float c = a.scale * kLog2e;
-  float bias[MASK ? R : 1][4];
-  if constexpr (MASK) load_mask<TY>(a.mask, mask_base, row0 + ty, a.Lq, col0 + tx, kv_len, bias);
+  const int ty = mask.ty, tx = mask.tx;
+  uint32_t hidden = 0;
+  if constexpr (MASK) {
+    if (!mask.additive()) {
+      hidden = mask.bits(row0, col0);
+      if (KEYS) __syncthreads();  // (P goes to the same place)
+    }
+  }
   float p[R][4], dp[R][4];
   product_nt<D, TY>(Qs, Ks, ty, tx, p);
   const bool edge = row0 + TS > a.Lq || col0 + TS > kv_len || (a.causal && col0 + TS - 1 > row0 + shift);
@@ -100,7 +106,10 @@ __device__ __forceinline__ void tile_p_ds(const BwdArgs& a, const float* Qs, con
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       float x = fmaf(p[i][j], c, -lse2);
-      if constexpr (MASK) x += bias[i][j];
+      if constexpr (MASK) {
+        if (mask.additive()) x = fmaf(Ps[r * LP + tx + 16 * j], kLog2e, x);
+        if (hidden >> (4 * i + j) & 1) x = -INFINITY;
+      }
       p[i][j] = exp2f(x);
       const int col = col0 + tx + 16 * j;
       if (edge && !(row < a.Lq && col < kv_len && (!a.causal || col <= row + shift))) p[i][j] = 0.f;
@@ -191,6 +200,7 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
   const int item = SPLIT ? blockIdx.x / cluster : blockIdx.x, rank = SPLIT ? blockIdx.x % cluster : 0;
   const bool keys = item < key_ctas;
   const int group = a.Hq / a.Hkv;
+  MaskTile<D, TY, NT, kPad> mask{a.mask, Ps, 0, ty, tx, tid};
 
   float2 acc0[R][D / 32], acc1[R][D / 32];
 #pragma unroll
@@ -233,14 +243,15 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
         __syncthreads();  // the tiles of the step before have been read
         load_tile<D, NT>(Qs, q, a.qs.s, row0, a.Lq, tid);
         load_tile<D, NT>(dOs, dO, a.dos.s, row0, a.Lq, tid);
+        mask.base = b * a.mask.sb + h * a.mask.sh;
+        if constexpr (MASK) mask.stage(row0, a.Lq, col0, kv_len);
         copies_commit();
         if (first) ptx::grid_dep_wait();  // launched early behind the delta pre-pass
         first = false;
         load_vectors(a, lse2_s, delta_s, base, row0, tid);
         copies_wait<0>();
         __syncthreads();
-        tile_p_ds<D, MASK, true>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift,
-                                 b * a.mask.sb + h * a.mask.sh, ty, tx);
+        tile_p_ds<D, MASK, true>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift, mask);
         __syncthreads();
         product_tn<D, TY>(Ps, dOs, ty, tx, acc0);
         product_tn<D, TY>(dSs, Qs, ty, tx, acc1);
@@ -286,6 +297,8 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
       load_tile<D, NT>(Ks, k, a.ks.s, t0 * TS, a.Skv, tid);
       load_tile<D, NT>(Vs, v, a.vs.s, t0 * TS, a.Skv, tid);
     }
+    mask.base = b * a.mask.sb + h * a.mask.sh;
+    if (MASK && n_tiles > t0) mask.stage(row0, a.Lq, t0 * TS, kv_len);
     copies_commit();
     ptx::grid_dep_wait();  // launched early behind the delta pre-pass
     load_vectors(a, lse2_s, delta_s, (static_cast<int64_t>(b) * a.Hq + h) * a.Lq, row0, tid);
@@ -293,10 +306,12 @@ __global__ void __launch_bounds__(Cfg<D>::NT, D == 64 ? 2 : 1) bwd_simt_kernel(c
       const int col0 = t * TS;
       copies_wait<0>();
       __syncthreads();
-      tile_p_ds<D, MASK, false>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, nullptr, dSs, row0, col0, kv_len, shift,
-                                b * a.mask.sb + h * a.mask.sh, ty, tx);
+      tile_p_ds<D, MASK, false>(a, Qs, Ks, Vs, dOs, lse2_s, delta_s, Ps, dSs, row0, col0, kv_len, shift, mask);
       __syncthreads();
-      if (t + 1 < n_tiles) load_tile<D, NT>(Vs, v, a.vs.s, col0 + TS, a.Skv, tid);
+      if (t + 1 < n_tiles) {
+        load_tile<D, NT>(Vs, v, a.vs.s, col0 + TS, a.Skv, tid);
+        if constexpr (MASK) mask.stage(row0, a.Lq, col0 + TS, kv_len);
+      }
       product_nn<D, TY>(dSs, Ks, ty, tx, acc0);
       __syncthreads();
       if (t + 1 < n_tiles) load_tile<D, NT>(Ks, k, a.ks.s, col0 + TS, a.Skv, tid);
@@ -353,13 +368,14 @@ cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   const int cluster = split_of(a, D);
   auto kern = cluster > 1 ? bwd_simt_kernel<D, MASK, true> : bwd_simt_kernel<D, MASK, false>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<D>::kSmemBytes);
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   const long long key_tiles = (a.Skv + TS - 1) / TS, q_tiles = (a.Lq + TS - 1) / TS;
   const long long key_ctas = a.dk || a.dv ? key_tiles * a.Hkv * a.B : 0, q_ctas = a.dq ? q_tiles * a.Hq * a.B : 0;
   if ((key_ctas + q_ctas) * cluster > 0x7fffffffll) return cudaErrorInvalidValue;
-  return launch_early(kern, dim3(static_cast<unsigned>((key_ctas + q_ctas) * cluster)), dim3(Cfg<D>::NT), Cfg<D>::kSmemBytes, stream,
-                      cluster, a, static_cast<int>(key_tiles), static_cast<int>(key_ctas), cluster);
+  return launch_early(kern, dim3(static_cast<unsigned>((key_ctas + q_ctas) * cluster)), dim3(Cfg<D>::NT),
+                   spread_smem(Cfg<D>::kSmemBytes, (key_ctas + q_ctas) * cluster, cluster), stream, cluster, a,
+                   static_cast<int>(key_tiles), static_cast<int>(key_ctas), cluster);
 }
 
 }  // namespace

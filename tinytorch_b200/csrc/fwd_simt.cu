@@ -11,7 +11,8 @@
 // Bound by the FMA pipes (74 TFLOP/s at 1965 MHz).  128 threads, 8 x 4 scores and 8 x D/16 outputs per thread
 // (simt_tile.cuh); the next K tile is copied in under the P V product and the next V tile under Q K^T; 3 CTAs of
 // D = 64 and 2 of D = 128 share an SM.  B4 H16 S2048 D64 causal: 1587 -> 958 us (21.7 -> 35.9 TFLOP/s) against scalar
-// shared-memory loads (eight per sixteen FMAs); ncu: FMA pipe 58 % busy, 2.7 warps per scheduler, the rest latency.
+// shared-memory loads (eight per sixteen FMAs); ncu: FMA pipe 58 % busy, 2.7 warps per scheduler, the rest latency.  The mask of
+// a tile comes through shared memory (MaskTile).  4 x 8 heads x 500, additive mask: D = 64 82 -> 76 us, D = 128 172 -> 128.
 //
 // Few query tiles leave most SMs idle for the time of the longest walk over the keys, 4 us (D = 64) or 8 us per key tile.
 // The key tiles are then divided among the CTAs of a cluster (SPLIT); their unnormalised O, maxima and sums meet in
@@ -27,18 +28,27 @@ namespace {
 using namespace simt;
 constexpr int kThreads = 128, TY = kThreads / 16, R = TS / TY;
 
-template <int D>
-constexpr int kSmemBytes = (3 * kTileFloats<D> + kScoreFloats) * static_cast<int>(sizeof(float));
+// With only K padded two CTAs of D = 128 fit an SM, to the byte (4 x 8 heads x 500: 136 -> 119 us).  Where there are too few for
+// two the padded tiles are the faster (8 heads x 512, divided: 39 us instead of 42).
+template <int D, bool SPLIT>
+struct Lay {
+  static constexpr bool kTight = D == 64 || !SPLIT;
+  static constexpr Layout Q = kTight ? kSwap : kPad, V = kTight ? kPlain : kPad, P = kTight ? kSwap : kPad;
+  static constexpr int kQ = kTight ? TS * D : kTileFloats<D>, kV = kQ, kP = kTight ? TS * TS : kScoreFloats;
+  static constexpr int kSmemBytes = (kQ + kTileFloats<D> + kV + kP) * static_cast<int>(sizeof(float));
+};
+static_assert(2 * (Lay<128, false>::kSmemBytes + 1024) <= 228 * 1024, "two CTAs of D = 128 to an SM");
 
 template <int D, bool MASK, bool SPLIT>
-__global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_kernel(const FwdArgs a, int cluster) {
+__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(const FwdArgs a, int cluster) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();  // launched early: everything below reads or writes global memory
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
-  float* Ks = Qs + kTileFloats<D>;
+  using LY = Lay<D, SPLIT>;
+  float* Ks = Qs + LY::kQ;
   float* Vs = Ks + kTileFloats<D>;
-  float* Ps = Vs + kTileFloats<D>;
+  float* Ps = Vs + LY::kV;
 
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const int n_mt = SPLIT ? gridDim.x / cluster : gridDim.x, rank = SPLIT ? blockIdx.x % cluster : 0;
@@ -62,11 +72,17 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
   const float c = a.scale * kLog2e;
   const int64_t mask_base = b * a.mask.sb + h * a.mask.sh;
 
+  MaskTile<D, TY, kThreads, LY::P> mask{a.mask, Ps, mask_base, ty, tx, tid};
+  float* mine = mask.mine();  // where this thread's scores go
   if (n_tiles > t0) {
-    load_tile<D, kThreads>(Qs, q, a.qs.s, row0, a.Lq, tid);
+    load_tile<D, kThreads, LY::Q>(Qs, q, a.qs.s, row0, a.Lq, tid);
     load_tile<D, kThreads>(Ks, k, a.ks.s, t0 * TS, kv_len, tid);
     copies_commit();
-    load_tile<D, kThreads>(Vs, v, a.vs.s, t0 * TS, kv_len, tid);
+    if constexpr (MASK) {
+      mask.stage(row0, a.Lq, t0 * TS, kv_len);
+      copies_commit();
+    }
+    load_tile<D, kThreads, LY::V>(Vs, v, a.vs.s, t0 * TS, kv_len, tid);
     copies_commit();
   }
 
@@ -81,15 +97,23 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
 
   for (int t = t0; t < n_tiles; ++t) {
     const int col0 = t * TS;
-    copies_wait<1>();  // Q and K of this tile; V may still be on its way
+    copies_wait<MASK ? 2 : 1>();  // Q and K of this tile; the mask and V may still be on their way
     __syncthreads();
-    float bias[MASK ? R : 1][4];
-    if constexpr (MASK) load_mask<TY>(a.mask, mask_base, row0 + ty, a.Lq, col0 + tx, kv_len, bias);
     float s[R][4];
-    product_nt<D, TY>(Qs, Ks, ty, tx, s);
+    product_nt<D, TY, LY::Q>(Qs, Ks, ty, tx, s);
+    if (MASK && !mask.additive()) copies_wait<1>();
     __syncthreads();  // K of this tile has been read
     if (t + 1 < n_tiles) load_tile<D, kThreads>(Ks, k, a.ks.s, col0 + TS, kv_len, tid);
     copies_commit();
+    uint32_t hidden = 0;
+    if constexpr (MASK) {
+      if (mask.additive()) {
+        copies_wait<2>();  // (of a thread's own)
+      } else {
+        hidden = mask.bits(row0, col0);
+        __syncthreads();
+      }
+    }
     const bool edge = col0 + TS > kv_len || (a.causal && col0 + TS - 1 > row0 + shift);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -98,7 +122,10 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         s[i][j] *= c;
-        if constexpr (MASK) s[i][j] += bias[i][j];
+        if constexpr (MASK) {
+          if (mask.additive()) s[i][j] = fmaf(mine[mask.at(i, j)], kLog2e, s[i][j]);
+          if (hidden >> (4 * i + j) & 1) s[i][j] = -INFINITY;
+        }
         const int col = col0 + tx + 16 * j;
         if (edge && !(col < kv_len && (!a.causal || col <= row + shift))) s[i][j] = -INFINITY;
         mx = fmaxf(mx, s[i][j]);
@@ -119,14 +146,18 @@ __global__ void __launch_bounds__(kThreads, D == 64 && !MASK ? 3 : 2) fwd_simt_k
       for (int j = 0; j < 4; ++j) {
         const float p = exp2f(s[i][j] - m_use);
         l[i] += p;
-        Ps[(ty + TY * i) * LP + tx + 16 * j] = p;
+        mine[mask.at(i, j)] = p;
       }
     }
     copies_wait<1>();  // V of this tile
     __syncthreads();
-    product_nn<D, TY>(Ps, Vs, ty, tx, acc);
+    product_nn<D, TY, LY::P, LY::V>(Ps, Vs, ty, tx, acc);
     __syncthreads();  // V and P have been read
-    if (t + 1 < n_tiles) load_tile<D, kThreads>(Vs, v, a.vs.s, col0 + TS, kv_len, tid);
+    if constexpr (MASK) {
+      if (t + 1 < n_tiles) mask.stage(row0, a.Lq, col0 + TS, kv_len);
+      copies_commit();
+    }
+    if (t + 1 < n_tiles) load_tile<D, kThreads, LY::V>(Vs, v, a.vs.s, col0 + TS, kv_len, tid);
     copies_commit();
   }
 
@@ -224,11 +255,13 @@ int split_of(const FwdArgs& a, int D) {
 
 template <int D, bool MASK>
 cudaError_t launch_t(const FwdArgs& a, cudaStream_t stream) {
-  const int cluster = split_of(a, D);
+  const int cluster = split_of(a, D), smem = cluster > 1 ? Lay<D, true>::kSmemBytes : Lay<D, false>::kSmemBytes;
   auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true> : fwd_simt_kernel<D, MASK, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes<D>);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
-  return launch_early(kern, dim3((a.Lq + TS - 1) / TS * cluster, a.Hq, a.B), dim3(kThreads), kSmemBytes<D>, stream, cluster, a, cluster);
+  const long long ctas = static_cast<long long>((a.Lq + TS - 1) / TS) * cluster * a.Hq * a.B;
+  return launch_early(kern, dim3((a.Lq + TS - 1) / TS * cluster, a.Hq, a.B), dim3(kThreads),
+                      spread_smem(smem, ctas, cluster), stream, cluster, a, cluster);
 }
 
 }  // namespace

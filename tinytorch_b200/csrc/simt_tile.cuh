@@ -4,7 +4,8 @@
 // A thread grid of 16 columns (tx) x TY rows (ty) works on a tile; a thread owns R = 64 / TY rows.  Every operand
 // comes from shared memory as 16-byte vectors: with R = 8 one vector feeds ten FMAs (the scalar loads these replace:
 // two), and a warp's vectors fall on at most two wavefronts.  Row strides carry 4 floats of padding, which puts eight
-// consecutive rows on different banks.  Sums run as fma.rn.f32x2: two fp32 FMAs per issued instruction, each rounded
+// consecutive rows on different banks.  An operand of which a warp reads two consecutive rows at a time (the first of a
+// product) can do without: kSwap exchanges neighbouring pieces of the odd rows instead.  Sums run as fma.rn.f32x2: two fp32 FMAs per issued instruction, each rounded
 // as the scalar one.  (Unrolling the vector loops 4 / 4 / 8 times: 3-5 % over 2 / 2 / 4; whole or not at all: slower.)
 #pragma once
 #include "common.cuh"
@@ -21,8 +22,12 @@ template <int D>
 constexpr int kTileFloats = TS * kLd<D>;
 constexpr int kScoreFloats = TS * LP;
 
-// rows [row0, row0 + 64) of src into dst[64][kLd<D>] by asynchronous 16-byte copies; rows at or beyond `valid` are zero
-template <int D, int NT>
+// How a tile lies in shared memory: padded rows; rows as they are; rows as they are, with neighbouring vectors of the odd
+// rows exchanged (of a score tile: neighbouring halves of 32 columns).
+enum Layout { kPad, kPlain, kSwap };
+
+// rows [row0, row0 + 64) of src into dst by asynchronous 16-byte copies; rows at or beyond `valid` are zero
+template <int D, int NT, Layout LAY = kPad>
 __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t row_stride, int row0, int valid, int tid) {
   const uint32_t base = ptx::smem_u32(dst);
 #pragma unroll
@@ -30,7 +35,7 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t 
     const int idx = tid + i * NT, r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
     const bool in = row0 + r < valid;
     const float* p = src + static_cast<int64_t>(in ? row0 + r : 0) * row_stride + c4;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (r * kLd<D> + c4) * 4), "l"(p), "r"(in ? 16 : 0)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (LAY == kPad ? r * kLd<D> + c4 : r * D + (LAY == kSwap ? c4 ^ (r & 1) * 4 : c4)) * 4), "l"(p), "r"(in ? 16 : 0)
                  : "memory");
   }
 }
@@ -44,24 +49,27 @@ __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x,
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
 // out[i][j] = sum_d A[ty + TY i][d] * B[tx + 16 j][d]
-template <int D, int TY>
+template <int D, int TY, Layout LA = kPad>
 __device__ __forceinline__ void product_nt(const float* A, const float* B, int ty, int tx, float (&out)[TS / TY][4]) {
-  constexpr int R = TS / TY;
+  constexpr int R = TS / TY, LDA = LA == kPad ? kLd<D> : D;
   float2 acc[R][4];
 #pragma unroll
   for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
-  const float* ap = A + ty * kLd<D>;
+  const int odd = LA == kSwap ? (ty & 1) * 4 : 0;  // (of all rows ty + TY i)
+  const float* ap[2] = {A + ty * LDA + odd, A + ty * LDA - odd};
   const float* bp = B + tx * kLd<D>;
-#pragma unroll 4
-  for (int d = 0; d < D; d += 4) {
+#pragma unroll 1
+  for (int d0 = 0; d0 < D; d0 += 16)
+#pragma unroll
+  for (int d = d0; d < d0 + 16; d += 4) {
     float4 b[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(bp + j * 16 * kLd<D> + d);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const float4 a = *reinterpret_cast<const float4*>(ap + i * TY * kLd<D> + d);
+      const float4 a = *reinterpret_cast<const float4*>(ap[(d - d0) / 4 & 1] + i * TY * LDA + d);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         acc[i][j] = ptx::fma2(lo2(a), lo2(b[j]), acc[i][j]);
@@ -76,20 +84,23 @@ __device__ __forceinline__ void product_nt(const float* A, const float* B, int t
 }
 
 // acc[i][.] += sum_k P[ty + TY i][k] * V[k][tx * 4 + 64 c ..]   (acc holds pairs of columns: 2 per group c of 4)
-template <int D, int TY>
+template <int D, int TY, Layout LPL = kPad, Layout LV = kPad>
 __device__ __forceinline__ void product_nn(const float* P, const float* V, int ty, int tx, float2 (&acc)[TS / TY][D / 32]) {
-  constexpr int R = TS / TY, DC = D / 64;
-  const float* pp = P + ty * LP;
-#pragma unroll 4
-  for (int k = 0; k < TS; k += 4) {
+  constexpr int R = TS / TY, DC = D / 64, LDP = LPL == kPad ? LP : TS, LDV = LV == kPad ? kLd<D> : D;
+  const int odd = LPL == kSwap ? (ty & 1) * 16 : 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < TS; k0 += 16) {
+  const float* pp = P + ty * LDP + (k0 ^ odd) - k0;
+#pragma unroll
+  for (int k = k0; k < k0 + 16; k += 4) {
     float4 v[4][DC];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int c = 0; c < DC; ++c) v[q][c] = *reinterpret_cast<const float4*>(V + (k + q) * kLd<D> + tx * 4 + c * 64);
+      for (int c = 0; c < DC; ++c) v[q][c] = *reinterpret_cast<const float4*>(V + (k + q) * LDV + tx * 4 + c * 64);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const float4 p4 = *reinterpret_cast<const float4*>(pp + i * TY * LP + k);
+      const float4 p4 = *reinterpret_cast<const float4*>(pp + i * TY * LDP + k);
       const float p[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -100,6 +111,7 @@ __device__ __forceinline__ void product_nn(const float* P, const float* V, int t
           acc[i][2 * c + 1] = ptx::fma2(pq, hi2(v[q][c]), acc[i][2 * c + 1]);
         }
     }
+  }
   }
 }
 
@@ -128,19 +140,81 @@ __device__ __forceinline__ void product_tn(const float* P, const float* X, int t
   }
 }
 
-// The mask elements (times log2 e) of this thread's scores: rows row, row + TY, .., columns col, col + 16, ..; 0 outside.
-template <int TY, int R>
-__device__ __forceinline__ void load_mask(const MaskArgs& m, int64_t base, int row, int n_rows, int col, int n_cols,
-                                          float (&bias)[R][4]) {
-  auto load = [&](auto* p, auto value) {  // (one loop per kind: nothing is decided per element)
-    p += base + row * m.sl + col;
+// The mask of a tile's scores.  Where thread (ty, tx) will write its probabilities, [(ty + TY i) LD + tx + 16 j] (kSwap: + 16 (j ^
+// (ty & 1))), the tile's shared memory holds before
+//   an additive mask   the thread's own elements, copied asynchronously one by one: nobody else has to wait for them;
+//   a boolean one      its bytes, a row in the first 68 bytes of a row (one row where all are the same): aligned words, copied by
+//                      all threads together.  Every thread has to take its own (bits) before any writes a probability.
+// (All elements in registers, fetched ahead of the product that comes first, are 32 of them: a CTA fewer to an SM.)  4 x 8
+// heads x 500 with an additive mask, D = 128: forward 172 -> 128 us, without a mask 119; D = 64: backward 221 -> 202, 186.
+template <int D, int TY, int NT, Layout LAY>
+struct MaskTile {
+  static constexpr int R = TS / TY, LD = LAY == kPad ? LP : TS;
+  const MaskArgs& m;
+  float* tile;
+  int64_t base;  // of (batch, head)
+  int ty, tx, tid;
+
+  __device__ __forceinline__ bool additive() const { return m.kind != TT_ATTN_MASK_BOOL; }
+  __device__ __forceinline__ float* mine() const { return tile + ty * LD + tx; }
+  __device__ __forceinline__ int at(int i, int j) const { return i * TY * LD + (LAY == kSwap ? j ^ (ty & 1) : j) * 16; }
+
+  // copies of the tile at (row0, col0) on their way; outside: 0 (added), anything (boolean)
+  __device__ __forceinline__ void stage(int row0, int n_rows, int col0, int n_cols) {
+    if (additive()) {
+      const int row = row0 + ty, col = col0 + tx;
+      const float* p = reinterpret_cast<const float*>(m.ptr) + base + row * m.sl + col;
+      const uint32_t dst = ptx::smem_u32(mine());
 #pragma unroll
-    for (int i = 0; i < R; ++i, p += TY * m.sl)
+      for (int i = 0; i < R; ++i, p += TY * m.sl)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bias[i][j] = row + TY * i < n_rows && col + 16 * j < n_cols ? value(p[16 * j]) : 0.f;
-  };
-  if (m.kind == TT_ATTN_MASK_BOOL) load(reinterpret_cast<const uint8_t*>(m.ptr), [](uint8_t x) { return x ? 0.f : -INFINITY; });
-  else load(reinterpret_cast<const float*>(m.ptr), [](float x) { return x * kLog2e; });
+        for (int j = 0; j < 4; ++j) {
+          const bool in = row + TY * i < n_rows && col + 16 * j < n_cols;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + at(i, j) * 4),
+                       "l"(in ? p + 16 * j : reinterpret_cast<const float*>(m.ptr)), "r"(in ? 4 : 0)
+                       : "memory");
+        }
+    } else {
+      constexpr int W = TS / 4 + 1;  // words that hold 64 bytes at any offset
+      const uint8_t* any = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(m.ptr) & ~uintptr_t(3));
+      for (int e = tid; e < (m.sl == 0 ? W : TS * W); e += NT) {
+        const int r = e / W, w = e - r * W;
+        const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + base + (row0 + r) * m.sl + col0;
+        const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);
+        const bool in = row0 + r < n_rows && w * 4 - mis < n_cols - col0 && w * 4 - mis < TS;  // some byte of it is looked at
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(tile + r * LD + w)),
+                     "l"(in ? p - mis + w * 4 : any), "r"(in ? 4 : 0)
+                     : "memory");
+      }
+    }
+  }
+  // boolean: bit 4 i + j: score (i, j) is hidden (or outside, where it does not count); the copies are complete and visible
+  __device__ __forceinline__ uint32_t bits(int row0, int col0) const {
+    const int first = m.sl == 0 ? 0 : ty, step = m.sl == 0 ? 0 : TY;
+    const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(m.ptr) + base + col0 + (row0 + first) * m.sl);
+    const uint8_t* p = reinterpret_cast<const uint8_t*>(tile + first * LD) + tx;
+    uint32_t b = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const uint8_t* q = p + i * step * LD * 4 + ((off + i * step * static_cast<uint32_t>(m.sl)) & 3);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b |= q[16 * j] ? 0u : 1u << (4 * i + j);
+    }
+    return b;
+  }
+};
+
+// Shared memory to ask for, so that no SM gets more CTAs than it has to: the CTAs of a cluster are put on as few SMs as hold
+// them, and a few of them then work two to an SM beside idle ones (D = 128, 8 heads x 512: 61 us instead of 39).  Clusters
+// of 4 and 8 do not fill every GPC, so that a grid close to the number of SMs is left as it is.
+inline int spread_smem(int need, long long ctas, int cluster) {
+  const int sms = cluster == 8 ? 128 : (cluster == 4 ? 136 : kSms);
+  for (int per_sm = 1; per_sm <= 2; ++per_sm)
+    if (ctas <= static_cast<long long>(per_sm) * sms) {
+      const int least = 228 * 1024 / (per_sm + 1) - 1024 + 128;  // too much for per_sm + 1 of them
+      return need > least ? need : least;
+    }
+  return need;
 }
 
 }  // namespace simt
