@@ -143,7 +143,7 @@ size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int 
     // delta [B,Hq,Lq] fp32; the fp16 / bf16 path adds an fp32 dQ accumulator [B,Hq,Lq,D]
     const size_t rows = static_cast<size_t>(B) * Hq * (Lq > 0 ? Lq : 0);
     // and the persistent kernel's work counter
-    if (dtype == TT_ATTN_F32) return round256(rows * sizeof(float));
+    if (dtype == TT_ATTN_F32) return round256(rows * sizeof(float)) + round256(bwd_ds_bytes(B, Hq, Hkv, Lq, Skv, D));
     // (and, where few key tiles are divided among several work items, their partial dK / dV)
     return round256(rows * sizeof(float)) + round256(rows * D * sizeof(float)) +
            round256(bwd_part_bytes(B, Hq, Hkv, Lq, Skv, D)) + round256(scratch_words(B) * sizeof(int));
@@ -242,6 +242,9 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
   size_t need = delta, part = 0;
   bool lens = false;
+  // fp32: dS tiles on their way from dK / dV to dQ, where all three are asked for and there is room
+  size_t ds = p->dtype == TT_ATTN_F32 && p->dq && (p->dk || p->dv) ? round256(bwd_ds_bytes(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) : 0;
+  if (delta + ds > room) ds = 0;
   if (p->dtype != TT_ATTN_F32) {
     // a buffer that is too small for the division (a small batch is divided further than a large one): fewer shares
     a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
@@ -251,8 +254,12 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
     lens = mask_lens_fit(a.mask, a.causal, p->B, room, need);
     need += lens ? round256(scratch_words(p->B) * sizeof(int)) : 256;
   }
-  if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
+  if (ds == 0 || ws.acquire(need + ds, p->workspace, p->workspace_bytes, p->alloc, p->device) != TT_ATTN_OK) {
+    ds = 0;  // (an allocator that has no more than before)
+    if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
+  }
   a.delta = static_cast<float*>(ws.ptr);
+  if (ds > 0) a.ds = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
   if (p->dtype != TT_ATTN_F32) {
     a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
     a.dkv_part = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta + accum);

@@ -74,6 +74,7 @@ struct BwdArgs {
   int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by the delta pre-pass
   int parts;          // tensor-core kernel: work items per key tile (see bwd_parts); > 1: each leaves its dK / dV in ...
   float* dkv_part;    // ... workspace [dK, dV][parts][B * Hkv][Skv][D] fp32
+  float* ds;          // fp32 kernels: dS tiles on their way from the dK / dV pass to the dQ pass, or null (see bwd_ds_bytes)
   void* dq;
   void* dk;
   void* dv;
@@ -129,6 +130,8 @@ cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t st
 int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal);
 size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
 size_t bwd_part_bytes_of(int parts, int B, int Hkv, int Skv, int D);
+// dS tiles of the fp32 backward (0: dQ recomputes them; a caller without room for them gets that too)
+size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
 // fp16 / bf16 backward on the tensor cores; needs a.delta, a.dq_accum and what a.parts asks for
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t stream);

@@ -23,8 +23,8 @@ constexpr int kTileFloats = TS * kLd<D>;
 constexpr int kScoreFloats = TS * LP;
 
 // How a tile lies in shared memory: padded rows; rows as they are; rows as they are, with neighbouring vectors of the odd
-// rows exchanged (of a score tile: neighbouring halves of 32 columns).
-enum Layout { kPad, kPlain, kSwap };
+// rows exchanged (of a score tile: neighbouring halves of 32 columns; kSwapHalves copies one in like that).
+enum Layout { kPad, kPlain, kSwap, kSwapHalves };
 
 // rows [row0, row0 + 64) of src into dst by asynchronous 16-byte copies; rows at or beyond `valid` are zero
 template <int D, int NT, Layout LAY = kPad>
@@ -35,7 +35,7 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t 
     const int idx = tid + i * NT, r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
     const bool in = row0 + r < valid;
     const float* p = src + static_cast<int64_t>(in ? row0 + r : 0) * row_stride + c4;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (LAY == kPad ? r * kLd<D> + c4 : r * D + (LAY == kSwap ? c4 ^ (r & 1) * 4 : c4)) * 4), "l"(p), "r"(in ? 16 : 0)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + (LAY == kPad ? r * kLd<D> + c4 : r * D + (LAY == kSwap ? c4 ^ (r & 1) * 4 : (LAY == kSwapHalves ? c4 ^ (r & 1) * 16 : c4))) * 4), "l"(p), "r"(in ? 16 : 0)
                  : "memory");
   }
 }
