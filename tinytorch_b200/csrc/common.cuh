@@ -171,8 +171,15 @@ cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  
 double linear_tile_us(const LinearCall& c, bool pair, int bn);  // what it, or pairs with 256 x 256, are expected to take
 cudaError_t launch_linear_tile(const LinearCall& c, bool pair, int bn);
 // ... for outputs with too few tiles to occupy the machine: contraction split over clusters (linear_split.cu)
-double linear_split_us(const LinearCall& c);  // what it is expected to take
-cudaError_t launch_linear_split(const LinearCall& c);
+struct SplitPlan {
+  int mt, tiles_m, tiles, cluster, stages, smem;
+  int per_sm, waves;
+  double hbm_rate;  // bytes per us
+  double us;        // what it is expected to take, among plans
+};
+SplitPlan plan_linear_split(const LinearCall& c);
+double linear_split_us(const LinearCall& c, const SplitPlan& p);  // ... beside the other kernels
+cudaError_t launch_linear_split(const LinearCall& c, const SplitPlan& p);
 // out[n] = sum over the rows of x[rows, n] (fused_ops.cu); n and ldx are multiples of 8
 // `beside`: the kernel launched just before is a linear_tc_kernel, beside which this one may run
 cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, bool beside,

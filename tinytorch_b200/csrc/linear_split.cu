@@ -257,13 +257,6 @@ __global__ void __launch_bounds__(kThreads)
   if (tid == 0 && ctl->abort_flag && a.status) atomicOr(a.status, kStatusWaitExpired);
 }
 
-struct Plan {
-  int mt, tiles_m, tiles, cluster, stages, smem;
-  int per_sm, waves;
-  double hbm_rate;  // bytes per us
-  double us;        // what it is expected to take
-};
-
 // How the problem is divided: the cheapest of the candidates by a model fitted to a sweep of 20 problems from 1 x 1024 x
 // 1024 to 2000 x 1024 x 1024 and 64 x 4096 x 28672 (B200; within 1.5 us of the measured time for the plans near the
 // best, and the plan it picks within 8 % of the best of the sweep):
@@ -278,9 +271,9 @@ struct Plan {
 // differ in size, so clusters of 8 leave up to a fifth of the SMs unused.  Asked once per device, size and share.
 int cluster_slots(int device, int cluster, int per_sm);
 
-Plan plan_split(int M, int N, int K, bool x_t, int device) {
+SplitPlan plan_split(int M, int N, int K, bool x_t, int device) {
   const int sms = sm_count(device);
-  Plan best{};
+  SplitPlan best{};
   best.us = 1e30;
   const int n_kb = (K + BK - 1) / BK, tiles_n = (N + BW - 1) / BW;
   const double bytes = 2.0 * K * (static_cast<double>(N) + M);
@@ -290,7 +283,7 @@ Plan plan_split(int M, int N, int K, bool x_t, int device) {
     const int mt = ((M + tm - 1) / tm + unit - 1) / unit * unit;
     if (mt == last_mt) continue;
     last_mt = mt;
-    Plan p;
+    SplitPlan p;
     p.mt = mt;
     p.tiles_m = (M + mt - 1) / mt;
     const long long tiles = static_cast<long long>(p.tiles_m) * tiles_n;
@@ -321,7 +314,7 @@ Plan plan_split(int M, int N, int K, bool x_t, int device) {
 }
 
 template <bool BF16, bool X_MN, bool W_MN>
-cudaError_t launch_t(const LinearCall& c, const Plan& p) {
+cudaError_t launch_t(const LinearCall& c, const SplitPlan& p) {
   auto kern = linear_split_kernel<BF16, X_MN, W_MN>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
@@ -337,7 +330,7 @@ cudaError_t launch_t(const LinearCall& c, const Plan& p) {
 }
 
 template <bool BF16>
-cudaError_t launch_bf(const LinearCall& c, const Plan& p) {
+cudaError_t launch_bf(const LinearCall& c, const SplitPlan& p) {
   if (c.x_t) return c.w_t ? launch_t<BF16, true, true>(c, p) : launch_t<BF16, true, false>(c, p);
   return c.w_t ? launch_t<BF16, false, true>(c, p) : launch_t<BF16, false, false>(c, p);
 }
@@ -374,8 +367,7 @@ int cluster_slots(int device, int cluster, int per_sm) {
 
 // What the plan is expected to take, for the choice between the kernels: as above, fitted to 170 problems (6 % rms) that the plans
 // themselves do not depend on: operands whose rows do not lie on cache lines, and the output's way to memory.
-double linear_split_us(const LinearCall& c) {
-  const Plan p = plan_split(c.M, c.N, c.K, c.x_t, c.device);
+double linear_split_us(const LinearCall& c, const SplitPlan& p) {
   const int n_kb = (c.K + BK - 1) / BK;
   const double lines = BW * row_lines(c.ldw) + p.mt * row_lines(c.ldx), bytes = 2.0 * c.K * (static_cast<double>(c.N) + c.M);
   const double sm_us = static_cast<double>(p.waves) * p.per_sm * ((n_kb + p.cluster - 1) / p.cluster) * lines * 128 / 137e3;
@@ -386,8 +378,9 @@ double linear_split_us(const LinearCall& c) {
   return body > out ? body + 0.1 * out : out + 0.1 * body;
 }
 
-cudaError_t launch_linear_split(const LinearCall& c) {
-  const Plan p = plan_split(c.M, c.N, c.K, c.x_t, c.device);
+SplitPlan plan_linear_split(const LinearCall& c) { return plan_split(c.M, c.N, c.K, c.x_t, c.device); }
+
+cudaError_t launch_linear_split(const LinearCall& c, const SplitPlan& p) {
   return c.dtype == TT_ATTN_BF16 ? launch_bf<true>(c, p) : launch_bf<false>(c, p);
 }
 

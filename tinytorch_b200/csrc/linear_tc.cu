@@ -307,16 +307,17 @@ struct Plan {
 // (linear_split.cu; always up to 128 rows).  Between the two lie problems for which a shape of linear_tile.cu puts a tile on nearly
 // every SM; it is taken where it is expected to save 6 % and 0.25 us (10 % where x is MN-major), about the error of the models.  Of 251 problems with more
 // than 128 rows that the models were not fitted to the mean is 0.94 of the time before (1.04 of the best shape's), the worst 1.03.
-Plan plan_of(const LinearCall& c) {
+Plan plan_of(const LinearCall& c, SplitPlan* split) {
   const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + BN - 1) / BN);
   if (tiles >= sm_count(c.device) / 2 * 2) return Plan{Plan::kPairs, false, 0};
+  *split = plan_linear_split(c);
   if (c.M <= HM) return Plan{Plan::kSplit, false, 0};
   Plan best{Plan::kPairs, false, 0};
   double us = linear_tile_us(c, true, BN);
   auto take = [&](const Plan& p, double t) {
     if (t < us) best = p, us = t;
   };
-  take(Plan{Plan::kSplit, false, 0}, linear_split_us(c));
+  take(Plan{Plan::kSplit, false, 0}, linear_split_us(c, *split));
   us = us * (c.x_t ? 0.9 : 0.94) - 0.25;
   if (!c.w_t) take(Plan{Plan::kTiles, true, 192}, linear_tile_us(c, true, 192));
   // (an MN-major w comes in blocks of 64 columns)
@@ -328,8 +329,9 @@ Plan plan_of(const LinearCall& c) {
 cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent) {
   if (persistent) *persistent = false;
   if (c.dtype != TT_ATTN_BF16 && c.dtype != TT_ATTN_F16) return cudaErrorInvalidValue;
-  const Plan p = plan_of(c);
-  if (p.kernel == Plan::kSplit) return launch_linear_split(c);
+  SplitPlan split;
+  const Plan p = plan_of(c, &split);
+  if (p.kernel == Plan::kSplit) return launch_linear_split(c, split);
   if (persistent) *persistent = true;
   if (p.kernel == Plan::kTiles) return launch_linear_tile(c, p.pair, p.bn);
   const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + BN - 1) / BN);
