@@ -61,19 +61,20 @@ __device__ __forceinline__ void product_nt(const float* A, const float* B, int t
   const float* ap[2] = {A + ty * LDA + odd, A + ty * LDA - odd};
   const float* bp = B + tx * kLd<D>;
 #pragma unroll 1
-  for (int d0 = 0; d0 < D; d0 += 16)
+  for (int d0 = 0; d0 < D; d0 += 16) {
 #pragma unroll
-  for (int d = d0; d < d0 + 16; d += 4) {
-    float4 b[4];
+    for (int d = d0; d < d0 + 16; d += 4) {
+      float4 b[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(bp + j * 16 * kLd<D> + d);
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(bp + j * 16 * kLd<D> + d);
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const float4 a = *reinterpret_cast<const float4*>(ap[(d - d0) / 4 & 1] + i * TY * LDA + d);
+      for (int i = 0; i < R; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(ap[(d - d0) / 4 & 1] + i * TY * LDA + d);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j] = ptx::fma2(lo2(a), lo2(b[j]), acc[i][j]);
-        acc[i][j] = ptx::fma2(hi2(a), hi2(b[j]), acc[i][j]);
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j] = ptx::fma2(lo2(a), lo2(b[j]), acc[i][j]);
+          acc[i][j] = ptx::fma2(hi2(a), hi2(b[j]), acc[i][j]);
+        }
       }
     }
   }
@@ -90,28 +91,28 @@ __device__ __forceinline__ void product_nn(const float* P, const float* V, int t
   const int odd = LPL == kSwap ? (ty & 1) * 16 : 0;
 #pragma unroll 1
   for (int k0 = 0; k0 < TS; k0 += 16) {
-  const float* pp = P + ty * LDP + (k0 ^ odd) - k0;
+    const float* pp = P + ty * LDP + (k0 ^ odd) - k0;
 #pragma unroll
-  for (int k = k0; k < k0 + 16; k += 4) {
-    float4 v[4][DC];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int c = 0; c < DC; ++c) v[q][c] = *reinterpret_cast<const float4*>(V + (k + q) * LDV + tx * 4 + c * 64);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const float4 p4 = *reinterpret_cast<const float4*>(pp + i * TY * LDP + k);
-      const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+    for (int k = k0; k < k0 + 16; k += 4) {
+      float4 v[4][DC];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int c = 0; c < DC; ++c) {
-          const float2 pq = make_float2(p[q], p[q]);
-          acc[i][2 * c] = ptx::fma2(pq, lo2(v[q][c]), acc[i][2 * c]);
-          acc[i][2 * c + 1] = ptx::fma2(pq, hi2(v[q][c]), acc[i][2 * c + 1]);
-        }
+        for (int c = 0; c < DC; ++c) v[q][c] = *reinterpret_cast<const float4*>(V + (k + q) * LDV + tx * 4 + c * 64);
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 p4 = *reinterpret_cast<const float4*>(pp + i * TY * LDP + k);
+        const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int c = 0; c < DC; ++c) {
+            const float2 pq = make_float2(p[q], p[q]);
+            acc[i][2 * c] = ptx::fma2(pq, lo2(v[q][c]), acc[i][2 * c]);
+            acc[i][2 * c + 1] = ptx::fma2(pq, hi2(v[q][c]), acc[i][2 * c + 1]);
+          }
+      }
     }
-  }
   }
 }
 
