@@ -12,7 +12,11 @@
 // (simt_tile.cuh); the next K tile is copied in under the P V product and the next V tile under Q K^T; 3 CTAs of
 // D = 64 and 2 of D = 128 share an SM.  B4 H16 S2048 D64 causal: 1587 -> 958 us (21.7 -> 35.9 TFLOP/s) against scalar
 // shared-memory loads (eight per sixteen FMAs); ncu: FMA pipe 58 % busy, 2.7 warps per scheduler, the rest latency.  The mask of
-// a tile comes through shared memory (MaskTile).  4 x 8 heads x 500, additive mask: D = 64 82 -> 76 us, D = 128 172 -> 128.
+// a tile comes through shared memory (MaskTile); one that is the same for all rows (MaskRow), and the bytes of a boolean one where
+// there is room for them (D = 64), as part of the K tile's copies, so that no barrier and no wait is spent on them.
+// Measured, us, elements loaded into registers -> now (all masks through MaskTile): 6 x 8 heads x 333, D = 64, padding 55.1 -> 53.6
+// (57.8), boolean 60.4 -> 55.9 (61.4), additive 60.3 -> 57.6 (59.3); 2 x 16/4 heads x 1100, D = 64, padding 295 -> 280 (301), boolean
+// 347 -> 295 (325); 4 x 8 heads x 500, D = 128, padding 159 -> 121 (126), boolean 184 -> 128 (132), additive 172 -> 125 (128).
 //
 // Few query tiles leave most SMs idle for the time of the longest walk over the keys, 4 us (D = 64) or 8 us per key tile.
 // The key tiles are then divided among the CTAs of a cluster (SPLIT); their unnormalised O, maxima and sums meet in
@@ -26,6 +30,7 @@ namespace ttattn {
 namespace {
 
 using namespace simt;
+enum MaskForm { kNoMask, kRowMask, kBoolMask, kAddMask };  // kRowMask: the same for all rows, of either kind
 constexpr int kThreads = 128, TY = kThreads / 16, R = TS / TY;
 
 // With only K padded two CTAs of D = 128 fit an SM, to the byte (4 x 8 heads x 500: 136 -> 119 us).  Where there are too few for
@@ -35,11 +40,15 @@ struct Lay {
   static constexpr bool kTight = D == 64 || !SPLIT;
   static constexpr Layout Q = kTight ? kSwap : kPad, V = kTight ? kPlain : kPad, P = kTight ? kSwap : kPad;
   static constexpr int kQ = kTight ? TS * D : kTileFloats<D>, kV = kQ, kP = kTight ? TS * TS : kScoreFloats;
-  static constexpr int kSmemBytes = (kQ + kTileFloats<D> + kV + kP) * static_cast<int>(sizeof(float));
+  static constexpr bool kApart = D == 64;  // a boolean mask's bytes have a place of their own, for two tiles
+  static constexpr int smem_bytes(MaskForm mask) {
+    return (kQ + kTileFloats<D> + kV + kP + (kApart && mask == kBoolMask ? 2 * TS * kByteRow : 0)) * static_cast<int>(sizeof(float));
+  }
 };
-static_assert(2 * (Lay<128, false>::kSmemBytes + 1024) <= 228 * 1024, "two CTAs of D = 128 to an SM");
+static_assert(2 * (Lay<128, false>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "two CTAs of D = 128 to an SM");
+static_assert(3 * (Lay<64, false>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "three CTAs of D = 64 to an SM");
 
-template <int D, bool MASK, bool SPLIT>
+template <int D, MaskForm MASK, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(const FwdArgs a, int cluster) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();  // launched early: everything below reads or writes global memory
@@ -73,13 +82,28 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(con
   const int64_t mask_base = b * a.mask.sb + h * a.mask.sh;
 
   MaskTile<D, TY, kThreads, LY::P> mask{a.mask, Ps, mask_base, ty, tx, tid};
+  const MaskRow<D> mask_row{a.mask, Ks, mask_base, tx, tid};
   float* mine = mask.mine();  // where this thread's scores go
+  // a tile's mask comes with its K, or (ASIDE) later, in a group of copies of its own, to where the scores go
+  constexpr bool APART = MASK == kBoolMask && LY::kApart, ASIDE = MASK == kAddMask || (MASK == kBoolMask && !APART);
+  auto apart = [&](int t) { return Ps + LY::kP + (t & 1) * TS * kByteRow; };
+  auto mask_with_k = [&](int t) {
+    if constexpr (MASK == kRowMask) mask_row.stage(t, kv_len);
+    if constexpr (APART) mask.template stage_bytes<kByteRow>(apart(t), row0, a.Lq, t * TS, kv_len);
+  };
+  auto mask_aside = [&](int col0) {
+    if constexpr (MASK == kBoolMask)
+      mask.template stage_bytes<mask.LD>(Ps, row0, a.Lq, col0, kv_len);
+    else  // (stage_added by itself: 124 bytes of spills instead of 40; 8 x 16 heads x 512, D = 64 256 us instead of 233)
+      mask.stage(row0, a.Lq, col0, kv_len);
+  };
   if (n_tiles > t0) {
     load_tile<D, kThreads, LY::Q>(Qs, q, a.qs.s, row0, a.Lq, tid);
     load_tile<D, kThreads>(Ks, k, a.ks.s, t0 * TS, kv_len, tid);
+    mask_with_k(t0);
     copies_commit();
-    if constexpr (MASK) {
-      mask.stage(row0, a.Lq, t0 * TS, kv_len);
+    if constexpr (ASIDE) {
+      mask_aside(t0 * TS);
       copies_commit();
     }
     load_tile<D, kThreads, LY::V>(Vs, v, a.vs.s, t0 * TS, kv_len, tid);
@@ -97,22 +121,27 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(con
 
   for (int t = t0; t < n_tiles; ++t) {
     const int col0 = t * TS;
-    copies_wait<MASK ? 2 : 1>();  // Q and K of this tile; the mask and V may still be on their way
+    copies_wait<ASIDE ? 2 : 1>();  // Q and K of this tile; the mask and V may still be on their way
     __syncthreads();
     float s[R][4];
     product_nt<D, TY, LY::Q>(Qs, Ks, ty, tx, s);
-    if (MASK && !mask.additive()) copies_wait<1>();
+    if (MASK == kBoolMask && ASIDE) copies_wait<1>();
     __syncthreads();  // K of this tile has been read
-    if (t + 1 < n_tiles) load_tile<D, kThreads>(Ks, k, a.ks.s, col0 + TS, kv_len, tid);
+    if (t + 1 < n_tiles) {
+      load_tile<D, kThreads>(Ks, k, a.ks.s, col0 + TS, kv_len, tid);
+      mask_with_k(t + 1);
+    }
     copies_commit();
     uint32_t hidden = 0;
-    if constexpr (MASK) {
-      if (mask.additive()) {
-        copies_wait<2>();  // (of a thread's own)
-      } else {
-        hidden = mask.bits(row0, col0);
-        __syncthreads();
-      }
+    if constexpr (MASK == kRowMask) {
+      mask_row.apply(t, c, s);
+    } else if constexpr (MASK == kAddMask) {
+      copies_wait<2>();  // (of a thread's own)
+    } else if constexpr (APART) {
+      mask.template apply<kByteRow>(apart(t), row0, col0, c, s);
+    } else if constexpr (MASK == kBoolMask) {
+      hidden = mask.bits(row0, col0);
+      __syncthreads();
     }
     const bool edge = col0 + TS > kv_len || (a.causal && col0 + TS - 1 > row0 + shift);
 #pragma unroll
@@ -121,11 +150,9 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(con
       float mx = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        s[i][j] *= c;
-        if constexpr (MASK) {
-          if (mask.additive()) s[i][j] = fmaf(mine[mask.at(i, j)], kLog2e, s[i][j]);
-          if (hidden >> (4 * i + j) & 1) s[i][j] = -INFINITY;
-        }
+        if (MASK == kNoMask || ASIDE) s[i][j] *= c;  // (the others have been)
+        if constexpr (MASK == kAddMask) s[i][j] = fmaf(mine[mask.at(i, j)], kLog2e, s[i][j]);
+        if (MASK == kBoolMask && ASIDE && (hidden >> (4 * i + j) & 1)) s[i][j] = -INFINITY;
         const int col = col0 + tx + 16 * j;
         if (edge && !(col < kv_len && (!a.causal || col <= row + shift))) s[i][j] = -INFINITY;
         mx = fmaxf(mx, s[i][j]);
@@ -153,8 +180,8 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(con
     __syncthreads();
     product_nn<D, TY, LY::P, LY::V>(Ps, Vs, ty, tx, acc);
     __syncthreads();  // V and P have been read
-    if constexpr (MASK) {
-      if (t + 1 < n_tiles) mask.stage(row0, a.Lq, col0 + TS, kv_len);
+    if constexpr (ASIDE) {
+      if (t + 1 < n_tiles) mask_aside(col0 + TS);
       copies_commit();
     }
     if (t + 1 < n_tiles) load_tile<D, kThreads, LY::V>(Vs, v, a.vs.s, col0 + TS, kv_len, tid);
@@ -253,9 +280,9 @@ int split_of(const FwdArgs& a, int D) {
   return cluster;
 }
 
-template <int D, bool MASK>
+template <int D, MaskForm MASK>
 cudaError_t launch_t(const FwdArgs& a, cudaStream_t stream) {
-  const int cluster = split_of(a, D), smem = cluster > 1 ? Lay<D, true>::kSmemBytes : Lay<D, false>::kSmemBytes;
+  const int cluster = split_of(a, D), smem = cluster > 1 ? Lay<D, true>::smem_bytes(MASK) : Lay<D, false>::smem_bytes(MASK);
   auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true> : fwd_simt_kernel<D, MASK, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
@@ -264,13 +291,19 @@ cudaError_t launch_t(const FwdArgs& a, cudaStream_t stream) {
                       spread_smem(smem, ctas, cluster), stream, cluster, a, cluster);
 }
 
+template <int D>
+cudaError_t launch_d(const FwdArgs& a, cudaStream_t stream) {
+  if (!a.mask.ptr) return launch_t<D, kNoMask>(a, stream);
+  if (a.mask.sl == 0) return launch_t<D, kRowMask>(a, stream);
+  return a.mask.kind == TT_ATTN_MASK_BOOL ? launch_t<D, kBoolMask>(a, stream) : launch_t<D, kAddMask>(a, stream);
+}
+
 }  // namespace
 
 cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, cudaStream_t stream) {
   if (dtype != TT_ATTN_F32) return cudaErrorInvalidValue;
-  const bool mask = a.mask.ptr != nullptr;
-  if (D == 64) return mask ? launch_t<64, true>(a, stream) : launch_t<64, false>(a, stream);
-  if (D == 128) return mask ? launch_t<128, true>(a, stream) : launch_t<128, false>(a, stream);
+  if (D == 64) return launch_d<64>(a, stream);
+  if (D == 128) return launch_d<128>(a, stream);
   return cudaErrorInvalidValue;
 }
 

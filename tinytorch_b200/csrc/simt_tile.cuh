@@ -141,13 +141,16 @@ __device__ __forceinline__ void product_tn(const float* P, const float* X, int t
   }
 }
 
+constexpr int kByteRow = TS / 4 + 1;  // words that hold the 64 bytes of a row at any offset
+
 // The mask of a tile's scores.  Where thread (ty, tx) will write its probabilities, [(ty + TY i) LD + tx + 16 j] (kSwap: + 16 (j ^
 // (ty & 1))), the tile's shared memory holds before
 //   an additive mask   the thread's own elements, copied asynchronously one by one: nobody else has to wait for them;
 //   a boolean one      its bytes, a row in the first 68 bytes of a row (one row where all are the same): aligned words, copied by
-//                      all threads together.  Every thread has to take its own (bits) before any writes a probability.
+//                      all threads together.  Every thread has to take its own (bits) before any writes a probability,
+//                      unless they lie somewhere else (stage_bytes, apply).
 // (All elements in registers, fetched ahead of the product that comes first, are 32 of them: a CTA fewer to an SM.)  4 x 8
-// heads x 500 with an additive mask, D = 128: forward 172 -> 128 us, without a mask 119; D = 64: backward 221 -> 202, 186.
+// heads x 500 with an additive mask, D = 128: forward 172 -> 125 us, without a mask 119; D = 64: backward 221 -> 202, 186.
 template <int D, int TY, int NT, Layout LAY>
 struct MaskTile {
   static constexpr int R = TS / TY, LD = LAY == kPad ? LP : TS;
@@ -161,32 +164,49 @@ struct MaskTile {
   __device__ __forceinline__ int at(int i, int j) const { return i * TY * LD + (LAY == kSwap ? j ^ (ty & 1) : j) * 16; }
 
   // copies of the tile at (row0, col0) on their way; outside: 0 (added), anything (boolean)
-  __device__ __forceinline__ void stage(int row0, int n_rows, int col0, int n_cols) {
-    if (additive()) {
-      const int row = row0 + ty, col = col0 + tx;
-      const float* p = reinterpret_cast<const float*>(m.ptr) + base + row * m.sl + col;
-      const uint32_t dst = ptx::smem_u32(mine());
+  __device__ __forceinline__ void stage(int row0, int n_rows, int col0, int n_cols) const {
+    if (additive())
+      stage_added(row0, n_rows, col0, n_cols);
+    else
+      stage_bytes<LD>(tile, row0, n_rows, col0, n_cols);
+  }
+  __device__ __forceinline__ void stage_added(int row0, int n_rows, int col0, int n_cols) const {
+    const int row = row0 + ty, col = col0 + tx;
+    const float* p = reinterpret_cast<const float*>(m.ptr) + base + row * m.sl + col;
+    const uint32_t dst = ptx::smem_u32(mine());
 #pragma unroll
-      for (int i = 0; i < R; ++i, p += TY * m.sl)
+    for (int i = 0; i < R; ++i, p += TY * m.sl)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const bool in = row + TY * i < n_rows && col + 16 * j < n_cols;
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + at(i, j) * 4),
-                       "l"(in ? p + 16 * j : reinterpret_cast<const float*>(m.ptr)), "r"(in ? 4 : 0)
-                       : "memory");
-        }
-    } else {
-      constexpr int W = TS / 4 + 1;  // words that hold 64 bytes at any offset
-      const uint8_t* any = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(m.ptr) & ~uintptr_t(3));
-      for (int e = tid; e < (m.sl == 0 ? W : TS * W); e += NT) {
-        const int r = e / W, w = e - r * W;
-        const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + base + (row0 + r) * m.sl + col0;
-        const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);
-        const bool in = row0 + r < n_rows && w * 4 - mis < n_cols - col0 && w * 4 - mis < TS;  // some byte of it is looked at
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(tile + r * LD + w)),
-                     "l"(in ? p - mis + w * 4 : any), "r"(in ? 4 : 0)
+      for (int j = 0; j < 4; ++j) {
+        const bool in = row + TY * i < n_rows && col + 16 * j < n_cols;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + at(i, j) * 4),
+                     "l"(in ? p + 16 * j : reinterpret_cast<const float*>(m.ptr)), "r"(in ? 4 : 0)
                      : "memory");
       }
+  }
+  template <int WORDS>  // of a row at `dst`
+  __device__ __forceinline__ void stage_bytes(float* dst, int row0, int n_rows, int col0, int n_cols) const {
+    const uint8_t* any = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(m.ptr) & ~uintptr_t(3));
+    for (int e = tid; e < (m.sl == 0 ? kByteRow : TS * kByteRow); e += NT) {
+      const int r = e / kByteRow, w = e - r * kByteRow;
+      const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + base + (row0 + r) * m.sl + col0;
+      const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);
+      const bool in = row0 + r < n_rows && w * 4 - mis < n_cols - col0 && w * 4 - mis < TS;  // some byte of it is looked at
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(dst + r * WORDS + w)),
+                   "l"(in ? p - mis + w * 4 : any), "r"(in ? 4 : 0)
+                   : "memory");
+    }
+  }
+  // boolean, bytes at `src`: scores of column col0 + tx + 16 j, scaled and masked
+  template <int WORDS>
+  __device__ __forceinline__ void apply(const float* src, int row0, int col0, float c, float (&s)[R][4]) const {
+    const uint32_t off = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(m.ptr) + base + col0 + (row0 + ty) * m.sl);
+    const uint8_t* p = reinterpret_cast<const uint8_t*>(src + ty * WORDS) + tx;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const uint8_t* q = p + i * TY * WORDS * 4 + ((off + i * TY * static_cast<uint32_t>(m.sl)) & 3);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = q[16 * j] ? s[i][j] * c : -INFINITY;
     }
   }
   // boolean: bit 4 i + j: score (i, j) is hidden (or outside, where it does not count); the copies are complete and visible
@@ -202,6 +222,55 @@ struct MaskTile {
       for (int j = 0; j < 4; ++j) b |= q[16 * j] ? 0u : 1u << (4 * i + j);
     }
     return b;
+  }
+};
+
+// A mask that is the same for all rows (padding), for the forward: its elements for a tile, 64 floats or the 17 words that hold 64
+// bytes, lie in the padding of the K tile, come with it and stay until the tile after next: nobody waits for them by themselves.
+template <int D>
+struct MaskRow {
+  const MaskArgs& m;
+  float* tile;   // K
+  int64_t base;  // of (batch, head)
+  int tx, tid;
+
+  __device__ __forceinline__ bool additive() const { return m.kind != TT_ATTN_MASK_BOOL; }
+  // word `w` of key tile t: four to a row, 16 or (bytes) 5 rows, those of odd tiles behind
+  static __device__ __forceinline__ int at(int t, int w) { return ((t & 1) * (TS / 4) + w / 4) * kLd<D> + D + w % 4; }
+
+  // the copy for key tile t; outside: 0 (added), anything (boolean)
+  __device__ __forceinline__ void stage(int t, int n_cols) const {
+    const int es = additive() ? 4 : 1, col0 = t * TS;
+    if (tid >= (additive() ? TS : kByteRow)) return;
+    const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + (base + col0) * es;
+    const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);  // (0 of floats)
+    const int first = tid * 4 - mis;                                       // of the word's bytes, counted from that of col0
+    const bool in = first < (n_cols - col0) * es && first < TS * es;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(tile + at(t, tid))), "l"(in ? p + first : p - mis),
+                 "r"(in ? 4 : 0)
+                 : "memory");
+  }
+  // scores of columns t TS + tx + 16 j, scaled and masked
+  template <int R>
+  __device__ __forceinline__ void apply(int t, float c, float (&s)[R][4]) const {
+    if (additive()) {
+      const float* p = tile + at(t, tx);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float add = p[j * 4 * kLd<D>];
+#pragma unroll
+        for (int i = 0; i < R; ++i) s[i][j] = fmaf(add, kLog2e, s[i][j] * c);
+      }
+    } else {
+      const int off = tx + static_cast<int>((reinterpret_cast<uintptr_t>(m.ptr) + base + t * TS) & 3);
+      const uint8_t* p = reinterpret_cast<const uint8_t*>(tile + at(t, off / 4)) + off % 4;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool seen = p[j * kLd<D> * 4] != 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) s[i][j] = seen ? s[i][j] * c : -INFINITY;
+      }
+    }
   }
 };
 
