@@ -449,7 +449,7 @@ template <int D>
 constexpr int kDqSmemBytes = 2 * (TS * TS + TS * D) * static_cast<int>(sizeof(float));
 
 template <int D>
-cudaError_t launch_dq(const BwdArgs& a, cudaStream_t stream) {
+cudaError_t launch_dq(const BwdArgs& a, int device, cudaStream_t stream) {
   const long long q_tiles = (a.Lq + TS - 1) / TS, items = q_tiles * a.Hq * a.B;
   const int k_tiles = (a.Skv + TS - 1) / TS;
   int cluster = 1;  // (steps of 2 us (D = 64) or 4 in a CTA alone)
@@ -458,12 +458,12 @@ cudaError_t launch_dq(const BwdArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   if (items * cluster > 0x7fffffffll) return cudaErrorInvalidValue;
-  return launch_early(kern, dim3(static_cast<unsigned>(items * cluster)), dim3(128), spread_smem(kDqSmemBytes<D>, items * cluster, cluster),
+  return launch_early(kern, dim3(static_cast<unsigned>(items * cluster)), dim3(128), spread_smem(kDqSmemBytes<D>, items * cluster, cluster, device),
                       stream, cluster, a, cluster);
 }
 
 template <int D, bool MASK>
-cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
+cudaError_t launch_t(const BwdArgs& a, int device, cudaStream_t stream) {
   cudaError_t e = launch_delta_t<float, D>(a, stream);
   if (e != cudaSuccess) return e;
   const bool store = a.ds != nullptr;
@@ -476,9 +476,9 @@ cudaError_t launch_t(const BwdArgs& a, cudaStream_t stream) {
   const long long key_ctas = a.dk || a.dv ? key_tiles * a.Hkv * a.B : 0, q_ctas = a.dq && !store ? q_tiles * a.Hq * a.B : 0;
   if ((key_ctas + q_ctas) * cluster > 0x7fffffffll) return cudaErrorInvalidValue;
   e = launch_early(kern, dim3(static_cast<unsigned>((key_ctas + q_ctas) * cluster)), dim3(Cfg<D>::NT),
-                   spread_smem(Cfg<D>::kSmemBytes, (key_ctas + q_ctas) * cluster, cluster), stream, cluster, a,
+                   spread_smem(Cfg<D>::kSmemBytes, (key_ctas + q_ctas) * cluster, cluster, device), stream, cluster, a,
                    static_cast<int>(key_tiles), static_cast<int>(key_ctas), cluster);
-  return e == cudaSuccess && store ? launch_dq<D>(a, stream) : e;
+  return e == cudaSuccess && store ? launch_dq<D>(a, device, stream) : e;
 }
 
 }  // namespace
@@ -501,11 +501,11 @@ size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   return bytes <= 192e6 && pairs >= (D == 64 ? 600 : 300) ? static_cast<size_t>(bytes) : 0;
 }
 
-cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, cudaStream_t stream) {
+cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream) {
   if (dtype != TT_ATTN_F32) return cudaErrorInvalidValue;
   const bool mask = a.mask.ptr != nullptr;
-  if (D == 64) return mask ? launch_t<64, true>(a, stream) : launch_t<64, false>(a, stream);
-  if (D == 128) return mask ? launch_t<128, true>(a, stream) : launch_t<128, false>(a, stream);
+  if (D == 64) return mask ? launch_t<64, true>(a, device, stream) : launch_t<64, false>(a, device, stream);
+  if (D == 128) return mask ? launch_t<128, true>(a, device, stream) : launch_t<128, false>(a, device, stream);
   return cudaErrorInvalidValue;
 }
 

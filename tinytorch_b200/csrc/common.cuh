@@ -122,8 +122,8 @@ struct DecodeArgs {
 
 // Each returns a cudaError_t from the launch (no synchronisation).
 cudaError_t launch_fwd_tc(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
-cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, cudaStream_t stream);
-cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
+cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
+cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 // rowsum(dO o O) into a.delta only (first step of every backward)
 cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
 // Work items per key tile of the tensor-core backward, and the workspace they need beside dq_accum (0 for one item)

@@ -281,29 +281,29 @@ int split_of(const FwdArgs& a, int D) {
 }
 
 template <int D, MaskForm MASK>
-cudaError_t launch_t(const FwdArgs& a, cudaStream_t stream) {
+cudaError_t launch_t(const FwdArgs& a, int device, cudaStream_t stream) {
   const int cluster = split_of(a, D), smem = cluster > 1 ? Lay<D, true>::smem_bytes(MASK) : Lay<D, false>::smem_bytes(MASK);
   auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true> : fwd_simt_kernel<D, MASK, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   const long long ctas = static_cast<long long>((a.Lq + TS - 1) / TS) * cluster * a.Hq * a.B;
   return launch_early(kern, dim3((a.Lq + TS - 1) / TS * cluster, a.Hq, a.B), dim3(kThreads),
-                      spread_smem(smem, ctas, cluster), stream, cluster, a, cluster);
+                      spread_smem(smem, ctas, cluster, device), stream, cluster, a, cluster);
 }
 
 template <int D>
-cudaError_t launch_d(const FwdArgs& a, cudaStream_t stream) {
-  if (!a.mask.ptr) return launch_t<D, kNoMask>(a, stream);
-  if (a.mask.sl == 0) return launch_t<D, kRowMask>(a, stream);
-  return a.mask.kind == TT_ATTN_MASK_BOOL ? launch_t<D, kBoolMask>(a, stream) : launch_t<D, kAddMask>(a, stream);
+cudaError_t launch_d(const FwdArgs& a, int device, cudaStream_t stream) {
+  if (!a.mask.ptr) return launch_t<D, kNoMask>(a, device, stream);
+  if (a.mask.sl == 0) return launch_t<D, kRowMask>(a, device, stream);
+  return a.mask.kind == TT_ATTN_MASK_BOOL ? launch_t<D, kBoolMask>(a, device, stream) : launch_t<D, kAddMask>(a, device, stream);
 }
 
 }  // namespace
 
-cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, cudaStream_t stream) {
+cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream) {
   if (dtype != TT_ATTN_F32) return cudaErrorInvalidValue;
-  if (D == 64) return launch_d<64>(a, stream);
-  if (D == 128) return launch_d<128>(a, stream);
+  if (D == 64) return launch_d<64>(a, device, stream);
+  if (D == 128) return launch_d<128>(a, device, stream);
   return cudaErrorInvalidValue;
 }
 

@@ -8,8 +8,11 @@
 // product) can do without: kSwap exchanges neighbouring pieces of the odd rows instead.  Sums run as fma.rn.f32x2: two fp32 FMAs per issued instruction, each rounded
 // as the scalar one.  (Unrolling the vector loops 4 / 4 / 8 times: 3-5 % over 2 / 2 / 4; whole or not at all: slower.)
 #pragma once
+#include <atomic>
+
 #include "common.cuh"
 #include "ptx.cuh"
+#include "tma_host.cuh"
 
 namespace ttattn {
 namespace simt {
@@ -274,14 +277,51 @@ struct MaskRow {
   }
 };
 
-// Shared memory to ask for, so that no SM gets more CTAs than it has to: the CTAs of a cluster are put on as few SMs as hold
-// them, and a few of them then work two to an SM beside idle ones (D = 128, 8 heads x 512: 61 us instead of 39).  Clusters
-// of 4 and 8 do not fill every GPC, so that a grid close to the number of SMs is left as it is.
-inline int spread_smem(int need, long long ctas, int cluster) {
-  const int sms = cluster == 8 ? 128 : (cluster == 4 ? 136 : kSms);
+// the least a CTA can ask for so that no more than per_sm fit an SM
+constexpr int least_smem(int per_sm) { return 228 * 1024 / (per_sm + 1) - 1024 + 128; }
+
+// CTAs of clusters of this size that can be resident at once where shared memory leaves room for `per_sm` (1 or 2) on an SM: a
+// cluster lives inside one GPC, and GPCs differ in size, from one chip to the next too.  Asked once per device.
+static __global__ void room_kernel() {}
+inline int cluster_room(int device, int cluster, int per_sm) {
+  static std::atomic<int> known[64][3][2];
+  if (device < 0 || device >= 64) return 0;
+  if (cluster == 1) return per_sm * sm_count(device);
+  std::atomic<int>& k = known[device][cluster == 2 ? 0 : (cluster == 4 ? 1 : 2)][per_sm - 1];
+  int n = k.load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(per_sm * sm_count(device) / cluster * cluster);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = least_smem(per_sm);
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, room_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    n = clusters > 0 ? clusters * cluster : -1;
+    k.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// Shared memory to ask for, so that no SM gets more CTAs than it has to, where all of them can be resident at once or two to an
+// SM: CTAs are put on as few SMs as hold them, and some then work two or three to an SM beside idle ones (D = 128, 8 heads x 512:
+// 61 us instead of 39; single CTAs, D = 64, 6 x 8 x 333: 72 instead of 53).  The launch attribute that asks for clusters to be
+// spread changes nothing.  The price: two such calls on two streams do not share an SM either (D = 64, 2 heads x 1024, alone 43 ->
+// 29 us, two at a time 47 -> 56; 8 heads x 512 29 -> 22 and 34 -> 37), and a successor that is launched early finds no room before
+// the CTAs of this grid end.
+// Clusters do not fill every GPC, so how many fit is asked of the device: one cluster more than that would wait for a whole round (16
+// clusters of 8 where 15 fit, 512 queries x 2 heads on 4000 keys, D = 64: 105 us; as it is 73, without the request 74).
+inline int spread_smem(int need, long long ctas, int cluster, int device) {
   for (int per_sm = 1; per_sm <= 2; ++per_sm)
-    if (ctas <= static_cast<long long>(per_sm) * sms) {
-      const int least = 228 * 1024 / (per_sm + 1) - 1024 + 128;  // too much for per_sm + 1 of them
+    if (ctas <= cluster_room(device, cluster, per_sm)) {
+      const int least = least_smem(per_sm);
       return need > least ? need : least;
     }
   return need;
