@@ -109,6 +109,8 @@ class FusedOracle:
     """fused_oracle.c: the reference's CPU fp32 siluMul / fusedAddRmsNorm, restated."""
 
     def __init__(self):
+        if not os.path.exists(ORACLE_SO):
+            build()
         self.lib = C.CDLL(ORACLE_SO)
         self.lib.oracle_silu_mul.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]
         self.lib.oracle_silu_mul.restype = None
