@@ -95,6 +95,13 @@ typedef struct tt_linear_params {
 } tt_linear_params;
 
 TT_ATTN_API int tt_linear(const tt_linear_params* p);
+
+/* For tests: the same projection with a tile of the caller's choice among those that tt_linear chooses
+ * from.  `shape`: the columns of a tile of single CTAs (64 .. 256 in steps of 32, with w_t of 64), or -192
+ * for pairs (not with w_t); TT_ATTN_ERR_SHAPE for any other.  0 launches nothing.  `planned` (host memory,
+ * or NULL with a shape) receives what tt_linear takes: such a number, -256 for pairs of 256 x 256, 0 for
+ * the contraction divided over a cluster.  x_sum is not written. */
+TT_ATTN_API int tt_linear_selftest(const tt_linear_params* p, int32_t shape, int32_t* planned);
 TT_ATTN_API int tt_fused_add_rms_norm(const tt_fused_add_rms_norm_params* p);
 TT_ATTN_API int tt_silu_mul(const tt_silu_mul_params* p);
 

@@ -89,6 +89,23 @@ def test_linear_rejects_bad_arguments():
     assert lib.tt_linear(C.byref(p)) == 0             # nothing to do
 
 
+def test_linear_tile_shapes_that_do_not_exist_are_refused():
+    """Pairs load half of 192 rows of w, which are not whole blocks of 64 where w is stored [K, N]."""
+    f = _capi.lib().tt_linear_selftest
+    f.argtypes, f.restype = [C.POINTER(_capi.LinearParams), C.c_int32, C.POINTER(C.c_int32)], C.c_int
+    p = _capi.LinearParams()
+    p.struct_size, p.dtype, p.M, p.N, p.K = C.sizeof(p), _capi.BF16, 256, 512, 64
+    p.x = p.w = p.y = 0x1000
+    bad = {0: (32, 48, 72, 288, -64, -128, -256, 2 ** 31 - 1, -2 ** 31), 1: (96, 160, 224, -192)}
+    for w_t, shapes in bad.items():
+        p.w_t = w_t
+        for shape in shapes:
+            assert f(C.byref(p), shape, None) == -3, (w_t, shape)
+    assert f(C.byref(p), 0, None) == -1               # nothing asked for
+    p.K = 60
+    assert f(C.byref(p), 64, None) == -5
+
+
 def test_library_exports_every_symbol_of_tt_fused_h():
     text = open(os.path.join(ROOT, "include", "tt_fused.h")).read()
     names = re.findall(r"TT_ATTN_API\s+[\w\s\*]+?\b(tt_\w+)\s*\(", text)

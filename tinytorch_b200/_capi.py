@@ -123,7 +123,7 @@ class LinearParams(C.Structure):
     ]
 
 
-FUSED_EXPORTS = ("tt_fused_add_rms_norm", "tt_silu_mul", "tt_linear")  # include/tt_fused.h
+FUSED_EXPORTS = ("tt_fused_add_rms_norm", "tt_silu_mul", "tt_linear", "tt_linear_selftest")  # include/tt_fused.h
 
 EXPORTS = ("tt_attn_fwd", "tt_attn_bwd", "tt_attn_decode", "tt_attn_decode_append", "tt_attn_decode_static",
            "tt_attn_selftest_wait_expiry", "tt_attn_workspace_bytes", "tt_attn_strerror",

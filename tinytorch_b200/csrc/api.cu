@@ -80,6 +80,32 @@ int check_common(int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D) {
 
 using namespace ttattn;
 
+// What tt_linear is asked for, checked; sums_only: just the sums of x (w and y, and what describes them, are not looked at).
+static int linear_call(const tt_linear_params* p, LinearCall* c, bool* sums_only) {
+  if (!p) return TT_ATTN_ERR_NULL;
+  const bool ext = p->struct_size == sizeof(tt_linear_params);
+  if (!ext && p->struct_size != offsetof(tt_linear_params, x_t)) return TT_ATTN_ERR_STRUCT;
+  if (p->dtype != TT_ATTN_F16 && p->dtype != TT_ATTN_BF16) return TT_ATTN_ERR_DTYPE;
+  if (p->M < 0 || p->N <= 0 || p->K <= 0 || p->M > 0x7fffffff || p->N > 0x7fffffff || p->K > 0x7fffffff)
+    return TT_ATTN_ERR_SHAPE;
+  const bool x_t = ext && p->x_t != 0, w_t = ext && p->w_t != 0;
+  const void* x_sum = ext ? p->x_sum : nullptr;
+  const int64_t x_cols = x_t ? p->M : p->K, w_cols = w_t ? p->N : p->K;  // the contiguous dimensions
+  const int64_t ldx = p->ldx ? p->ldx : x_cols, ldw = p->ldw ? p->ldw : w_cols, ldy = p->ldy ? p->ldy : p->N;
+  *c = LinearCall{p->dtype, p->x, p->w, p->bias, p->y, static_cast<int>(p->M), static_cast<int>(p->N), static_cast<int>(p->K),
+                  ldx, ldw, ldy, x_t, w_t, p->status, p->device, static_cast<cudaStream_t>(p->stream)};
+  *sums_only = x_sum && !p->w && !p->y;
+  if (p->M == 0) return TT_ATTN_OK;
+  if (!p->x || (!*sums_only && (!p->w || !p->y))) return TT_ATTN_ERR_NULL;
+  if (x_sum && !x_t) return TT_ATTN_ERR_SHAPE;
+  if (ldx < x_cols || ldw < w_cols || ldy < p->N) return TT_ATTN_ERR_SHAPE;
+  auto odd = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 2 != 0; };
+  if (x_cols % 8 || ldx % 8 || !aligned16(p->x) || odd(x_sum)) return TT_ATTN_ERR_ALIGN;
+  if (!*sums_only && (w_cols % 8 || p->N % 8 || ldw % 8 || ldy % 8 || !aligned16(p->w) || !aligned16(p->y) || odd(p->bias)))
+    return TT_ATTN_ERR_ALIGN;
+  return TT_ATTN_OK;
+}
+
 extern "C" {
 
 int tt_attn_version(void) { return TT_ATTN_ABI_VERSION; }
@@ -428,37 +454,31 @@ int tt_silu_mul(const tt_silu_mul_params* p) {
 }
 
 int tt_linear(const tt_linear_params* p) {
-  if (!p) return TT_ATTN_ERR_NULL;
-  const bool ext = p->struct_size == sizeof(tt_linear_params);
-  if (!ext && p->struct_size != offsetof(tt_linear_params, x_t)) return TT_ATTN_ERR_STRUCT;
-  if (p->dtype != TT_ATTN_F16 && p->dtype != TT_ATTN_BF16) return TT_ATTN_ERR_DTYPE;
-  if (p->M < 0 || p->N <= 0 || p->K <= 0 || p->M > 0x7fffffff || p->N > 0x7fffffff || p->K > 0x7fffffff)
-    return TT_ATTN_ERR_SHAPE;
-  if (p->M == 0) return TT_ATTN_OK;
-  const bool x_t = ext && p->x_t != 0, w_t = ext && p->w_t != 0;
-  void* x_sum = ext ? p->x_sum : nullptr;
-  const bool sums_only = x_sum && !p->w && !p->y;
-  if (!p->x || (!sums_only && (!p->w || !p->y))) return TT_ATTN_ERR_NULL;
-  if (x_sum && !x_t) return TT_ATTN_ERR_SHAPE;
-  const int64_t x_cols = x_t ? p->M : p->K, w_cols = w_t ? p->N : p->K;  // the contiguous dimensions
-  const int64_t ldx = p->ldx ? p->ldx : x_cols, ldw = p->ldw ? p->ldw : w_cols, ldy = p->ldy ? p->ldy : p->N;
-  if (ldx < x_cols || ldw < w_cols || ldy < p->N) return TT_ATTN_ERR_SHAPE;
-  // (sums alone: w and y, and what describes them, are not looked at any further)
-  if (sums_only ? x_cols % 8 || ldx % 8 || !aligned16(p->x) || reinterpret_cast<uintptr_t>(x_sum) % 2 : x_cols % 8 || w_cols % 8 || p->N % 8 || ldx % 8 || ldw % 8 || ldy % 8 || !aligned16(p->x) || !aligned16(p->w) ||
-      !aligned16(p->y) || (p->bias && reinterpret_cast<uintptr_t>(p->bias) % 2) || reinterpret_cast<uintptr_t>(x_sum) % 2)
-    return TT_ATTN_ERR_ALIGN;
+  LinearCall c;
+  bool sums_only;
+  if (int rc = linear_call(p, &c, &sums_only)) return rc;
+  if (c.M == 0) return TT_ATTN_OK;
+  void* x_sum = p->struct_size == sizeof(tt_linear_params) ? p->x_sum : nullptr;
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
-  cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  if (sums_only) {
-    cudaError_t e = launch_column_sums(p->dtype, p->x, x_sum, p->K, p->M, ldx, false, stream);
-    return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
-  }
-  const LinearCall c{p->dtype, p->x, p->w, p->bias, p->y, static_cast<int>(p->M), static_cast<int>(p->N),
-                     static_cast<int>(p->K), ldx, ldw, ldy, x_t, w_t, p->status, p->device, stream};
   bool persistent = false;
-  cudaError_t e = launch_linear_tc(c, &persistent);
-  if (e == cudaSuccess && x_sum) e = launch_column_sums(p->dtype, p->x, x_sum, p->K, p->M, ldx, persistent, stream);
+  cudaError_t e = sums_only ? cudaSuccess : launch_linear_tc(c, &persistent);
+  if (e == cudaSuccess && x_sum) e = launch_column_sums(c.dtype, c.x, x_sum, c.K, c.M, c.ldx, persistent, c.stream);
+  return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
+}
+
+int tt_linear_selftest(const tt_linear_params* p, int32_t shape, int32_t* planned) {
+  LinearCall c;
+  bool sums_only;
+  if (int rc = linear_call(p, &c, &sums_only)) return rc;
+  const bool pair = shape < 0;
+  const int bn = shape < -1024 ? 0 : (pair ? -shape : shape);
+  if (sums_only || c.M == 0 || (shape != 0 && !linear_tile_fits(c, pair, bn))) return TT_ATTN_ERR_SHAPE;
+  if (shape == 0 && !planned) return TT_ATTN_ERR_NULL;
+  DeviceGuard guard(p->device);
+  if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
+  if (planned) *planned = linear_shape(c);
+  cudaError_t e = shape != 0 ? launch_linear_tile(c, pair, bn) : cudaSuccess;
   return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
 }
 

@@ -167,8 +167,11 @@ struct LinearCall {
 // sectors instead of four where they are not a multiple of a sector (from the fits in linear_tile.cu and linear_split.cu).
 inline double row_lines(int64_t ld) { return ld % 16 ? 1.74 : (ld % 64 ? 1.17 : 1.0); }
 cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  // *persistent: the CTAs let the next kernel in once all before them is complete
+// What it takes: 0, the contraction divided; single CTAs: the columns of a tile; pairs: minus the columns of a tile.
+int linear_shape(const LinearCall& c);
 // ... with tiles made to measure (linear_tile.cu): single CTAs with 128 x `bn`, or pairs with 256 x 192
 double linear_tile_us(const LinearCall& c, bool pair, int bn);  // what it, or pairs with 256 x 256, are expected to take
+bool linear_tile_fits(const LinearCall& c, bool pair, int bn);  // whether there is such a tile for operands stored like these
 cudaError_t launch_linear_tile(const LinearCall& c, bool pair, int bn);
 // ... for outputs with too few tiles to occupy the machine: contraction split over clusters (linear_split.cu)
 struct SplitPlan {

@@ -326,6 +326,12 @@ Plan plan_of(const LinearCall& c, SplitPlan* split) {
 }
 }  // namespace
 
+int linear_shape(const LinearCall& c) {
+  SplitPlan split;
+  const Plan p = plan_of(c, &split);
+  return p.kernel == Plan::kSplit ? 0 : (p.kernel == Plan::kPairs ? -BN : (p.pair ? -p.bn : p.bn));
+}
+
 cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent) {
   if (persistent) *persistent = false;
   if (c.dtype != TT_ATTN_BF16 && c.dtype != TT_ATTN_F16) return cudaErrorInvalidValue;

@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                      const __grid_constant__ CUtensorMap tmY, const LinArgs a) {
   using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   constexpr bool PAIR = PAIR_BN != 0;
+  static_assert(!(PAIR && W_MN), "the 96 columns of w that a CTA of a pair loads are not whole blocks of 64");
   constexpr int BM = PAIR ? 2 * HM : HM, CW = kOutCols<PAIR>, OB = kOutBytes<PAIR>;
   extern __shared__ __align__(1024) uint8_t smem[];
   const int bn = PAIR ? PAIR_BN : a.bn, stages = PAIR ? kPairStages : a.stages, sbytes = stage_bytes<PAIR>(bn);
@@ -180,12 +181,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             load(sa, &tmX, bar, kb * BK, m0);  // rows beyond M read as zero
           }
           if constexpr (W_MN) {
-            if constexpr (PAIR) {
-              load(sa + kABytes, &tmW, bar, n0, kb * BK);
-              load(sa + kABytes + kMnBlock, &tmW, bar, n0 + 64, kb * BK);
-            } else {
-              for (int c = 0; c < wn; c += 64) load(sa + kABytes + c * (BK * 2), &tmW, bar, n0 + c, kb * BK);
-            }
+            for (int c = 0; c < wn; c += 64) load(sa + kABytes + c * (BK * 2), &tmW, bar, n0 + c, kb * BK);
           } else {
             load(sa + kABytes, &tmW, bar, kb * BK, n0);
           }
@@ -376,7 +372,12 @@ double linear_tile_us(const LinearCall& c, bool pair, int bn) {
   return 2.1 + (pair ? 1.6 : 0.0) + (body > out ? body + 0.1 * out : out + 0.1 * body) + epi;
 }
 
+bool linear_tile_fits(const LinearCall& c, bool pair, int bn) {
+  return pair ? bn == 192 && !c.w_t : bn >= 64 && bn <= kMaxBN && bn % (c.w_t ? 64 : 32) == 0;
+}
+
 cudaError_t launch_linear_tile(const LinearCall& c, bool pair, int bn) {
+  if (!linear_tile_fits(c, pair, bn)) return cudaErrorInvalidValue;
   return c.dtype == TT_ATTN_BF16 ? launch_bf<true>(c, pair, bn) : launch_bf<false>(c, pair, bn);
 }
 
