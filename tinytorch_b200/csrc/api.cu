@@ -268,7 +268,7 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
   size_t need = delta, part = 0;
   bool lens = false;
-  // fp32: dS tiles on their way from dK / dV to dQ, where all three are asked for and there is room
+  // fp32: dS tiles on their way from dK / dV to dQ, where dQ and at least one of the others are asked for and there is room
   size_t ds = p->dtype == TT_ATTN_F32 && p->dq && (p->dk || p->dv) ? round256(bwd_ds_bytes(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) : 0;
   if (delta + ds > room) ds = 0;
   if (p->dtype != TT_ATTN_F32) {
