@@ -1,7 +1,8 @@
 """GPU: the projection kernels and their gradient products at the edges of their tiles and dispatch rules.
 
-linear_split.cu takes outputs with few tiles (any M up to 128, or fewer 256 x 256 tiles than about two rounds of CTA
-pairs, by cost), linear_tc.cu the rest; both read operands stored with the contraction slow or fast.  Reference: the
+linear_split.cu takes outputs with few tiles (any M up to 128, and where it is expected to be the fastest), linear_tc.cu those with two
+rounds of 256 x 256 tiles, linear_tile.cu (test_linear_tiles_gpu.py) what lies between; all read operands stored with the
+contraction slow or fast.  Reference: the
 same sums in fp64.  Bound per element: half a unit in the last place of the tensor dtype for the one rounding, plus
 fp32 accumulation in any order: (terms + 2) * 2^-24 * sum of |products|.
 """
@@ -26,9 +27,9 @@ def _check(got, a, b, bias, dtype):  # got ~ a b (+ bias), a [m, k], b [k, n] in
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,K,N", [
     (1, 8, 8), (16, 64, 128), (17, 72, 136), (3, 4096, 264),                 # one tile of x; clusters of 1 .. 8
-    (128, 520, 1024), (129, 1032, 4096), (255, 64, 4096), (300, 1024, 3000),  # several tiles of x, K tails
+    (128, 520, 1024), (129, 1032, 4096), (255, 64, 4096), (300, 1024, 3000),  # several tiles of x, K tails; dW: tiles made to measure
     (511, 192, 264), (257, 4160, 512),
-    (1100, 72, 9736), (2050, 456, 4872), (4000, 64, 2568),                    # the persistent pairs, ragged on every side
+    (1100, 72, 9736), (2050, 456, 4872), (4000, 64, 2568),                    # forward: the persistent pairs, ragged on every side
 ])
 def test_projection_and_gradients_at_tile_edges(dtype, M, K, N):
     from tinytorch_b200 import fused

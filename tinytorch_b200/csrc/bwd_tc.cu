@@ -91,17 +91,6 @@ struct Cfg128 {
 // First of the n steps of a key tile that belongs to part p of `parts`.
 __device__ __forceinline__ int part_begin(int n, int p, int parts) { return parts == 1 ? p * n : n * p / parts; }
 
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  } else {
-    __half2 t = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  }
-}
-
 // The mask of 16 queries and this thread's key, as stored: adjacent threads read adjacent keys.  Fetched before the scores
 // arrive, all loads in flight together (one by one inside the arithmetic they made a step ten times as long): B5 H32/16
 // L1620 D64 with an additive bf16 mask 3447 -> 620 us, without a mask 380; D128, 2 x 16/4 heads x 2048: 319, 213.  `off`:

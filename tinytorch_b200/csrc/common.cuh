@@ -23,6 +23,18 @@ constexpr int kStatusBadSmemAlign = 2;   // dynamic shared memory did not start 
 constexpr int kStatusCacheFull = 4;      // decode-append: no free row in the cache of some sequence
 constexpr int kStatusRopeRange = 8;      // decode-append: position beyond the rotary tables
 
+// two values, rounded to the 16-bit type, in one register
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  if constexpr (BF16) {
+    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&t);
+  } else {
+    __half2 t = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&t);
+  }
+}
+
 struct Str3 {
   int64_t b, h, s;
 };
@@ -166,7 +178,8 @@ struct LinearCall {
 // Cache lines that 128 bytes of a row cost: rows of `ld` 16-bit elements that are not a multiple of a line long touch two, and five
 // sectors instead of four where they are not a multiple of a sector (from the fits in linear_tile.cu and linear_split.cu).
 inline double row_lines(int64_t ld) { return ld % 16 ? 1.74 : (ld % 64 ? 1.17 : 1.0); }
-cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);  // *persistent: the CTAs let the next kernel in once all before them is complete
+// *persistent: a kernel was taken beside which launch_column_sums may run
+cudaError_t launch_linear_tc(const LinearCall& c, bool* persistent = nullptr);
 // What it takes: 0, the contraction divided; single CTAs: the columns of a tile; pairs: minus the columns of a tile.
 int linear_shape(const LinearCall& c);
 // ... with tiles made to measure (linear_tile.cu): single CTAs with 128 x `bn`, or pairs with 256 x 192
@@ -184,7 +197,8 @@ SplitPlan plan_linear_split(const LinearCall& c);
 double linear_split_us(const LinearCall& c, const SplitPlan& p);  // ... beside the other kernels
 cudaError_t launch_linear_split(const LinearCall& c, const SplitPlan& p);
 // out[n] = sum over the rows of x[rows, n] (fused_ops.cu); n and ldx are multiples of 8
-// `beside`: the kernel launched just before is a linear_tc_kernel, beside which this one may run
+// `beside`: the kernel launched just before is linear_tc_kernel or linear_tile_kernel, whose CTAs let this one in once all before
+// them is complete (grid_dep_launch behind grid_dep_wait) and leave the 1.5 KB of shared memory that a CTA here takes
 cudaError_t launch_column_sums(int dtype, const void* x, void* out, int64_t rows, int64_t n, int64_t ldx, bool beside,
                                cudaStream_t stream);
 

@@ -96,17 +96,6 @@ constexpr int smem_bytes() {
   return (QT + 2 * NSTAGE) * tile_bytes<D>() + QT * kStageBytes + kMaskExtra<D, GEN> + 1024 /*alignment slack*/ + 512 /*SmemCtl*/;
 }
 
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  } else {
-    __half2 t = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  }
-}
-
 // GEN: 1: the variant for a causal triangle that is not top-left aligned, 2: that and a mask; the fast variant (0) compiles
 // all of that out.
 // KEYS: `per_head` items (query blocks) per (batch, kv head), `rank` of `cluster` shares of the key tiles; else pairs.

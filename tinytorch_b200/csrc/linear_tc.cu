@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "linear_order.cuh"
 #include "ptx.cuh"
 #include "tma_host.cuh"
 
@@ -52,29 +53,9 @@ static_assert(kSmemBytes <= 232448, "exceeds the shared memory a CTA may request
 struct LinArgs {
   const void* bias;  // [N] in the tensor dtype, or null
   int M, N, K;
-  int group_m;       // row-tiles per L2 group (see launch_t)
+  int group_m;       // row-tiles per L2 group (see rows_per_group)
   int32_t* status;
 };
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  } else {
-    __half2 t = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  }
-}
-
-__device__ __forceinline__ void tile_of(int t, int group_m, int tiles_m, int tiles_n, int* m_tile, int* n_tile) {
-  const int per_group = group_m * tiles_n;
-  const int g = t / per_group, in_g = t - g * per_group;
-  const int first_m = g * group_m;
-  const int gm = tiles_m - first_m < group_m ? tiles_m - first_m : group_m;
-  *m_tile = first_m + in_g % gm;
-  *n_tile = in_g / gm;
-}
 
 template <bool BF16, bool X_MN, bool W_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
@@ -274,17 +255,8 @@ cudaError_t launch_t(const LinearCall& c, int ctas) {
       !make_map_2d(&tw, c.dtype, c.w, W_MN ? c.N : c.K, W_MN ? c.K : c.N, c.ldw, W_MN ? BK : HN) ||
       !make_map_2d(&ty, c.dtype, c.y, c.N, c.M, c.ldy, HM))
     return cudaErrorInvalidValue;
-  // Row-tiles per L2 group.  The pairs running at one time work on one group: its rows of x are read from HBM once as long
-  // as they stay in L2 while w streams by, and w once per group.  So: as many row-tiles (a power of two) as take 60 MB of
-  // the 126; where w itself stays in L2 (up to 40 MB), 4, so that x does not push it out.  Under sustained load, us, with 4
-  // before: 4096 x 4096 -> 12288 342 -> 312, 16384 x 4096 -> 12288 1341 -> 1225, 8192 cubed 893 -> 861, 2000 x 4096 -> 28672
-  // 387 -> 362 (and 32 or 64 instead of 16 for the second: 1377, 1625).
-  const long long x_tile = 2ll * BM * c.K, w_bytes = 2ll * c.N * c.K;
-  int group_m = 4;
-  if (w_bytes > 40 << 20)
-    while (group_m < 64 && group_m * 2 * x_tile <= 60 << 20) group_m *= 2;
   return launch_early(kern, dim3(ctas), dim3(kThreads), kSmemBytes, c.stream, 1,
-                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, group_m, c.status});
+                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, rows_per_group(c, BM), c.status});
 }
 
 template <bool BF16>

@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "linear_order.cuh"
 #include "ptx.cuh"
 #include "tma_host.cuh"
 
@@ -66,30 +67,10 @@ struct LinArgs {
   const void* bias;  // [N] in the tensor dtype, or null
   int M, N, K;
   int bn, stages;    // columns of a tile; ring depth
-  int group_m;       // row-tiles per L2 group (see launch_t)
+  int group_m;       // row-tiles per L2 group (see rows_per_group)
   uint32_t tmem_cols;
   int32_t* status;
 };
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  } else {
-    __half2 t = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&t);
-  }
-}
-
-__device__ __forceinline__ void tile_of(int t, int group_m, int tiles_m, int tiles_n, int* m_tile, int* n_tile) {
-  const int per_group = group_m * tiles_n;
-  const int g = t / per_group, in_g = t - g * per_group;
-  const int first_m = g * group_m;
-  const int gm = tiles_m - first_m < group_m ? tiles_m - first_m : group_m;
-  *m_tile = first_m + in_g % gm;
-  *n_tile = in_g / gm;
-}
 
 // PAIR_BN: a pair's columns, or 0: a single CTA, whose tile width comes as an argument.
 template <bool BF16, bool X_MN, bool W_MN, int PAIR_BN>
@@ -334,17 +315,12 @@ cudaError_t launch_t(const LinearCall& c, int tile_bn) {
       !make_map_2d(&tw, c.dtype, c.w, W_MN ? c.N : c.K, W_MN ? c.K : c.N, c.ldw, W_MN ? BK : (PAIR ? bn / 2 : bn)) ||
       !make_map_2d(&ty, c.dtype, c.y, c.N, c.M, c.ldy, HM, kOutCols<PAIR>))
     return cudaErrorInvalidValue;
-  // row-tiles per L2 group: as in linear_tc.cu
-  const long long x_tile = 2ll * BM * c.K, w_bytes = 2ll * c.N * c.K;
-  int group_m = 4;
-  if (w_bytes > 40 << 20)
-    while (group_m < 64 && group_m * 2 * x_tile <= 60 << 20) group_m *= 2;
   uint32_t cols = 64;  // two accumulators
   while (static_cast<int>(cols) < 2 * bn) cols *= 2;
   const long long tiles = static_cast<long long>((c.M + BM - 1) / BM) * ((c.N + bn - 1) / bn);
   const int slots = sm_count(c.device) / (PAIR ? 2 : 1), ctas = static_cast<int>(tiles < slots ? tiles : slots) * (PAIR ? 2 : 1);
   return launch_early(kern, dim3(ctas), dim3(kThreads), smem_bytes<PAIR>(bn, stages), c.stream, PAIR ? 2 : 1,
-                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, bn, stages, group_m, cols, c.status});
+                      tx, tw, ty, LinArgs{c.bias, c.M, c.N, c.K, bn, stages, rows_per_group(c, BM), cols, c.status});
 }
 
 template <bool BF16>
