@@ -29,14 +29,6 @@ constexpr int kScoreFloats = TS * LP;
 // rows exchanged (of a score tile: neighbouring halves of 32 columns; kSwapHalves copies one in like that).
 enum Layout { kPad, kPlain, kSwap, kSwapHalves };
 
-// where the vector of columns c4.. of row r lies
-template <int D, Layout LAY>
-__device__ __forceinline__ int place(int r, int c4) {
-  if (LAY == kPad) return r * kLd<D> + c4;
-  const int swap = LAY == kSwap ? 4 : (LAY == kSwapHalves ? 16 : 0);
-  return r * D + (c4 ^ (r & 1) * swap);
-}
-
 // rows [row0, row0 + 64) of src into dst by asynchronous 16-byte copies; rows at or beyond `valid` are zero
 template <int D, int NT, Layout LAY = kPad>
 __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t row_stride, int row0, int valid, int tid) {
@@ -46,7 +38,8 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t 
     const int idx = tid + i * NT, r = idx / (D / 4), c4 = (idx % (D / 4)) * 4;
     const bool in = row0 + r < valid;
     const float* p = src + static_cast<int64_t>(in ? row0 + r : 0) * row_stride + c4;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + place<D, LAY>(r, c4) * 4), "l"(p), "r"(in ? 16 : 0)
+    const int swap = LAY == kSwap ? 4 : (LAY == kSwapHalves ? 16 : 0), at = r * (LAY == kPad ? kLd<D> : D) + (c4 ^ (r & 1) * swap);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + at * 4), "l"(p), "r"(in ? 16 : 0)
                  : "memory");
   }
 }
