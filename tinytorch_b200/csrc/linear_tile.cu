@@ -1,6 +1,6 @@
 // y[M,N] = x[M,K] w[N,K]^T + bias[N] and its gradient products for outputs between those of linear_tc.cu and linear_split.cu: too
 // few tiles of 256 x 256 to fill the machine evenly, too many to divide the contraction.  They are bound by the way of the operands
-// into the SMs that have a tile (about 80 bytes a clock each) and by a last round of tiles that is not full, so the tile is made
+// into the SMs that have a tile (119-135 bytes a ns each, measured with up to 160 columns) and by a last round of tiles that is not full, so the tile is made
 // to measure: 128 rows by 64..256 columns in steps of 32 for single CTAs, and 256 x 192 for pairs of them (clusters of two, tcgen05
 // cta_group::2, each CTA with 128 rows of the tile and of x and HALF of its rows of w).  Persistent, one CTA per SM.
 //   warp 0     producer (both CTAs): cp.async.bulk.tensor loads (128-byte swizzle) of 64 contraction elements of its rows of x and
