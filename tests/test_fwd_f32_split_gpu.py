@@ -71,3 +71,25 @@ def test_no_round_for_a_cluster_too_many(fewer, more):
         q, k = torch.randn(1, heads, 64, 64, device="cuda"), torch.randn(1, heads, 4000, 64, device="cuda")
         us.append(min(_median_us(lambda: op.sdpAttentionFwd(q, k, k)) for _ in range(3)))
     assert us[1] <= 1.7 * us[0], us
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 128, 129, 192])  # either side of what counts as a short walk
+@pytest.mark.parametrize("causal,lens", [(False, False), (True, False), ("bottom-right", True)])
+def test_short_undivided_walks_fp32(D, S, causal, lens):
+    """Against the composition in fp64; more query tiles than are ever divided."""
+    from tinytorch_b200 import op
+    B, Hq, Hkv, L = 10, 32, 8, 70
+    gen = torch.Generator("cuda").manual_seed(S + D)
+    q, k, v = (torch.randn(s, device="cuda", generator=gen) for s in ((B, Hq, L, D), (B, Hkv, S, D), (B, Hkv, S, D)))
+    n = torch.randint(0, S + 1, (B,), dtype=torch.int32, device="cuda", generator=gen) if lens else None
+    o, lse = op.sdpAttentionFwd(q, k, v, isCausal=causal, kvLens=n)
+    rows = torch.full((B, 1, 1, 1), S, device="cuda") if n is None else n.view(B, 1, 1, 1).long()
+    i, j = torch.arange(L, device="cuda").view(1, 1, L, 1), torch.arange(S, device="cuda")
+    seen = (j < rows) & (j <= i + (rows - L if causal == "bottom-right" else 0) if causal else j >= 0)
+    s = q.double() @ k.double().repeat_interleave(Hq // Hkv, 1).transpose(2, 3) * D ** -0.5
+    s = s.masked_fill(~seen, float("-inf"))
+    want = torch.nan_to_num(s.softmax(-1)) @ v.double().repeat_interleave(Hq // Hkv, 1)
+    assert float((o.double() - want).abs().max()) <= TOL_REL_FP32 * max(1.0, float(want.abs().max()))
+    some = seen.any(-1).expand(B, Hq, L)
+    assert float((lse.double() - s.logsumexp(-1))[some].abs().max()) <= 1e-4 and bool(torch.isneginf(lse[~some]).all())

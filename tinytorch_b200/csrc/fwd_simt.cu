@@ -33,11 +33,15 @@ using namespace simt;
 enum MaskForm { kNoMask, kRowMask, kBoolMask, kAddMask };  // kRowMask: the same for all rows, of either kind
 constexpr int kThreads = 128, TY = kThreads / 16, R = TS / TY;
 
-// With only K padded two CTAs of D = 128 fit an SM, to the byte (4 x 8 heads x 500: 136 -> 119 us).  Where there are too few for
-// two the padded tiles are the faster (8 heads x 512, divided: 39 us instead of 42).
-template <int D, bool SPLIT>
+// TIGHT: only K is padded, so that two CTAs of D = 128 fit an SM, to the byte (4 x 8 heads x 500: 136 -> 119 us).  Where there are too
+// few for two the padded tiles are the faster (8 heads x 512, divided: 39 us instead of 42).  Three CTAs of D = 64 fit either way: tight
+// tiles are the faster but for walks of one or two key tiles without a mask (kShortWalk), whose start the kernel's spills weigh on:
+// padded and tight, 11 x 32/8 heads x 22 14.7 and 15.2 us, 40 x 8 x 60 16.5 and 17.0, 16 x 12 x 128 27.3 and 27.7; 12 x 4 x 250 29.9 and
+// 29.4, 4 x 8 x 500 73.0 and 72.4.
+constexpr int kShortWalk = 2;
+template <int D, bool TIGHT>
 struct Lay {
-  static constexpr bool kTight = D == 64 || !SPLIT;
+  static constexpr bool kTight = TIGHT;
   static constexpr Layout Q = kTight ? kSwap : kPad, V = kTight ? kPlain : kPad, P = kTight ? kSwap : kPad;
   static constexpr int kQ = kTight ? TS * D : kTileFloats<D>, kV = kQ, kP = kTight ? TS * TS : kScoreFloats;
   static constexpr bool kApart = D == 64;  // a boolean mask's bytes have a place of their own, for two tiles
@@ -45,16 +49,17 @@ struct Lay {
     return (kQ + kTileFloats<D> + kV + kP + (kApart && mask == kBoolMask ? 2 * TS * kByteRow : 0)) * static_cast<int>(sizeof(float));
   }
 };
-static_assert(2 * (Lay<128, false>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "two CTAs of D = 128 to an SM");
-static_assert(3 * (Lay<64, false>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "three CTAs of D = 64 to an SM");
+static_assert(2 * (Lay<128, true>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "two CTAs of D = 128 to an SM");
+static_assert(3 * (Lay<64, false>::smem_bytes(kNoMask) + 1024) <= 228 * 1024, "three CTAs of D = 64 to an SM");
+static_assert(3 * (Lay<64, true>::smem_bytes(kBoolMask) + 1024) <= 228 * 1024, "three CTAs of D = 64 to an SM");
 
-template <int D, MaskForm MASK, bool SPLIT>
+template <int D, MaskForm MASK, bool SPLIT, bool TIGHT>
 __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) fwd_simt_kernel(const FwdArgs a, int cluster) {
   ptx::grid_dep_launch();
   ptx::grid_dep_wait();  // launched early: everything below reads or writes global memory
   extern __shared__ __align__(16) float sm[];
   float* Qs = sm;
-  using LY = Lay<D, SPLIT>;
+  using LY = Lay<D, TIGHT>;
   float* Ks = Qs + LY::kQ;
   float* Vs = Ks + kTileFloats<D>;
   float* Ps = Vs + LY::kV;
@@ -282,8 +287,12 @@ int split_of(const FwdArgs& a, int D) {
 
 template <int D, MaskForm MASK>
 cudaError_t launch_t(const FwdArgs& a, int device, cudaStream_t stream) {
-  const int cluster = split_of(a, D), smem = cluster > 1 ? Lay<D, true>::smem_bytes(MASK) : Lay<D, false>::smem_bytes(MASK);
-  auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true> : fwd_simt_kernel<D, MASK, false>;
+  const int cluster = split_of(a, D);
+  constexpr bool SPLIT_TIGHT = D == 64;
+  auto kern = cluster > 1 ? fwd_simt_kernel<D, MASK, true, SPLIT_TIGHT> : fwd_simt_kernel<D, MASK, false, true>;
+  int smem = cluster > 1 ? Lay<D, SPLIT_TIGHT>::smem_bytes(MASK) : Lay<D, true>::smem_bytes(MASK);
+  if constexpr (D == 64 && MASK == kNoMask)
+    if (cluster == 1 && a.Skv <= kShortWalk * TS) kern = fwd_simt_kernel<D, MASK, false, false>, smem = Lay<D, false>::smem_bytes(MASK);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
   const long long ctas = static_cast<long long>((a.Lq + TS - 1) / TS) * cluster * a.Hq * a.B;
