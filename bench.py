@@ -448,7 +448,7 @@ def run_ours(args, w, wname):
         train = wl["kind"] == "fwdbwd"
         # the kernel that takes most of the step's device time (profiles/launch_list_bench_default.md)
         kern = (("decode_tc_kernel" if wl["Hq"] != wl["Hkv"] else "decode_kernel") if decode
-                else ("fwd_simt_kernel" if wl["dtype"] == "f32" else
+                else ("fwd_f32_kernel" if wl["dtype"] == "f32" else
                       (("bwd_tc64_kernel" if wl["D"] == 64 else "bwd_tc_kernel") if train else "fwd_tc_kernel")))
         # algorithmic bytes of that kernel's launch (backward: Q, K, V, dO read, dK, dV and the fp32 dQ written)
         alg_bytes = work if decode else (fwd_bytes(wl) if wl["kind"] == "fwd" else (

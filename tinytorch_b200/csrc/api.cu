@@ -222,7 +222,7 @@ int tt_attn_fwd(const tt_attn_fwd_params* p) {
   a.sched = static_cast<int*>(ws.ptr);
   a.mask_lens = lens ? a.sched + 1 : nullptr;
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_fwd_simt(p->dtype, p->D, a, p->device, stream)
+  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_fwd_f32(p->D, a, p->device, stream)
                                           : launch_fwd_tc(p->dtype, p->D, a, p->device, stream);
   return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
 }

@@ -52,7 +52,7 @@ struct MaskArgs {
   bool wide;        // every row starts on a 16-byte boundary
 };
 
-// Arguments common to the prefill kernels (SIMT and tensor-core).
+// Arguments common to the prefill kernels.
 struct FwdArgs {
   const void* q;
   const void* k;
@@ -134,7 +134,7 @@ struct DecodeArgs {
 
 // Each returns a cudaError_t from the launch (no synchronisation).
 cudaError_t launch_fwd_tc(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
-cudaError_t launch_fwd_simt(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
+cudaError_t launch_fwd_f32(int D, const FwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 // rowsum(dO o O) into a.delta only (first step of every backward)
 cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t stream);

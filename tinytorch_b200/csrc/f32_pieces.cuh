@@ -1,0 +1,148 @@
+// fp32 matrix products on the tensor cores: every operand is written as the sum of three bf16 pieces.
+//
+// A float has 24 significant bits, a bf16 has 8: x rounded to bf16, what is left rounded to bf16, and what is left then are three
+// bf16 whose sum is x, exactly, over the range of exponents.  Of the nine products of pieces the six that reach 2^-24 of the result are
+// taken and accumulated in fp32 in TMEM, the small ones first, over one tile only (64 terms of the contraction for probabilities, D for
+// scores): the tensor cores truncate where they accumulate, so the sums over tiles are made in registers, by rounded additions.  Error
+// of a product against 64 bits, relative (2-norm), beside that of a chain of fp32 FMAs: 64 terms 0.8e-7 (1.4e-7), 128 terms 1.3e-7 (2.0e-7);
+// truncated instead of rounded pieces, all of whose left-out products have one sign, 1.2e-7 and 1.7e-7.  Six bf16 products at
+// 2.2 PFLOP/s are worth five times the FMA pipes' 74 TFLOP/s.
+//
+// Infinities: where a piece is zero its product with an infinite piece of the other operand would be NaN where x * inf is inf, and
+// pieces of other signs than x would subtract infinities.  Kernels therefore walk their tiles again with the CAREFUL split once they
+// have met a value that is not finite (or too large for a bf16): truncated pieces, which all have the sign of x, none of them zero
+// (2^-40 of the value in its place) unless x is, and all infinite where x is.
+#pragma once
+#include "common.cuh"
+#include "ptx.cuh"
+
+namespace ttattn {
+namespace pieces {
+
+// What the truncations take, on average, from a sum of 64 products of mixed signs (four steps of the contraction at full size): given
+// back where sums are added or scaled anyway.  (128 terms: twice that.)  With 32 terms or fewer nothing is.  Relative error of gradients,
+// 4 x 8 heads x 500, without and with (and of fp32 FMAs): D = 64 dQ 4.2e-7, 3.6e-7 (3.8e-7), D = 128 5.2e-7, 3.5e-7 (4.2e-7).
+constexpr float kLoss = 0.75e-7f;
+constexpr int kFewTerms = 32;
+
+constexpr int kPieces = 3;
+constexpr int kProducts = 6;
+// the products taken, small ones first: piece of A and piece of B (0: leading), a nibble each
+constexpr uint32_t kPieceA = 0x001012, kPieceB = 0x010210;
+__host__ __device__ constexpr uint32_t piece_a(int p) { return kPieceA >> (4 * p) & 3; }
+__host__ __device__ constexpr uint32_t piece_b(int p) { return kPieceB >> (4 * p) & 3; }
+static_assert(piece_a(0) == 2 && piece_b(0) == 0 && piece_a(1) == 1 && piece_b(1) == 1 && piece_a(2) == 0 && piece_b(2) == 2 &&
+                  piece_a(3) == 1 && piece_b(3) == 0 && piece_a(4) == 0 && piece_b(4) == 1 && piece_a(5) == 0 && piece_b(5) == 0,
+              "every pair of pieces that reaches 2^-24, the small ones first");
+
+__device__ __forceinline__ float lead(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ uint32_t pack_lead(float x0, float x1) {  // leading halves of two floats, x0 below
+  return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
+}
+// the float that the next piece is the lead of, where it must not be zero
+__device__ __forceinline__ float never_zero(float rest, float x) {
+  return copysignf(fmaxf(fabsf(rest), fabsf(x) * 0x1p-40f), x);  // (fmaxf(NaN, inf) = inf: inf - inf is not taken)
+}
+
+// Pieces of two neighbouring elements.  `odd` turns NaN where the first pieces are not both finite.
+template <bool CAREFUL>
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l, float2& odd) {
+  if constexpr (CAREFUL) {
+    h = pack_lead(x0, x1);
+    const float2 r = make_float2(x0 - lead(x0), x1 - lead(x1)), q = make_float2(r.x - lead(r.x), r.y - lead(r.y));
+    m = pack_lead(never_zero(r.x, x0), never_zero(r.y, x1));
+    l = pack_lead(never_zero(q.x, x0), never_zero(q.y, x1));
+  } else {
+    const float2 minus = make_float2(-1.f, -1.f);
+    auto floats = [](uint32_t two) { return make_float2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u)); };
+    h = pack2<true>(x0, x1);
+    const float2 r = ptx::fma2(floats(h), minus, make_float2(x0, x1));
+    m = pack2<true>(r.x, r.y);
+    const float2 q = ptx::fma2(floats(m), minus, r);
+    l = pack2<true>(q.x, q.y);
+    odd = ptx::fma2(r, make_float2(0.f, 0.f), odd);
+  }
+}
+// ... of probabilities, which are finite where the others are
+template <bool CAREFUL>
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+  float2 unused = make_float2(0.f, 0.f);
+  split2<CAREFUL>(x0, x1, h, m, l, unused);
+}
+
+// The two sums of a product: with the first plane, whose truncations count, and with the others.
+__device__ __forceinline__ float2 both(const float2& x, const float2& y, float loss) {
+  return ptx::add2(x, ptx::fma2(x, make_float2(loss, loss), y));
+}
+
+// Eight consecutive floats as 16 bytes of each piece, `plane` bytes apart, at shared-memory addresses; N times, side by side.
+template <bool CAREFUL, int N>
+__device__ __forceinline__ void store8(const uint32_t (&dst)[N], uint32_t plane, const float4 (&x)[N][2], float2& odd) {
+  uint32_t p[N][kPieces][4];
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      split2<CAREFUL>(x[i][e].x, x[i][e].y, p[i][0][2 * e], p[i][1][2 * e], p[i][2][2 * e], odd);
+      split2<CAREFUL>(x[i][e].z, x[i][e].w, p[i][0][2 * e + 1], p[i][1][2 * e + 1], p[i][2][2 * e + 1], odd);
+    }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int e = 0; e < kPieces; ++e)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst[i] + e * plane), "r"(p[i][e][0]), "r"(p[i][e][1]), "r"(p[i][e][2]),
+                   "r"(p[i][e][3])
+                   : "memory");
+}
+__device__ __forceinline__ bool was_odd(const float2& odd) { return !(odd.x + odd.y == 0.f); }
+
+// A tile of ROWS x D floats on its way from global memory into three planes of bf16 in shared memory, in the layout that both
+// K-major and MN-major descriptors read: rows of 128 bytes with the 128-byte swizzle; the planes of 64 columns one after the other, so that
+// two of them serve as one operand of twice the rows (K-major) or columns (MN-major), then those of the next 64.  NT threads
+// take chunks of eight floats, neighbouring threads neighbouring chunks.
+template <int ROWS, int D, int NT>
+struct Tile {
+  static constexpr int kPlane = ROWS * 128;
+  static constexpr int kBlock = kPlane * kPieces;      // 64 columns
+  static constexpr int kBytes = kBlock * (D / 64);
+  static constexpr int kChunks = ROWS * (D / 8) / NT;  // of a thread
+  static_assert(ROWS * (D / 8) % NT == 0 && NT % (D / 8) == 0, "chunks");
+
+  static __device__ __forceinline__ int row(int tid, int i) { return tid / (D / 8) + i * (NT / (D / 8)); }
+  static __device__ __forceinline__ int col(int tid) { return tid % (D / 8) * 8; }
+  static __device__ __forceinline__ uint32_t at(int tid, int i) {  // of chunk i in the first plane
+    const int r = row(tid, i), c = tid % (D / 8);
+    return (c / 8) * kBlock + r * 128 + (((c % 8) ^ (r & 7)) << 4);
+  }
+  // chunks i .. i + N - 1
+  template <int N>
+  static __device__ __forceinline__ void put(uint32_t base, int tid, int i, const float4 (&x)[N][2], bool careful, float2& odd) {
+    uint32_t dst[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) dst[e] = base + at(tid, i + e);
+    if (careful)
+      store8<true, N>(dst, kPlane, x, odd);
+    else
+      store8<false, N>(dst, kPlane, x, odd);
+  }
+};
+
+// Rows of a group's queries: query by query, the heads of the group together.
+struct Group {
+  int n;            // heads
+  uint32_t magic;   // row / n is the upper word of row * magic; 0: by a division
+  __device__ __forceinline__ Group(int heads, int rows)
+      : n(heads), magic(heads > 1 && static_cast<uint64_t>(rows + 256u) * heads < (1ull << 32) ? 0xffffffffu / heads + 1 : 0) {}
+  // (magic = (2^32 + e) / n with e < n: exact while row * e < 2^32)
+  __device__ __forceinline__ int query(int row) const { return n == 1 ? row : (magic ? static_cast<int>(__umulhi(row, magic)) : row / n); }
+  __device__ __forceinline__ int head(int row) const { return row - query(row) * n; }  // of the group
+};
+
+__device__ __forceinline__ float4 load4_or_zero(const float* p, bool in) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (in) v = __ldg(reinterpret_cast<const float4*>(p));
+  return v;
+}
+
+}  // namespace pieces
+}  // namespace ttattn

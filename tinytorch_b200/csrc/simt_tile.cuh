@@ -1,4 +1,4 @@
-// Building blocks of the fp32 attention kernels (fwd_simt.cu, bwd_simt.cu): 64-row tiles in shared memory and the two
+// Building blocks of the fp32 backward kernels (bwd_simt.cu): 64-row tiles in shared memory and the two
 // forms of product on them, on CUDA cores with packed fp32 FMAs.
 //
 // A thread grid of 16 columns (tx) x TY rows (ty) works on a tile; a thread owns R = 64 / TY rows.  Every operand
@@ -226,55 +226,6 @@ struct MaskTile {
       for (int j = 0; j < 4; ++j) b |= q[16 * j] ? 0u : 1u << (4 * i + j);
     }
     return b;
-  }
-};
-
-// A mask that is the same for all rows (padding), for the forward: its elements for a tile, 64 floats or the 17 words that hold 64
-// bytes, lie in the padding of the K tile, come with it and stay until the tile after next: nobody waits for them by themselves.
-template <int D>
-struct MaskRow {
-  const MaskArgs& m;
-  float* tile;   // K
-  int64_t base;  // of (batch, head)
-  int tx, tid;
-
-  __device__ __forceinline__ bool additive() const { return m.kind != TT_ATTN_MASK_BOOL; }
-  // word `w` of key tile t: four to a row, 16 or (bytes) 5 rows, those of odd tiles behind
-  static __device__ __forceinline__ int at(int t, int w) { return ((t & 1) * (TS / 4) + w / 4) * kLd<D> + D + w % 4; }
-
-  // the copy for key tile t; outside: 0 (added), anything (boolean)
-  __device__ __forceinline__ void stage(int t, int n_cols) const {
-    const int es = additive() ? 4 : 1, col0 = t * TS;
-    if (tid >= (additive() ? TS : kByteRow)) return;
-    const uint8_t* p = reinterpret_cast<const uint8_t*>(m.ptr) + (base + col0) * es;
-    const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(p) & 3);  // (0 of floats)
-    const int first = tid * 4 - mis;                                       // of the word's bytes, counted from that of col0
-    const bool in = first < (n_cols - col0) * es && first < TS * es;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(ptx::smem_u32(tile + at(t, tid))), "l"(in ? p + first : p - mis),
-                 "r"(in ? 4 : 0)
-                 : "memory");
-  }
-  // scores of columns t TS + tx + 16 j, scaled and masked
-  template <int R>
-  __device__ __forceinline__ void apply(int t, float c, float (&s)[R][4]) const {
-    if (additive()) {
-      const float* p = tile + at(t, tx);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float add = p[j * 4 * kLd<D>];
-#pragma unroll
-        for (int i = 0; i < R; ++i) s[i][j] = fmaf(add, kLog2e, s[i][j] * c);
-      }
-    } else {
-      const int off = tx + static_cast<int>((reinterpret_cast<uintptr_t>(m.ptr) + base + t * TS) & 3);
-      const uint8_t* p = reinterpret_cast<const uint8_t*>(tile + at(t, off / 4)) + off % 4;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool seen = p[j * kLd<D> * 4] != 0;
-#pragma unroll
-        for (int i = 0; i < R; ++i) s[i][j] = seen ? s[i][j] * c : -INFINITY;
-      }
-    }
   }
 };
 
