@@ -1,4 +1,4 @@
-"""GPU: the fp32 forward, whose products are sums of bf16 ones on the tensor cores (csrc/f32_pieces.cuh), and the backward behind it: the edges of
+"""GPU: fp32 attention, forward and backward, whose products are sums of bf16 ones on the tensor cores (csrc/f32_pieces.cuh): the edges of
 its tiles (128 rows of a group's queries, 64 keys), strided operands, scales of both signs and zero, masks at any offset, walks divided
 over clusters, and values that are not finite.
 
@@ -76,13 +76,10 @@ def test_edges(D, B, Hq, Hkv, L, S, causal, lens):
     if n is not None:  # rows behind the lengths are not looked at
         for b, m in enumerate(lens):
             k[b, :, m:], v[b, :, m:] = math.nan, math.inf
-    from tinytorch_b200 import op
-    o, _ = op.sdpAttentionFwd(q, k, v, isCausal=causal, kvLens=n)
+    got = _run(q, k, v, g, causal=causal, lens=n)
     for t in (k, v):
         t.nan_to_num_(0.0, 0.0)
-    want = _reference(q, k, v, g, causal=causal, lens=n)
-    _check((o,), want)
-    _check(_run(q, k, v, g, causal=causal, lens=n), want)
+    _check(got, _reference(q, k, v, g, causal=causal, lens=n))
 
 
 @pytest.mark.parametrize("D", [64, 128])
@@ -141,3 +138,17 @@ def test_values_that_are_not_finite(D, where):
     assert torch.equal(torch.sign(o[torch.isinf(o)]).double(), torch.sign(want[torch.isinf(want)]))
     ok = torch.isfinite(want)
     assert bool(((o.double() - want)[ok].abs() <= TOL_REL_FP32 * torch.clamp(want[ok].abs(), min=1.0)).all())
+
+
+def test_gradients_of_infinite_inputs_are_not_spread():
+    """An infinite element of dO reaches its row of dQ and its column of dV, and the keys' gradients, and nothing else."""
+    q, k, v, g = _tensors(2, 2, 2, 140, 150, 64)
+    g[0, 0, 131, 5] = math.inf
+    o, dq, dk, dv = _run(q, k, v, g)
+    assert bool(torch.isposinf(dv[0, 0, :, 5]).all())
+    bad = [~torch.isfinite(t) for t in (dq, dk, dv)]
+    assert int(bad[0].sum()) == 64 and bool(bad[0][0, 0, 131].all()) and int(bad[1].sum()) == 150 * 64 and int(bad[2].sum()) == 150
+    g[0, 0, 131, 5] = 0.0
+    want = _reference(q, k, v, g)
+    for t, w, b in zip((dq, dk, dv), want[1:], bad):
+        assert float((t.double() - w)[~b].abs().max()) <= TOL_REL_FP32 * max(1.0, float(w.abs().max()))

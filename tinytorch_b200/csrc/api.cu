@@ -293,7 +293,7 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
     a.mask_lens = lens ? a.sched + 1 : nullptr;
   }
   cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_simt(p->dtype, p->D, a, p->device, stream)
+  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_f32(p->D, a, p->device, stream)
                                           : launch_bwd_tc(p->dtype, p->D, a, p->device, stream);
   return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
 }

@@ -86,7 +86,7 @@ struct BwdArgs {
   int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by the delta pre-pass
   int parts;          // tensor-core kernel: work items per key tile (see bwd_parts); > 1: each leaves its dK / dV in ...
   float* dkv_part;    // ... workspace [dK, dV][parts][B * Hkv][Skv][D] fp32
-  float* ds;          // fp32 kernels: dS tiles on their way from the dK / dV pass to the dQ pass, or null (see bwd_ds_bytes)
+  float* ds;          // fp32 kernels: dS on its way from the dK / dV pass to the dQ pass, or null (see bwd_ds_bytes)
   void* dq;
   void* dk;
   void* dv;
@@ -135,14 +135,14 @@ struct DecodeArgs {
 // Each returns a cudaError_t from the launch (no synchronisation).
 cudaError_t launch_fwd_tc(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_fwd_f32(int D, const FwdArgs& a, int device, cudaStream_t stream);
-cudaError_t launch_bwd_simt(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
+cudaError_t launch_bwd_f32(int D, const BwdArgs& a, int device, cudaStream_t stream);
 // rowsum(dO o O) into a.delta only (first step of every backward)
 cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
 // Work items per key tile of the tensor-core backward, and the workspace they need beside dq_accum (0 for one item)
 int bwd_parts(int B, int Hq, int Hkv, int Lq, int Skv, int D, bool causal);
 size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
 size_t bwd_part_bytes_of(int parts, int B, int Hkv, int Skv, int D);
-// dS tiles of the fp32 backward (0: dQ recomputes them; a caller without room for them gets that too)
+// dS of the fp32 backward (0: dQ recomputes it; a caller without room for it gets that too)
 size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
 // fp16 / bf16 backward on the tensor cores; needs a.delta, a.dq_accum and what a.parts asks for
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
