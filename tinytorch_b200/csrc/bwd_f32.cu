@@ -8,8 +8,9 @@
 // two tiles in shared memory, all as three bf16 planes.  Every tile's product is read from TMEM and added to the sums in registers.
 //   warps 0-7   two warpgroups, the halves of the 64 columns: P and dS; then the tile's products into the sums: key CTAs dV the
 //               first, dK the second, query CTAs half the columns of dQ each
-//   warps 8-11  the other side's first operand (Q or K) into its pieces, with what goes with its rows (log-sum-exp, delta)
-//   warps 12-15 its second operand (dO or V), and masks
+//   warps 8-15  the other side's tiles into their pieces, with what goes with their rows (log-sum-exp, delta); D = 64: the first operand (Q or
+//               K) by one warpgroup, the second (dO or V) by the other; D = 128, where a tile waits for its one place: by both together.
+//               The second warpgroup brings masks too
 //   warp 16     issues the MMAs of S and dP: of the next tile as soon as what lies in their places has been used
 //   warp 17     issues those of dV and dK (dQ)
 // so that P is made under dK of the tile before and dP, and dS under dV.  (One warp for all four spends 1700 of 6100 clocks per tile in waits.)
@@ -47,7 +48,8 @@ struct Ctl {
 template <int D, MaskForm MASK>
 struct Lay {
   using TA = Tile<BM, D, kWork>;
-  using TB = Tile<BN, D, 128>;
+  static constexpr int kLoad = D == 64 ? 128 : 256;  // threads that bring a tile
+  using TB = Tile<BN, D, kLoad>;
   static constexpr int kStages = D == 64 ? 2 : 1;  // of the other side's tiles
   static constexpr int kMaskBytes = MASK == kNoMask ? 0 : (MASK == kBoolMask ? BM * 8 : BM * BN * 4);
   static constexpr int kA2 = 0, kB1 = TA::kBytes, kB2 = kB1 + kStages * TB::kBytes, kM = kB2 + kStages * TB::kBytes;
@@ -416,21 +418,26 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
   } else if (warp < kIssueWarp) {
     // ---------------------------------------------------------------------------- the other side's tiles, masks --
     ptx::setmaxnreg_dec<LY::kLoadRegs>();
-    const bool first = warp < 12;
-    const int lt = tid & 127;
-    uint64_t* full = first ? ctl->b1_full : ctl->b2_full;
-    uint64_t* free = first ? ctl->b1_free : ctl->b2_free;
-    const uint32_t dst = base + (first ? LY::kB1 : LY::kB2);
+    const int lt = tid & (LY::kLoad - 1);
     constexpr int kHeld = D == 64 ? 4 : 2;  // chunks in flight
     float4 raw[kHeld][2];
-    const float* from = (KEYS ? (first ? qp + head0 * a.qs.h : gp + head0 * a.dos.h) : (first ? kp : vp)) + TB::col(lt);
-    const int64_t st_s = KEYS ? (first ? a.qs.s : a.dos.s) : (first ? a.ks.s : a.vs.s), st_h = first ? a.qs.h : a.dos.h;
-    auto fetch = [&](int t, int i0) {
+    // (D = 64: which of the operands is a number of the warp's, and the code for both is one: as two copies it is 15 % slower)
+    struct Operand {
+      const float* rows;
+      int64_t st_s, st_h;
+    };
+    auto operand = [&](bool first) {
+      return Operand{(KEYS ? (first ? qp + head0 * a.qs.h : gp + head0 * a.dos.h) : (first ? kp : vp)) + TB::col(lt),
+                     KEYS ? (first ? a.qs.s : a.dos.s) : (first ? a.ks.s : a.vs.s), first ? a.qs.h : a.dos.h};
+    };
+    const Operand mine = operand(warp < 12);
+    auto fetch = [&](bool first, int t, int i0) {
+      const Operand x = LY::kLoad == 128 ? mine : operand(first);
 #pragma unroll
       for (int i = 0; i < kHeld; ++i) {
         const int row = (begin + t) * BN + TB::row(lt, i0 + i);
-        const float* p = KEYS ? from + rw.query(row) * st_s : from + row * st_s;
-        if (KEYS && group > 1) p += rw.head(row) * st_h;
+        const float* p = KEYS ? x.rows + rw.query(row) * x.st_s : x.rows + row * x.st_s;
+        if (KEYS && group > 1) p += rw.head(row) * x.st_h;
         raw[i][0] = load4_or_zero(p, row < other_rows), raw[i][1] = load4_or_zero(p + 4, row < other_rows);
       }
     };
@@ -439,6 +446,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
       float2 odd = make_float2(0.f, 0.f);
       auto put_mask = [&](int t) {
         const uint32_t at = done + t;
+        const int mt_id = tid & 127;
         const int col0 = (begin + t) * BN, w = warp & 3;
         if (t > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->m_free, (at - 1) & 1, abort_flag))) return false;
         const int64_t mask_b = b * a.mask.sb + head0 * a.mask.sh;
@@ -446,7 +454,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         auto row_at = [&](int r) { return mask_b + rw.head(r) * a.mask.sh + rw.query(r) * a.mask.sl; };
         if constexpr (MASK == kBoolMask) {
           // 64 keys of a row to bits, by a thread: the aligned words that hold their bytes, shifted into place
-          const int r = KEYS ? col0 + lt % BN : own0 + lt, key = KEYS ? own0 + lt / BN * 64 : col0;
+          const int r = KEYS ? col0 + mt_id % BN : own0 + mt_id, key = KEYS ? own0 + mt_id / BN * 64 : col0;
           const uintptr_t at_b = reinterpret_cast<uintptr_t>(a.mask.ptr) + row_at(r) + key;
           const int mis = static_cast<int>(at_b & 3), end = r < rows ? min(64, kv_len - key) + mis : 0;
           const uint32_t* words = reinterpret_cast<const uint32_t*>(at_b - mis);
@@ -461,10 +469,10 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
             x = y;
           }
           if constexpr (KEYS) {  // words of 32 keys, one per column
-            uint32_t* to = reinterpret_cast<uint32_t*>(smem + LY::kM) + lt / BN * 2 * BN + lt % BN;
+            uint32_t* to = reinterpret_cast<uint32_t*>(smem + LY::kM) + mt_id / BN * 2 * BN + mt_id % BN;
             to[0] = two[0], to[BN] = two[1];
           } else {  // two words a row
-            *reinterpret_cast<uint2*>(smem + LY::kM + lt * 8) = make_uint2(two[0], two[1]);
+            *reinterpret_cast<uint2*>(smem + LY::kM + mt_id * 8) = make_uint2(two[0], two[1]);
           }
           ptx::mbar_arrive(&ctl->m_full);
         } else if constexpr (MASK == kAddMask) {
@@ -521,11 +529,11 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         }
         return true;
       };
-      if (n > 0) fetch(0, 0);
-      for (int t = 0; t < n; ++t) {
+      auto bring = [&](bool first, int t) {  // (its first chunks have been asked for); false: a wait has run out
         const uint32_t at = done + t, stage = at % LY::kStages, use = at / LY::kStages;
         // (the first operand's place is free once dK or dQ of its last user has been made, the second's once dP and dV have)
-        if (use > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(&free[stage], (use - 1) & 1, abort_flag))) break;
+        if (use > 0 && !__all_sync(0xffffffffu, ptx::mbar_wait(first ? &ctl->b1_free[stage] : &ctl->b2_free[stage], (use - 1) & 1, abort_flag)))
+          return false;
         if (KEYS && first && lt < BN) {
           const int r = (begin + t) * BN + lt;
           const float l = r < rows ? a.lse[stat_at(r)] : 0.f;
@@ -535,15 +543,33 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         }
 #pragma unroll
         for (int i0 = 0; i0 < TB::kChunks; i0 += kHeld) {
-          if (i0 > 0) fetch(t, i0);
+          if (i0 > 0) fetch(first, t, i0);
 #pragma unroll
           for (int i = 0; i < kHeld; ++i)
-            TB::put(dst + stage * TB::kBytes, lt, i0 + i, reinterpret_cast<const float4(&)[1][2]>(raw[i]), careful, odd);
+            TB::put(base + (first ? LY::kB1 : LY::kB2) + stage * TB::kBytes, lt, i0 + i, reinterpret_cast<const float4(&)[1][2]>(raw[i]), careful, odd);
         }
         ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive(&full[stage]);
-        if (t + 1 < n) fetch(t + 1, 0);
-        if (MASK != kNoMask && !first && !put_mask(t)) break;
+        ptx::mbar_arrive(first ? &ctl->b1_full[stage] : &ctl->b2_full[stage]);
+        return true;
+      };
+      if constexpr (LY::kLoad == 128) {
+        const bool first = warp < 12;
+        if (n > 0) fetch(first, 0, 0);
+        for (int t = 0; t < n; ++t) {
+          if (!bring(first, t)) break;
+          if (t + 1 < n) fetch(first, t + 1, 0);
+          if (MASK != kNoMask && !first && !put_mask(t)) break;
+        }
+      } else {
+        // (the second operand's place is the first to be free)
+        if (n > 0) fetch(false, 0, 0);
+        for (int t = 0; t < n; ++t) {
+          if (!bring(false, t)) break;
+          fetch(true, t, 0);
+          if (MASK != kNoMask && warp >= 12 && !put_mask(t)) break;
+          if (!bring(true, t)) break;
+          if (t + 1 < n) fetch(false, t + 1, 0);
+        }
       }
       if (was_odd(odd)) ctl->bad = 1;
       if (last_pass(careful)) break;
@@ -685,8 +711,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_f32_kernel(const BwdArgs a, i
     ptx::mbar_init(&ctl->a_full, kWork);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&ctl->b1_full[i], 128), ptx::mbar_init(&ctl->b1_free[i], 1);
-      ptx::mbar_init(&ctl->b2_full[i], 128), ptx::mbar_init(&ctl->b2_free[i], keys ? 2 : 1);  // (dP, and dV)
+      ptx::mbar_init(&ctl->b1_full[i], LY::kLoad), ptx::mbar_init(&ctl->b1_free[i], 1);
+      ptx::mbar_init(&ctl->b2_full[i], LY::kLoad), ptx::mbar_init(&ctl->b2_free[i], keys ? 2 : 1);  // (dP, and dV)
     }
     ptx::mbar_init(&ctl->s_full, 1);
     ptx::mbar_init(&ctl->dp_full, 1);

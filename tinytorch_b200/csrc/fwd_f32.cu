@@ -5,7 +5,7 @@
 //   warps 0-3    softmax: thread r owns row r (TMEM lane r).  Per key tile S from TMEM, mask, running maximum and sum, P as three bf16
 //                planes into TMEM, and the factor that the row's older sums shrink by
 //   warps 4-7    O: each tile's P V is read from TMEM and added to the rows' sums in registers
-//   warps 8-11   K tiles into their pieces; warps 12-15 V tiles
+//   warps 8-15   K and V tiles into their pieces: a warpgroup each (D = 64), or both together K first (D = 128, see below)
 //   warps 16, 17 issue the MMAs of S and of P V: S of the next tile as soon as the softmax has read this one's, P V of a tile under
 //                the softmax of the next.  (One warp for both spends 850 of 3100 clocks per tile in waits for what is there already.)
 //   warps 18, 19 masks
@@ -42,7 +42,8 @@ struct Ctl {
 template <int D, MaskForm MASK>
 struct Lay {
   using TQ = Tile<BM, D, 256>;
-  using TK = Tile<BN, D, 128>;
+  static constexpr int kLoad = D == 64 ? 128 : 256;  // threads that bring a tile
+  using TK = Tile<BN, D, kLoad>;
   static constexpr int kStages = D == 64 ? 2 : 1;  // of K, and of V
   static constexpr bool kWideV = D == 64;
   // a boolean mask: two words of bits per row; an additive one: 64 floats, of one row or of each
@@ -83,8 +84,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
     ptx::mbar_init(&ctl->q_full, 256);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      ptx::mbar_init(&ctl->k_full[i], 128);
-      ptx::mbar_init(&ctl->v_full[i], 128);
+      ptx::mbar_init(&ctl->k_full[i], LY::kLoad);
+      ptx::mbar_init(&ctl->v_full[i], LY::kLoad);
       ptx::mbar_init(&ctl->k_free[i], 1);
       ptx::mbar_init(&ctl->v_free[i], 1);
       ptx::mbar_init(&ctl->p_full[i], BM);
@@ -381,45 +382,55 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
   } else if (warp < kIssueWarp) {
     // --------------------------------------------------------------------------------------------- K or V, by tile --
     ptx::setmaxnreg_dec<LY::kLoadRegs>();
-    const bool keys = warp < 12;
-    const int ht = tid & 127;
-    const Str3& st = keys ? a.ks : a.vs;
-    const float* src = reinterpret_cast<const float*>(keys ? a.k : a.v) + b * st.b + hk * st.h + TK::col(ht);
-    uint64_t* full = keys ? ctl->k_full : ctl->v_full;
-    const uint32_t dst = base + (keys ? LY::kK : LY::kV);
-    // Chunks in flight: asked for together, as the place of those before in the registers is free, and converted together.  (Each asked
-    // for as the one before leaves: D = 128 34.5 -> 38 us, 4 x 8 heads x 500; two warpgroups per operand 39, K's next tile as it is in shared memory 42.6.)
-    constexpr int kHeld = 4;
-    float4 raw[kHeld][2];
-    auto fetch = [&](int t, int i0) {  // rows at or beyond the length are zero
+    // A thread's chunks of a tile are in flight together, asked for as those of the tile before leave the registers, and are
+    // converted two at a time.  (Each asked for as the one before leaves: D = 128 34.5 -> 38 us, 4 x 8 heads x 500; K's next tile as it is in
+    // shared memory: 42.6.)
+    // D = 128: K's tiles have one place, and wait for it: a tile's time is K into its place, 2500 clocks by one warpgroup, and S,
+    // 1800.  Both warpgroups bring K, then V.
+    constexpr bool kBoth = D == 128;
+    const bool keys = !kBoth && warp < 12;
+    const int ht = tid & (LY::kLoad - 1);
+    const float* k = reinterpret_cast<const float*>(a.k) + b * a.ks.b + hk * a.ks.h + TK::col(ht);
+    const float* v = reinterpret_cast<const float*>(a.v) + b * a.vs.b + hk * a.vs.h + TK::col(ht);
+    static_assert(TK::kChunks == 4, "chunks of a thread");
+    float4 raw[4][2];
+    auto fetch = [&](bool of_k, int t) {  // rows at or beyond the length are zero
+      const float* src = of_k ? k : v;
+      const int64_t stride = of_k ? a.ks.s : a.vs.s;
 #pragma unroll
-      for (int i = 0; i < kHeld; ++i) {
-        const int r = (t0 + t) * BN + TK::row(ht, i0 + i);
-        const float* p = src + static_cast<int64_t>(r) * st.s;
+      for (int i = 0; i < 4; ++i) {
+        const int r = (t0 + t) * BN + TK::row(ht, i);
+        const float* p = src + static_cast<int64_t>(r) * stride;
         raw[i][0] = load4_or_zero(p, r < kv_len), raw[i][1] = load4_or_zero(p + 4, r < kv_len);
       }
     };
     bool careful = false;
     for (int done = 0;; done += n, careful = true) {
       float2 odd = make_float2(0.f, 0.f);
-      if (n > 0) fetch(0, 0);
-      for (int t = 0; t < n; ++t) {
+      auto put = [&](bool of_k, int t) {  // false: a wait has run out
         const uint32_t at = done + t, stage = at % kStages, last = at - kStages;
         if (t >= kStages) {  // the stage's last user has been read
-          if (!uwait(keys ? &ctl->k_free[last & 1] : &ctl->v_free[last & 1], last >> 1)) break;
+          if (!uwait(of_k ? &ctl->k_free[last & 1] : &ctl->v_free[last & 1], last >> 1)) return false;
         }
+        const uint32_t dst = base + (of_k ? LY::kK : LY::kV) + stage * TK::kBytes;
+        float2 seen = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int i0 = 0; i0 < TK::kChunks; i0 += kHeld) {
-          if (i0 > 0) fetch(t, i0);
-#pragma unroll
-          for (int i = 0; i < kHeld; i += 2)
-            TK::put(dst + stage * TK::kBytes, ht, i0 + i, reinterpret_cast<const float4(&)[2][2]>(raw[i]), careful, odd);
-        }
+        for (int i = 0; i < 4; i += 2) TK::put(dst, ht, i, reinterpret_cast<const float4(&)[2][2]>(raw[i]), careful, seen);
+        if (!of_k) odd = ptx::add2(odd, seen);
         ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive(&full[stage]);
-        if (t + 1 < n) fetch(t + 1, 0);
+        ptx::mbar_arrive(of_k ? &ctl->k_full[stage] : &ctl->v_full[stage]);
+        return true;
+      };
+      if (n > 0) fetch(kBoth || keys, 0);
+      for (int t = 0; t < n; ++t) {
+        if (!put(kBoth || keys, t)) break;
+        if (kBoth) {
+          fetch(false, t);
+          if (!put(false, t)) break;
+        }
+        if (t + 1 < n) fetch(kBoth || keys, t + 1);
       }
-      if (!keys && was_odd(odd)) ctl->bad = 1;
+      if (was_odd(odd)) ctl->bad = 1;
       if (last_pass(careful)) break;
     }
     if (SPLIT) ptx::cluster_sync(), ptx::cluster_sync();
