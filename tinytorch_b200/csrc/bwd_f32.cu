@@ -183,7 +183,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
             uint32_t w[kPieces][8];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              if (careful) {
+              if (rare(careful)) {
                 split2<true>(x[e].x, x[e].y, w[0][2 * e], w[1][2 * e], w[2][2 * e], odd);
                 split2<true>(x[e].z, x[e].w, w[0][2 * e + 1], w[1][2 * e + 1], w[2][2 * e + 1], odd);
               } else {
@@ -264,7 +264,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         float p[32];  // in the order of the blocks
         auto planes = [&](uint32_t at, const float* x) {  // pieces of a block's 16 columns
           uint32_t w[kPieces][8];
-          if (careful) {
+          if (rare(careful)) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) split2<true>(x[2 * e], x[2 * e + 1], w[0][e], w[1][e], w[2][e], odd);
           } else {
@@ -887,7 +887,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
               if (col0 + e >= limit) x[e] = 0.f;
           }
           uint32_t w[kPieces][8];
-          if (careful) {
+          if (rare(careful)) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) split2<true>(x[2 * e], x[2 * e + 1], w[0][e], w[1][e], w[2][e], odd);
           } else {

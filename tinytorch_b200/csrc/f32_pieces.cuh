@@ -44,6 +44,9 @@ __device__ __forceinline__ float never_zero(float rest, float x) {
   return copysignf(fmaxf(fabsf(rest), fabsf(x) * 0x1p-40f), x);  // (fmaxf(NaN, inf) = inf: inf - inf is not taken)
 }
 
+// the second pass: its code out of the way (the kernels' loops are long for the instruction caches)
+__device__ __forceinline__ bool rare(bool careful) { return __builtin_expect(careful, 0); }
+
 // Pieces of two neighbouring elements.  `odd` turns NaN where the first pieces are not both finite.
 template <bool CAREFUL>
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l, float2& odd) {
@@ -120,7 +123,7 @@ struct Tile {
     uint32_t dst[N];
 #pragma unroll
     for (int e = 0; e < N; ++e) dst[e] = base + at(tid, i + e);
-    if (careful)
+    if (rare(careful))
       store8<true, N>(dst, kPlane, x, odd);
     else
       store8<false, N>(dst, kPlane, x, odd);

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
           if (!uwait(&ctl->v_free[two], (at - 2) >> 1)) break;
           ptx::tc_fence_after();
         }
-        if (careful)
+        if (rare(careful))
           probabilities(std::true_type{});
         else
           probabilities(std::false_type{});
