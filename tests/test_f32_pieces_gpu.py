@@ -152,3 +152,29 @@ def test_gradients_of_infinite_inputs_are_not_spread():
     want = _reference(q, k, v, g)
     for t, w, b in zip((dq, dk, dv), want[1:], bad):
         assert float((t.double() - w)[~b].abs().max()) <= TOL_REL_FP32 * max(1.0, float(w.abs().max()))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("value", [-2.0e38, -1.0e38, 2.0e38, -math.inf, torch.finfo(torch.float32).min])
+def test_masks_of_large_values(D, value):
+    """A row whose mask is one large value for all keys: their mean (the scores are lost in it); nothing where the value times log2(e),
+    the unit of the exponents, is -inf.  A row that has it for some keys: the others'."""
+    from tinytorch_b200 import op
+    q, k, v, _ = _tensors(1, 2, 2, 70, 90, D)
+    mask = torch.zeros(1, 1, 70, 90, device="cuda")
+    mask[:, :, 5] = value
+    mask[:, :, 6, 40:] = value
+    o, lse = op.sdpAttentionFwd(q, k, v, attnMask=mask)
+    plain = abs(value) * 1.4426950408889634 < 3.4028235e38
+    # rounded additions of up to 90 terms of size 1, equally weighted
+    want = v.double().mean(2) if plain else torch.zeros(1, 2, D, device="cuda", dtype=torch.float64)
+    assert (o[:, :, 5] - want).abs().max() < 90 * 2.0 ** -24
+    if not plain:
+        assert torch.isneginf(lse[:, :, 5]).all()
+    part = slice(40, 90) if value > 0 else slice(0, 40)
+    if value < 0:
+        want, = _reference(q[:, :, 6:7], k[:, :, part], v[:, :, part])
+        assert (o[:, :, 6:7] - want).norm() < 1e-6 * want.norm()
+    else:
+        assert (o[:, :, 6] - v[:, :, part].double().mean(2)).abs().max() < 90 * 2.0 ** -24
+    assert torch.isfinite(o).all()

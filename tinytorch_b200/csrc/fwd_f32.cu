@@ -13,11 +13,12 @@
 // of K (and of V, D = 64) are read as one operand of 128.  S and O come as two sums then, with the first plane and with the others.
 //
 // Bound by the chain of a tile: softmax 2000 clocks and 300 until S is seen (D = 64: a tile 2400; the MMAs take 2100 of them), for D = 128,
-// where only one K tile fits, K into pieces 2500, then S 1800 (a tile 5700).  Against the same in fp32 FMAs on CUDA cores (64 x 64 tiles,
-// whose FMA pipes were 58 % busy), us: D = 64, 4 x 8 heads x 500 72 -> 19 (additive mask 74 -> 29, 6 x 333 padding 52 -> 19), causal 16 x 2048 293 -> 55,
-// 11 x 32/8 heads x 22 14.5 -> 9.3, one query on one key 7.2 -> 6.4; D = 128, 4 x 8 x 500 117 -> 36 (additive 125 -> 44), causal 4 x 4096 506 -> 115.
+// where only one K tile fits, K into pieces, then S 1800.  Against the same in fp32 FMAs on CUDA cores (64 x 64 tiles, whose FMA pipes were
+// 58 % busy), us: D = 64, 4 x 8 heads x 500 72 -> 19 (additive mask 74 -> 29, 6 x 333 padding 52 -> 19), causal 16 x 2048 293 -> 54,
+// 11 x 32/8 heads x 22 14.5 -> 9.2, one query on one key 7.2 -> 6.3; D = 128, 4 x 8 x 500 117 -> 33 (additive 125 -> 43), causal 4 x 4096 506 -> 107.
 // Relative error against 64 bits: 4 x 8 x 500 3.5e-7 -> 1.6e-7 and 4.7e-7 -> 2.0e-7.
 // Tried: P over the S that it is made of, two such buffers, S up to two tiles ahead: 2700 clocks a tile.  One place for P: 3150.
+// Additive rows by bulk copies of 256 bytes: 29.7 -> 32.3, D = 128 43 -> 53.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -273,9 +274,16 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
 #pragma unroll
             for (int j = 0; j < BN; j += 4) {
               const float4 m4 = ptx::ld_shared_f4(mask_at + (MASK == kAddRow ? j * 4 : tid * BN * 4 + (((j / 4) ^ (tid & 7)) << 4)));
-              const float mk[4] = {m4.x, m4.y, m4.z, m4.w};
+              if constexpr (D == 64) {  // (29.8 -> 28.6, 2048 queries 56.8 -> 54.0; D = 128, with fewer registers, 43.6 -> 44.1 and 82.2 -> 81.1)
+                const float2 c2 = make_float2(c, c), log2e = make_float2(kLog2e, kLog2e);
+                const float2 lo = ptx::fma2(make_float2(m4.x, m4.y), log2e, ptx::mul2(make_float2(s[j], s[j + 1]), c2));
+                const float2 hi = ptx::fma2(make_float2(m4.z, m4.w), log2e, ptx::mul2(make_float2(s[j + 2], s[j + 3]), c2));
+                s[j] = lo.x, s[j + 1] = lo.y, s[j + 2] = hi.x, s[j + 3] = hi.y;
+              } else {
+                const float mk[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e) s[j + e] = fmaf(mk[e], kLog2e, s[j + e] * c);
+                for (int e = 0; e < 4; ++e) s[j + e] = fmaf(mk[e], kLog2e, s[j + e] * c);
+              }
             }
           }
           ptx::mbar_arrive(&ctl->m_free[stage]);
