@@ -20,9 +20,9 @@
 // of it: one product instead of the query CTAs' three.
 //
 // Bound by the tensor pipe and the waits around it: D = 64, a tile 5700 clocks, of them 4 x 1050 in MMAs; D = 128, where only one tile of the other
-// side fits, 14400, its two operands' conversion among them.  Against the same in fp32 FMAs on CUDA cores, us, with the delta pass: D = 64, 4 x 8
-// heads x 500 156 -> 62 (additive mask 170 -> 76), causal 8 x 8 x 1024 784 -> 257, 2 x 16/2 x 700 219 -> 86; D = 128, 4 x 8 x 500 296 -> 124, causal
-// 4 x 8 x 1024 719 -> 267.  Relative error of dQ against 64 bits: 3.9e-7 -> 3.2e-7 and 4.3e-7 -> 3.5e-7, of dK 4.5e-7 -> 3.2e-7 and 5.6e-7 -> 3.5e-7.
+// side fits, its two operands' conversion besides.  Against the same in fp32 FMAs on CUDA cores, us, with the delta pass: D = 64, 4 x 8 heads x 500
+// 156 -> 61 (additive mask 170 -> 75), causal 8 x 8 x 1024 784 -> 257, 2 x 16/2 x 700 217 -> 84; D = 128, 4 x 8 x 500 295 -> 110 (additive mask 304 -> 136),
+// causal 4 x 8 x 1024 719 -> 203.  Relative error of dQ against 64 bits: 3.9e-7 -> 3.2e-7 and 4.3e-7 -> 3.5e-7, of dK 4.5e-7 -> 3.2e-7 and 5.6e-7 -> 3.5e-7.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
