@@ -213,7 +213,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         ptx::mbar_arrive(&ctl->a_full);
       }
       const float c = a.scale * kLog2e;
-      const float loss = (KEYS ? rows : kv_len) > kFewTerms ? kLoss : 0.f;  // of sums over the other side's rows
+      const float loss = (KEYS ? rows : kv_len) > kFewTerms ? kLoss : kNoLoss;  // of sums over the other side's rows
       // what the row takes part in: other rows lo .. hi - 1
       int lo = 0, hi;
       float lse2 = 0.f, delta = 0.f;  // query CTAs: the row's
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     // keys that the row sees: what lies behind has not been written
     const int limit = own0 + r < rows ? (a.causal ? min(kv_len, rw.query(own0 + r) + shift + 1) : kv_len) : 0;
-    const float loss = limit > kFewTerms ? kLoss : 0.f;
+    const float loss = limit > kFewTerms ? kLoss : kNoLoss;
     const int pitch = ds_pitch(a), n_rows = ds_rows(a) - own0;
     const float* ds = ds_of(a, b, hk) + static_cast<int64_t>(own0) * pitch;
     auto fetch = [&](int t) {  // two rows of 64 floats a warp at a time, neighbouring vectors exchanged by row

@@ -24,6 +24,7 @@ namespace pieces {
 // 4 x 8 heads x 500, without and with (and of fp32 FMAs): D = 64 dQ 4.2e-7, 3.6e-7 (3.8e-7), D = 128 5.2e-7, 3.5e-7 (4.2e-7).
 constexpr float kLoss = 0.75e-7f;
 constexpr int kFewTerms = 32;
+constexpr float kNoLoss = 0x1p-60f;  // adds nothing to a finite sum, and leaves an infinite one what it is (0 would make NaN of it)
 
 constexpr int kPieces = 3;
 constexpr int kProducts = 6;

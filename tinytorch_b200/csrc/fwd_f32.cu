@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
     // ------------------------------------------------------------------------------------------------------ O --
     ptx::setmaxnreg_inc<LY::kSumRegs>();
     // (of the terms that a row has, as far as lengths and alignment tell)
-    const float loss = (a.causal ? min(kv_len, query_of(tid - 128) + shift + 1) : kv_len) > kFewTerms ? kLoss : 0.f;
+    const float loss = (a.causal ? min(kv_len, query_of(tid - 128) + shift + 1) : kv_len) > kFewTerms ? kLoss : kNoLoss;
     const uint32_t from = tmem_o + (static_cast<uint32_t>((warp - 4) * 32) << 16);
     float2 acc[D / 2];
     bool careful = false;
