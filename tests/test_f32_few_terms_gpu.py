@@ -1,6 +1,6 @@
 """GPU: fp32 attention whose rows have few terms.  An infinity, or a sum that is too large for a float, stays an infinity whatever the number of
 terms: with 1, 7, 32 and 33 keys (queries, for the keys' gradients), under a causal mask, where the first rows of every call have few, and
-in both head dimensions.
+in both head dimensions; and so does one whose factor is so small that the lower pieces of it are below what a bf16 holds.
 
 Reference: the composition in fp64, formula by formula; which elements are infinite or NaN has to agree."""
 import math
@@ -107,3 +107,38 @@ def test_dq_that_overflows(S, D):
     rest = torch.ones(D, dtype=torch.bool, device="cuda")
     rest[3] = False
     assert bool(torch.isfinite(dq[0, 0][:, rest]).all()) and bool(torch.isfinite(dq[0, 1]).all()) and bool(torch.isfinite(dq[1]).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S", [2, 90])
+def test_infinities_with_small_probabilities(S, D):
+    """Probabilities from 1 down to 2^-118 (and 1 / 89 of that), with an infinite V and with an infinite dO."""
+    from tinytorch_b200 import op
+    L = 252
+    q, k, v, g = (torch.zeros((1, 1, n, D), device="cuda") for n in (L, S, S, L))
+    v.normal_(), g.normal_()
+    steps = torch.arange(L, device="cuda") * 0.47  # what the last key's exponents are below the others
+    q[0, 0, :, 0], k[0, 0, S - 1, 0] = steps, -1.0
+    v[0, 0, S - 1, 3], g[0, 0, :, 5] = math.inf, -math.inf
+    o, lse = op.sdpAttentionFwd(q, k, v, scale=math.log(2.0))
+    assert bool(torch.isposinf(o[..., 3]).all()) and int((~torch.isfinite(o)).sum()) == L
+    v[0, 0, S - 1, 3] = 0.0
+    o, lse = op.sdpAttentionFwd(q, k, v, scale=math.log(2.0))
+    for row in (slice(0, L), slice(200, 201), slice(L - 1, L)):  # all rows; one whose probability of the last key is small
+        dv = op.sdpAttentionBwd(g[:, :, row], q[:, :, row], k, v, o[:, :, row], lse[:, :, row].clone(), scale=math.log(2.0))[2]
+        assert bool(torch.isneginf(dv[..., 5]).all()) and int((~torch.isfinite(dv)).sum()) == S
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("small", [0.5, 1e-30, 1e-34, 1e-37, 2.0 ** -126, 2.0 ** -133, 1e-42])
+def test_keys_hidden_by_small_queries(small, D):
+    """A small number times -inf is -inf: the key takes no part, and the others are what they would be without it."""
+    from tinytorch_b200 import op
+    q, k, v, _ = _tensors(40, 90, D)
+    q[..., 3], k[..., 3] = small, 0.0
+    k[:, :, 70, 3] = -math.inf
+    o, lse = op.sdpAttentionFwd(q, k, v)
+    others = torch.arange(90, device="cuda") != 70
+    want = _probabilities(q, k[:, :, others], False) @ v[:, :, others].double()
+    _same(o, want)
+    assert bool(torch.isfinite(lse).all())

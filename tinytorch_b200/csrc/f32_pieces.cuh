@@ -11,7 +11,7 @@
 // Infinities: where a piece is zero its product with an infinite piece of the other operand would be NaN where x * inf is inf, and
 // pieces of other signs than x would subtract infinities.  Kernels therefore walk their tiles again with the CAREFUL split once they
 // have met a value that is not finite (or too large for a bf16): truncated pieces, which all have the sign of x, none of them zero
-// (2^-40 of the value in its place) unless x is, and all infinite where x is.
+// (2^-40 of the value in its place, or the smallest bf16, 2^-133, where that is less) unless x is, and all infinite where x is.
 #pragma once
 #include "common.cuh"
 #include "ptx.cuh"
@@ -40,9 +40,11 @@ __device__ __forceinline__ float lead(float x) { return __uint_as_float(__float_
 __device__ __forceinline__ uint32_t pack_lead(float x0, float x1) {  // leading halves of two floats, x0 below
   return __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
 }
-// the float that the next piece is the lead of, where it must not be zero
+// The float that a piece of x is the lead of, where it must not be zero unless x is: `rest`, or 2^-40 of x, or the smallest bf16 there is.
 __device__ __forceinline__ float never_zero(float rest, float x) {
-  return copysignf(fmaxf(fabsf(rest), fabsf(x) * 0x1p-40f), x);  // (fmaxf(NaN, inf) = inf: inf - inf is not taken)
+  float least = fabsf(x) * 0x1p-40f;
+  if (least < 0x1p-133f && x != 0.f) least = 0x1p-133f;
+  return copysignf(fmaxf(fabsf(rest), least), x);  // (fmaxf(NaN, inf) = inf: inf - inf is not taken)
 }
 
 // the second pass: its code out of the way (the kernels' loops are long for the instruction caches)
@@ -52,7 +54,7 @@ __device__ __forceinline__ bool rare(bool careful) { return __builtin_expect(car
 template <bool CAREFUL>
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l, float2& odd) {
   if constexpr (CAREFUL) {
-    h = pack_lead(x0, x1);
+    h = pack_lead(never_zero(x0, x0), never_zero(x1, x1));
     const float2 r = make_float2(x0 - lead(x0), x1 - lead(x1)), q = make_float2(r.x - lead(r.x), r.y - lead(r.y));
     m = pack_lead(never_zero(r.x, x0), never_zero(r.y, x1));
     l = pack_lead(never_zero(q.x, x0), never_zero(q.y, x1));
