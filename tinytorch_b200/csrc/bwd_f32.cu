@@ -22,7 +22,7 @@
 // Bound by the tensor pipe and the waits around it: D = 64, a tile 5700 clocks, of them 4 x 1050 in MMAs; D = 128, where only one tile of the other
 // side fits, its two operands' conversion besides.  Against the same in fp32 FMAs on CUDA cores, us, with the delta pass: D = 64, 4 x 8 heads x 500
 // 156 -> 61 (additive mask 170 -> 75), causal 8 x 8 x 1024 784 -> 257, 2 x 16/2 x 700 217 -> 84; D = 128, 4 x 8 x 500 295 -> 110 (additive mask 304 -> 136),
-// causal 4 x 8 x 1024 719 -> 203.  Relative error of dQ against 64 bits: 3.9e-7 -> 3.2e-7 and 4.3e-7 -> 3.5e-7, of dK 4.5e-7 -> 3.2e-7 and 5.6e-7 -> 3.5e-7.
+// causal 4 x 8 x 1024 719 -> 203.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -53,12 +53,13 @@ struct Lay {
   static constexpr int kStages = D == 64 ? 2 : 1;  // of the other side's tiles
   static constexpr int kMaskBytes = MASK == kNoMask ? 0 : (MASK == kBoolMask ? BM * 8 : BM * BN * 4);
   static constexpr int kA2 = 0, kB1 = TA::kBytes, kB2 = kB1 + kStages * TB::kBytes, kM = kB2 + kStages * TB::kBytes;
-  static constexpr int kVec = kM + kMaskBytes;  // [2][lse, delta][64]
-  static constexpr int kCtl = kVec + 4 * BN * 4;
+  static constexpr int kVec = kM + kMaskBytes;  // [2][lse, weight, delta][64]
+  static constexpr int kVecBytes = 3 * BN * 4;
+  static constexpr int kCtl = kVec + 2 * kVecBytes;
   static constexpr int kBytes = kCtl + 256;
   static constexpr int kLdO = D + 4;  // floats a row of the sums on their way out
   // TMEM: planes of the own side's first operand | S, then P | dP, then dS | product of a tile.
-  // kWide: products of 64 columns come as two sums, with the first plane and with the others (see fwd_f32.cu).  The planes of 16 columns
+  // kWide: products of 64 columns come as two sums (f32_pieces.cuh).  The planes of 16 columns
   // of P and dS lie over the scores that they are made of.  Without (TMEM is full), scores lie in columns 16..79 of a region and the
   // planes of 16 columns in 24 each: written first to last by the one warpgroup and last to first by the other, they come to lie over
   // scores that have been read.
@@ -76,15 +77,15 @@ struct Lay {
 static_assert(sizeof(Ctl) <= 256, "control block");
 static_assert(Lay<128, kAddMask>::kBytes <= 227 * 1024, "shared memory");
 
-// the two sums of a product, or (not WIDE) its one, held as words, with what truncations took
-template <bool WIDE>
-__device__ __forceinline__ void add_to(uint32_t (&x)[16], const uint32_t (&y)[16], float loss) {
-#pragma unroll
-  for (int e = 0; e < 16; e += 2) {
-    const float2 a = make_float2(__uint_as_float(x[e]), __uint_as_float(x[e + 1])), b = make_float2(__uint_as_float(y[e]), __uint_as_float(y[e + 1]));
-    const float2 z = WIDE ? both(a, b, loss) : ptx::fma2(a, make_float2(loss, loss), a);
-    x[e] = __float_as_uint(z.x), x[e + 1] = __float_as_uint(z.y);
-  }
+// two neighbouring words of accumulators
+__device__ __forceinline__ float2 floats2(const uint32_t (&x)[16], int i) { return make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])); }
+// A row's log-sum-exp in units of the exponents without an integer of 0 .. log2(n), n: how many keys the row may see; negated.  2 to minus that
+// integer is the row's weight.  What a key of average probability has for an exponent is near 0 then, and so is its rounding, where it would be
+// near -log2(n): relative error of dQ against 64 bits, 4 x 8 heads x 500, 3.8e-7 -> 3.2e-7 (D = 64; fp32 FMAs 3.8e-7), 4.4e-7 -> 3.8e-7 (D = 128; 4.2e-7).
+__device__ __forceinline__ float minus_lse2(float lse, int n, float& weight) {
+  const float x = lse * kLog2e, whole = fminf(fmaxf(rintf(x), 0.f), static_cast<float>(31 - __clz(max(n, 1))));
+  weight = __int_as_float((127 - static_cast<int>(whole)) << 23);
+  return lse == -INFINITY ? -INFINITY : whole - x;  // (a row without any participating key: P is 0)
 }
 
 // where dS waits for the dQ pass: for each (batch, kv head) the queries' rows, in whole tiles, of keys, in whole tiles
@@ -213,10 +214,9 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         ptx::mbar_arrive(&ctl->a_full);
       }
       const float c = a.scale * kLog2e;
-      const float loss = (KEYS ? rows : kv_len) > kFewTerms ? kLoss : kNoLoss;  // of sums over the other side's rows
       // what the row takes part in: other rows lo .. hi - 1
       int lo = 0, hi;
-      float lse2 = 0.f, delta = 0.f;  // query CTAs: the row's
+      float lse2 = 0.f, weight = 1.f, delta = 0.f;  // query CTAs: the row's
       int all_lo = 0, all_hi;         // what every row of the CTA takes part in
       if constexpr (KEYS) {
         const int key = own0 + r;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         hi = own0 + r < rows ? (a.causal ? min(kv_len, i_q + shift + 1) : kv_len) : 0;
         all_hi = a.causal ? min(kv_len, rw.query(own0) + shift + 1) : kv_len;
         const float l = own0 + r < rows ? a.lse[stat_at(own0 + r)] : 0.f;
-        lse2 = l == -INFINITY ? INFINITY : l * kLog2e;  // (a row without any participating key: P is 0)
+        lse2 = minus_lse2(l, kv_len, weight);
         delta = own0 + r < rows ? a.delta[stat_at(own0 + r)] : 0.f;
       }
       // a tile's product into the sums
@@ -245,9 +245,9 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           ptx::tmem_ld16(from + 2 * j, o);
           if (LY::kWide) ptx::tmem_ld16(from + D + 2 * j, o2);
           ptx::tmem_wait_ld();
-          add_to<LY::kWide>(o, o2, loss);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[j + e] = ptx::add2(acc[j + e], make_float2(__uint_as_float(o[2 * e]), __uint_as_float(o[2 * e + 1])));
+          for (int e = 0; e < 8; ++e)
+            acc[j + e] = ptx::add2(acc[j + e], LY::kWide ? ptx::add2(floats2(o, 2 * e), floats2(o2, 2 * e)) : floats2(o, 2 * e));
         }
         ptx::tc_fence_before();
         ptx::mbar_arrive(free);
@@ -256,7 +256,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
       for (int t = 0; t < n; ++t) {
         const uint32_t at = done + t, par = at & 1;
         const int col0 = (begin + t) * BN;
-        const uint32_t vec = base + LY::kVec + par * (2 * BN * 4);  // key CTAs: lse of the columns; delta behind
+        const uint32_t vec = base + LY::kVec + par * LY::kVecBytes;  // key CTAs: of the columns
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->s_full, par, abort_flag))) break;
         if constexpr (MASK != kNoMask)
           if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->m_full, par, abort_flag))) break;
@@ -296,13 +296,13 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
             }
           }
           ptx::tmem_wait_ld();
-          add_to<LY::kWide>(s, s2, D == 64 ? kLoss : 2 * kLoss);
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            float l4[4] = {lse2, lse2, lse2, lse2};
+            float l4[4] = {lse2, lse2, lse2, lse2}, w4[4] = {weight, weight, weight, weight};
             if constexpr (KEYS) {
-              const float4 v = ptx::ld_shared_f4(vec + (j0 + j) * 4);
+              const float4 v = ptx::ld_shared_f4(vec + (j0 + j) * 4), w = ptx::ld_shared_f4(vec + (BN + j0 + j) * 4);
               l4[0] = v.x, l4[1] = v.y, l4[2] = v.z, l4[3] = v.w;
+              w4[0] = w.x, w4[1] = w.y, w4[2] = w.z, w4[3] = w.w;
             }
             float mk[4];
             if constexpr (MASK == kAddMask) {
@@ -315,10 +315,15 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
               }
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float x = fmaf(__uint_as_float(s[j + e]), c, -l4[e]);
-              if constexpr (MASK == kAddMask) x = fmaf(mk[e], kLog2e, x);
-              pb[j + e] = ptx::ex2(x);
+            for (int e = 0; e < 4; e += 2) {
+              const float2 c2 = make_float2(c, c), l2 = make_float2(l4[e], l4[e + 1]);
+              float2 x = LY::kWide ? ptx::add2(floats2(s, j + e), floats2(s2, j + e)) : floats2(s, j + e);
+              if constexpr (MASK == kAddMask)  // (the forward's sum, with its roundings)
+                x = ptx::add2(ptx::fma2(make_float2(mk[e], mk[e + 1]), make_float2(kLog2e, kLog2e), ptx::mul2(x, c2)), l2);
+              else
+                x = ptx::fma2(x, c2, l2);
+              x = ptx::mul2(make_float2(ptx::ex2(x.x), ptx::ex2(x.y)), make_float2(w4[e], w4[e + 1]));
+              pb[j + e] = x.x, pb[j + e + 1] = x.y;
             }
           }
           const bool edge = col0 + j0 < all_lo || col0 + j0 + 16 > all_hi;
@@ -344,16 +349,19 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           ptx::tmem_ld16(y_at + LY::kScores + j0, s);
           if (LY::kWide) ptx::tmem_ld16(y_at + BN + j0, s2);
           ptx::tmem_wait_ld();
-          add_to<LY::kWide>(s, s2, D == 64 ? kLoss : 2 * kLoss);
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
             float d4[4] = {delta, delta, delta, delta};
             if constexpr (KEYS) {
-              const float4 v = ptx::ld_shared_f4(vec + BN * 4 + (j0 + j) * 4);
+              const float4 v = ptx::ld_shared_f4(vec + 2 * BN * 4 + (j0 + j) * 4);
               d4[0] = v.x, d4[1] = v.y, d4[2] = v.z, d4[3] = v.w;
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) pb[j + e] *= __uint_as_float(s[j + e]) - d4[e];  // dS, without the scale
+            for (int e = 0; e < 4; e += 2) {  // dS, without the scale
+              const float2 dp = LY::kWide ? ptx::add2(floats2(s, j + e), floats2(s2, j + e)) : floats2(s, j + e);
+              const float2 x = ptx::mul2(make_float2(pb[j + e], pb[j + e + 1]), ptx::add2(dp, make_float2(-d4[e], -d4[e + 1])));
+              pb[j + e] = x.x, pb[j + e + 1] = x.y;
+            }
           }
           planes(y_at + LY::plane_at(0, j0 / 16), pb);
           if (KEYS && a.ds && own0 + r < ds_pitch(a)) {
@@ -537,9 +545,10 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         if (KEYS && first && lt < BN) {
           const int r = (begin + t) * BN + lt;
           const float l = r < rows ? a.lse[stat_at(r)] : 0.f;
-          float* vec = reinterpret_cast<float*>(smem + LY::kVec) + (at & 1) * 2 * BN;
-          vec[lt] = r >= rows || l == -INFINITY ? INFINITY : l * kLog2e;
-          vec[BN + lt] = r < rows ? a.delta[stat_at(r)] : 0.f;
+          float w, *vec = reinterpret_cast<float*>(smem + LY::kVec + (at & 1) * LY::kVecBytes);
+          vec[lt] = minus_lse2(r < rows ? l : -INFINITY, kv_len, w);
+          vec[BN + lt] = w;
+          vec[2 * BN + lt] = r < rows ? a.delta[stat_at(r)] : 0.f;
         }
 #pragma unroll
         for (int i0 = 0; i0 < TB::kChunks; i0 += kHeld) {
@@ -590,21 +599,12 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
       const uint32_t b2 = ptx::smem_desc_lo(base + LY::kB2, 16);
       constexpr int kLbo = LY::kWide ? TB::kPlane : TB::kBlock;
       const uint32_t b1_mn = ptx::smem_desc_lo(base + LY::kB1, kLbo), b2_mn = ptx::smem_desc_lo(base + LY::kB2, kLbo);
-      // The pairs of pieces, small ones first.  Wide: (l, h) into the first sum, (h, l) into the second, then m and h with (h, m) into both.
-      constexpr int kSteps = LY::kWide ? 4 : kProducts;
-      struct Step {
-        uint32_t a, b;
-        bool second, two, onto;
-      };
-      auto step_of = [](int p) {
-        if (LY::kWide) return Step{p == 0 ? 2u : (p == 2 ? 1u : 0u), p == 1 ? 2u : 0u, p == 1, p >= 2, p >= 2};
-        return Step{piece_a(p), piece_b(p), false, false, p > 0};
-      };
+      constexpr Sums kSums = LY::kWide ? kLeadApart : kOneSum;
       // product of a tile: A's planes from TMEM region `region`, B MN-major
       auto issue_t = [&](uint32_t region, uint32_t b_mn) {
 #pragma unroll 1  // (all products at once: the addresses do not fit this warp's registers)
-        for (int p = 0; p < kSteps; ++p) {
-          const Step st = step_of(p);
+        for (int p = 0; p < steps_of(kSums); ++p) {
+          const Step st = step_of(kSums, p);
           const uint32_t d = tmem + LY::kT + (st.second ? D : 0), ap = tmem + region + LY::plane_at(st.a, 0), bp = b_mn + st.b * kPB;
           const uint32_t idesc = st.two ? kIdescT2 : kIdescT1;
 #pragma unroll
@@ -619,8 +619,8 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         if (!uwait(&ctl->b1_full[stage], at / LY::kStages & 1) || !(t == 0 ? uwait(&ctl->a_full, pass & 1) : uwait(&ctl->x_free, (at - 1) & 1))) return false;
         ptx::tc_fence_after();
 #pragma unroll 1
-        for (int p = 0; p < kSteps; ++p) {
-          const Step st = step_of(p);
+        for (int p = 0; p < steps_of(kSums); ++p) {
+          const Step st = step_of(kSums, p);
           const uint32_t d = tmem + LY::kX + LY::kScores + (st.second ? BN : 0), ap = tmem + LY::kA1 + st.a * (D / 2), bp = b1 + stage_at + st.b * kPB;
           const uint32_t idesc = st.two ? kIdescS2 : kIdescS1;
 #pragma unroll
@@ -636,8 +636,8 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         if (!uwait(&ctl->b2_full[stage], at / LY::kStages & 1) || !(t == 0 ? uwait(&ctl->a_full, pass & 1) : uwait(&ctl->y_free, (at - 1) & 1))) return false;
         ptx::tc_fence_after();
 #pragma unroll 1
-        for (int p = 0; p < kSteps; ++p) {
-          const Step st = step_of(p);
+        for (int p = 0; p < steps_of(kSums); ++p) {
+          const Step st = step_of(kSums, p);
           const uint32_t d = tmem + LY::kY + LY::kScores + (st.second ? BN : 0), ap = a2 + st.a * kPA, bp = b2s + st.b * kPB;
           const uint32_t idesc = st.two ? kIdescS2 : kIdescS1;
 #pragma unroll
@@ -828,7 +828,6 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     // keys that the row sees: what lies behind has not been written
     const int limit = own0 + r < rows ? (a.causal ? min(kv_len, rw.query(own0 + r) + shift + 1) : kv_len) : 0;
-    const float loss = limit > kFewTerms ? kLoss : kNoLoss;
     const int pitch = ds_pitch(a), n_rows = ds_rows(a) - own0;
     const float* ds = ds_of(a, b, hk) + static_cast<int64_t>(own0) * pitch;
     auto fetch = [&](int t) {  // two rows of 64 floats a warp at a time, neighbouring vectors exchanged by row
@@ -858,9 +857,9 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
           ptx::tmem_ld16(from + 2 * j, o);
           if (LY::kWide) ptx::tmem_ld16(from + D + 2 * j, o2);
           ptx::tmem_wait_ld();
-          add_to<LY::kWide>(o, o2, loss);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[j + e] = ptx::add2(acc[j + e], make_float2(__uint_as_float(o[2 * e]), __uint_as_float(o[2 * e + 1])));
+          for (int e = 0; e < 8; ++e)
+            acc[j + e] = ptx::add2(acc[j + e], LY::kWide ? ptx::add2(floats2(o, 2 * e), floats2(o2, 2 * e)) : floats2(o, 2 * e));
         }
         ptx::tc_fence_before();
       };
@@ -984,16 +983,15 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
         const uint32_t at = done + t, two = at & 1;
         if (!uwait(&ctl->b_full[two], at >> 1) || !uwait(&ctl->a_full[two], at >> 1)) break;
         ptx::tc_fence_after();
-        constexpr int kSteps = LY::kWide ? 4 : kProducts;
+        constexpr Sums kSums = LY::kWide ? kLeadApart : kOneSum;
 #pragma unroll 1
-        for (int p = 0; p < kSteps; ++p) {  // pairs of pieces, as in walk
-          const uint32_t pa = LY::kWide ? (p == 0 ? 2u : (p == 2 ? 1u : 0u)) : piece_a(p), pb = LY::kWide ? (p == 1 ? 2u : 0u) : piece_b(p);
-          const uint32_t d = tmem + LY::kT + two * LY::kBufT + (LY::kWide && p == 1 ? D : 0), ap = tmem + LY::kA + two * LY::kBufA + pa * 32;
-          const uint32_t bp = b_mn + two * (TB::kBytes >> 4) + pb * kPB, idesc = LY::kWide && p >= 2 ? kIdesc2 : kIdesc1;
-          const bool onto = LY::kWide ? p >= 2 : p > 0;
+        for (int p = 0; p < steps_of(kSums); ++p) {
+          const Step st = step_of(kSums, p);
+          const uint32_t d = tmem + LY::kT + two * LY::kBufT + (st.second ? D : 0), ap = tmem + LY::kA + two * LY::kBufA + st.a * 32;
+          const uint32_t bp = b_mn + two * (TB::kBytes >> 4) + st.b * kPB, idesc = st.two ? kIdesc2 : kIdesc1;
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
-            if (leader) ptx::mma_ts2(d, ap + ks * 8, bp + ks * (2048 >> 4), kHi, idesc, onto || ks > 0 ? 1u : 0u);
+            if (leader) ptx::mma_ts2(d, ap + ks * 8, bp + ks * (2048 >> 4), kHi, idesc, st.onto || ks > 0 ? 1u : 0u);
         }
         if (leader) {
           ptx::mma_commit(&ctl->b_free[two]);

@@ -3,10 +3,16 @@
 // A float has 24 significant bits, a bf16 has 8: x rounded to bf16, what is left rounded to bf16, and what is left then are three
 // bf16 whose sum is x, exactly, over the range of exponents.  Of the nine products of pieces the six that reach 2^-24 of the result are
 // taken and accumulated in fp32 in TMEM, the small ones first, over one tile only (64 terms of the contraction for probabilities, D for
-// scores): the tensor cores truncate where they accumulate, so the sums over tiles are made in registers, by rounded additions.  Error
-// of a product against 64 bits, relative (2-norm), beside that of a chain of fp32 FMAs: 64 terms 0.8e-7 (1.4e-7), 128 terms 1.3e-7 (2.0e-7);
-// truncated instead of rounded pieces, all of whose left-out products have one sign, 1.2e-7 and 1.7e-7.  Six bf16 products at
-// 1.63 PFLOP/s are 271 TFLOP/s of fp32, 3.7 times the FMA pipes' 74.
+// scores): the tensor cores truncate where they accumulate, so the sums over tiles are made in registers, by rounded additions.  What the
+// truncations take is not given back: on average it is 0.75e-7 of a sum of 64 products of mixed signs, but other data lose other shares, sums of
+// few or of few bits none, and dP - delta makes much of little (operands of [0.5, 1.5], D = 128: dK 2.8e-7 off as it is, 15.5e-7 with that
+// average added).  Relative error against 64 bits (2-norm), 4 x 8 heads x 500, and that of fp32 FMAs, 1e-7:
+//                   D = 64: O, dQ, dK, dV                                D = 128
+//   N(0, 1)           1.9 (3.5)  3.2 (3.8)  3.2 (4.5)  2.9 (4.3)           2.5 (4.7)  3.8 (4.2)  3.8 (5.6)  3.2 (5.4)
+//   ... 3 Q, 3 K      3.8 (7.0)  11.3 (17)  11.3 (17)  10.5 (13.5)         5.6 (9.2)  18 (21)    18 (21)    16.1 (14.6)
+//   [0.5, 1.5]        0.8 (1.7)  dQ is 0 but for errors  1.2 (2.2)  0.7 (1.8)      0.9 (3.3)             2.8 (4.9)  2.7 (4.5)
+//   Q, K in -2 .. 2   1.6 (3.2)  4.8 (6.9)  4.7 (6.8)  4.6 (5.7)           1.5 (3.4)  8.3 (10.7) 8.3 (10.8) 8.1 (9.2)
+// Six bf16 products at 1.63 PFLOP/s are 271 TFLOP/s of fp32, 3.7 times the FMA pipes' 74.
 //
 // Infinities: where a piece is zero its product with an infinite piece of the other operand would be NaN where x * inf is inf, and
 // pieces of other signs than x would subtract infinities.  Kernels therefore walk their tiles again with the CAREFUL split once they
@@ -19,13 +25,6 @@
 namespace ttattn {
 namespace pieces {
 
-// What the truncations take, on average, from a sum of 64 products of mixed signs (four steps of the contraction at full size): given
-// back where sums are added or scaled anyway.  (128 terms: twice that.)  With 32 terms or fewer nothing is.  Relative error of gradients,
-// 4 x 8 heads x 500, without and with (and of fp32 FMAs): D = 64 dQ 4.2e-7, 3.6e-7 (3.8e-7), D = 128 5.2e-7, 3.5e-7 (4.2e-7).
-constexpr float kLoss = 0.75e-7f;
-constexpr int kFewTerms = 32;
-constexpr float kNoLoss = 0x1p-60f;  // adds nothing to a finite sum, and leaves an infinite one what it is (0 would make NaN of it)
-
 constexpr int kPieces = 3;
 constexpr int kProducts = 6;
 // the products taken, small ones first: piece of A and piece of B (0: leading), a nibble each
@@ -35,6 +34,26 @@ __host__ __device__ constexpr uint32_t piece_b(int p) { return kPieceB >> (4 * p
 static_assert(piece_a(0) == 2 && piece_b(0) == 0 && piece_a(1) == 1 && piece_b(1) == 1 && piece_a(2) == 0 && piece_b(2) == 2 &&
                   piece_a(3) == 1 && piece_b(3) == 0 && piece_a(4) == 0 && piece_b(4) == 1 && piece_a(5) == 0 && piece_b(5) == 0,
               "every pair of pieces that reaches 2^-24, the small ones first");
+
+// How the products of a tile are summed.  kOneSum: in one accumulator.  The others have a second one beside it, and an MMA whose second
+// operand is the two first planes as one of twice the rows fills both.  kTwoSums: (l, h), (m, h), (h, h) in the first, the rest in the second.
+// kLeadApart: (h, h) alone in the first.  Its truncations are those of a sum of the leading pieces alone then, none where these are few or
+// fit 24 bits, and the same whichever operand comes first, in the forward and in the backward.  Two MMAs of 64 columns in the place of one of 128: D = 64 forward
+// 18.1 -> 18.4 us (4 x 8 heads x 500), backward 58.8 -> 59.3; relative error of dV against 64 bits, scores of standard deviation 9, 18.6e-7 -> 13.0e-7
+// (fp32 FMAs 13.5e-7), of dK, operands of [0.5, 1.5], 2.8e-7 -> 1.5e-7 (2.2e-7).
+enum Sums { kOneSum, kTwoSums, kLeadApart };
+struct Step {
+  uint32_t a, b;  // pieces
+  bool second;    // into the second sum
+  bool two;       // pieces b and b + 1, into both
+  bool onto;      // what there is
+};
+__host__ __device__ constexpr int steps_of(Sums s) { return s == kOneSum ? kProducts : (s == kTwoSums ? 4 : 5); }
+__host__ __device__ constexpr Step step_of(Sums s, int p) {
+  return s == kOneSum    ? Step{piece_a(p), piece_b(p), false, false, p > 0}
+         : s == kTwoSums ? Step{p == 0 ? 2u : (p == 2 ? 1u : 0u), p == 1 ? 2u : 0u, p == 1, p >= 2, p >= 2}
+                         : Step{p == 1 ? 2u : (p >= 3 ? 1u : 0u), p == 2 ? 2u : (p == 4 ? 1u : 0u), p > 0, p == 0, p > 0};
+}
 
 __device__ __forceinline__ float lead(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack_lead(float x0, float x1) {  // leading halves of two floats, x0 below
@@ -74,11 +93,6 @@ template <bool CAREFUL>
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
   float2 unused = make_float2(0.f, 0.f);
   split2<CAREFUL>(x0, x1, h, m, l, unused);
-}
-
-// The two sums of a product: with the first plane, whose truncations count, and with the others.
-__device__ __forceinline__ float2 both(const float2& x, const float2& y, float loss) {
-  return ptx::add2(x, ptx::fma2(x, make_float2(loss, loss), y));
 }
 
 // Eight consecutive floats as 16 bytes of each piece, `plane` bytes apart, at shared-memory addresses; N times, side by side.

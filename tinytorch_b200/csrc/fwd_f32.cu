@@ -10,13 +10,12 @@
 //                the softmax of the next.  (One warp for both spends 850 of 3100 clocks per tile in waits for what is there already.)
 //   warps 18, 19 masks
 // An MMA of 64 columns takes 52 (A from TMEM) or 66 clocks (from shared memory) where 32 would do and 128 columns take 64: the first two planes
-// of K (and of V, D = 64) are read as one operand of 128.  S and O come as two sums then, with the first plane and with the others.
+// of K (and of V, D = 64) are read as one operand of 128.  S and O come as two sums then (f32_pieces.cuh).
 //
 // Bound by the chain of a tile: softmax 2000 clocks and 300 until S is seen (D = 64: a tile 2400; the MMAs take 2100 of them), for D = 128,
 // where only one K tile fits, K into pieces, then S 1800.  Against the same in fp32 FMAs on CUDA cores (64 x 64 tiles, whose FMA pipes were
 // 58 % busy), us: D = 64, 4 x 8 heads x 500 72 -> 19 (additive mask 74 -> 29, 6 x 333 padding 52 -> 19), causal 16 x 2048 293 -> 54,
 // 11 x 32/8 heads x 22 14.5 -> 9.2, one query on one key 7.2 -> 6.3; D = 128, 4 x 8 x 500 117 -> 33 (additive 125 -> 43), causal 4 x 4096 506 -> 107.
-// Relative error against 64 bits: 4 x 8 x 500 3.5e-7 -> 1.6e-7 and 4.7e-7 -> 2.0e-7.
 // Tried: P over the S that it is made of, two such buffers, S up to two tiles ahead: 2700 clocks a tile.  One place for P: 3150.
 // Additive rows by bulk copies of 256 bytes: 29.7 -> 32.3, D = 128 43 -> 53.
 #include <algorithm>
@@ -254,8 +253,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
           ptx::tmem_wait_ld();
 #pragma unroll
           for (int e = 0; e < 32; e += 2) {
-            const float2 z = both(make_float2(__uint_as_float(x[e]), __uint_as_float(x[e + 1])),
-                                  make_float2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])), D == 64 ? kLoss : 2 * kLoss);
+            const float2 z = ptx::add2(make_float2(__uint_as_float(x[e]), __uint_as_float(x[e + 1])),
+                                       make_float2(__uint_as_float(y[e]), __uint_as_float(y[e + 1])));
             s[j + e] = z.x, s[j + e + 1] = z.y;
           }
         }
@@ -308,31 +307,37 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
         reinterpret_cast<float*>(smem + LY::kAlpha)[(at & 3) * BM + tid] = alpha;
         float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         const float2 c2 = make_float2(c, c), neg2 = make_float2(-m_use, -m_use);
-        auto probabilities = [&](auto keep_signs) {
+        auto probabilities = [&](auto keep_signs, const float* sp, int j) {  // of 16 scores, those of columns j ..
+          uint32_t ph[8], pm[8], pl[8];
 #pragma unroll
-          for (int j = 0; j < BN; j += 16) {
-            uint32_t ph[8], pm[8], pl[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float2 sc = make_float2(s[j + 2 * e], s[j + 2 * e + 1]);
-              const float2 y = SCALED ? ptx::add2(sc, neg2) : ptx::fma2(sc, c2, neg2);
-              const float2 p = make_float2(ptx::ex2(y.x), ptx::ex2(y.y));
-              sum[e & 1] = ptx::add2(sum[e & 1], p);
-              split2<decltype(keep_signs)::value>(p.x, p.y, ph[e], pm[e], pl[e]);
-            }
-            ptx::tmem_st8(p_at + j / 2, ph);
-            ptx::tmem_st8(p_at + 32 + j / 2, pm);
-            ptx::tmem_st8(p_at + 64 + j / 2, pl);
+          for (int e = 0; e < 8; ++e) {
+            const float2 sc = make_float2(sp[2 * e], sp[2 * e + 1]);
+            const float2 y = SCALED ? ptx::add2(sc, neg2) : ptx::fma2(sc, c2, neg2);
+            const float2 p = make_float2(ptx::ex2(y.x), ptx::ex2(y.y));
+            sum[e & 1] = ptx::add2(sum[e & 1], p);
+            split2<decltype(keep_signs)::value>(p.x, p.y, ph[e], pm[e], pl[e]);
           }
+          ptx::tmem_st8(p_at + j / 2, ph);
+          ptx::tmem_st8(p_at + 32 + j / 2, pm);
+          ptx::tmem_st8(p_at + 64 + j / 2, pl);
         };
         if (t >= 2) {  // P of two tiles before has been read
           if (!uwait(&ctl->v_free[two], (at - 2) >> 1)) break;
           ptx::tc_fence_after();
         }
-        if (rare(careful))
-          probabilities(std::true_type{});
-        else
-          probabilities(std::false_type{});
+        if (rare(careful)) {
+          // With a mask its code stands once, and s moves up: four times it costs the other pass registers (additive, 4 x 8 heads x 500:
+          // 28.7 us, boolean 23.5; once 27.8 and 22.8).  Without one it is four times: 18.3; once 18.7.
+#pragma unroll(MASK == kNoMask ? 4 : 1)
+          for (int j = 0; j < BN; j += 16) {
+            probabilities(std::true_type{}, s, j);
+#pragma unroll
+            for (int e = 0; e < BN - 16; ++e) s[e] = s[e + 16];
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN; j += 16) probabilities(std::false_type{}, s + j, j);
+        }
         sum[0] = ptx::add2(sum[0], sum[1]);
         l_row = fmaf(l_row, alpha, sum[0].x + sum[0].y);
         ptx::tmem_wait_st();
@@ -349,8 +354,6 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
   } else if (warp < 8) {
     // ------------------------------------------------------------------------------------------------------ O --
     ptx::setmaxnreg_inc<LY::kSumRegs>();
-    // (of the terms that a row has, as far as lengths and alignment tell)
-    const float loss = (a.causal ? min(kv_len, query_of(tid - 128) + shift + 1) : kv_len) > kFewTerms ? kLoss : kNoLoss;
     const uint32_t from = tmem_o + (static_cast<uint32_t>((warp - 4) * 32) << 16);
     float2 acc[D / 2];
     bool careful = false;
@@ -374,8 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
           for (int e = 0; e < 8; ++e) {
             const float2 z = make_float2(__uint_as_float(x[2 * e]), __uint_as_float(x[2 * e + 1]));
             acc[j / 2 + e] = ptx::fma2(acc[j / 2 + e], alpha2,
-                                       LY::kWideV ? both(z, make_float2(__uint_as_float(y[2 * e]), __uint_as_float(y[2 * e + 1])), loss)
-                                                  : ptx::fma2(z, make_float2(loss, loss), z));
+                                       LY::kWideV ? ptx::add2(z, make_float2(__uint_as_float(y[2 * e]), __uint_as_float(y[2 * e + 1]))) : z);
           }
         }
         ptx::tc_fence_before();
@@ -456,18 +458,18 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
       constexpr uint32_t kPQ = TQ::kPlane >> 4, kPK = TK::kPlane >> 4;
       const uint32_t qlo = ptx::smem_desc_lo(base + LY::kQ, 16), klo = ptx::smem_desc_lo(base + LY::kK, 16);
       const uint32_t vlo = ptx::smem_desc_lo(base + LY::kV, LY::kWideV ? TK::kPlane : TK::kBlock);
-      // pieces (l, h) into the first sum, (h, l) into the second, then m and h with (h, m) into both
+      constexpr Sums kSumsS = D == 64 ? kLeadApart : kTwoSums, kSumsO = LY::kWideV ? kLeadApart : kOneSum;
       auto issue_qk = [&](uint32_t at) {
         const uint32_t d = tmem, k0 = klo + at % kStages * (TK::kBytes >> 4);
 #pragma unroll 1
-        for (int p = 0; p < 4; ++p) {
-          const uint32_t qo = qlo + (p == 0 ? 2 * kPQ : (p == 2 ? kPQ : 0)), ko = k0 + (p == 1 ? 2 * kPK : 0), to = d + (p == 1 ? BN : 0);
-          const uint32_t idesc = p < 2 ? idesc_s1 : idesc_s2;
+        for (int p = 0; p < steps_of(kSumsS); ++p) {
+          const Step st = step_of(kSumsS, p);
+          const uint32_t qo = qlo + st.a * kPQ, ko = k0 + st.b * kPK, to = d + (st.second ? BN : 0), idesc = st.two ? idesc_s2 : idesc_s1;
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks)
             if (leader)
               ptx::mma_ss2(to, qo + (((ks >> 2) * TQ::kBlock + (ks & 3) * 32) >> 4), kHi, ko + (((ks >> 2) * TK::kBlock + (ks & 3) * 32) >> 4), kHi,
-                           idesc, p > 1 || ks > 0 ? 1u : 0u);
+                           idesc, st.onto || ks > 0 ? 1u : 0u);
         }
         if (leader) {
           ptx::mma_commit(&ctl->k_free[at & 1]);
@@ -476,20 +478,13 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
       };
       auto issue_pv = [&](uint32_t at) {
         const uint32_t p0 = tmem + LY::kP + (at & 1) * LY::kBufP, v0 = vlo + at % kStages * (TK::kBytes >> 4);
-        constexpr int kSteps = LY::kWideV ? 4 : kProducts;
 #pragma unroll 1
-        for (int p = 0; p < kSteps; ++p) {
-          uint32_t po, vo, to = tmem_o, idesc = kIdescO1;
-          if (LY::kWideV) {
-            po = p0 + (p == 0 ? 64 : (p == 2 ? 32 : 0)), vo = v0 + (p == 1 ? 2 * kPK : 0), to += p == 1 ? D : 0;
-            if (p >= 2) idesc = kIdescO2;
-          } else {
-            po = p0 + piece_a(p) * 32, vo = v0 + piece_b(p) * kPK;
-          }
-          const bool onto = LY::kWideV ? p > 1 : p > 0;
+        for (int p = 0; p < steps_of(kSumsO); ++p) {
+          const Step st = step_of(kSumsO, p);
+          const uint32_t po = p0 + st.a * 32, vo = v0 + st.b * kPK, to = tmem_o + (st.second ? D : 0), idesc = st.two ? kIdescO2 : kIdescO1;
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
-            if (leader) ptx::mma_ts2(to, po + ks * 8, vo + ks * (2048 >> 4), kHi, idesc, onto || ks > 0 ? 1u : 0u);
+            if (leader) ptx::mma_ts2(to, po + ks * 8, vo + ks * (2048 >> 4), kHi, idesc, st.onto || ks > 0 ? 1u : 0u);
         }
         if (leader) {
           ptx::mma_commit(&ctl->v_free[at & 1]);
