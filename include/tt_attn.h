@@ -297,7 +297,9 @@ TT_ATTN_API int tt_attn_selftest_wait_expiry(int device, void* stream, uint64_t 
  *    padding mask uses; with 256 bytes such a mask is read in full;
  *  - backward: rowsum(dO o O) and, fp16 / bf16, the fp32 dQ accumulator and the words above;
  *    where key tiles are few also shares of dK / dV, as many as fit; fp32: dS, where it
- *    comes to 192 MB at most and fits (else dQ recomputes it);
+ *    comes to 192 MB at most and fits (else dQ recomputes it), and with an additive mask 8
+ *    bytes a row, if they fit behind that, for rows whose log-sum-exp is beyond 4096 (all keys
+ *    masked by -1e9, say; without, those beyond 2^18 count for nothing in the gradients);
  *  - decode: partial results of the pieces a cache is divided into, in longer pieces if need be,
  *    and a work counter for several query heads per key head.
  * TT_ATTN_ERR_WORKSPACE comes when not even the least of this fits. */

@@ -169,7 +169,10 @@ size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int 
     // delta [B,Hq,Lq] fp32; the fp16 / bf16 path adds an fp32 dQ accumulator [B,Hq,Lq,D]
     const size_t rows = static_cast<size_t>(B) * Hq * (Lq > 0 ? Lq : 0);
     // and the persistent kernel's work counter
-    if (dtype == TT_ATTN_F32) return round256(rows * sizeof(float)) + round256(bwd_ds_bytes(B, Hq, Hkv, Lq, Skv, D));
+    if (dtype == TT_ATTN_F32) {
+      const size_t ds = round256(bwd_ds_bytes(B, Hq, Hkv, Lq, Skv, D));
+      return round256(rows * sizeof(float)) + ds + (ds > 0 ? round256(rows * sizeof(float2)) : 0);
+    }
     // (and, where few key tiles are divided among several work items, their partial dK / dV)
     return round256(rows * sizeof(float)) + round256(rows * D * sizeof(float)) +
            round256(bwd_part_bytes(B, Hq, Hkv, Lq, Skv, D)) + round256(scratch_words(B) * sizeof(int));
@@ -263,7 +266,7 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   DeviceGuard guard(p->device);
   if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
   Workspace ws;
-  // delta | dQ accumulator | shares of dK / dV | work counter and, if they fit, a padding mask's lengths
+  // delta | dQ accumulator | shares of dK / dV | work counter and, if they fit, a padding mask's lengths; fp32: delta | dS | rows' maxima and sums
   const size_t rows = static_cast<size_t>(p->B) * p->Hq * p->Lq, delta = round256(rows * sizeof(float));
   const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
   size_t need = delta, part = 0;
@@ -271,6 +274,9 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
   // fp32: dS tiles on their way from dK / dV to dQ, where dQ and at least one of the others are asked for and there is room
   size_t ds = p->dtype == TT_ATTN_F32 && p->dq && (p->dk || p->dv) ? round256(bwd_ds_bytes(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) : 0;
   if (delta + ds > room) ds = 0;
+  // ... and, with an additive mask, maxima and sums of the rows whose log-sum-exp is too large to say both
+  size_t stats = p->dtype == TT_ATTN_F32 && a.mask.ptr && a.mask.kind != TT_ATTN_MASK_BOOL ? round256(rows * sizeof(float2)) : 0;
+  if (delta + ds + stats > room) stats = 0;
   if (p->dtype != TT_ATTN_F32) {
     // a buffer that is too small for the division (a small batch is divided further than a large one): fewer shares
     a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
@@ -280,12 +286,13 @@ int tt_attn_bwd(const tt_attn_bwd_params* p) {
     lens = mask_lens_fit(a.mask, a.causal, p->B, room, need);
     need += lens ? round256(scratch_words(p->B) * sizeof(int)) : 256;
   }
-  if (ds == 0 || ws.acquire(need + ds, p->workspace, p->workspace_bytes, p->alloc, p->device) != TT_ATTN_OK) {
-    ds = 0;  // (an allocator that has no more than before)
+  if (ds + stats == 0 || ws.acquire(need + ds + stats, p->workspace, p->workspace_bytes, p->alloc, p->device) != TT_ATTN_OK) {
+    ds = stats = 0;  // (an allocator that has no more than before)
     if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
   }
   a.delta = static_cast<float*>(ws.ptr);
   if (ds > 0) a.ds = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
+  if (stats > 0) a.row_stats = reinterpret_cast<float2*>(static_cast<char*>(ws.ptr) + delta + ds);
   if (p->dtype != TT_ATTN_F32) {
     a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
     a.dkv_part = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta + accum);

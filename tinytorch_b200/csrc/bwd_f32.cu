@@ -53,7 +53,7 @@ struct Lay {
   static constexpr int kStages = D == 64 ? 2 : 1;  // of the other side's tiles
   static constexpr int kMaskBytes = MASK == kNoMask ? 0 : (MASK == kBoolMask ? BM * 8 : BM * BN * 4);
   static constexpr int kA2 = 0, kB1 = TA::kBytes, kB2 = kB1 + kStages * TB::kBytes, kM = kB2 + kStages * TB::kBytes;
-  static constexpr int kVec = kM + kMaskBytes;  // [2][lse, weight, delta][64]
+  static constexpr int kVec = kM + kMaskBytes;  // [2][exponent base, factor, delta][64]
   static constexpr int kVecBytes = 3 * BN * 4;
   static constexpr int kCtl = kVec + 2 * kVecBytes;
   static constexpr int kBytes = kCtl + 256;
@@ -79,15 +79,6 @@ static_assert(Lay<128, kAddMask>::kBytes <= 227 * 1024, "shared memory");
 
 // two neighbouring words of accumulators
 __device__ __forceinline__ float2 floats2(const uint32_t (&x)[16], int i) { return make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])); }
-// A row's log-sum-exp in units of the exponents without an integer of 0 .. log2(n), n: how many keys the row may see; negated.  2 to minus that
-// integer is the row's weight.  What a key of average probability has for an exponent is near 0 then, and so is its rounding, where it would be
-// near -log2(n): relative error of dQ against 64 bits, 4 x 8 heads x 500, 3.8e-7 -> 3.2e-7 (D = 64; fp32 FMAs 3.8e-7), 4.4e-7 -> 3.8e-7 (D = 128; 4.2e-7).
-__device__ __forceinline__ float minus_lse2(float lse, int n, float& weight) {
-  const float x = lse * kLog2e, whole = fminf(fmaxf(rintf(x), 0.f), static_cast<float>(31 - __clz(max(n, 1))));
-  weight = __int_as_float((127 - static_cast<int>(whole)) << 23);
-  return lse == -INFINITY ? -INFINITY : whole - x;  // (a row without any participating key: P is 0)
-}
-
 // where dS waits for the dQ pass: for each (batch, kv head) the queries' rows, in whole tiles, of keys, in whole tiles
 __device__ __forceinline__ int ds_pitch(const BwdArgs& a) { return (a.Skv + BN - 1) / BN * BN; }
 __device__ __forceinline__ int ds_rows(const BwdArgs& a) { return (a.Lq * (a.Hq / a.Hkv) + BN - 1) / BN * BN; }
@@ -152,6 +143,13 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
   const int own_rows = (KEYS ? kv_len : rows) - own0, other_rows = KEYS ? rows : kv_len;  // (own ones may be fewer than none)
   const int64_t stat_base = static_cast<int64_t>(b) * a.Hq * a.Lq;  // of lse and delta
   auto stat_at = [&](int r) { return stat_base + static_cast<int64_t>(head0 + rw.head(r)) * a.Lq + rw.query(r); };
+  auto stats_of = [&](int r) {  // of the query in row r
+    if (r >= rows) return make_float2(-INFINITY, 1.f);
+    if (MASK == kAddMask && a.row_stats) return a.row_stats[stat_at(r)];
+    const float lse = a.lse[stat_at(r)];
+    // (too large for its exponents to be right within a few per cent, and no room for better: the row counts for nothing)
+    return MASK == kAddMask && fabsf(lse) >= 0x1p18f ? make_float2(-INFINITY, 1.f) : exponent_base(lse, kv_len);
+  };
 
   auto last_pass = [&](bool careful) {  // by all threads at the end of a pass
     ptx::named_barrier(1, kThreads);
@@ -216,7 +214,8 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
       const float c = a.scale * kLog2e;
       // what the row takes part in: other rows lo .. hi - 1
       int lo = 0, hi;
-      float lse2 = 0.f, weight = 1.f, delta = 0.f;  // query CTAs: the row's
+      float2 stats = make_float2(0.f, 1.f);  // query CTAs: the row's
+      float delta = 0.f;
       int all_lo = 0, all_hi;         // what every row of the CTA takes part in
       if constexpr (KEYS) {
         const int key = own0 + r;
@@ -230,8 +229,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
         const int i_q = rw.query(own0 + r);
         hi = own0 + r < rows ? (a.causal ? min(kv_len, i_q + shift + 1) : kv_len) : 0;
         all_hi = a.causal ? min(kv_len, rw.query(own0) + shift + 1) : kv_len;
-        const float l = own0 + r < rows ? a.lse[stat_at(own0 + r)] : 0.f;
-        lse2 = minus_lse2(l, kv_len, weight);
+        stats = stats_of(own0 + r);
         delta = own0 + r < rows ? a.delta[stat_at(own0 + r)] : 0.f;
       }
       // a tile's product into the sums
@@ -298,7 +296,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           ptx::tmem_wait_ld();
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            float l4[4] = {lse2, lse2, lse2, lse2}, w4[4] = {weight, weight, weight, weight};
+            float l4[4] = {stats.x, stats.x, stats.x, stats.x}, w4[4] = {stats.y, stats.y, stats.y, stats.y};
             if constexpr (KEYS) {
               const float4 v = ptx::ld_shared_f4(vec + (j0 + j) * 4), w = ptx::ld_shared_f4(vec + (BN + j0 + j) * 4);
               l4[0] = v.x, l4[1] = v.y, l4[2] = v.z, l4[3] = v.w;
@@ -544,10 +542,9 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           return false;
         if (KEYS && first && lt < BN) {
           const int r = (begin + t) * BN + lt;
-          const float l = r < rows ? a.lse[stat_at(r)] : 0.f;
-          float w, *vec = reinterpret_cast<float*>(smem + LY::kVec + (at & 1) * LY::kVecBytes);
-          vec[lt] = minus_lse2(r < rows ? l : -INFINITY, kv_len, w);
-          vec[BN + lt] = w;
+          const float2 stats = stats_of(r);
+          float* vec = reinterpret_cast<float*>(smem + LY::kVec + (at & 1) * LY::kVecBytes);
+          vec[lt] = stats.x, vec[BN + lt] = stats.y;
           vec[2 * BN + lt] = r < rows ? a.delta[stat_at(r)] : 0.f;
         }
 #pragma unroll

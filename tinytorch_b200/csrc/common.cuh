@@ -86,6 +86,7 @@ struct BwdArgs {
   int* sched;         // tensor-core kernel: work counter in scratch memory, zeroed by the delta pre-pass
   int parts;          // tensor-core kernel: work items per key tile (see bwd_parts); > 1: each leaves its dK / dV in ...
   float* dkv_part;    // ... workspace [dK, dV][parts][B * Hkv][Skv][D] fp32
+  float2* row_stats;  // fp32 kernels with an additive mask: workspace [B, Hq, Lq] for what a row's probabilities are made with (see exponent_base), or null
   float* ds;          // fp32 kernels: dS on its way from the dK / dV pass to the dQ pass, or null (see bwd_ds_bytes)
   void* dq;
   void* dk;
