@@ -290,6 +290,12 @@ TT_ATTN_API int tt_attn_decode_static(const tt_attn_decode_params* p);
 TT_ATTN_API int tt_attn_selftest_wait_expiry(int device, void* stream, uint64_t limit_ns, int32_t* status,
                                              unsigned long long* waited_ns);
 
+/* For tests: the fp32 backward (TT_ATTN_ERR_DTYPE for others) with dQ made the way the caller chooses.  `path`: 0, dS is
+ * recomputed; 1, dS is stored by the pass that makes dK and dV, whatever its size (TT_ATTN_ERR_SHAPE where dQ or both
+ * of the others are not asked for); -1 launches nothing, and `planned` (host memory, else not written) receives
+ * what tt_attn_bwd takes with this scratch memory. */
+TT_ATTN_API int tt_attn_bwd_selftest(const tt_attn_bwd_params* p, int32_t path, int32_t* planned);
+
 /* Scratch bytes with which the given call runs at its best (0 if none).  Skv is the cache
  * capacity for TT_ATTN_KIND_DECODE.  A buffer sized for a batch serves every smaller one,
  * although a small batch, which is divided further, would like more:

@@ -142,3 +142,41 @@ def test_keys_hidden_by_small_queries(small, D):
     want = _probabilities(q, k[:, :, others], False) @ v[:, :, others].double()
     _same(o, want)
     assert bool(torch.isfinite(lse).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("small", [1e-20, 1e-30, 3e-33])
+@pytest.mark.parametrize("large", [3.4e38, math.inf])
+def test_small_values_beside_large_ones(large, small, D):
+    """What has been split a second time, into truncated pieces, is as accurate relative to itself, however small.  (The products of pieces that are left out all
+    have the sign of the whole then, and take up to 2^-20 of it; the third pieces of 3e-33 are the smallest numbers that a bf16 has.)"""
+    from tinytorch_b200 import op
+    q, k, v, g = _tensors(140, 150, D)
+    v[0, 0, 11, 1] = large
+    v[0, 0, :, 2] = small * (1 + torch.rand(150, device="cuda"))
+    g[1, 1, 7, 3] = large
+    g[1, 1, :, 4] = small * (1 + torch.rand(140, device="cuda"))
+    o, lse = op.sdpAttentionFwd(q, k, v)
+    p = _probabilities(q, k, False)
+    want = (p @ v.double())[0, 0, :, 2]
+    assert bool(((o[0, 0, :, 2].double() - want).abs() <= TOL_REL_FP32 * want).all())
+    v[0, 0, 11, 1] = 0.0
+    o, lse = op.sdpAttentionFwd(q, k, v)
+    dv = op.sdpAttentionBwd(g, q, k, v, o, lse)[2]
+    want = (p.transpose(2, 3) @ g.double())[1, 1, :, 4]
+    assert bool(((dv[1, 1, :, 4].double() - want).abs() <= TOL_REL_FP32 * want).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("exponent,bits", [(-100, 23), (-108, 23), (-115, 18), (-120, 13), (-124, 9)])
+def test_how_accurate_small_values_are(exponent, bits, D):
+    """One key: O is V.  A float is the sum of its pieces, exactly, down to 2^-110; below, the last piece is a multiple of 2^-133 and the
+    value is off by half of that at most, 2^(-134 - exponent) of itself."""
+    from tinytorch_b200 import op
+    q, k, v, g = _tensors(40, 1, D)
+    v = (1 + torch.rand_like(v)) * 2.0 ** exponent
+    o, lse = op.sdpAttentionFwd(q, k, v)
+    assert bool(((o - v).abs().double() <= 2.0 ** -bits * v.double()).all())
+    dv = op.sdpAttentionBwd(v.expand(2, 2, 40, D).contiguous(), q, k, v, o, lse)[2]
+    want = 40 * v.double()
+    assert bool(((dv - want).abs() <= (2.0 ** -bits + TOL_REL_FP32) * want).all())

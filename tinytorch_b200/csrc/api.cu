@@ -158,6 +158,93 @@ size_t append_bytes(int dtype, int B, int Hq, int Hkv, int D) {
 }
 }  // namespace
 
+// The backward, and how the fp32 one comes to dQ: as planned, as the selftest says, or not at all (kAsked: the plan is asked for).
+enum BwdPath { kPlanned, kAsked, kRecompute, kStore };
+static int bwd_call(const tt_attn_bwd_params* p, BwdPath path, int32_t* planned) {
+  if (!p) return TT_ATTN_ERR_NULL;
+  const bool v2 = p->struct_size == sizeof(tt_attn_bwd_params);
+  if (!v2 && p->struct_size != offsetof(tt_attn_bwd_params, mask)) return TT_ATTN_ERR_STRUCT;
+  if (int rc = check_common(p->dtype, p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) return rc;
+  if (!p->q || !p->k || !p->v || !p->o || !p->d_o || !p->lse) return TT_ATTN_ERR_NULL;
+  if (path != kPlanned && p->dtype != TT_ATTN_F32) return TT_ATTN_ERR_DTYPE;
+  if (path == kStore && !(p->dq && (p->dk || p->dv))) return TT_ATTN_ERR_SHAPE;
+  if (path == kAsked) *planned = 0;
+  if (!p->dq && !p->dk && !p->dv) return TT_ATTN_OK;
+  const size_t es = elem_size(p->dtype);
+  BwdArgs a{};
+  a.q = p->q, a.k = p->k, a.v = p->v, a.o = p->o, a.d_o = p->d_o, a.lse = p->lse;
+  a.dq = p->dq, a.dk = p->dk, a.dv = p->dv;
+  a.qs = dense_or(p->q_strides, p->Hq, p->Lq, p->D);
+  a.ks = dense_or(p->k_strides, p->Hkv, p->Skv, p->D);
+  a.vs = dense_or(p->v_strides, p->Hkv, p->Skv, p->D);
+  a.os = dense_or(p->o_strides, p->Hq, p->Lq, p->D);
+  a.dos = dense_or(p->do_strides, p->Hq, p->Lq, p->D);
+  a.dqs = dense_or(p->dq_strides, p->Hq, p->Lq, p->D);
+  a.dks = dense_or(p->dk_strides, p->Hkv, p->Skv, p->D);
+  a.dvs = dense_or(p->dv_strides, p->Hkv, p->Skv, p->D);
+  const void* ptrs[] = {p->q, p->k, p->v, p->o, p->d_o, p->dq, p->dk, p->dv, p->lse};
+  for (const void* q : ptrs)
+    if (!aligned16(q)) return TT_ATTN_ERR_ALIGN;
+  const Str3* sts[] = {&a.qs, &a.ks, &a.vs, &a.os, &a.dos, &a.dqs, &a.dks, &a.dvs};
+  for (const Str3* s : sts)
+    if (!strides_ok(*s, es)) return TT_ATTN_ERR_ALIGN;
+  a.B = p->B, a.Hq = p->Hq, a.Hkv = p->Hkv, a.Lq = p->Lq, a.Skv = p->Skv;
+  if (p->is_causal < 0 || p->is_causal > TT_ATTN_CAUSAL_BOTTOM_RIGHT) return TT_ATTN_ERR_SHAPE;
+  a.causal = p->is_causal;
+  a.scale = p->scale;
+  a.kv_lens = p->kv_lens;
+  a.status = p->status;
+  if (v2)
+    if (int rc = take_mask(p->mask, p->mask_kind, p->mask_strides, &a.mask)) return rc;
+  DeviceGuard guard(p->device);
+  if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
+  Workspace ws;
+  // delta | dQ accumulator | shares of dK / dV | work counter and, if they fit, a padding mask's lengths; fp32: delta | dS | rows' maxima and sums
+  const size_t rows = static_cast<size_t>(p->B) * p->Hq * p->Lq, delta = round256(rows * sizeof(float));
+  const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
+  size_t need = delta, part = 0;
+  bool lens = false;
+  // fp32: dS tiles on their way from dK / dV to dQ, where dQ and at least one of the others are asked for and there is room
+  size_t ds = p->dtype == TT_ATTN_F32 && p->dq && (p->dk || p->dv) ? round256(bwd_ds_bytes(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) : 0;
+  if (path == kStore) ds = round256(static_cast<size_t>(bwd_ds_bytes_of(p->B, p->Hq, p->Lq, p->Skv)));
+  if (path == kRecompute || delta + ds > room) ds = 0;
+  if (path == kStore && ds == 0) return TT_ATTN_ERR_WORKSPACE;
+  // ... and, with an additive mask, maxima and sums of the rows whose log-sum-exp is too large to say both
+  size_t stats = p->dtype == TT_ATTN_F32 && a.mask.ptr && a.mask.kind != TT_ATTN_MASK_BOOL ? round256(rows * sizeof(float2)) : 0;
+  if (delta + ds + stats > room) stats = 0;
+  if (p->dtype != TT_ATTN_F32) {
+    // a buffer that is too small for the division (a small batch is divided further than a large one): fewer shares
+    a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
+    while (a.parts > 1 && delta + accum + round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D)) + 256 > room) --a.parts;
+    part = round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D));
+    need = delta + accum + part;
+    lens = mask_lens_fit(a.mask, a.causal, p->B, room, need);
+    need += lens ? round256(scratch_words(p->B) * sizeof(int)) : 256;
+  }
+  if (path == kAsked) {
+    *planned = ds > 0 && bwd_f32_takes_ds(p->D, a, p->device);
+    return TT_ATTN_OK;
+  }
+  if (ds + stats == 0 || ws.acquire(need + ds + stats, p->workspace, p->workspace_bytes, p->alloc, p->device) != TT_ATTN_OK) {
+    ds = stats = 0;  // (an allocator that has no more than before)
+    if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
+  }
+  a.delta = static_cast<float*>(ws.ptr);
+  if (ds > 0) a.ds = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
+  if (stats > 0) a.row_stats = reinterpret_cast<float2*>(static_cast<char*>(ws.ptr) + delta + ds);
+  if (p->dtype != TT_ATTN_F32) {
+    a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
+    a.dkv_part = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta + accum);
+    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + delta + accum + part);
+    a.mask_lens = lens ? a.sched + 1 : nullptr;
+  }
+  if (path == kStore && ds == 0) return TT_ATTN_ERR_WORKSPACE;
+  cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_f32(p->D, a, path == kStore, p->device, stream)
+                                          : launch_bwd_tc(p->dtype, p->D, a, p->device, stream);
+  return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
+}
+
 extern "C" {
 
 size_t tt_attn_workspace_bytes(int kind, int dtype, int B, int Hq, int Hkv, int Lq, int Skv, int D) {
@@ -230,79 +317,12 @@ int tt_attn_fwd(const tt_attn_fwd_params* p) {
   return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
 }
 
-int tt_attn_bwd(const tt_attn_bwd_params* p) {
-  if (!p) return TT_ATTN_ERR_NULL;
-  const bool v2 = p->struct_size == sizeof(tt_attn_bwd_params);
-  if (!v2 && p->struct_size != offsetof(tt_attn_bwd_params, mask)) return TT_ATTN_ERR_STRUCT;
-  if (int rc = check_common(p->dtype, p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) return rc;
-  if (!p->q || !p->k || !p->v || !p->o || !p->d_o || !p->lse) return TT_ATTN_ERR_NULL;
-  if (!p->dq && !p->dk && !p->dv) return TT_ATTN_OK;
-  const size_t es = elem_size(p->dtype);
-  BwdArgs a{};
-  a.q = p->q, a.k = p->k, a.v = p->v, a.o = p->o, a.d_o = p->d_o, a.lse = p->lse;
-  a.dq = p->dq, a.dk = p->dk, a.dv = p->dv;
-  a.qs = dense_or(p->q_strides, p->Hq, p->Lq, p->D);
-  a.ks = dense_or(p->k_strides, p->Hkv, p->Skv, p->D);
-  a.vs = dense_or(p->v_strides, p->Hkv, p->Skv, p->D);
-  a.os = dense_or(p->o_strides, p->Hq, p->Lq, p->D);
-  a.dos = dense_or(p->do_strides, p->Hq, p->Lq, p->D);
-  a.dqs = dense_or(p->dq_strides, p->Hq, p->Lq, p->D);
-  a.dks = dense_or(p->dk_strides, p->Hkv, p->Skv, p->D);
-  a.dvs = dense_or(p->dv_strides, p->Hkv, p->Skv, p->D);
-  const void* ptrs[] = {p->q, p->k, p->v, p->o, p->d_o, p->dq, p->dk, p->dv, p->lse};
-  for (const void* q : ptrs)
-    if (!aligned16(q)) return TT_ATTN_ERR_ALIGN;
-  const Str3* sts[] = {&a.qs, &a.ks, &a.vs, &a.os, &a.dos, &a.dqs, &a.dks, &a.dvs};
-  for (const Str3* s : sts)
-    if (!strides_ok(*s, es)) return TT_ATTN_ERR_ALIGN;
-  a.B = p->B, a.Hq = p->Hq, a.Hkv = p->Hkv, a.Lq = p->Lq, a.Skv = p->Skv;
-  if (p->is_causal < 0 || p->is_causal > TT_ATTN_CAUSAL_BOTTOM_RIGHT) return TT_ATTN_ERR_SHAPE;
-  a.causal = p->is_causal;
-  a.scale = p->scale;
-  a.kv_lens = p->kv_lens;
-  a.status = p->status;
-  if (v2)
-    if (int rc = take_mask(p->mask, p->mask_kind, p->mask_strides, &a.mask)) return rc;
-  DeviceGuard guard(p->device);
-  if (!guard.ok) return TT_ATTN_ERR_NO_DEVICE;
-  Workspace ws;
-  // delta | dQ accumulator | shares of dK / dV | work counter and, if they fit, a padding mask's lengths; fp32: delta | dS | rows' maxima and sums
-  const size_t rows = static_cast<size_t>(p->B) * p->Hq * p->Lq, delta = round256(rows * sizeof(float));
-  const size_t accum = round256(rows * p->D * sizeof(float)), room = p->workspace ? p->workspace_bytes : SIZE_MAX;
-  size_t need = delta, part = 0;
-  bool lens = false;
-  // fp32: dS tiles on their way from dK / dV to dQ, where dQ and at least one of the others are asked for and there is room
-  size_t ds = p->dtype == TT_ATTN_F32 && p->dq && (p->dk || p->dv) ? round256(bwd_ds_bytes(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D)) : 0;
-  if (delta + ds > room) ds = 0;
-  // ... and, with an additive mask, maxima and sums of the rows whose log-sum-exp is too large to say both
-  size_t stats = p->dtype == TT_ATTN_F32 && a.mask.ptr && a.mask.kind != TT_ATTN_MASK_BOOL ? round256(rows * sizeof(float2)) : 0;
-  if (delta + ds + stats > room) stats = 0;
-  if (p->dtype != TT_ATTN_F32) {
-    // a buffer that is too small for the division (a small batch is divided further than a large one): fewer shares
-    a.parts = bwd_parts(p->B, p->Hq, p->Hkv, p->Lq, p->Skv, p->D, p->is_causal != 0);
-    while (a.parts > 1 && delta + accum + round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D)) + 256 > room) --a.parts;
-    part = round256(bwd_part_bytes_of(a.parts, p->B, p->Hkv, p->Skv, p->D));
-    need = delta + accum + part;
-    lens = mask_lens_fit(a.mask, a.causal, p->B, room, need);
-    need += lens ? round256(scratch_words(p->B) * sizeof(int)) : 256;
-  }
-  if (ds + stats == 0 || ws.acquire(need + ds + stats, p->workspace, p->workspace_bytes, p->alloc, p->device) != TT_ATTN_OK) {
-    ds = stats = 0;  // (an allocator that has no more than before)
-    if (int rc = ws.acquire(need, p->workspace, p->workspace_bytes, p->alloc, p->device)) return rc;
-  }
-  a.delta = static_cast<float*>(ws.ptr);
-  if (ds > 0) a.ds = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
-  if (stats > 0) a.row_stats = reinterpret_cast<float2*>(static_cast<char*>(ws.ptr) + delta + ds);
-  if (p->dtype != TT_ATTN_F32) {
-    a.dq_accum = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta);
-    a.dkv_part = reinterpret_cast<float*>(static_cast<char*>(ws.ptr) + delta + accum);
-    a.sched = reinterpret_cast<int*>(static_cast<char*>(ws.ptr) + delta + accum + part);
-    a.mask_lens = lens ? a.sched + 1 : nullptr;
-  }
-  cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-  cudaError_t e = p->dtype == TT_ATTN_F32 ? launch_bwd_f32(p->D, a, p->device, stream)
-                                          : launch_bwd_tc(p->dtype, p->D, a, p->device, stream);
-  return e == cudaSuccess ? TT_ATTN_OK : launch_failed(e);
+int tt_attn_bwd(const tt_attn_bwd_params* p) { return bwd_call(p, kPlanned, nullptr); }
+
+int tt_attn_bwd_selftest(const tt_attn_bwd_params* p, int32_t path, int32_t* planned) {
+  if (path < -1 || path > 1) return TT_ATTN_ERR_SHAPE;
+  if (path < 0 && !planned) return TT_ATTN_ERR_NULL;
+  return bwd_call(p, path < 0 ? kAsked : (path == 0 ? kRecompute : kStore), planned);
 }
 
 int tt_attn_decode(const tt_attn_decode_params* p) {

@@ -1044,6 +1044,28 @@ Plan plan_of(const Items& x, const Items& y, double item_us, double merge_us, in
   return best;
 }
 
+// dQ by CTAs of its own, in one launch with those of dK and dV, or of their dS in another.
+struct Plans {
+  Plan recomputed, stored, dq;
+  bool take_ds;
+};
+Plans plans_of(int D, const BwdArgs& a, int device) {
+  const double heads = static_cast<double>(a.B) * a.Hkv, rows = static_cast<double>(a.Lq) * (a.Hq / a.Hkv);
+  const double key_walk = std::ceil(rows / BN), query_walk = std::ceil(static_cast<double>(a.Skv) / BN);
+  const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.55 : 1.0;  // of all tiles
+  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, D == 64 ? 3.1 : 8.5};
+  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, D == 64 ? 2.4 : 5.3};
+  const double item = D == 64 ? 6.5 : 18.0, merge = 6.5;
+  const Items none{0.0, 0.0, 0.0, 0.0};
+  Plans p{plan_of(keys, queries, item, merge, device), plan_of(keys, none, item, merge, device), {1, 0.0}, false};
+  // The pass that reads dS, where it is the faster, with 7 us for a launch and for dS (D = 128: wherever there is dS).  D = 64: 4 x 8 x 500 67 -> 62 us, 6 x 8 x 333 66 -> 59, 2 x 16/2 x 700 causal
+  // 117 -> 86; not for causal 3 x 1000 (33; 37) and 2 x 8/2 x 130 on 1500 (39; 43).  D = 128: 2 x 8/2 x 130 on 1500 79 -> 60, 4 x 8 x 500 143 -> 124.
+  queries.step_us = D == 64 ? 1.2 : 1.8;
+  p.dq = plan_of(queries, none, 5.0, 3.0, device);
+  p.take_ds = D == 128 || p.stored.us + p.dq.us + 7.0 < p.recomputed.us;
+  return p;
+}
+
 template <int D>
 cudaError_t launch_d(const BwdArgs& a, int cluster, int device, cudaStream_t stream) {
   if (!a.mask.ptr) return launch_t<D, kNoMask>(a, cluster, device, stream);
@@ -1063,39 +1085,29 @@ cudaError_t launch_dq(const BwdArgs& a, int cluster, int device, cudaStream_t st
 
 }  // namespace
 
+constexpr double kPairBytes = BN * BN * sizeof(float);
+double bwd_ds_bytes_of(int B, int Hq, int Lq, int Skv) {
+  return static_cast<double>(B) * Hq * ((Lq + BN - 1) / BN) * ((Skv + BN - 1) / BN) * kPairBytes;
+}
 // Where there is room for dS, dQ is one product more instead of three, by a kernel of its own: 16 KB of scratch for 64 queries and 64
 // keys, written and read once.  Up to 192 MB of it; and from as many pairs on as make up for the launch.
 size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (B <= 0 || Hq <= 0 || Lq <= 0 || Skv <= 0) return 0;
-  const double pairs = static_cast<double>(B) * Hq * ((Lq + BN - 1) / BN) * ((Skv + BN - 1) / BN), bytes = pairs * BN * BN * sizeof(float);
-  return bytes <= 192e6 && pairs >= (D == 64 ? 600 : 300) ? static_cast<size_t>(bytes) : 0;
+  const double bytes = bwd_ds_bytes_of(B, Hq, Lq, Skv);
+  return bytes <= 192e6 && bytes >= (D == 64 ? 600 : 300) * kPairBytes ? static_cast<size_t>(bytes) : 0;
 }
 
-cudaError_t launch_bwd_f32(int D, const BwdArgs& args, int device, cudaStream_t stream) {
+bool bwd_f32_takes_ds(int D, const BwdArgs& a, int device) { return plans_of(D, a, device).take_ds; }
+
+cudaError_t launch_bwd_f32(int D, const BwdArgs& args, bool take_ds, int device, cudaStream_t stream) {
   BwdArgs a = args;
-  const double heads = static_cast<double>(a.B) * a.Hkv, rows = static_cast<double>(a.Lq) * (a.Hq / a.Hkv);
-  const double key_walk = std::ceil(rows / BN), query_walk = std::ceil(static_cast<double>(a.Skv) / BN);
-  const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.55 : 1.0;  // of all tiles
-  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, D == 64 ? 3.1 : 8.5};
-  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, D == 64 ? 2.4 : 5.3};
-  const double item = D == 64 ? 6.5 : 18.0, merge = 6.5;
-  const Items none{0.0, 0.0, 0.0, 0.0};
-  Plan plan = plan_of(keys, queries, item, merge, device), dq{1, 0.0};
-  if (a.ds) {
-    // The pass that reads dS, where it is the faster, with 7 us for a launch and for dS (D = 128: wherever there is dS).  D = 64: 4 x 8 x 500 67 -> 62 us, 6 x 8 x 333 66 -> 59, 2 x 16/2 x 700 causal
-    // 117 -> 86; not for causal 3 x 1000 (33; 37) and 2 x 8/2 x 130 on 1500 (39; 43).  D = 128: 2 x 8/2 x 130 on 1500 79 -> 60, 4 x 8 x 500 143 -> 124.
-    queries.step_us = D == 64 ? 1.2 : 1.8;
-    const Plan store = plan_of(keys, none, item, merge, device);
-    dq = plan_of(queries, none, 5.0, 3.0, device);
-    if (D == 128 || store.us + dq.us + 7.0 < plan.us)
-      plan = store;
-    else
-      a.ds = nullptr;
-  }
+  const Plans plans = plans_of(D, a, device);
+  if (!take_ds && !plans.take_ds) a.ds = nullptr;
+  const int cluster = a.ds ? plans.stored.cluster : plans.recomputed.cluster;
   cudaError_t e = launch_bwd_delta(TT_ATTN_F32, D, a, stream);
-  if (e == cudaSuccess) e = D == 64 ? launch_d<64>(a, plan.cluster, device, stream) : launch_d<128>(a, plan.cluster, device, stream);
+  if (e == cudaSuccess) e = D == 64 ? launch_d<64>(a, cluster, device, stream) : launch_d<128>(a, cluster, device, stream);
   if (e != cudaSuccess || !a.ds) return e;
-  return D == 64 ? launch_dq<64>(a, dq.cluster, device, stream) : launch_dq<128>(a, dq.cluster, device, stream);
+  return D == 64 ? launch_dq<64>(a, plans.dq.cluster, device, stream) : launch_dq<128>(a, plans.dq.cluster, device, stream);
 }
 
 }  // namespace ttattn

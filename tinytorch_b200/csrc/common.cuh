@@ -136,7 +136,8 @@ struct DecodeArgs {
 // Each returns a cudaError_t from the launch (no synchronisation).
 cudaError_t launch_fwd_tc(int dtype, int D, const FwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_fwd_f32(int D, const FwdArgs& a, int device, cudaStream_t stream);
-cudaError_t launch_bwd_f32(int D, const BwdArgs& a, int device, cudaStream_t stream);
+// (take_ds: dQ of a.ds, if it is there, as planned or in any case)
+cudaError_t launch_bwd_f32(int D, const BwdArgs& a, bool take_ds, int device, cudaStream_t stream);
 // rowsum(dO o O) into a.delta only (first step of every backward)
 cudaError_t launch_bwd_delta(int dtype, int D, const BwdArgs& a, cudaStream_t stream);
 // Work items per key tile of the tensor-core backward, and the workspace they need beside dq_accum (0 for one item)
@@ -145,6 +146,8 @@ size_t bwd_part_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
 size_t bwd_part_bytes_of(int parts, int B, int Hkv, int Skv, int D);
 // dS of the fp32 backward (0: dQ recomputes it; a caller without room for it gets that too)
 size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D);
+double bwd_ds_bytes_of(int B, int Hq, int Lq, int Skv);  // ... of any size
+bool bwd_f32_takes_ds(int D, const BwdArgs& a, int device);  // whether the call makes dQ of it, given room
 // fp16 / bf16 backward on the tensor cores; needs a.delta, a.dq_accum and what a.parts asks for
 cudaError_t launch_bwd_tc(int dtype, int D, const BwdArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_decode(int dtype, int D, const DecodeArgs& a, cudaStream_t stream);
