@@ -596,12 +596,12 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
       const uint32_t b2 = ptx::smem_desc_lo(base + LY::kB2, 16);
       constexpr int kLbo = LY::kWide ? TB::kPlane : TB::kBlock;
       const uint32_t b1_mn = ptx::smem_desc_lo(base + LY::kB1, kLbo), b2_mn = ptx::smem_desc_lo(base + LY::kB2, kLbo);
-      constexpr Sums kSums = LY::kWide ? kLeadApart : kOneSum;
+      constexpr Sums kSums = LY::kWide ? kLeadApart : kOneSum, kSumsT = LY::kWide ? kTwoSums : kOneSum;
       // product of a tile: A's planes from TMEM region `region`, B MN-major
       auto issue_t = [&](uint32_t region, uint32_t b_mn) {
 #pragma unroll 1  // (all products at once: the addresses do not fit this warp's registers)
-        for (int p = 0; p < steps_of(kSums); ++p) {
-          const Step st = step_of(kSums, p);
+        for (int p = 0; p < steps_of(kSumsT); ++p) {
+          const Step st = step_of(kSumsT, p);
           const uint32_t d = tmem + LY::kT + (st.second ? D : 0), ap = tmem + region + LY::plane_at(st.a, 0), bp = b_mn + st.b * kPB;
           const uint32_t idesc = st.two ? kIdescT2 : kIdescT1;
 #pragma unroll
@@ -980,10 +980,10 @@ __global__ void __launch_bounds__(kDqThreads, 1) bwd_f32_dq_kernel(const BwdArgs
         const uint32_t at = done + t, two = at & 1;
         if (!uwait(&ctl->b_full[two], at >> 1) || !uwait(&ctl->a_full[two], at >> 1)) break;
         ptx::tc_fence_after();
-        constexpr Sums kSums = LY::kWide ? kLeadApart : kOneSum;
+        constexpr Sums kSumsT = LY::kWide ? kTwoSums : kOneSum;
 #pragma unroll 1
-        for (int p = 0; p < steps_of(kSums); ++p) {
-          const Step st = step_of(kSums, p);
+        for (int p = 0; p < steps_of(kSumsT); ++p) {
+          const Step st = step_of(kSumsT, p);
           const uint32_t d = tmem + LY::kT + two * LY::kBufT + (st.second ? D : 0), ap = tmem + LY::kA + two * LY::kBufA + st.a * 32;
           const uint32_t bp = b_mn + two * (TB::kBytes >> 4) + st.b * kPB, idesc = st.two ? kIdesc2 : kIdesc1;
 #pragma unroll
@@ -1020,9 +1020,8 @@ cudaError_t launch_t(const BwdArgs& a, int cluster, int device, cudaStream_t str
 }
 
 // CTAs per cluster, that share a walk: what is expected to take the least time, with one CTA to an SM, items whose walk takes `step_us` a
-// tile and whose rest `item_us`.  `walk` and `mean`: the longest and the average walk in tiles.  Constants from a sweep of 21 shapes with
-// 1, 2, 4 and 8.  Measured, us, undivided -> chosen: D = 64, causal 3 x 1000 58 -> 33 (3), 2 x 16/2 heads x 700 causal 314 -> 86 (5), 2 x 4 x 128
-// 14.6 (2: 17.5); D = 128, 8/1 heads x 33 on 1000 104 -> 26 (8), 2 x 8/2 x 130 on 1500 111 -> 60.
+// tile and whose rest `item_us`.  `walk` and `mean`: the longest and the average walk in tiles.  Measured, us, undivided -> chosen: D = 64,
+// causal 3 x 1000 58 -> 32 (3), 2 x 16/2 heads x 700 causal 314 -> 85 (6), 2 x 4 x 128 14.6 (2: 17.1); D = 128, 8/1 heads x 33 on 1000 104 -> 25 (8).
 struct Items {
   double count, walk, mean, step_us;
 };
@@ -1044,7 +1043,10 @@ Plan plan_of(const Items& x, const Items& y, double item_us, double merge_us, in
   return best;
 }
 
-// dQ by CTAs of its own, in one launch with those of dK and dV, or of their dS in another.
+// dQ by CTAs of its own, in one launch with those of dK and dV, or of their dS in another: what is expected to take less.  The constants are fitted to 22
+// shapes, each both ways; the choice is right in all of them.  us, recomputed and stored: D = 64, 4 x 8 heads x 500 63.0 and 58.2, causal 45.9 and 56.3, 16 x 16 x 128
+// causal 55.6 and 49.1, 3 x 1000 causal 32.6 and 40.0, 2 x 16/2 x 700 causal 124 and 85, 2 x 8/2 x 130 on 1500 39.2 and 43.1; D = 128, 4 x 8 x 500 123 and 109, causal
+// 91 and 104 (it was stored wherever there was room: 108 -> 91), 3 x 1000 causal 52 and 62, 4 x 8 x 200 43 and 47, 8 x 8 x 512 252 and 221, 1 x 16/4 x 2000 on 300 332 and 189.
 struct Plans {
   Plan recomputed, stored, dq;
   bool take_ds;
@@ -1053,16 +1055,15 @@ Plans plans_of(int D, const BwdArgs& a, int device) {
   const double heads = static_cast<double>(a.B) * a.Hkv, rows = static_cast<double>(a.Lq) * (a.Hq / a.Hkv);
   const double key_walk = std::ceil(rows / BN), query_walk = std::ceil(static_cast<double>(a.Skv) / BN);
   const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.55 : 1.0;  // of all tiles
-  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, D == 64 ? 3.1 : 8.5};
-  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, D == 64 ? 2.4 : 5.3};
-  const double item = D == 64 ? 6.5 : 18.0, merge = 6.5;
+  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, D == 64 ? 3.25 : 6.9};
+  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, D == 64 ? 1.87 : 4.6};
+  const double item = D == 64 ? 9.54 : 14.8, merge = D == 64 ? 4.0 : 3.0;
   const Items none{0.0, 0.0, 0.0, 0.0};
   Plans p{plan_of(keys, queries, item, merge, device), plan_of(keys, none, item, merge, device), {1, 0.0}, false};
-  // The pass that reads dS, where it is the faster, with 7 us for a launch and for dS (D = 128: wherever there is dS).  D = 64: 4 x 8 x 500 67 -> 62 us, 6 x 8 x 333 66 -> 59, 2 x 16/2 x 700 causal
-  // 117 -> 86; not for causal 3 x 1000 (33; 37) and 2 x 8/2 x 130 on 1500 (39; 43).  D = 128: 2 x 8/2 x 130 on 1500 79 -> 60, 4 x 8 x 500 143 -> 124.
-  queries.step_us = D == 64 ? 1.2 : 1.8;
-  p.dq = plan_of(queries, none, 5.0, 3.0, device);
-  p.take_ds = D == 128 || p.stored.us + p.dq.us + 7.0 < p.recomputed.us;
+  // The pass that reads dS, where the two launches take less than the one.
+  queries.step_us = D == 64 ? 1.61 : 2.35;
+  p.dq = plan_of(queries, none, D == 64 ? 5.4 : 7.9, 3.0, device);
+  p.take_ds = p.stored.us + p.dq.us < p.recomputed.us;
   return p;
 }
 
@@ -1090,7 +1091,9 @@ double bwd_ds_bytes_of(int B, int Hq, int Lq, int Skv) {
   return static_cast<double>(B) * Hq * ((Lq + BN - 1) / BN) * ((Skv + BN - 1) / BN) * kPairBytes;
 }
 // Where there is room for dS, dQ is one product more instead of three, by a kernel of its own: 16 KB of scratch for 64 queries and 64
-// keys, written and read once.  Up to 192 MB of it; and from as many pairs on as make up for the launch.
+// keys, written and read once.  Up to 192 MB of it, and from as many pairs of tiles on as storing can pay for (whether it does is the plan's, which knows
+// the device and the causal form).  us, recomputed and stored: D = 64, 256 pairs (2 x 8 x 256 causal) 21.7 and 26.7, 512 (4 x 8 x 200) 24.8 and 33.8, 864 (3 x 8 x 333)
+// 31.7 and 37.1, 1024 (16 x 16 x 128 causal) 55.6 and 49.1; D = 128, 256 33.3 and 36.1, 512 (32 x 4 x 100) 48.4 and 42.0, 576 (8 x 8 x 130 causal) 54.2 and 47.6.
 size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (B <= 0 || Hq <= 0 || Lq <= 0 || Skv <= 0) return 0;
   const double bytes = bwd_ds_bytes_of(B, Hq, Lq, Skv);

@@ -10,7 +10,7 @@
 //                   D = 64: O, dQ, dK, dV                                D = 128
 //   N(0, 1)           1.9 (3.5)  3.2 (3.8)  3.2 (4.5)  2.9 (4.3)           2.5 (4.7)  3.8 (4.2)  3.8 (5.6)  3.2 (5.4)
 //   ... 3 Q, 3 K      3.8 (7.0)  11.3 (17)  11.3 (17)  10.5 (13.5)         5.6 (9.2)  18 (21)    18 (21)    16.1 (14.6)
-//   [0.5, 1.5]        0.8 (1.7)  dQ is 0 but for errors  1.2 (2.2)  0.7 (1.8)      0.9 (3.3)             2.8 (4.9)  2.7 (4.5)
+//   [0.5, 1.5]        0.8 (1.7)  dQ is 0 but for errors  1.1 (2.2)  0.6 (1.8)      0.9 (3.3)             2.8 (4.9)  2.7 (4.5)
 //   Q, K in -2 .. 2   1.6 (3.2)  4.8 (6.9)  4.7 (6.8)  4.6 (5.7)           1.5 (3.4)  8.3 (10.7) 8.3 (10.8) 8.1 (9.2)
 // Six bf16 products at 1.63 PFLOP/s are 271 TFLOP/s of fp32, 3.7 times the FMA pipes' 74.
 //
@@ -38,9 +38,10 @@ static_assert(piece_a(0) == 2 && piece_b(0) == 0 && piece_a(1) == 1 && piece_b(1
 // How the products of a tile are summed.  kOneSum: in one accumulator.  The others have a second one beside it, and an MMA whose second
 // operand is the two first planes as one of twice the rows fills both.  kTwoSums: (l, h), (m, h), (h, h) in the first, the rest in the second.
 // kLeadApart: (h, h) alone in the first.  Its truncations are those of a sum of the leading pieces alone then, none where these are few or
-// fit 24 bits, and the same whichever operand comes first, in the forward and in the backward.  Two MMAs of 64 columns in the place of one of 128: D = 64 forward
-// 18.1 -> 18.4 us (4 x 8 heads x 500), backward 58.8 -> 59.3; relative error of dV against 64 bits, scores of standard deviation 9, 18.6e-7 -> 13.0e-7
-// (fp32 FMAs 13.5e-7), of dK, operands of [0.5, 1.5], 2.8e-7 -> 1.5e-7 (2.2e-7).
+// fit 24 bits, and the same whichever operand comes first, in the forward and in the backward.  D = 64, for scores, dP and the forward's O.  Two MMAs of
+// 64 columns in the place of one of 128: forward 18.1 -> 18.4 us (4 x 8 heads x 500), backward 58.8 -> 59.1; relative error of dV against 64 bits, scores of standard
+// deviation 9, 18.6e-7 -> 13.0e-7 (fp32 FMAs 13.5e-7), of dK, operands of [0.5, 1.5], 2.8e-7 -> 1.1e-7 (2.2e-7; scores alone so, and dP not: 12.7e-7).  dV, dK and dQ
+// are as exact with either.
 enum Sums { kOneSum, kTwoSums, kLeadApart };
 struct Step {
   uint32_t a, b;  // pieces
