@@ -483,9 +483,6 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           ptx::mbar_arrive(&ctl->m_full);
         } else if constexpr (MASK == kAddMask) {
           const float* any = reinterpret_cast<const float*>(a.mask.ptr);
-          auto copy4 = [&](uint32_t dst, const float* p, bool in) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(in ? p : any), "r"(in ? 4 : 0) : "memory");
-          };
           // every `step`-th of the rows from r0 on, `count` of them, without a division for each
           auto each_row = [&](int r0, int step, int count, auto f) {
             int r = r0, g = rw.head(r0);
@@ -509,9 +506,12 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
                 ptx::cp_async16(to + e * BM * 4 + lane * 16, in ? any + p + key : any, in ? left * 4 : 0);
               });
             } else {
+              const int key = own0 + lane, last = kv_len - own0 - lane;  // (keys beyond the length are left as they are: they are hidden)
               each_row(col0 + w * kCols, 1, kCols, [&](int e, bool in, int64_t p) {
-#pragma unroll
-                for (int j = lane; j < BM; j += 32) copy4(to + (e * BM + j) * 4, any + p + own0 + j, in && own0 + j < kv_len);
+                const uint32_t dst = to + (e * BM + lane) * 4;
+                const float* from = in ? any + p + key : any;
+                copies4(dst, from, in, last > 0, last > 32);
+                copies4(dst + 256, from + 64, in, last > 64, last > 96);
               });
             }
           } else {  // [row][64], neighbouring vectors exchanged by row; 32 rows a warp
@@ -525,9 +525,8 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
             } else {
               each_row(own0 + w * kOwn, 1, kOwn, [&](int e, bool in, int64_t p) {
                 const int rr = w * kOwn + e;
-#pragma unroll
-                for (int j = lane; j < BN; j += 32)
-                  copy4(base + LY::kM + rr * BN * 4 + (((j / 4) ^ (rr & 7)) << 4) + (j % 4) * 4, any + p + col0 + j, in && col0 + j < kv_len);
+                copies4(base + LY::kM + rr * BN * 4 + (((lane / 4) ^ (rr & 7)) << 4) + (lane % 4) * 4, in ? any + p + col0 + lane : any, in,
+                        col0 + lane < kv_len, col0 + lane + 32 < kv_len);
               });
             }
           }

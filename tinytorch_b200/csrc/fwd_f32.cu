@@ -575,10 +575,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
                 ptx::cp_async16(mask_at + r * BN * 4 + ((ch ^ (r & 7)) << 4), in ? any + p + ch * 4 : any, in ? left * 4 : 0);
               });
             } else {
+              // (keys beyond the length are left as they are: they are hidden)
+              const bool in0 = col0 + lane < kv_len, in1 = col0 + lane + 32 < kv_len;
               each_row(1, 64, [&](int r, bool in, int64_t p) {
-#pragma unroll
-                for (int j = lane; j < BN; j += 32)
-                  copy4(mask_at + r * BN * 4 + (((j / 4) ^ (r & 7)) << 4) + (j % 4) * 4, any + p + j, in && col0 + j < kv_len);
+                const uint32_t to = mask_at + r * BN * 4 + (((lane / 4) ^ (r & 7)) << 4) + (lane % 4) * 4;
+                copies4(to, in ? any + p + lane : any, in, in0, in1);
               });
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(ptx::smem_u32(&ctl->m_full[stage])) : "memory");
