@@ -468,9 +468,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
 #pragma unroll 4
           for (int i = 0; i < 16; ++i) {
             const uint32_t y = 4 * i + 4 < end ? __ldg(words + i + 1) : 0;
-            uint32_t v = __funnelshift_r(x, y, 8 * mis);
-            v |= v >> 4, v |= v >> 2, v = (v | v >> 1) & 0x01010101u;  // whether a byte is not zero
-            v = (v * 0x01020408u >> 24 & 15) << (4 * (i % 8));
+            const uint32_t v = mask_bits(x, y, mis) << (4 * (i % 8));
             two[0] |= i < 8 ? v : 0, two[1] |= i < 8 ? 0 : v;
             x = y;
           }
@@ -483,18 +481,8 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
           ptx::mbar_arrive(&ctl->m_full);
         } else if constexpr (MASK == kAddMask) {
           const float* any = reinterpret_cast<const float*>(a.mask.ptr);
-          // every `step`-th of the rows from r0 on, `count` of them, without a division for each
           auto each_row = [&](int r0, int step, int count, auto f) {
-            int r = r0, g = rw.head(r0);
-            int64_t p = row_at(r0);
-            const int dg = step % group;
-            const int64_t dp = step / group * a.mask.sl + dg * a.mask.sh, wrap = a.mask.sl - group * a.mask.sh;
-#pragma unroll 2
-            for (int e = 0; e < count; ++e) {
-              f(e * step, r < rows, p);
-              r += step, g += dg, p += dp;
-              if (g >= group) g -= group, p += wrap;
-            }
+            each_mask_row<2>(a.mask, group, rows, r0, rw.head(r0), row_at(r0), step, count, f);
           };
           if constexpr (KEYS) {  // [column][key], 16 columns a warp
             constexpr int kCols = BN / 4;

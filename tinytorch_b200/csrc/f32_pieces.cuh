@@ -168,6 +168,27 @@ __device__ __forceinline__ float2 exponent_base(float lse, int n) {
   return make_float2(lse == -INFINITY ? -INFINITY : whole - x, __int_as_float((127 - static_cast<int>(whole)) << 23));
 }
 
+// Four bytes of a boolean mask, from byte `mis` of two words on, as bits: whether they are not zero.
+__device__ __forceinline__ uint32_t mask_bits(uint32_t lo, uint32_t hi, int mis) {
+  uint32_t v = __funnelshift_r(lo, hi, 8 * mis);
+  v |= v >> 4, v |= v >> 2, v = (v | v >> 1) & 0x01010101u;
+  return v * 0x01020408u >> 24 & 15;
+}
+
+// Every `step`-th of a group's rows (`rows` of them) from row r on, whose head is g and whose mask begins at `at`, `count` times and without a division for each:
+// f(which of them, whether there is such a row, where its mask begins).
+template <int UNROLL, typename F>
+__device__ __forceinline__ void each_mask_row(const MaskArgs& m, int group, int rows, int r, int g, int64_t at, int step, int count, F f) {
+  const int dg = step % group;
+  const int64_t d = step / group * m.sl + dg * m.sh, wrap = m.sl - group * m.sh;
+#pragma unroll UNROLL
+  for (int e = 0; e < count; ++e) {
+    f(e * step, r < rows, at);
+    r += step, g += dg, at += d;
+    if (g >= group) g -= group, at += wrap;
+  }
+}
+
 // Two floats of a mask's row, 32 apart, global -> shared by asynchronous copies, where the key (a, b) takes part; zeros where there is no such row.  By predicates:
 // as zero-filling copies (two selects more each) 2 x 8/4 heads x 99 on 131 keys took 11.7 us forward, by branches 12.5, so 11.0; 8 x 8 x 127 12.7, 14.0, 11.0.
 __device__ __forceinline__ void copies4(uint32_t dst, const float* src, bool row, bool a, bool b) {

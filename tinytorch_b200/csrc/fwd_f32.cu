@@ -519,18 +519,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
           const uint32_t stage = at % LY::kMaskStages, use = at / LY::kMaskStages, mask_at = base + LY::kM + stage * LY::kMaskBytes;
           if (use > 0 && !uwait(&ctl->m_free[stage], use - 1)) break;
           const int64_t mask_b = b * a.mask.sb + hk * group * a.mask.sh + col0;
-          // every `step`-th row from r0 on, `count` of them, without a division for each
-          auto each_row = [&](int step, int count, auto f) {
-            int i_q = first_iq, g = first_g;
-            const int dq = step / group, dg = step % group;
-            int64_t p = mask_b + g * a.mask.sh + i_q * a.mask.sl;
-            const int64_t dp = dq * a.mask.sl + dg * a.mask.sh, wrap = a.mask.sl - group * a.mask.sh;
-#pragma unroll 8
-            for (int e = 0; e < count; ++e) {
-              f(r0 + e * step, i_q < a.Lq, p);
-              i_q += dq, g += dg, p += dp;
-              if (g >= group) g -= group, ++i_q, p += wrap;
-            }
+          auto each_row = [&](int step, int count, auto f) {  // from r0 on
+            each_mask_row<8>(a.mask, group, rows, row0 + r0, first_g, mask_b + first_g * a.mask.sh + first_iq * a.mask.sl, step, count,
+                             [&](int e, bool in, int64_t p) { f(r0 + e, in, p); });
           };
           if constexpr (MASK == kBoolMask) {
             // a row's 64 bytes to bits: the aligned words that hold them, shifted into place
@@ -546,11 +537,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
               }
               uint32_t two[2] = {0, 0};
 #pragma unroll
-              for (int i = 0; i < BN / 4; ++i) {
-                uint32_t v = __funnelshift_r(x[i], x[i + 1], 8 * mis);
-                v |= v >> 4, v |= v >> 2, v = (v | v >> 1) & 0x01010101u;  // whether a byte is not zero
-                two[i / 8] |= (v * 0x01020408u >> 24 & 15) << (4 * (i % 8));
-              }
+              for (int i = 0; i < BN / 4; ++i) two[i / 8] |= mask_bits(x[i], x[i + 1], mis) << (4 * (i % 8));
               if (same)
                 asm volatile("st.shared.v4.u32 [%0], {%1, %2, %1, %2};" ::"r"(mask_at + mt_id * 16), "r"(two[0]), "r"(two[1]) : "memory");
               else
