@@ -1030,10 +1030,12 @@ Plan plan_of(const Items& x, const Items& y, double item_us, double merge_us, in
   return best;
 }
 
-// dQ by CTAs of its own, in one launch with those of dK and dV, or of their dS in another: what is expected to take less.  The constants are fitted to 22
-// shapes, each both ways; the choice is right in all of them.  us, recomputed and stored: D = 64, 4 x 8 heads x 500 63.0 and 58.2, causal 45.9 and 56.3, 16 x 16 x 128
-// causal 55.6 and 49.1, 3 x 1000 causal 32.6 and 40.0, 2 x 16/2 x 700 causal 124 and 85, 2 x 8/2 x 130 on 1500 39.2 and 43.1; D = 128, 4 x 8 x 500 123 and 109, causal
-// 91 and 104 (it was stored wherever there was room: 108 -> 91), 3 x 1000 causal 52 and 62, 4 x 8 x 200 43 and 47, 8 x 8 x 512 252 and 221, 1 x 16/4 x 2000 on 300 332 and 189.
+// dQ by CTAs of its own, in one launch with those of dK and dV, or of their dS in another: what is expected to take less.  The constants are fitted to
+// 148 calls timed both ways (35 shapes, plain, causal, with boolean and additive masks); the choice is the faster way but for four, by 2, 3, 3 and 20 % (D = 64,
+// 3 x 1000: 40 stored, 48 as clusters for which there is no room at once).
+// us, recomputed and stored: D = 64, 4 x 8 heads x 500 63.0 and 58.2, causal 45.4 and 56.0, additive mask 83 and 77, 16 x 16 x 128 causal 55.6 and 49.1,
+// 3 x 1000 causal 31.6 and 40.2, boolean mask 50.9 and 44.1, 2 x 16/2 x 700 204 and 151 with it; D = 128, 4 x 8 x 500 123 and 109, causal 90 and 97, additive
+// mask 169 and 142, 3 x 1000 causal 52.7 and 57.8, 4 x 8 x 200 43 and 47, additive 59 and 53, 8 x 8 x 512 252 and 221.
 struct Plans {
   Plan recomputed, stored, dq;
   bool take_ds;
@@ -1041,15 +1043,16 @@ struct Plans {
 Plans plans_of(int D, const BwdArgs& a, int device) {
   const double heads = static_cast<double>(a.B) * a.Hkv, rows = static_cast<double>(a.Lq) * (a.Hq / a.Hkv);
   const double key_walk = std::ceil(rows / BN), query_walk = std::ceil(static_cast<double>(a.Skv) / BN);
-  const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.55 : 1.0;  // of all tiles
-  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, D == 64 ? 3.25 : 6.9};
-  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, D == 64 ? 1.87 : 4.6};
+  const double seen = a.causal == TT_ATTN_CAUSAL_TOP_LEFT ? 0.5 : 1.0;  // of all tiles
+  const double mask = a.mask.ptr ? (D == 64 ? 0.8 : 2.6) : 0.0;          // us a tile, of both walks
+  const Items keys{a.dk || a.dv ? heads * std::ceil(static_cast<double>(a.Skv) / BM) : 0.0, key_walk, seen * key_walk, (D == 64 ? 3.25 : 6.9) + mask};
+  Items queries{a.dq ? heads * std::ceil(rows / BM) : 0.0, query_walk, seen * query_walk, (D == 64 ? 1.87 : 4.6) + mask};
   const double item = D == 64 ? 9.54 : 14.8, merge = D == 64 ? 4.0 : 3.0;
   const Items none{0.0, 0.0, 0.0, 0.0};
   Plans p{plan_of(keys, queries, item, merge, device), plan_of(keys, none, item, merge, device), {1, 0.0}, false};
   // The pass that reads dS, where the two launches take less than the one.
   queries.step_us = D == 64 ? 1.61 : 2.35;
-  p.dq = plan_of(queries, none, D == 64 ? 5.4 : 7.9, 3.0, device);
+  p.dq = plan_of(queries, none, D == 64 ? 5.2 : 7.6, 3.0, device);
   p.take_ds = p.stored.us + p.dq.us < p.recomputed.us;
   return p;
 }
@@ -1079,12 +1082,12 @@ double bwd_ds_bytes_of(int B, int Hq, int Lq, int Skv) {
 }
 // Where there is room for dS, dQ is one product more instead of three, by a kernel of its own: 16 KB of scratch for 64 queries and 64
 // keys, written and read once.  Up to 192 MB of it, and from as many pairs of tiles on as storing can pay for (whether it does is the plan's, which knows
-// the device and the causal form).  us, recomputed and stored: D = 64, 256 pairs (2 x 8 x 256 causal) 21.7 and 26.7, 512 (4 x 8 x 200) 24.8 and 33.8, 864 (3 x 8 x 333)
-// 31.7 and 37.1, 1024 (16 x 16 x 128 causal) 55.6 and 49.1; D = 128, 256 33.3 and 36.1, 512 (32 x 4 x 100) 48.4 and 42.0, 576 (8 x 8 x 130 causal) 54.2 and 47.6.
+// the device, causal form and mask).  us, recomputed and stored: D = 64, 256 pairs (2 x 8 x 256) 21.2 and 26.5 causal, additive mask 25.4 and 29.2, 512
+// (16 x 8 x 128) 31.2 and 27.5, 36.3 and 31.7; D = 128, 256 pairs 33.4 and 36.0, 41.4 and 40.2, 512 52.3 and 46.8, 62.6 and 52.0.
 size_t bwd_ds_bytes(int B, int Hq, int Hkv, int Lq, int Skv, int D) {
   if (B <= 0 || Hq <= 0 || Lq <= 0 || Skv <= 0) return 0;
   const double bytes = bwd_ds_bytes_of(B, Hq, Lq, Skv);
-  return bytes <= 192e6 && bytes >= (D == 64 ? 600 : 300) * kPairBytes ? static_cast<size_t>(bytes) : 0;
+  return bytes <= 192e6 && bytes >= (D == 64 ? 500 : 250) * kPairBytes ? static_cast<size_t>(bytes) : 0;
 }
 
 bool bwd_f32_takes_ds(int D, const BwdArgs& a, int device) { return plans_of(D, a, device).take_ds; }
