@@ -19,10 +19,10 @@
 // Where there is room for dS and work enough for one more launch (bwd_ds_bytes), the key CTAs leave theirs and bwd_f32_dq_kernel makes dQ
 // of it: one product instead of the query CTAs' three.
 //
-// Bound by the tensor pipe and the waits around it: D = 64, a tile 5700 clocks, of them 4 x 1050 in MMAs; D = 128, where only one tile of the other
-// side fits, its two operands' conversion besides.  Against the same in fp32 FMAs on CUDA cores, us, with the delta pass: D = 64, 4 x 8 heads x 500
-// 156 -> 61 (additive mask 170 -> 75), causal 8 x 8 x 1024 784 -> 257, 2 x 16/2 x 700 217 -> 84; D = 128, 4 x 8 x 500 295 -> 110 (additive mask 304 -> 136),
-// causal 4 x 8 x 1024 719 -> 203.
+// Bound by the tensor pipe and the waits around it; D = 128, where only one tile of the other side fits, by its two operands' conversion
+// besides.  Against the same in fp32 FMAs on CUDA cores, us, with the delta pass: D = 64, 4 x 8 heads x 500 156 -> 58 (additive mask 170 -> 74),
+// causal 8 x 8 x 1024 785 -> 245, 2 x 16/2 x 700 218 -> 86, but one tile of 4 x 16 x 57 12.5 -> 15.3; D = 128, 4 x 8 x 500 296 -> 110 (additive mask
+// 304 -> 137), causal 4 x 8 x 1024 718 -> 203.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -596,7 +596,7 @@ __device__ __forceinline__ void walk(const BwdArgs& a, uint8_t* smem, uint32_t b
             if (leader) ptx::mma_ts2(d, ap + LY::plane_at(0, ks), bp + ks * (2048 >> 4), kHi, idesc, st.onto || ks > 0 ? 1u : 0u);
         }
       };
-      // (Every lane polls every barrier: with a lane for each the warp came to its MMAs in parts, and they faulted.)
+      // (Every lane polls every barrier: tcgen05.mma wants the warp together, and lanes that wait for different barriers come apart.)
       // S = K Q^T (Q K^T), tile t; a_full: the own side is there
       auto issue_s = [&](int t) {
         const uint32_t at = done + t, stage = at % LY::kStages, stage_at = stage * (TB::kBytes >> 4);

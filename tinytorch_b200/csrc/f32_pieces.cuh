@@ -1,7 +1,8 @@
 // fp32 matrix products on the tensor cores: every operand is written as the sum of three bf16 pieces.
 //
 // A float has 24 significant bits, a bf16 has 8: x rounded to bf16, what is left rounded to bf16, and what is left then are three
-// bf16 whose sum is x, exactly, over the range of exponents.  Of the nine products of pieces the six that reach 2^-24 of the result are
+// bf16 whose sum is x: exactly from 2^-110 on; below, the last piece is a multiple of 2^-133 and x is off by half of that at most (2^-19 of itself at
+// 2^-115, 2^-9 at 2^-125).  Of the nine products of pieces the six that reach 2^-24 of the result are
 // taken and accumulated in fp32 in TMEM, the small ones first, over one tile only (64 terms of the contraction for probabilities, D for
 // scores): the tensor cores truncate where they accumulate, so the sums over tiles are made in registers, by rounded additions.  What the
 // truncations take is not given back: on average it is 0.75e-7 of a sum of 64 products of mixed signs, but other data lose other shares, sums of

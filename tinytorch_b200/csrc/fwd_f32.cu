@@ -11,11 +11,14 @@
 //   warps 18, 19 masks
 // An MMA of 64 columns takes 52 (A from TMEM) or 66 clocks (from shared memory) where 32 would do and 128 columns take 64: the first two planes
 // of K (and of V, D = 64) are read as one operand of 128.  S and O come as two sums then (f32_pieces.cuh).
+// A probability that is 0 takes part in P V, as in the composition: what is not finite in V spoils the rows that share a tile with it (all 128 that walk
+// as far, also those whose causal limit lies before it), and no others.
 //
-// Bound by the chain of a tile: softmax 2000 clocks and 300 until S is seen (D = 64: a tile 2400; the MMAs take 2100 of them), for D = 128,
+// Bound by the chain of a tile: softmax 2000 clocks and 300 until S is seen (D = 64: a tile 2400, the MMAs under them), for D = 128,
 // where only one K tile fits, K into pieces, then S 1800.  Against the same in fp32 FMAs on CUDA cores (64 x 64 tiles, whose FMA pipes were
-// 58 % busy), us: D = 64, 4 x 8 heads x 500 72 -> 19 (additive mask 74 -> 29, 6 x 333 padding 52 -> 19), causal 16 x 2048 293 -> 54,
-// 11 x 32/8 heads x 22 14.5 -> 9.2, one query on one key 7.2 -> 6.3; D = 128, 4 x 8 x 500 117 -> 33 (additive 125 -> 43), causal 4 x 4096 506 -> 107.
+// 58 % busy), us: D = 64, 4 x 8 heads x 500 72 -> 18.4 (additive mask 74 -> 27, 6 x 333 padding 53 -> 19), causal 16 x 2048 294 -> 54.5,
+// 11 x 32/8 heads x 22 14.7 -> 9.1, one query on one key 7.2 -> 6.4, but 2 x 8/4 heads x 99 on 131 with an additive mask 10.4 -> 11.0; D = 128,
+// 4 x 8 x 500 117 -> 32 (additive 126 -> 38), causal 4 x 4096 506 -> 107.
 // Tried: P over the S that it is made of, two such buffers, S up to two tiles ahead: 2700 clocks a tile.  One place for P: 3150.
 // Additive rows by bulk copies of 256 bytes: 29.7 -> 32.3, D = 128 43 -> 53.
 #include <algorithm>
@@ -326,9 +329,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_f32_kernel(const FwdArgs a, i
           ptx::tc_fence_after();
         }
         if (rare(careful)) {
-          // With a mask its code stands once, and s moves up: four times it costs the other pass registers (additive, 4 x 8 heads x 500:
-          // 28.7 us, boolean 23.5; once 27.8 and 22.8).  Without one it is four times: 18.3; once 18.7.
-#pragma unroll(MASK == kNoMask ? 4 : 1)
+          // Its code stands once, and s moves up: four times it costs the other pass registers (additive mask, 4 x 8 heads x 500: 28.7 us,
+          // boolean 23.5; once 27.8 and 22.8; D = 128, 4 x 4096 causal 110.7 and 107.3).  D = 64 without a mask has it four times: 18.3; once 18.7.
+#pragma unroll(MASK == kNoMask && D == 64 ? 4 : 1)
           for (int j = 0; j < BN; j += 16) {
             probabilities(std::true_type{}, s, j);
 #pragma unroll
