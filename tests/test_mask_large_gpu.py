@@ -88,3 +88,23 @@ def test_a_workspace_without_room_for_the_rows(D):
         assert all(bool(torch.isfinite(t).all()) for t in grads)
         if zero:
             _check(grads, q, k, v, g, mask, large, -1.0e9)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_grouped_heads_and_one_large_mask(D):
+    """Query heads that share a kv head, each with a mask of its own."""
+    from tinytorch_b200 import op
+    B, H, group, L, S, value = 2, 2, 3, 70, 90, -1.0e9
+    q, _, _, g, _, large = _case(B, H * group, L, S, D, value, False)
+    _, k, v, _, _, _ = _case(B, H, L, S, D, value, False)
+    mask = torch.randn((1, H * group, L, S), device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    mask[:, :, large] = value
+    o, lse = op.sdpAttentionFwd(q, k, v, attnMask=mask)
+    dq, dk, dv = op.sdpAttentionBwd(g, q, k, v, o, lse, attnMask=mask)
+    _check((dq,), q, *(t.repeat_interleave(group, 1) for t in (k, v)), g, mask, large, value)
+    # the kv heads' gradients: the sums of what each query head gives with a copy of its own
+    kk, vv = (t.repeat_interleave(group, 1).contiguous() for t in (k, v))
+    each = op.sdpAttentionBwd(g, q, kk, vv, o, lse, attnMask=mask)
+    for t, w in zip((dk, dv), each[1:]):
+        w = w.double().unflatten(1, (H, group)).sum(2)
+        assert float((t.double() - w).abs().max()) <= TOL_REL_FP32 * max(1.0, float(w.abs().max()))
